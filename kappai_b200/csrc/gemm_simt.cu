@@ -3,8 +3,19 @@
 // This is the matrix product of the true 32-bit path (no tensor-core mode of
 // reduced precision is involved) and the general fallback of the bfloat16 path
 // for shapes the tensor-core kernels refuse.  W is row-major [out][in] as in
-// the reference (src/backend/cpu/scalar/quants.c:1367-1414); each output
-// element sums k = 0..K-1 in order, so a row's result does not depend on M.
+// the reference (src/backend/cpu/scalar/quants.c:1367-1414).
+//
+// float32 operands with 16-byte rows run one of two kernels.  Both add an output's products in the same order,
+// whatever M is: k is cut into stretches of 256, a stretch's even and odd k are two chains of FMAs from zero that are added
+// at its end, and the stretches' sums are added in the order of k.  So a row's result does not depend on the rows beside it, the rows of a step can be
+// cut anywhere, and long sums lose less than in one chain of K.
+//
+//  * gemm_f32_rows_kernel: few rows.  Bound by reading W once (4 bytes a weight).
+//  * gemm_f32_tile_kernel: many rows.  Bound by the FMA rate (about 70 TFLOP/s of scalar FMA was measured on B200; the
+//    packed two-element form gains nothing in rate but takes half the issue slots).
+//
+// Everything else (bfloat16 operands, rows that are not 16-byte aligned) runs gemm_nt_simt_kernel, which sums
+// k = 0..K-1 in order.  The choice between the orders depends on type and alignment only, never on M.
 #include "common.cuh"
 
 #define EPI_STORE 0      // C (type T) = acc
@@ -87,11 +98,335 @@ static int launch(const void* A, const void* W, const float* bias, void* C, int 
     return kp_launch_status();
 }
 
+// ------------------------------------------------------------------------------------------ float32, aligned rows
+
+constexpr int F32_GROUP = 256;                       // k's of one chain of FMAs (see above)
+
+struct F32Args {
+    const float* A; const float* W; const float* bias; float* C;
+    int M, N, K, lda, ldw, ldc;
+};
+
+// 16 bytes to shared memory without a register between; `ok` false: zeros, nothing is read
+__device__ __forceinline__ void f32_cp16(void* dst, const float* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void f32_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void f32_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// two FMAs in one instruction: the chains of the even and of the odd k's
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void f32_fma2(f32x2& d, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float f32_halves(f32x2 v) {
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+
+template <int EPI> __device__ __forceinline__ void f32_store(const F32Args& p, int m, int n, float v) {
+    if (p.bias) v += p.bias[n];
+    float* c = p.C + (size_t)m * p.ldc + n;
+    *c = EPI == EPI_ACCUM_F32 ? *c + v : v;
+}
+
+// Few rows.  A CTA owns 8 R rows of W; its warps cut K into jobs of 1024 columns = 4 stretches, and a lane (r, q) of a job
+// sums stretch q of the rows r, r + 8, ... for MB rows of A, so that every chain stays in one lane.  A warp brings its
+// job's W (and A) through a ring of its own in stages of 32 columns, by cp.async; nothing in the main loop waits for
+// another warp.  The stages of W that the ring holds are on their way before the wait on the kernel before (weights
+// depend on no kernel), those of A behind it.  In shared memory the eight 16-byte chunks of a row's stage are permuted
+// by the row (chunk c of row r at c ^ r), so the eight rows of a quarter warp read all banks once.
+//
+// More rows than MB take the grid's y; W then comes from L2.  Measured (W from HBM): 8 rows by 2048 x 5632 in 13.3 us
+// (3.5 TB/s; 608 us with tiles of 64 x 64 and a chain of K), 11264 x 2048 in 23 us, 65536 x 2048 in 93 us (5.8 TB/s); one
+// row 10.6, 15.7 and 78 us (6.9 TB/s).  R = 4, MB = 16 reads shared memory least for its FMAs: 64 rows by 2048 x 5632 in
+// 77 us against 84 with R = 2, MB = 8.
+#define F32R_COLS 32                                  // columns of a stage
+#define F32R_JOB (4 * F32_GROUP)                      // columns of a job
+#define F32R_MAX_WARPS 8
+
+template <int R, int MB, int EPI>
+__global__ void __launch_bounds__(F32R_MAX_WARPS * 32)
+gemm_f32_rows_kernel(const F32Args p, int n_stages) {
+    constexpr int W_BYTES = 8 * R * 4 * F32R_COLS * 4, A_BYTES = MB * 4 * F32R_COLS * 4, STAGE = W_BYTES + A_BYTES;
+    constexpr int PER_JOB = F32_GROUP / F32R_COLS;    // stages of a job
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    const int r = lane & 7, q = lane >> 3;
+    const int n0 = blockIdx.x * 8 * R, m0 = blockIdx.y * MB;
+    const int K = p.K, n_jobs = (K + F32R_JOB - 1) / F32R_JOB;
+    unsigned char* ring = smem + (size_t)warp * n_stages * STAGE;
+    float* red = reinterpret_cast<float*>(smem + (size_t)n_warps * n_stages * STAGE);     // [stretch][MB][8 R]
+    const int mine = n_jobs > warp ? (n_jobs - warp - 1) / n_warps + 1 : 0;               // jobs of this warp
+    const int total = mine * PER_JOB;
+
+    auto col_of = [&](int it) { return (warp + (it / PER_JOB) * n_warps) * F32R_JOB + (it % PER_JOB) * F32R_COLS; };
+    // (a warp's 32 copies are 4 rows of a stretch by 8 chunks)
+    const int cr = lane >> 3, cc = lane & 7;
+    auto load_w = [&](int it) {
+        unsigned char* dst = ring + (size_t)(it % n_stages) * STAGE;
+        const int k0 = col_of(it) + cc * 4;
+#pragma unroll
+        for (int g = 0; g < 4; g++)
+#pragma unroll
+            for (int i = 0; i < 2 * R; i++) {
+                const int row = i * 4 + cr, k = k0 + g * F32_GROUP;                       // row of the CTA's 8 R
+                const float* src = p.W + (size_t)min(n0 + row, p.N - 1) * p.ldw + k;
+                f32_cp16(dst + ((((row >> 3) * 4 + g) * 8 + (row & 7)) * 8 + (cc ^ (row & 7))) * 16, src, k < K);
+            }
+    };
+    auto load_a = [&](int it) {
+        unsigned char* dst = ring + (size_t)(it % n_stages) * STAGE + W_BYTES;
+        const int k = col_of(it) + cc * 4 + cr * F32_GROUP;                               // stretch cr, chunk cc
+#pragma unroll
+        for (int m = 0; m < MB; m++)
+            f32_cp16(dst + ((m * 4 + cr) * 8 + ((cc + 2 * cr) & 7)) * 16, p.A + (size_t)min(m0 + m, p.M - 1) * p.lda + k, k < K);
+    };
+
+    const int ahead = n_stages - 1;
+    KP_TRACE_MARK(0);
+    for (int it = 0; it < ahead && it < total; it++) load_w(it);
+    pdl_wait();
+    KP_TRACE_MARK(1);
+    pdl_launch_dependents();
+    // (the first stages' W is part of the first stage's group: it was asked for first and comes first)
+    for (int it = 0; it < ahead; it++) {
+        if (it < total) load_a(it);
+        f32_cp_commit();
+    }
+
+    f32x2 acc[R][MB];
+    for (int it = 0; it < total; it++) {
+        if (it % PER_JOB == 0) {
+#pragma unroll
+            for (int i = 0; i < R; i++)
+#pragma unroll
+                for (int m = 0; m < MB; m++) acc[i][m] = 0;
+        }
+        // stage `it` has come: all but the ahead - 1 groups behind it
+        switch (ahead) {
+            case 1: f32_cp_wait<0>(); break;
+            case 2: f32_cp_wait<1>(); break;
+            case 3: f32_cp_wait<2>(); break;
+            case 4: f32_cp_wait<3>(); break;
+            case 5: f32_cp_wait<4>(); break;
+            case 6: f32_cp_wait<5>(); break;
+            default: f32_cp_wait<6>(); break;
+        }
+        __syncwarp();
+        if (it + ahead < total) { load_w(it + ahead); load_a(it + ahead); }
+        f32_cp_commit();
+        const unsigned char* st = ring + (size_t)(it % n_stages) * STAGE;
+        const ulonglong2* wr = reinterpret_cast<const ulonglong2*>(st) + (q * 8 + r) * 8;
+        const ulonglong2* ar = reinterpret_cast<const ulonglong2*>(st + W_BYTES) + q * 8;
+#pragma unroll
+        for (int c = 0; c < F32R_COLS / 4; c++) {
+            ulonglong2 w[R];
+#pragma unroll
+            for (int i = 0; i < R; i++) w[i] = wr[i * 256 + (c ^ r)];
+#pragma unroll
+            for (int m = 0; m < MB; m++) {
+                const ulonglong2 a = ar[m * 32 + ((c + 2 * q) & 7)];
+#pragma unroll
+                for (int i = 0; i < R; i++) { f32_fma2(acc[i][m], a.x, w[i].x); f32_fma2(acc[i][m], a.y, w[i].y); }
+            }
+        }
+        if (it % PER_JOB == PER_JOB - 1) {
+            const int g = (warp + (it / PER_JOB) * n_warps) * 4 + q;
+#pragma unroll
+            for (int i = 0; i < R; i++)
+#pragma unroll
+                for (int m = 0; m < MB; m++) red[((size_t)g * MB + m) * 8 * R + i * 8 + r] = f32_halves(acc[i][m]);
+        }
+    }
+    __syncthreads();
+    const int n_groups = (K + F32_GROUP - 1) / F32_GROUP;
+    for (int e = threadIdx.x; e < MB * 8 * R; e += blockDim.x) {
+        const int m = m0 + e / (8 * R), n = n0 + e % (8 * R);
+        if (m >= p.M || n >= p.N) continue;
+        float v = 0.f;
+        for (int g = 0; g < n_groups; g++) v += red[(size_t)g * MB * 8 * R + e];
+        f32_store<EPI>(p, m, n, v);
+    }
+}
+
+// Many rows.  A CTA of 256 threads computes 64 x 64 of C, a thread 4 x 4 of it (rows ty + 16 i, columns tx + 16 j).
+// Stages of 32 columns of A and W come by cp.async as they lie in memory; a thread reads four k's of a row at a time (no
+// transposed copy is needed), chunks permuted by the row as above.  A 16-byte read that neighbouring lanes share costs
+// two slots of shared memory, one that lanes eight apart share four (measured), so lane bits 1 to 3 choose the row of A
+// and bits 0 and 4 that of W.  Two CTAs an SM.
+// Measured: 2,048 rows by 6144 x 2048 in 1.21 ms, 43 TFLOP/s, 513 rows by 2048 x 5632 in 325 us (one thread a 4 x 4 of a
+// tile read with scalar, transposed copies: 647 us).  What is left is the dispatch of FMAs with three operands from
+// registers of the same bank; 128 x 64 tiles (8 x 4 a thread) were within 4 % either way.
+#define F32T_COLS 32
+#define F32T_STAGES 3
+#define F32T_SMEM (F32T_STAGES * 128 * F32T_COLS * 4 + 4 * 256 * 16)
+template <int EPI>
+__global__ void __launch_bounds__(256, 2)
+gemm_f32_tile_kernel(const F32Args p) {
+    constexpr int TMt = 4, ROWS = 16 * TMt, STAGE = (ROWS + 64) * F32T_COLS * 4;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ty = (warp & 1) * 8 + ((lane >> 1) & 7), tx = (warp >> 1) * 4 + (lane & 1) + ((lane >> 4) << 1);
+    const int m0 = blockIdx.y * ROWS, n0 = blockIdx.x * 64;
+    const int K = p.K, n_st = (K + F32T_COLS - 1) / F32T_COLS;
+    const int lr = threadIdx.x >> 3, lc = threadIdx.x & 7;               // copies: 32 rows by 8 chunks at a time
+    auto load = [&](int it, bool a, bool w) {
+        unsigned char* dst = smem + (it % F32T_STAGES) * STAGE;
+        const int k = it * F32T_COLS + lc * 4;
+        if (a) {
+#pragma unroll
+            for (int i = 0; i < ROWS / 32; i++) {
+                const int row = i * 32 + lr;
+                f32_cp16(dst + (row * 8 + (lc ^ (row & 7))) * 16, p.A + (size_t)min(m0 + row, p.M - 1) * p.lda + k, k < K);
+            }
+        }
+        if (w) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int row = i * 32 + lr;
+                f32_cp16(dst + ((ROWS + row) * 8 + (lc ^ (row & 7))) * 16, p.W + (size_t)min(n0 + row, p.N - 1) * p.ldw + k, k < K);
+            }
+        }
+    };
+    KP_TRACE_MARK(0);
+    for (int it = 0; it < F32T_STAGES - 1 && it < n_st; it++) load(it, false, true);
+    pdl_wait();
+    KP_TRACE_MARK(1);
+    pdl_launch_dependents();
+    for (int it = 0; it < F32T_STAGES - 1; it++) {
+        if (it < n_st) load(it, true, false);
+        f32_cp_commit();
+    }
+    f32x2 acc[TMt][4];
+    // the outputs' sums over the stretches so far lie in shared memory (registers are short), each thread's its own
+    float4* sum = reinterpret_cast<float4*>(smem + F32T_STAGES * STAGE) + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < TMt; i++) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0;
+        sum[i * 256] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int it = 0; it < n_st; it++) {
+        f32_cp_wait<F32T_STAGES - 2>();
+        __syncthreads();                                                 // the stage has come; the one before has been read
+        if (it + F32T_STAGES - 1 < n_st) load(it + F32T_STAGES - 1, true, true);
+        f32_cp_commit();
+        const ulonglong2* as = reinterpret_cast<const ulonglong2*>(smem + (it % F32T_STAGES) * STAGE);
+        const ulonglong2* ws = as + ROWS * 8;
+#pragma unroll
+        for (int c = 0; c < F32T_COLS / 4; c++) {
+            ulonglong2 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[j] = ws[(tx + 16 * j) * 8 + (c ^ (tx & 7))];
+#pragma unroll
+            for (int i = 0; i < TMt; i++) {
+                const ulonglong2 a = as[(ty + 16 * i) * 8 + (c ^ (ty & 7))];
+#pragma unroll
+                for (int j = 0; j < 4; j++) f32_fma2(acc[i][j], a.x, w[j].x);
+#pragma unroll
+                for (int j = 0; j < 4; j++) f32_fma2(acc[i][j], a.y, w[j].y);
+            }
+        }
+        if (it % (F32_GROUP / F32T_COLS) == F32_GROUP / F32T_COLS - 1 || it == n_st - 1) {
+#pragma unroll
+            for (int i = 0; i < TMt; i++) {
+                float4 v = sum[i * 256];
+                v.x += f32_halves(acc[i][0]); v.y += f32_halves(acc[i][1]); v.z += f32_halves(acc[i][2]); v.w += f32_halves(acc[i][3]);
+                sum[i * 256] = v;
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = 0;
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TMt; i++) {
+        const int m = m0 + ty + 16 * i;
+        if (m >= p.M) continue;
+        const float4 v = sum[i * 256];
+        const float out[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int n = n0 + tx + 16 * j;
+            if (n < p.N) f32_store<EPI>(p, m, n, out[j]);
+        }
+    }
+}
+
+static int f32_n_sm() {
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    }
+    return n;
+}
+
+template <typename Kern, typename... Args>
+static int f32_launch(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return (int)kp_launch_pdl(kern, grid, dim3(threads), smem, s, args...);
+}
+
+template <int R, int MB, int EPI>
+static int f32_rows(const F32Args& p, cudaStream_t s) {
+    const int n_jobs = (p.K + F32R_JOB - 1) / F32R_JOB;
+    const int stage = (8 * R + MB) * 4 * F32R_COLS * 4;
+    const int most = R == 4 ? 4 : F32R_MAX_WARPS;
+    const int warps = n_jobs < most ? n_jobs : (n_jobs + (n_jobs + most - 1) / most - 1) / ((n_jobs + most - 1) / most);
+    const size_t red = (size_t)n_jobs * 4 * MB * 8 * R * 4;
+    const dim3 grid((p.N + 8 * R - 1) / (8 * R), (p.M + MB - 1) / MB);
+    // one CTA an SM: all the ring that pays (a job has 8 stages); more: a third of the SM's memory each
+    const size_t room = (int)(grid.x * grid.y) <= f32_n_sm() ? 200 * 1024 : 74 * 1024;
+    int stages = red < room ? (int)((room - red) / ((size_t)warps * stage)) : 0;
+    if (stages > 8) stages = 8;
+    if (stages < 2) stages = 2;
+    const size_t smem = (size_t)warps * stages * stage + red;
+    if (smem > 220 * 1024) return KP_ERR_UNSUPPORTED;
+    return f32_launch(gemm_f32_rows_kernel<R, MB, EPI>, grid, warps * 32, smem, s, p, stages);
+}
+
+// Which kernel (K counts in every kernel alike, so the rule compares rounds over the SMs; measured at widths of 1024 to
+// 11264, us, with rows of 8 | rows of 16 | tiles):
+//   up to 24 rows: rows of 8 (16 rows by 2048 x 5632: 25 | 38 | 172; by 1024 x 1024: 8 | 19 | 32), but not for a wide W
+//   with one job of K, whose CTAs are single warps (16 rows by 9216 x 1024: 30 | 21 | 40);
+//   a round of rows of 16 takes 7.2 us for 1,000 k, one of tiles 30.5 (128 rows by 2048 x 5632: 165 | 152 | 172; 160 rows:
+//   - | 190 | 173; 96 rows by 6144 x 2048: 98 | 82 | 121; 256 rows by 1024 x 1024: - | 22 | 33; 400 rows: - | 42 | 33).
+template <int EPI>
+static int f32_run(const F32Args& p, cudaStream_t s) {
+    const int sms = f32_n_sm();
+    const auto rounds = [&](long long ctas) { return (ctas + sms - 1) / sms; };
+    const auto cuts = [](int n, int size) { return (long long)((n + size - 1) / size); };
+    int st = KP_ERR_UNSUPPORTED;                                         // (a K too long for the sums of its stretches: tiles)
+    if (p.M <= 8 || (p.M <= 24 && (p.K > F32R_JOB || p.N <= 32 * sms))) {
+        const bool narrow = cuts(p.N, 16) < sms;                         // 8 rows of W a CTA where 16 leave SMs idle
+#define F32_ROWS(MB_) st = narrow ? f32_rows<1, MB_, EPI>(p, s) : f32_rows<2, MB_, EPI>(p, s)
+        if (p.M == 1) F32_ROWS(1);
+        else if (p.M == 2) F32_ROWS(2);
+        else if (p.M <= 4) F32_ROWS(4);
+        else F32_ROWS(8);
+#undef F32_ROWS
+    } else if (rounds(cuts(p.M, 16) * cuts(p.N, 32)) * 72 < rounds(cuts(p.M, 64) * cuts(p.N, 64)) * 305) {
+        st = f32_rows<4, 16, EPI>(p, s);
+    }
+    if (st != KP_ERR_UNSUPPORTED) return st;
+    return f32_launch(gemm_f32_tile_kernel<EPI>, dim3((p.N + 63) / 64, (p.M + 63) / 64), 256, F32T_SMEM, s, p);
+}
+
 extern "C" int kp_gemm_nt_simt(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int lda,
                                int ldw, int ldc, int epi, int dtype, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return KP_ERR_BAD_ARG;
     if ((long long)((M + BM - 1) / BM) > 65535) return KP_ERR_UNSUPPORTED;
+    if (dtype == KP_DTYPE_F32 && !((K | lda | ldw) & 3) && !(((uintptr_t)A | (uintptr_t)W) & 15)) {
+        const F32Args p = {(const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc};
+        if (epi == EPI_STORE || epi == EPI_STORE_F32) return f32_run<EPI_STORE>(p, (cudaStream_t)stream);
+        if (epi == EPI_ACCUM_F32) return f32_run<EPI_ACCUM_F32>(p, (cudaStream_t)stream);
+        return KP_ERR_BAD_ARG;
+    }
     KP_DISPATCH_DTYPE(dtype, T, return launch<T>(A, W, bias, C, M, N, K, lda, ldw, ldc, epi, (cudaStream_t)stream));
     return 0;
 }

@@ -1,0 +1,44 @@
+"""The float32 product with 16-byte rows (csrc/gemm_simt.cu): its two kernels at the edges of their tiles, stretches and
+jobs against float64, and one order of summation whatever the number of rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROWS = (1, 2, 3, 4, 5, 8, 9, 16, 24, 25, 40, 64, 65, 130)      # few-row kernels of 1, 2, 4, 8 and 16 rows a pass, tiles of 64
+
+
+@pytest.mark.parametrize("N,K", [(1, 4), (33, 252), (72, 256), (100, 260), (2050, 1024), (200, 1028), (331, 4100), (64, 9000),
+                                 (5000, 512)])
+def test_against_float64_and_one_order_for_every_number_of_rows(N, K):
+    from kappai_b200.ops import kernels as Kn
+    g = torch.Generator(device="cuda").manual_seed(N * 10007 + K)
+    a = torch.randn(max(ROWS), K + 4, device="cuda", generator=g)[:, :K]        # (rows longer than K)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    bias = torch.randn(N, device="cuda", generator=g)
+    exact = a.double() @ w.double().T
+    # a chain of 128 FMAs, its partner, one sum a stretch of 256: each rounds at most eps/2 of the sum of magnitudes
+    bound = (128 + 1 + -(-K // 256) + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T + bias.double().abs()) * 1.01
+    whole = None
+    for M in reversed(ROWS):
+        out = Kn.gemm_nt_simt(a[:M], w, torch.full((M, N), float("nan"), device="cuda"))
+        assert bool(((out.double() - exact[:M]).abs() <= bound[:M]).all()), (M, N, K)
+        whole = out if whole is None else whole
+        assert torch.equal(out, whole[:M]), f"{M} rows: another order of summation"
+        acc = torch.ones(M, N, device="cuda")
+        Kn.gemm_nt_simt(a[:M], w, acc, bias, accumulate=True)
+        assert torch.equal(acc, 1.0 + (out + bias)), M
+    last = Kn.gemm_nt_simt(a[-1:], w, torch.empty(1, N, device="cuda"))
+    assert torch.equal(last[0], whole[-1])
+
+
+def test_rows_that_are_not_16_byte_aligned_take_the_general_kernel():
+    from kappai_b200.ops import kernels as Kn
+    base = torch.randn(9, 130, device="cuda")
+    w = torch.randn(70, 130, device="cuda")
+    for a_ in (base[:, :127], base[:, 1:128], base):                            # K, address and pitch that are none
+        k = a_.shape[1]
+        out = Kn.gemm_nt_simt(a_, w[:, :k], torch.empty(9, 70, device="cuda"))
+        exact = a_.double() @ w[:, :k].double().T
+        bound = (k + 2) * 2.0 ** -24 * (a_.double().abs() @ w[:, :k].double().abs().T)
+        assert bool(((out.double() - exact).abs() <= bound).all())
