@@ -44,7 +44,8 @@
 #define EPI_SWIGLU 3
 #define EPI_ACT 6                            // store bf16 behind an ungated activation (common.cuh, kp_act_plain)
 #define EPI_GLU 4                            // inside this file only: EPI_SWIGLU whose unit is the one with limits (act code 3)
-#define TC_GATED(E) ((E) == EPI_SWIGLU || (E) == EPI_GLU)
+#define EPI_GATED_RT 5                       // inside this file only: EPI_SWIGLU with an activation other than silu, chosen at run time
+#define TC_GATED(E) ((E) == EPI_SWIGLU || (E) == EPI_GLU || (E) == EPI_GATED_RT)
 
 #define TC_BM 128
 #define TC_BK 64
@@ -88,6 +89,32 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&t);
 }
 
+// Biases of W sums g (and u: the up half, gated) of the output columns from n_base on, those below n_lim.
+template <int EPI, int W>
+__device__ __forceinline__ void tc_bias(const TcArgs& p, int n_lim, float (&g)[W], float (&u)[W], int n_base) {
+    if (!p.bias) return;
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+        if (n_base + j < n_lim) {
+            g[j] += p.bias[n_base + j];
+            if TC_GATED(EPI) u[j] += p.bias[p.ff + n_base + j];
+        }
+    }
+}
+// What becomes of a sum.  silu has instantiations of its own: with the activation chosen at run time every one of the 32
+// unrolled outputs carried the code of all of them, and the epilogue waited for instructions (200 rows by gate/up
+// 11264 x 2048: 24.1 us a product against 20.7; the kernel of pairs 31.6 against 20.2).
+template <int EPI>
+__device__ __forceinline__ float tc_value(const TcArgs& p, float g, float u) {
+    if TC_GATED(EPI) {
+        // gate and up are rounded to the storage type first, as the unfused path stores them
+        const float gq = to_f32(from_f32<bf16>(g)), uq = to_f32(from_f32<bf16>(u));
+        if (EPI == EPI_GLU) return kp_glu_clamped(gq, uq, p.glu_limit, p.glu_alpha, p.glu_shift);
+        return (EPI == EPI_SWIGLU ? kp_act<KP_ACT_SILU>(gq) : kp_act_epilogue(p.act, gq)) * uq;
+    }
+    return EPI == EPI_ACT ? kp_act_plain(p.act, g) : g;
+}
+
 // A piece of W output columns (32, or 4 in the split's reduction) of row m, from its sums g (and u: the up half,
 // SwiGLU), to C: bias, SwiGLU or accumulation, and the store (vector stores where rows of C are 16-byte aligned).
 template <int EPI, int W>
@@ -96,17 +123,12 @@ __device__ __forceinline__ void tc_finish(const TcArgs& p, int n_lim, const floa
     float v[W];
 #pragma unroll
     for (int j = 0; j < W; j++) {
-        float x = g[j];
-        if (p.bias && n_base + j < n_lim) x += p.bias[n_base + j];
-        if TC_GATED(EPI) {
-            float up = u[j];
-            if (p.bias && n_base + j < n_lim) up += p.bias[p.ff + n_base + j];
-            // gate and up are rounded to the storage type first, as the unfused path stores them
-            const float gq = to_f32(from_f32<bf16>(x)), uq = to_f32(from_f32<bf16>(up));
-            x = EPI == EPI_GLU ? kp_glu_clamped(gq, uq, p.glu_limit, p.glu_alpha, p.glu_shift) : kp_act_epilogue(p.act, gq) * uq;
+        float x = g[j], up = u[j];
+        if (p.bias && n_base + j < n_lim) {
+            x += p.bias[n_base + j];
+            if TC_GATED(EPI) up += p.bias[p.ff + n_base + j];
         }
-        if (EPI == EPI_ACT) x = kp_act_plain(p.act, x);
-        v[j] = x;
+        v[j] = tc_value<EPI>(p, x, up);
     }
     const bool whole = p.vec_ok && n_base + W <= n_lim;                  // vector stores of the whole piece
     if (EPI == EPI_STORE || EPI == EPI_ACT || TC_GATED(EPI)) {
@@ -403,6 +425,213 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == 1) kp_tmem_dealloc(tmem_base, 2 * BN);
 }
 
+// ------------------------------------------------------------------------------------------ pairs of CTAs
+// Products of many rows: a pair of CTAs (a cluster of two, cta_group::2) computes tiles of 256 x BN, each CTA 128 of the
+// rows.  What bounds the one-CTA kernel there is the bytes that an SM brings into shared memory: for 128 x 256 outputs it
+// reads 48 KB a k-block, about 770 cycles' worth from L2 for 512 cycles of MMAs.  A pair reads A once a CTA and each half
+// of W once a pair: 32 KB an SM.  The roles are those of gemm_tc_kernel; the first CTA's MMA warp issues for both, both
+// CTAs' loads count at its "full" barriers, and its commits free the stages and hand over the accumulators in both.
+// The sums run in the same order as in gemm_tc_kernel (the same bits).  Measured, us, one CTA a tile | pairs: 2,048 rows by
+// 11264 x 2048 (gated) 77.0 | 67.0, 1.41 PFLOP/s; 2048 x 5632 44.8 | 37.2; 6144 x 2048 46.8 | 37.7; 2048 x 2048 25.3 | 19.3;
+// 512 rows by 65536 x 1024 92.8 | 65.1.
+//
+// The epilogue warps pass their pieces (128 bytes of 32 rows) through shared memory, so that a warp writes, and for an
+// accumulated output reads, four whole rows' stretches of 128 bytes at a time instead of 16 bytes of 32 rows; the old
+// values of an accumulated output are asked for before the piece is read from tensor memory.
+#define TC_PAIR_STAGES(BN) ((BN) == 256 ? 5 : 7)
+#define TC_PAIR_SMEM(BN) ((size_t)TC_PAIR_STAGES(BN) * (128 + (BN) / 2) * TC_BK * 2 + TC_EPI_PER_Q * 4 * 4096 + (2 * TC_PAIR_STAGES(BN) + 4) * 8 + 16 + 1024)
+
+template <int BN, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const TcArgs p) {
+    constexpr int STAGES = TC_PAIR_STAGES(BN);
+    constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN / 2 * TC_BK * 2, STAGE = A_BYTES + B_BYTES;
+    constexpr int N_OUT_TILE = TC_GATED(EPI) ? BN / 2 : BN;
+    extern __shared__ unsigned char smem[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
+    unsigned char* pieces = tiles + (size_t)STAGES * STAGE;                // 4 KB an epilogue warp
+    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + TC_EPI_PER_Q * 4 * 4096);   // (the first CTA's are used)
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;                                  // [2]
+    uint64_t* acc_empty = acc_full + 2;                                   // [2] (the first CTA's are used)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    const int n_kb = (p.K + TC_BK - 1) / TC_BK;
+    const int n_out = TC_GATED(EPI) ? p.ff : p.N;
+    const int tiles_m = (p.M + 2 * TC_BM - 1) / (2 * TC_BM), tiles_n = (n_out + N_OUT_TILE - 1) / N_OUT_TILE;
+    const int n_tiles = tiles_m * tiles_n;
+
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
+        for (int s = 0; s < STAGES; s++) { kp_mbar_init(&full[s], 1); kp_mbar_init(&empty[s], 1); }
+        for (int b2 = 0; b2 < 2; b2++) { kp_mbar_init(&acc_full[b2], 1); kp_mbar_init(&acc_empty[b2], 2 * 4 * TC_EPI_PER_Q); }
+        *abort_flag = 0;
+        kp_mbar_init_fence();
+    }
+    if (warp == 1) kp_tmem_alloc_pair(tmem_slot, 2 * BN);
+    kp_tc_fence_before();
+    __syncthreads();
+    kp_cluster_sync();                                                    // both CTAs' barriers and tensor memory are there
+    kp_tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            auto load_w = [&](int s, int kb, int n0) {
+                // this CTA's half of the W tile: gate rows or up rows, or the first or second BN / 2 rows
+                const int row = TC_GATED(EPI) ? rank * p.ff + n0 : n0 + rank * (BN / 2);
+                kp_tma_load_2d_pair(tiles + (size_t)s * STAGE + A_BYTES, &tmW, kb * TC_BK, row, kp_cluster_addr(&full[s], 0));
+            };
+            int pre = 0;
+            if (pair < n_tiles) {
+                const int n0 = (pair / tiles_m) * N_OUT_TILE;
+                pre = min(STAGES, n_kb);
+                for (int i = 0; i < pre; i++) {
+                    if (rank == 0) kp_mbar_expect_tx(&full[i], 2 * STAGE);
+                    load_w(i, i, n0);
+                }
+            }
+            KP_TRACE_MARK_LANE(0);
+            pdl_wait();
+            KP_TRACE_MARK_LANE(1);
+            pdl_launch_dependents();
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+                const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
+                for (int kb = 0; kb < n_kb; kb++) {
+                    if (pre > 0) {
+                        pre--;
+                    } else {
+                        if (*abort_flag || !kp_mbar_wait_bounded(&empty[s], ph ^ 1)) { *abort_flag = 1; ok = false; break; }
+                        if (rank == 0) kp_mbar_expect_tx(&full[s], 2 * STAGE);
+                        load_w(s, kb, n0);
+                    }
+                    kp_tma_load_2d_pair(tiles + (size_t)s * STAGE, &tmA, kb * TC_BK, m0, kp_cluster_addr(&full[s], 0));
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        kp_pdl_begin();
+        if (rank == 0) {                                                  // (the whole warp in step: one elected lane issues)
+            constexpr uint32_t idesc = kp_umma_idesc(2 * TC_BM, BN);
+            int s = 0, ti = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ti++) {
+                const int b2 = ti & 1;
+                ok = !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], ((ti >> 1) & 1) ^ 1);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) { *abort_flag = 1; break; }
+                kp_tc_fence_after();
+                const uint32_t tmem_d = tmem_base + (uint32_t)(b2 * BN);
+                for (int kb = 0; kb < n_kb; kb++) {
+                    ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
+                    if (!ok) { *abort_flag = 1; break; }
+                    kp_tc_fence_after();
+                    const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * STAGE);
+                    kp_umma_bf16_box_pair(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, kb != 0);
+                    kp_umma_commit_pair(&empty[s]);
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+                if (ok) kp_umma_commit_pair(&acc_full[b2]);
+            }
+        }
+    } else {
+        kp_pdl_begin();
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        unsigned char* piece = pieces + (size_t)(warp - 2) * 4096;
+        constexpr bool NARROW = EPI == EPI_STORE || EPI == EPI_ACT || TC_GATED(EPI);   // 16-bit outputs: a piece is 64 columns
+        constexpr int PW = NARROW ? 64 : 32;
+        int ti = 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ti++) {
+            const int b2 = ti & 1;
+            const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM + q * 32, n0 = (tile / tiles_m) * N_OUT_TILE;
+            if (!kp_mbar_wait_bounded(&acc_full[b2], (ti >> 1) & 1) || *abort_flag) { ok = false; break; }
+            kp_tc_fence_after();
+            const uint32_t lane_base = tmem_base + (uint32_t)(b2 * BN) + ((uint32_t)(q * 32) << 16);
+            const int m = m0 + lane;
+#pragma unroll 1
+            for (int c = half * PW; c < N_OUT_TILE && m0 < p.M; c += PW * TC_EPI_PER_Q) {
+                const bool staged = p.vec_ok && n0 + c + PW <= n_out;     // (the same for the whole warp)
+                const int prow = lane >> 3, pch = lane & 7;               // a pass through the piece: rows prow, prow + 4, ...
+                float4 old[8];
+                if (EPI == EPI_ACCUM_F32 && staged) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int row = m0 + i * 4 + prow;
+                        old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (row < p.M) old[i] = *reinterpret_cast<const float4*>((const float*)p.C + (size_t)row * p.ldc + n0 + c + pch * 4);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < PW / 32; h++) {
+                    uint32_t r[32], u[32];
+                    kp_tmem_ld32(lane_base + c + h * 32, r);
+                    if TC_GATED(EPI) kp_tmem_ld32(lane_base + BN / 2 + c + h * 32, u);
+                    const int n_base = n0 + c + h * 32;
+                    float v[32], up[32];
+#pragma unroll
+                    for (int j = 0; j < 32; j++) { v[j] = __uint_as_float(r[j]); up[j] = TC_GATED(EPI) ? __uint_as_float(u[j]) : 0.f; }
+                    if (!staged) {
+                        if (m < p.M) tc_finish<EPI, 32>(p, n_out, v, up, m, n_base);
+                        continue;
+                    }
+                    // (rows beyond the last hold zeros, on which the activation's division is slow: they are left alone)
+                    if (m < p.M) {
+                        tc_bias<EPI, 32>(p, n_out, v, up, n_base);
+#pragma unroll
+                        for (int j = 0; j < 32; j++) v[j] = tc_value<EPI>(p, v[j], up[j]);
+                    }
+                    if (NARROW) {
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            *reinterpret_cast<uint4*>(piece + lane * 128 + (((h * 4 + j) ^ (lane & 7)) * 16)) =
+                                make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]), pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; j++)
+                            *reinterpret_cast<float4*>(piece + lane * 128 + ((j ^ (lane & 7)) * 16)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    }
+                }
+                if (!staged) continue;
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int row = i * 4 + prow;
+                    if (m0 + row >= p.M) continue;
+                    const unsigned char* src = piece + row * 128 + ((pch ^ (row & 7)) * 16);
+                    if (NARROW) {
+                        *reinterpret_cast<uint4*>((bf16*)p.C + (size_t)(m0 + row) * p.ldc + n0 + c + pch * 8) = *reinterpret_cast<const uint4*>(src);
+                    } else {
+                        float4 o = *reinterpret_cast<const float4*>(src);
+                        if (EPI == EPI_ACCUM_F32) { o.x += old[i].x; o.y += old[i].y; o.z += old[i].z; o.w += old[i].w; }
+                        *reinterpret_cast<float4*>((float*)p.C + (size_t)(m0 + row) * p.ldc + n0 + c + pch * 4) = o;
+                    }
+                }
+                __syncwarp();
+            }
+            kp_tc_fence_before();
+            __syncwarp();
+            if (lane == 0) kp_mbar_arrive_cluster(kp_cluster_addr(&acc_empty[b2], 0));
+        }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(&g_tc_status, 1); }
+    }
+    kp_tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) kp_linger_after_failure();
+    if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
+    kp_cluster_sync();                                                    // the other CTA may still signal barriers here
+    if (warp == 1) kp_tmem_dealloc_pair(tmem_base, 2 * BN);
+}
+
 // ------------------------------------------------------------------------------------------ host side
 #define TC_SMEM_KB 208                       // shared memory for the ring
 #ifndef TC_SPLIT_MAX_M_TILES
@@ -499,6 +728,21 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaSt
     return kp_launch_status();
 }
 
+template <int BN, int EPI>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcArgs& a, cudaStream_t s) {
+    auto kern = gemm_tc_pair_kernel<BN, EPI>;
+    static bool ready = false;
+    if (!ready) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_PAIR_SMEM(BN));
+        if (e != cudaSuccess) return (int)e;
+        ready = true;
+    }
+    const int n_out = TC_GATED(EPI) ? a.ff : a.N, n_tile = TC_GATED(EPI) ? BN / 2 : BN;
+    const int n_tiles = ((n_out + n_tile - 1) / n_tile) * ((a.M + 2 * TC_BM - 1) / (2 * TC_BM));
+    const int pairs = tc_n_sm() / 2;
+    return (int)kp_launch_pdl(kern, dim3(2 * (n_tiles < pairs ? n_tiles : pairs)), dim3(TC_THREADS), TC_PAIR_SMEM(BN), s, ta, tw, a);
+}
+
 // Clusters of `cluster` CTAs that run at once, for the tile width and epilogue of a launch.
 static int tc_max_clusters(int bn, int epi, int cluster, int a_rows) {
     int stages = 0;
@@ -592,6 +836,9 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
     a.splits = 1;
     a.kb_per_split = (K + TC_BK - 1) / TC_BK;
     a.a_rows = M >= TC_BM ? TC_BM : (M + 7) / 8 * 8;
+    // what the choice so far brings into the busiest SM, and below what others would
+    const int n_kb_all = (K + TC_BK - 1) / TC_BK;
+    long long cost_now = ((long long)tiles_at(bn) * m_tiles + sms - 1) / sms * n_kb_all * (TC_BK * 2) * (bn + a.a_rows);
     if (m_tiles <= TC_SPLIT_MAX_M_TILES && M > 16 && split) {
         // (the same holds for a few rows of tiles -- a prompt portion or decoded tokens beside one, 129 to 1024
         // rows -- where the product has few tiles and a long K: 264 rows by 2048 x 5632 are 48 tiles of 88 k-blocks)
@@ -619,18 +866,47 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
                 if (best < 0 || cost < best) { best = cost; best_bn = w; best_sp = sp; }
             }
         }
+        if (best >= 0 && (best_sp > 1 || m_tiles > 1)) cost_now = best;
         if (best_sp > 1) {
             bn = best_bn;
             a.splits = best_sp;
             a.kb_per_split = (n_kb + best_sp - 1) / best_sp;
         }
     }
+    // Pairs of CTAs for more than one row of tiles, where they bring in less.  A split's exchange of sums costs more than
+    // its bytes: 1.5 times its cost and 90 KB separate the two (measured, us, split | pairs: 200 rows by 1024 x 1024
+    // 8.6 | 9.7, 300 rows by 2048 x 2048 18.7 | 14.2, 512 rows by 2048 x 5632 22.7 | 29.1, 768 rows 34.3 | 29.9, 200 rows
+    // by 3072 x 2048 14.4 | 11.1).
+    int pair_bn = 0;
+    if (m_tiles > 1) {
+        if (a.splits > 1) cost_now += cost_now / 2 + 90 * 1024;
+        for (int w = 256; w >= 128; w /= 2) {
+            const long long tiles = (long long)tiles_at(w) * ((M + 2 * TC_BM - 1) / (2 * TC_BM));
+            const long long cost = (tiles + sms / 2 - 1) / (sms / 2) * n_kb_all * (TC_BK * 2) * (w / 2 + TC_BM);
+            if (cost <= cost_now) { cost_now = cost; pair_bn = w; }
+        }
+    }
+    cudaStream_t s = (cudaStream_t)stream;
     alignas(64) CUtensorMap ta, tw;
     int st = kp_make_map_bf16_2d(&ta, A, (unsigned long long)M, K, lda, TC_BK, a.a_rows);
     if (st) return st;
-    st = kp_make_map_bf16_2d(&tw, W, (unsigned long long)N, K, ldw, TC_BK, epi == EPI_SWIGLU ? bn / 2 : bn);
+    st = kp_make_map_bf16_2d(&tw, W, (unsigned long long)N, K, ldw, TC_BK, pair_bn ? pair_bn / 2 : (epi == EPI_SWIGLU ? bn / 2 : bn));
     if (st) return st;
-    cudaStream_t s = (cudaStream_t)stream;
+    if (pair_bn) {
+#define TC_PAIR(EPI) return pair_bn == 256 ? launch_pair<256, EPI>(ta, tw, a, s) : launch_pair<128, EPI>(ta, tw, a, s)
+        switch (epi) {
+            case EPI_STORE: TC_PAIR(EPI_STORE);
+            case EPI_STORE_F32: TC_PAIR(EPI_STORE_F32);
+            case EPI_ACCUM_F32: TC_PAIR(EPI_ACCUM_F32);
+            case EPI_ACT: TC_PAIR(EPI_ACT);
+            case EPI_SWIGLU:
+                if (a.act == KP_ACT_GLU_CLAMPED) TC_PAIR(EPI_GLU);
+                if (a.act != KP_ACT_SILU) TC_PAIR(EPI_GATED_RT);
+                TC_PAIR(EPI_SWIGLU);
+            default: return KP_ERR_BAD_ARG;
+        }
+#undef TC_PAIR
+    }
 #define TC_PICK(EPI)                                               \
     switch (bn) {                                                  \
         case 256: return launch<256, EPI>(ta, tw, a, s);           \
@@ -644,20 +920,18 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
         case EPI_ACCUM_F32: TC_PICK(EPI_ACCUM_F32)
         case EPI_ACT: TC_PICK(EPI_ACT)
         case EPI_SWIGLU:
-            if (a.act == KP_ACT_GLU_CLAMPED) {           // an instantiation of its own: the others' epilogues stay as they were
-                switch (bn) {
-                    case 256: return launch<256, EPI_GLU>(ta, tw, a, s);
-                    case 128: return launch<128, EPI_GLU>(ta, tw, a, s);
-                    default: return launch<64, EPI_GLU>(ta, tw, a, s);
-                }
-            }
-            switch (bn) {
-                case 256: return launch<256, EPI_SWIGLU>(ta, tw, a, s);
-                case 128: return launch<128, EPI_SWIGLU>(ta, tw, a, s);
-                default: return launch<64, EPI_SWIGLU>(ta, tw, a, s);
-            }
+#define TC_PICK_GATED(EPI)                                         \
+    switch (bn) {                                                  \
+        case 256: return launch<256, EPI>(ta, tw, a, s);           \
+        case 128: return launch<128, EPI>(ta, tw, a, s);           \
+        default: return launch<64, EPI>(ta, tw, a, s);             \
+    }
+            if (a.act == KP_ACT_GLU_CLAMPED) TC_PICK_GATED(EPI_GLU)
+            if (a.act != KP_ACT_SILU) TC_PICK_GATED(EPI_GATED_RT)
+            TC_PICK_GATED(EPI_SWIGLU)
         default: return KP_ERR_BAD_ARG;
     }
+#undef TC_PICK_GATED
 #undef TC_PICK
 }
 

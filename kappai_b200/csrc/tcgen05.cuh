@@ -99,6 +99,49 @@ __device__ __forceinline__ void kp_tmem_st32(uint32_t taddr, const uint32_t (&r)
 }
 __device__ __forceinline__ void kp_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// ---- pairs of CTAs (cta_group::2): one MMA over two SMs, M = 256, each CTA with its half of A, of B's rows and of the output.
+// One warp of each CTA allocates; the columns are the same in both.
+__device__ __forceinline__ void kp_tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(kp_smem_u32(dst_smem)), "r"(ncols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+}
+__device__ __forceinline__ void kp_tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
+}
+// Four MMAs along K over one 128-byte box of a K-major A and B (64 elements), by an elected lane of the pair's first CTA;
+// the descriptors' addresses hold in both CTAs.  `accumulate` is that of the first.
+__device__ __forceinline__ void kp_umma_bf16_box_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n .reg .pred p, e;\n .reg .b64 a, b;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+                 " @e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+                 " add.s64 a, %1, 2;\n add.s64 b, %2, 2;\n setp.eq.b32 p, 0, 0;\n"
+                 " @e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n"
+                 " add.s64 a, %1, 4;\n add.s64 b, %2, 4;\n"
+                 " @e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n"
+                 " add.s64 a, %1, 6;\n add.s64 b, %2, 6;\n"
+                 " @e tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n}"
+                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate ? 1u : 0u) : "memory");
+}
+// the mbarrier at this place of both CTAs gets one arrival when the pair's MMAs issued so far have completed (elected lane)
+__device__ __forceinline__ void kp_umma_commit_pair(uint64_t* bar) {
+    asm volatile("{\n .reg .pred e;\n .reg .b16 both;\n elect.sync _|e, 0xffffffff;\n mov.b16 both, 3;\n"
+                 " @e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n}"
+                 ::"r"(kp_smem_u32(bar)) : "memory");
+}
+// the address of this CTA's shared-memory place in the cluster's CTA `rank`
+__device__ __forceinline__ uint32_t kp_cluster_addr(const void* p, int rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(kp_smem_u32(p)), "r"(rank));
+    return ra;
+}
+// a box of the 2-D tensor to this CTA's shared memory, its bytes counted at a barrier of either CTA of the pair
+__device__ __forceinline__ void kp_tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void kp_mbar_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
 // Shared-memory matrix descriptor of an operand tile whose rows are 128 bytes (64 bf16), stored with the
 // 128-byte swizzle in atoms of 8 rows (1024 bytes): start address, leading offset 1 (16 bytes; unused by these
 // layouts), stride offset 1024 bytes between 8-row groups, version 1, layout SWIZZLE_128B.  For a K-major
