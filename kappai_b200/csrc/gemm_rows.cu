@@ -1,0 +1,324 @@
+// C[M,N] = A[M,K] * W[N,K]^T for up to 8 rows of bfloat16: the products of a decode step.
+//
+// Such a product is a few microseconds long, and a step is a chain of a hundred of them.  Back to back, the time of
+// gemm_stream.cu hardly depends on whether the weights come from HBM or lie in L2 (2048 x 5632: 8.3 us against 8.1), nor on
+// its loads of A or its epilogue: what it waits for is the hand over of its rings between a producer and eight warps, a
+// stage of 8 rows at a time, on two or three CTAs an SM.  Here nothing is handed over:
+//
+//  * Persistent CTAs of 256 threads, one an SM, walk tiles of W rows: 16 rows, or 8 where that spreads the rows more evenly; 8 gate and
+//    the 8 matching up rows (gated epilogue); the 8 matching rows of B, C and X (conv step).
+//  * The eight warps cut K: of every 512 columns warp w takes the blocks of 32 at w and w + 8.  Each brings its blocks of
+//    the tile's rows (and of A) through a ring of its own by cp.async; no warp waits for another inside a tile.  The
+//    rings are filled with weights, which depend on no earlier kernel, before the wait on the kernel before.
+//  * W rows are the m side of mma.m16n8k16, the batch rows the n side.  A lane's operands are 16 bytes of one row (the
+//    same permutation of k on both sides); the 16-byte chunks of odd rows are stored four places on, so that the eight
+//    lanes of a quarter warp read all banks once.
+//  * At a tile's end the warps' partial sums are added in warp order from zero.  The order of every sum is that of
+//    gemm_stream.cu, so a row's result does not depend on which of the two ran.
+//
+// Measured back to back, us, gemm_stream | this, one row and 8: 2048 x 5632 7.8 | 6.5, 7.9 | 7.1; 6144 x 2048 6.8 | 5.2,
+// 6.9 | 5.7; 2048 x 2048 3.8 | 2.6, 3.8 | 2.8; at 16 rows it loses (8.2 | 9.0), as A then weighs as much as W.  A decode
+// step of the 1.2B shape: one request 601 -> 506 us, eight 607 -> 550; of the 350M shape 376 -> 343.  One CTA must have an
+// SM to itself: with rings of 100 KB two fit, the next product's CTAs come in early and unevenly, two on some SMs and none
+// on others, and a step takes 613 us.  Rings of 122 KB 524, 155 KB 506, 190 KB 511, 210 KB 542.
+//
+// Epilogues as in gemm_stream.cu.  K a multiple of 512.
+#include "mma.cuh"
+
+#define EPI_STORE 0
+#define EPI_STORE_F32 1
+#define EPI_ACCUM_F32 2
+#define EPI_SWIGLU 3
+#define EPI_CONV_STEP 4
+#define EPI_ACT 6
+
+#define RW_WARPS 8
+#define RW_SMEM (155 * 1024)                 // shared memory of the rings: more than half an SM's, see above
+#define RW_MAX_STAGES 8
+
+struct RowsArgs {
+    const bf16* A; int lda;
+    const bf16* W; int ldw;
+    const float* bias;
+    void* C; int ldc;
+    int M, N, K, ff;                         // ff: output columns of an epilogue that joins rows of W (gated: N / 2; conv step: N / 3)
+    int act;
+    float glu_limit, glu_alpha, glu_shift;
+    const float* conv_w; const float* conv_bias; float* conv_state;
+    const int* seg_pos; const int* seg_slot;
+    int conv_k;
+};
+
+// WR: rows of W a tile (8, 16, or 24: the conv step).
+template <int WR, int EPI>
+__global__ void __launch_bounds__(RW_WARPS * 32, 1)
+gemm_rows_kernel(const RowsArgs p) {
+    constexpr int MT = (WR + 15) / 16;                                   // m16 tiles (of a 24-row tile's second one half is empty)
+    constexpr int JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
+    constexpr int TROWS = WR / JOINS;                                    // output columns a tile
+    constexpr int W_BYTES = WR * 128, STAGE = W_BYTES + 8 * 128;
+    constexpr int S = RW_SMEM / (RW_WARPS * STAGE) > RW_MAX_STAGES ? RW_MAX_STAGES : RW_SMEM / (RW_WARPS * STAGE);
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int M = p.M, n_out = JOINS > 1 ? p.ff : p.N;
+    const int n_tiles = (n_out + TROWS - 1) / TROWS, n_ch = p.K / 512;   // chunks of 64 columns a warp and tile
+    unsigned char* ring = smem + (size_t)warp * S * STAGE;
+    float* red = reinterpret_cast<float*>(smem + (size_t)RW_WARPS * S * STAGE);   // [2][warp][MT][4][32]
+    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - blockIdx.x - 1) / gridDim.x + 1 : 0;
+    const int total = my_tiles * n_ch;
+
+    const int cr = lane >> 3, cc = lane & 7;                             // copies: 4 rows by 8 chunks at a time
+    const int col0 = warp * 32 + (cc >> 2) * 256 + (cc & 3) * 8;         // this lane's column of a warp's chunk 0
+    int ld_tile = blockIdx.x, ld_c = 0, ld_s = 0;                        // the next stage to be asked for
+    auto load_w = [&](int tile, int c, int s) {
+        unsigned char* dst = ring + (size_t)s * STAGE;
+        const int n0 = tile * TROWS;
+#pragma unroll
+        for (int i = 0; i < WR / 4; i++) {
+            const int row = i * 4 + cr;                                  // row of the tile
+            const int wrow = JOINS > 1 ? (row >> 3) * p.ff + min(n0 + (row & 7), n_out - 1) : min(n0 + row, n_out - 1);
+            cp_async16(dst + row * 128 + ((cc ^ ((row & 1) << 2)) * 16), p.W + (size_t)wrow * p.ldw + c * 512 + col0, true);
+        }
+    };
+    auto load_a = [&](int c, int s) {
+        unsigned char* dst = ring + (size_t)s * STAGE + W_BYTES;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int row = i * 4 + cr;
+            if (row < M) cp_async16(dst + row * 128 + ((cc ^ ((row & 1) << 2)) * 16), p.A + (size_t)row * p.lda + c * 512 + col0, true);
+        }
+    };
+    auto advance = [&]() {
+        if (++ld_c == n_ch) { ld_c = 0; ld_tile += gridDim.x; }
+        if (++ld_s == S) ld_s = 0;
+    };
+
+    KP_TRACE_MARK(0);
+    pdl_launch_dependents();                                             // (what comes next reads nothing before its own wait)
+    for (int i = 0; i < S; i++) {
+        if (i < total) { load_w(ld_tile, ld_c, ld_s); advance(); }
+        cp_async_commit();
+    }
+    pdl_wait();
+    KP_TRACE_MARK(1);
+    for (int i = 0; i < S; i++) {
+        if (i < total) load_a(i % n_ch, i);
+        cp_async_commit();
+    }
+
+    int s = 0, buf = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
+        const int n0 = tile * TROWS;
+        // what the epilogue needs beside the sums is asked for now: its trips to L2 run under the main loop
+        float pre_c = 0.f, pre_hist[3] = {0.f, 0.f, 0.f}, pre_cw[4] = {0.f, 0.f, 0.f, 0.f};
+        const int om = threadIdx.x / TROWS, on = n0 + threadIdx.x % TROWS;   // this thread's output (the first TROWS * M threads)
+        const bool mine = om < M && on < n_out;
+        if (mine) {
+            if (EPI == EPI_ACCUM_F32) pre_c = ((const float*)p.C)[(size_t)om * p.ldc + on];
+            if (EPI == EPI_CONV_STEP && p.conv_k <= 4) {
+                const bool fresh = p.seg_pos[om] == 0;
+                const float* st = p.conv_state + (size_t)p.seg_slot[om] * (p.conv_k - 1) * p.ff;
+                const float* cw = p.conv_w + (size_t)on * p.conv_k;
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    if (k < p.conv_k - 1) pre_hist[k] = fresh ? 0.f : st[(size_t)k * p.ff + on];
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (k < p.conv_k) pre_cw[k] = cw[k];
+            }
+        }
+        float acc[MT][4];
+#pragma unroll
+        for (int a = 0; a < MT; a++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[a][i] = 0.f;
+        for (int c = 0; c < n_ch; c++) {
+            cp_async_wait<S - 1>();                                      // this stage has come, all but the S - 1 behind it
+            __syncwarp();
+            const unsigned char* st = ring + (size_t)s * STAGE;
+#pragma unroll
+            for (int b = 0; b < 2; b++) {                                // the blocks of 32 columns
+                const int at = ((b * 4 + t) ^ ((g & 1) << 2)) * 16;
+                uint4 w[2 * MT];
+#pragma unroll
+                for (int i = 0; i < 2 * MT; i++) w[i] = i * 8 < WR ? *reinterpret_cast<const uint4*>(st + (i * 8 + g) * 128 + at) : make_uint4(0, 0, 0, 0);
+                const uint4 x = *reinterpret_cast<const uint4*>(st + W_BYTES + g * 128 + at);   // (rows beyond M: any values, nobody reads their sums)
+#pragma unroll
+                for (int a = 0; a < MT; a++) {
+                    mma_bf16(acc[a], w[2 * a].x, w[2 * a + 1].x, w[2 * a].y, w[2 * a + 1].y, x.x, x.y);
+                    mma_bf16(acc[a], w[2 * a].z, w[2 * a + 1].z, w[2 * a].w, w[2 * a + 1].w, x.z, x.w);
+                }
+            }
+            __syncwarp();                                                // the stage has been read
+            if (ld_tile < n_tiles) { load_w(ld_tile, ld_c, ld_s); load_a(ld_c, ld_s); advance(); }
+            cp_async_commit();
+            if (++s == S) s = 0;
+        }
+        // acc[a]: rows of W 16 a + g (elements 0, 1) and 16 a + g + 8 (2, 3), batch rows 2 t, 2 t + 1
+        float* r = red + (size_t)buf * RW_WARPS * MT * 128;
+#pragma unroll
+        for (int a = 0; a < MT; a++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) r[(warp * MT + a) * 128 + i * 32 + lane] = acc[a][i];
+        __syncthreads();                                                 // (the other half of `red` is free: its readers were here)
+        if (mine) {
+            // the sum of W row `row` of the tile for this thread's batch row, over the warps in order
+            auto sum_of = [&](int row) {
+                const int a = row >> 4, i = ((row & 8) ? 2 : 0) + (om & 1), l = (row & 7) * 4 + (om >> 1);
+                float v = 0.f;
+#pragma unroll
+                for (int w8 = 0; w8 < RW_WARPS; w8++) v += r[(w8 * MT + a) * 128 + i * 32 + l];
+                return v;
+            };
+            const int m = om, n = on, lr = on - n0;
+            float v = sum_of(lr);
+            if (p.bias) v += p.bias[n];
+            const size_t o = (size_t)m * p.ldc + n;
+            if (EPI == EPI_CONV_STEP) {
+                float cg = sum_of(8 + lr), xv = sum_of(16 + lr);
+                if (p.bias) { cg += p.bias[p.ff + n]; xv += p.bias[2 * p.ff + n]; }
+                // B, C and X as the separate product stores them, then shortconv.cu's decode step: every product and
+                // sum rounded on its own (src/backend/cpu/common.c:2393-2431)
+                const float b = to_f32(from_f32<bf16>(v)), cq = to_f32(from_f32<bf16>(cg)), xq = to_f32(from_f32<bf16>(xv));
+                const int d = p.ff, Kc = p.conv_k;
+                float* st = p.conv_state + (size_t)p.seg_slot[m] * (Kc - 1) * d;
+                const float bx = __fmul_rn(b, xq);
+                float hist[15], tap[16];
+                if (Kc <= 4) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) hist[k] = pre_hist[k];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) tap[k] = pre_cw[k];
+                } else {
+                    const bool fresh = p.seg_pos[m] == 0;
+                    const float* cw = p.conv_w + (size_t)n * Kc;
+                    for (int k = 0; k < Kc - 1; k++) hist[k] = fresh ? 0.f : st[(size_t)k * d + n];
+                    for (int k = 0; k < Kc; k++) tap[k] = cw[k];
+                }
+                float sum;
+                if (Kc == 3) {
+                    sum = __fadd_rn(__fadd_rn(__fmul_rn(hist[0], tap[0]), __fmul_rn(hist[1], tap[1])), __fmul_rn(bx, tap[2]));
+                } else {
+                    sum = __fmul_rn(bx, tap[Kc - 1]);
+                    for (int k = 0; k < Kc - 1; k++) sum = __fadd_rn(sum, __fmul_rn(hist[k], tap[k]));
+                }
+                if (p.conv_bias) sum = __fadd_rn(sum, p.conv_bias[n]);
+                ((bf16*)p.C)[o] = from_f32<bf16>(__fmul_rn(cq, sum));
+                for (int k = 0; k + 1 < Kc - 1; k++) st[(size_t)k * d + n] = hist[k + 1];
+                st[(size_t)(Kc - 2) * d + n] = bx;
+            } else if (EPI == EPI_SWIGLU) {
+                float u = sum_of(8 + lr);
+                if (p.bias) u += p.bias[p.ff + n];
+                // gate and up are rounded to the storage type before the activation, as the unfused path stores them
+                const float gq = to_f32(from_f32<bf16>(v)), uq = to_f32(from_f32<bf16>(u));
+                ((bf16*)p.C)[o] = from_f32<bf16>(kp_gated_epilogue(p.act, gq, uq, p.glu_limit, p.glu_alpha, p.glu_shift));
+            } else if (EPI == EPI_STORE) {
+                ((bf16*)p.C)[o] = from_f32<bf16>(v);
+            } else if (EPI == EPI_ACT) {
+                ((bf16*)p.C)[o] = from_f32<bf16>(kp_act_plain(p.act, v));
+            } else if (EPI == EPI_STORE_F32) {
+                ((float*)p.C)[o] = v;
+            } else {
+                ((float*)p.C)[o] = pre_c + v;
+            }
+        }
+    }
+    KP_TRACE_MARK(2);
+}
+
+static int rw_n_sm() {
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    }
+    return n;
+}
+
+template <int WR, int EPI>
+static int rows_launch(const RowsArgs& a, cudaStream_t s) {
+    constexpr int MT = (WR + 15) / 16, JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
+    constexpr int STAGE = WR * 128 + 8 * 128;
+    constexpr int S = RW_SMEM / (RW_WARPS * STAGE) > RW_MAX_STAGES ? RW_MAX_STAGES : RW_SMEM / (RW_WARPS * STAGE);
+    constexpr size_t smem = (size_t)RW_WARPS * S * STAGE + sizeof(float) * 2 * RW_WARPS * MT * 128;
+    auto kern = gemm_rows_kernel<WR, EPI>;
+    static bool ready = false;
+    if (!ready) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        ready = true;
+    }
+    const int n_out = JOINS > 1 ? a.ff : a.N, n_tiles = (n_out + WR / JOINS - 1) / (WR / JOINS);
+    return (int)kp_launch_pdl(kern, dim3(n_tiles < rw_n_sm() ? n_tiles : rw_n_sm()), dim3(RW_WARPS * 32), smem, s, a);
+}
+
+static int rows_run(const RowsArgs& a, int epi, cudaStream_t s) {
+    // tiles of 8 rows where the busiest SM then has fewer rows of W (3072 rows: 24 against 32; 1024 rows: 8 against 16)
+    const int sms = rw_n_sm();
+    const auto busiest = [&](int rows) { return ((a.N + rows - 1) / rows + sms - 1) / sms * rows; };
+    const bool narrow = busiest(8) < busiest(16);
+#define RW_PICK(EPI) return narrow ? rows_launch<8, EPI>(a, s) : rows_launch<16, EPI>(a, s)
+    switch (epi) {
+        case EPI_STORE: RW_PICK(EPI_STORE);
+        case EPI_STORE_F32: RW_PICK(EPI_STORE_F32);
+        case EPI_ACCUM_F32: RW_PICK(EPI_ACCUM_F32);
+        case EPI_ACT: RW_PICK(EPI_ACT);
+        case EPI_SWIGLU: return rows_launch<16, EPI_SWIGLU>(a, s);
+        case EPI_CONV_STEP: return rows_launch<24, EPI_CONV_STEP>(a, s);
+        default: return KP_ERR_BAD_ARG;
+    }
+#undef RW_PICK
+}
+
+static int rows_check(const RowsArgs& a) {
+    if (a.M > 8 || a.K < 512 || (a.K % 512) || (a.lda & 7) || (a.ldw & 7) || ((uintptr_t)a.A & 15) || ((uintptr_t)a.W & 15))
+        return KP_ERR_UNSUPPORTED;
+    return 0;
+}
+
+extern "C" {
+
+// epi and glu as in gemm_stream.cu
+int kp_gemm_rows(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K,
+                 int epi, float limit, float alpha, float shift, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    RowsArgs a = {};
+    a.A = (const bf16*)A; a.lda = lda; a.W = (const bf16*)W; a.ldw = ldw; a.bias = bias; a.C = C; a.ldc = ldc;
+    a.M = M; a.N = N; a.K = K;
+    a.act = KP_EPI_ACT(epi);
+    epi = KP_EPI_KIND(epi);
+    if (a.act != KP_ACT_SILU && a.act != KP_ACT_RELU && a.act != KP_ACT_GELU_TANH && !(a.act == KP_ACT_GLU_CLAMPED && epi == EPI_SWIGLU) &&
+        !(a.act == KP_ACT_RELU_SQ && epi == EPI_ACT)) return KP_ERR_UNSUPPORTED;
+    a.glu_limit = limit; a.glu_alpha = alpha; a.glu_shift = shift;
+    if (epi == EPI_CONV_STEP) return KP_ERR_BAD_ARG;
+    if (epi == EPI_SWIGLU) {
+        if (N & 1) return KP_ERR_BAD_ARG;
+        a.ff = N / 2;
+    }
+    int st = rows_check(a);
+    if (st) return st;
+    return rows_run(a, epi, (cudaStream_t)stream);
+}
+
+// The in_proj of the gated short convolution with the conv step of a decode step in its epilogue: W = [B; C; X]
+// ([3 d, K]), C = [M, d] bfloat16; conv_w [d][conv_k], conv_bias [d] or null, state [slots][conv_k - 1][d], and
+// for each of the M <= 8 rows its position (seg_pos) and state slot (seg_slot).  Rows are one-row segments.
+int kp_gemm_rows_conv_step(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N,
+                           int K, const float* conv_w, const float* conv_bias, float* conv_state, const int* seg_pos,
+                           const int* seg_slot, int conv_k, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    RowsArgs a = {};
+    a.A = (const bf16*)A; a.lda = lda; a.W = (const bf16*)W; a.ldw = ldw; a.bias = bias; a.C = C; a.ldc = ldc;
+    a.M = M; a.N = N; a.K = K; a.ff = N / 3;
+    if (N % 3) return KP_ERR_BAD_ARG;
+    int st = rows_check(a);
+    if (st) return st;
+    if (conv_k < 2 || conv_k > 16 || !conv_w || !conv_state || !seg_pos || !seg_slot) return KP_ERR_UNSUPPORTED;
+    a.conv_w = conv_w; a.conv_bias = conv_bias; a.conv_state = conv_state; a.seg_pos = seg_pos; a.seg_slot = seg_slot;
+    a.conv_k = conv_k;
+    return rows_run(a, EPI_CONV_STEP, (cudaStream_t)stream);
+}
+
+}  // extern "C"

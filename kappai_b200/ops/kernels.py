@@ -1629,6 +1629,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[
 
 
 STREAM_MAX_M = 64          # rows up to which the bulk-copy kernel is preferred
+ROWS_MAX_M = 8             # of them, rows up to which csrc/gemm_rows.cu runs instead: the same sums in the same order
 USE_STREAM = True         # few-row products go to the bulk-copy kernel where their shape fits it
 
 
@@ -1677,8 +1678,9 @@ def gemm_stream_conv_step(a: torch.Tensor, w_in: torch.Tensor, bias: Optional[to
             _need(t, nm, torch.float32)
             if t.numel() != n:
                 raise KernelError(f"gemm_stream_conv_step: {nm} size")
-    lib = load_library("gemm_stream")
-    _run("gemm_stream_conv_step", lib.kp_gemm_stream_conv_step, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
+    few = M <= ROWS_MAX_M
+    lib = load_library("gemm_rows" if few else "gemm_stream")
+    _run("gemm_stream_conv_step", lib.kp_gemm_rows_conv_step if few else lib.kp_gemm_stream_conv_step, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
          _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, _ptr(conv_w), _ptr(conv_bias), _ptr(state), _ptr(seg_pos),
          _ptr(seg_slot), conv_k, STREAM, tag=f" {N}x{K}", work=_gemm_work(M, N, K, a, w_in, out))
     return out
@@ -1693,6 +1695,9 @@ def _glu_floats(glu):
     if not limit > 0:
         raise KernelError("the gated unit's limit must be positive")
     return ctypes.c_float(limit), ctypes.c_float(alpha), ctypes.c_float(shift)
+
+
+_NO_LIMITS = (ctypes.c_float(0.0),) * 3
 
 
 def _fused_activation(name: str) -> int:
@@ -1757,6 +1762,11 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optio
     if plain_activation is not None:
         epi = _plain_epilogue(epi, plain_activation)
     consts = _glu_floats(glu) if swiglu and glu is not None else ()
+    if USE_STREAM and stream_fits(K, swiglu) and stream_pays(N, K) and M <= ROWS_MAX_M:
+        lib = load_library("gemm_rows")
+        _run("gemm_stream", lib.kp_gemm_rows, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
+             _rows_2d(out, "out"), M, N, K, epi, *(consts or _NO_LIMITS), STREAM, tag=f" {N}x{K}", work=_gemm_work(M, N, K, a, w, out))
+        return out
     if USE_STREAM and stream_fits(K, swiglu) and stream_pays(N, K) and M <= STREAM_MAX_M:
         lib = load_library("gemm_stream")
         _run("gemm_stream", lib.kp_gemm_stream_glu if consts else lib.kp_gemm_stream, _ptr(a), _rows_2d(a, "a"), _ptr(w),
