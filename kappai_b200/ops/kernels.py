@@ -47,8 +47,11 @@ def _stream() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+_NULL = ctypes.c_void_p(0)
+
+
+def _ptr(t: Optional[torch.Tensor], _p=ctypes.c_void_p) -> ctypes.c_void_p:
+    return _NULL if t is None else _p(t.data_ptr())
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:
@@ -130,7 +133,8 @@ def _run(what: str, fn, *args, tag: str = "", work=None) -> None:
     answer.  ``tag`` and ``work`` = (flops, bytes) describe the call to a :class:`KernelTimer`."""
     timer = TIMER[0]
     if timer is None:
-        _check(fn(*[_stream() if a is STREAM else a for a in args]), what)
+        # (nearly every launcher takes the stream last)
+        _check(fn(*args[:-1], _stream()) if args[-1] is STREAM else fn(*[_stream() if a is STREAM else a for a in args]), what)
         if LAUNCH_LOG[0] is not None and tag:
             LAUNCH_LOG[0][-1] += tag
         return
@@ -143,6 +147,16 @@ def _run(what: str, fn, *args, tag: str = "", work=None) -> None:
 
 def _gemm_work(M: int, N: int, K: int, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor):
     return (2 * M * N * K, M * K * a.element_size() + N * K * w.element_size() + out.numel() * out.element_size())
+
+
+def _run_gemm(what: str, fn, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *args) -> None:
+    """:func:`_run` for a matrix product; what describes it to a timer or a log is made only where one listens (a step
+    launches about a hundred products from Python)."""
+    if TIMER[0] is None and LAUNCH_LOG[0] is None:
+        _run(what, fn, *args)
+    else:
+        (M, K), N = a.shape, w.shape[0]
+        _run(what, fn, *args, tag=f" {N}x{K}", work=_gemm_work(M, N, K, a, w, out))
 
 
 LAUNCH_LOG = [None]        # a list: every launch appends its name (bench.py --probe timeline names a step's kernels by it)
@@ -163,9 +177,10 @@ def _check(status: int, what: str) -> None:
 
 def _rows_2d(t: torch.Tensor, name: str) -> int:
     """Leading dimension (in elements) of a 2-D tensor whose rows are contiguous."""
-    if t.dim() != 2 or t.stride(1) != 1:
+    s = t.stride()
+    if len(s) != 2 or s[1] != 1:
         raise KernelError(f"{name}: expected a 2-D tensor with contiguous rows")
-    return t.stride(0)
+    return s[0]
 
 
 # --------------------------------------------------------------- status words
@@ -618,8 +633,8 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
     else:
         raise KernelError("gemm: output dtype must be the operand dtype or float32")
     lib = load_library("gemm_simt")
-    _run("gemm_nt_simt", lib.kp_gemm_nt_simt, _ptr(a), _ptr(w), _ptr(bias), _ptr(out), M, N, K, lda, ldw, ldc, epi,
-         dtype_code(a.dtype), STREAM, tag=f" {N}x{K}", work=_gemm_work(M, N, K, a, w, out))
+    _run_gemm("gemm_nt_simt", lib.kp_gemm_nt_simt, a, w, out, _ptr(a), _ptr(w), _ptr(bias), _ptr(out), M, N, K, lda, ldw, ldc, epi,
+         dtype_code(a.dtype), STREAM)
     return out
 
 
@@ -1559,24 +1574,31 @@ EPI_SWIGLU = 3
 EPI_ACT = 6
 
 
+def _rows_16_bytes(t: torch.Tensor) -> bool:
+    """Is every row of a 2-D bfloat16 tensor contiguous and 16-byte aligned?"""
+    ld, one = t.stride()
+    return one == 1 and ld % 8 == 0 and t.data_ptr() % 16 == 0
+
+
 def skinny_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Can the weight-streaming kernel take this product?"""
-    return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.shape[0] <= SKINNY_MAX_M
-            and a.shape[1] % 32 == 0 and a.stride(1) == 1 and w.stride(1) == 1 and a.stride(0) % 8 == 0
-            and w.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    M, K = a.shape
+    return (M <= SKINNY_MAX_M and K % 32 == 0 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+            and _rows_16_bytes(a) and _rows_16_bytes(w))
 
 
 USE_TC = True              # bfloat16 products of more than 64 rows (and some of fewer) run on tcgen05 tensor cores
 
 
-TC_HEAD_FROM_M = 2         # rows from which a 65536-row head goes to the tcgen05 kernel (measured: one row ties)
+TC_HEAD_FROM_M = 1         # rows from which a 65536-row head goes to the tcgen05 kernel (a step of one row 509 -> 501 us, of
+                           # the 350M shape 344 -> 334: its first weights are on their way before the wait on the norm)
 TC_SPLIT_FROM_M = 17       # rows from which every product goes to the tcgen05 kernel (cut along K where that pays)
 
 
 def tc_pays_for_few_rows(M: int, N: int, swiglu: bool) -> bool:
     """Few-row products that the tcgen05 kernel runs faster than the weight-streaming
     kernels (measured on B200, K = 2048, inside a decode step): the 65536-row head from
-    2 rows on (a step of 2 rows 638 -> 602 us, of 4 rows 661 -> 624; one row ties), every
+    1 row on (a step of 2 rows 638 -> 602 us, of 4 rows 661 -> 624, of one 509 -> 501), every
     product from 17 rows on (there the kernel cuts the product along K: a step of 64 rows
     1600 -> 1320 us), and below that wide products from 32 rows on."""
     if M >= TC_SPLIT_FROM_M:
@@ -1588,9 +1610,8 @@ def tc_pays_for_few_rows(M: int, N: int, swiglu: bool) -> bool:
 
 def tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Can the tcgen05 kernel take this product (bfloat16, 16-byte aligned rows, K a multiple of 8)?"""
-    return (USE_TC and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.shape[1] % 8 == 0
-            and a.stride(1) == 1 and w.stride(1) == 1 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
-            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    return (USE_TC and a.shape[1] % 8 == 0 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+            and _rows_16_bytes(a) and _rows_16_bytes(w))
 
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -1615,16 +1636,14 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[
     lib = load_library("gemm_tc")
     if swiglu and glu is not None:
         epi = _skinny_epilogue(out, accumulate, swiglu) | (ACT_GLU_CLAMPED << 8)
-        _run("gemm_tc", lib.kp_gemm_tc_split_glu, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
-             _rows_2d(out, "out"), M, N, K, epi, 1 if split else 0, *_glu_floats(glu), STREAM, tag=f" {N}x{K}",
-             work=_gemm_work(M, N, K, a, w, out))
+        _run_gemm("gemm_tc", lib.kp_gemm_tc_split_glu, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
+             _rows_2d(out, "out"), M, N, K, epi, 1 if split else 0, *_glu_floats(glu), STREAM)
         return out
     epi = _skinny_epilogue(out, accumulate, swiglu) | (_fused_activation(activation) << 8 if swiglu else 0)
     if plain_activation is not None:
         epi = _plain_epilogue(epi, plain_activation)
-    _run("gemm_tc", lib.kp_gemm_tc_split, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
-         _rows_2d(out, "out"), M, N, K, epi, 1 if split else 0, STREAM, tag=f" {N}x{K}",
-         work=_gemm_work(M, N, K, a, w, out))
+    _run_gemm("gemm_tc", lib.kp_gemm_tc_split, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
+         _rows_2d(out, "out"), M, N, K, epi, 1 if split else 0, STREAM)
     return out
 
 
@@ -1680,9 +1699,9 @@ def gemm_stream_conv_step(a: torch.Tensor, w_in: torch.Tensor, bias: Optional[to
                 raise KernelError(f"gemm_stream_conv_step: {nm} size")
     few = M <= ROWS_MAX_M
     lib = load_library("gemm_rows" if few else "gemm_stream")
-    _run("gemm_stream_conv_step", lib.kp_gemm_rows_conv_step if few else lib.kp_gemm_stream_conv_step, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
+    _run_gemm("gemm_stream_conv_step", lib.kp_gemm_rows_conv_step if few else lib.kp_gemm_stream_conv_step, a, w_in, out, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
          _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, _ptr(conv_w), _ptr(conv_bias), _ptr(state), _ptr(seg_pos),
-         _ptr(seg_slot), conv_k, STREAM, tag=f" {N}x{K}", work=_gemm_work(M, N, K, a, w_in, out))
+         _ptr(seg_slot), conv_k, STREAM)
     return out
 
 
@@ -1764,19 +1783,17 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optio
     consts = _glu_floats(glu) if swiglu and glu is not None else ()
     if USE_STREAM and stream_fits(K, swiglu) and stream_pays(N, K) and M <= ROWS_MAX_M:
         lib = load_library("gemm_rows")
-        _run("gemm_stream", lib.kp_gemm_rows, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
-             _rows_2d(out, "out"), M, N, K, epi, *(consts or _NO_LIMITS), STREAM, tag=f" {N}x{K}", work=_gemm_work(M, N, K, a, w, out))
+        _run_gemm("gemm_stream", lib.kp_gemm_rows, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
+             _rows_2d(out, "out"), M, N, K, epi, *(consts or _NO_LIMITS), STREAM)
         return out
     if USE_STREAM and stream_fits(K, swiglu) and stream_pays(N, K) and M <= STREAM_MAX_M:
         lib = load_library("gemm_stream")
-        _run("gemm_stream", lib.kp_gemm_stream_glu if consts else lib.kp_gemm_stream, _ptr(a), _rows_2d(a, "a"), _ptr(w),
-             _rows_2d(w, "w"), _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, epi, *consts, STREAM, tag=f" {N}x{K}",
-             work=_gemm_work(M, N, K, a, w, out))
+        _run_gemm("gemm_stream", lib.kp_gemm_stream_glu if consts else lib.kp_gemm_stream, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w),
+             _rows_2d(w, "w"), _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, epi, *consts, STREAM)
         return out
     lib = load_library("gemm_skinny")
-    _run("gemm_skinny", lib.kp_gemm_skinny_glu if consts else lib.kp_gemm_skinny, _ptr(a), _rows_2d(a, "a"), _ptr(w),
-         _rows_2d(w, "w"), _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, epi, *consts, STREAM, tag=f" {N}x{K}",
-         work=_gemm_work(M, N, K, a, w, out))
+    _run_gemm("gemm_skinny", lib.kp_gemm_skinny_glu if consts else lib.kp_gemm_skinny, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w),
+         _rows_2d(w, "w"), _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, epi, *consts, STREAM)
     return out
 
 
