@@ -83,8 +83,9 @@ class PagePool:
         return _ceil_div(n_tokens // self.every, self.page_size)
 
     def pages_needed(self, req: Hashable, new_len: int) -> int:
-        have = len(self._tables.get(req, ()))
-        return max(0, self.pages_for(new_len) - have)
+        # (asked for every request of every step: no further calls)
+        need = -(-(new_len // self.every) // self.page_size) - len(self._tables.get(req, ()))
+        return need if need > 0 else 0
 
     def slot(self, req: Hashable, pos: int) -> int:
         """Physical slot (page * page_size + offset) of the entry that position ``pos`` writes: its own, or in a pool
@@ -242,6 +243,7 @@ class CacheManager:
 
     def __init__(self, groups: Dict[Hashable, tuple], n_slots: int):
         self.pools: Dict[Hashable, PagePool] = {k: PagePool(*v) for k, v in groups.items()}
+        self._releasing = [p for p in self.pools.values() if p.window is not None or p.block is not None]
         self.slots = SlotPool(n_slots)
         self.requests: Dict[Hashable, RequestCache] = {}
 
@@ -272,9 +274,12 @@ class CacheManager:
     def try_extend(self, req: Hashable, new_len: int) -> bool:
         """:meth:`extend` that answers False (and takes nothing) where it would raise OutOfPages."""
         pools = self.pools.values()
-        needs = [p.pages_needed(req, new_len) for p in pools]
-        if not any(needs):
+        for p in pools:                          # (most decoded tokens fill a page that is there)
+            if p.pages_needed(req, new_len):
+                break
+        else:
             return True
+        needs = [p.pages_needed(req, new_len) for p in pools]
         if any(n > p.n_free for n, p in zip(needs, pools)):
             return False
         for p in pools:
@@ -287,7 +292,7 @@ class CacheManager:
         if new_len < rc.length:
             raise CacheError("a request's length cannot shrink")
         rc.length = new_len
-        for p in self.pools.values():
+        for p in self._releasing:
             p.release_behind(req, new_len)
 
     # -- end

@@ -150,51 +150,42 @@ def lay_out_step(segments: Sequence[Segment], groups: Dict[Hashable, int], vocab
     """
     if not segments:
         raise BatchError("a step needs at least one segment")
+    n_seg = len(segments)
+    seg_len = [len(s.tokens) for s in segments]
     seen = set()
-    n_rows = 0
-    token_arrays = []
-    for s in segments:
+    for s, n in zip(segments, seg_len):
         if s.req in seen:
             raise BatchError(f"request {s.req!r} appears twice in one step")
         seen.add(s.req)
-        if len(s.tokens) < 1:
+        if n < 1:
             raise BatchError(f"request {s.req!r}: a segment needs at least one token")
-        if s.pos_start < 0 or s.pos_start + len(s.tokens) > max_positions:
-            raise BatchError(f"request {s.req!r}: positions {s.pos_start}..{s.pos_start + len(s.tokens) - 1} "
+        if s.pos_start < 0 or s.pos_start + n > max_positions:
+            raise BatchError(f"request {s.req!r}: positions {s.pos_start}..{s.pos_start + n - 1} "
                              f"exceed the engine's limit of {max_positions}")
-        ids = np.asarray(s.tokens, dtype=np.int64)
-        if ids.min() < 0 or ids.max() >= vocab_size:
-            t = int(ids[(ids < 0) | (ids >= vocab_size)][0])
-            raise BatchError(f"request {s.req!r}: token id {t} outside the vocabulary of {vocab_size}")
-        token_arrays.append(ids)
         for w in s.want:
-            if not (0 <= int(w) < len(s.tokens)):
-                raise BatchError(f"request {s.req!r}: wanted index {w} outside its {len(s.tokens)} tokens")
-        n_rows += len(s.tokens)
-    n_seg = len(segments)
+            if not (0 <= int(w) < n):
+                raise BatchError(f"request {s.req!r}: wanted index {w} outside its {n} tokens")
+    n_rows = sum(seg_len)
 
-    token_ids = np.empty(n_rows, np.int32)
-    positions = np.empty(n_rows, np.int32)
-    row_seg = np.empty(n_rows, np.int32)
+    # rows by arrays over all segments (a step may have hundreds of one row)
+    ids = np.asarray([t for s in segments for t in s.tokens], dtype=np.int64)
+    lens = np.asarray(seg_len, dtype=np.int64)
     cu_rows = np.zeros(n_seg + 1, np.int32)
-    seg_pos = np.empty(n_seg, np.int32)
-    seg_slot = np.empty(n_seg, np.int32)
-    logit_rows: List[int] = []
-    r = 0
-    for i, s in enumerate(segments):
-        n = len(s.tokens)
-        token_ids[r:r + n] = token_arrays[i]
-        positions[r:r + n] = np.arange(s.pos_start, s.pos_start + n)
-        row_seg[r:r + n] = i
-        seg_pos[i], seg_slot[i] = s.pos_start, s.slot
-        logit_rows.extend(r + int(w) for w in s.want)
-        r += n
-        cu_rows[i + 1] = r
+    np.cumsum(lens, out=cu_rows[1:])
+    row_seg = np.repeat(np.arange(n_seg, dtype=np.int32), lens)
+    bad = (ids < 0) | (ids >= vocab_size)
+    if bad.any():
+        r = int(np.argmax(bad))
+        raise BatchError(f"request {segments[row_seg[r]].req!r}: token id {int(ids[r])} outside the vocabulary of {vocab_size}")
+    token_ids = ids.astype(np.int32)
+    seg_pos = np.asarray([s.pos_start for s in segments], dtype=np.int32)
+    seg_slot = np.asarray([s.slot for s in segments], dtype=np.int32)
+    positions = np.arange(n_rows, dtype=np.int32) + (seg_pos - cu_rows[:-1])[row_seg]
+    logit_rows: List[int] = [r + int(w) for s, r in zip(segments, cu_rows.tolist()) for w in s.want]
     if len(set(seg_slot.tolist())) != n_seg:
         raise BatchError("two segments of one step name the same state slot")
 
     parts = [token_ids, positions, row_seg, cu_rows, seg_pos, seg_slot, np.asarray(logit_rows, dtype=np.int32)]
-    seg_len = [len(s.tokens) for s in segments]
     host_segs = StepSegments(n_rows, n_seg, cu_rows, seg_pos, seg_len, max(seg_len), all(n == 1 for n in seg_len))
     part_tables = []                                   # (key, [(name, index into parts)], scalars)
     for key, builder in (table_builders or {}).items():
@@ -212,20 +203,19 @@ def lay_out_step(segments: Sequence[Segment], groups: Dict[Hashable, int], vocab
         if round_blocks is not None:
             max_blocks = int(round_blocks(max_blocks))
         bt = np.full((n_seg, max_blocks), -1, np.int32)
-        sm = np.empty(n_rows, np.int32)
-        r = 0
-        for i, s in enumerate(segments):
+        slots: List[int] = []
+        per_entry = (every or {}).get(gk, 1)
+        for i, (s, n) in enumerate(zip(segments, seg_len)):
             t = s.block_tables.get(gk)
             ts = s.token_slots.get(gk)
-            n = len(s.tokens)
             if t is None or ts is None or len(ts) != n:
                 raise BatchError(f"request {s.req!r}: no block table / token slots for page group {gk!r}")
-            need = -(-((s.pos_start + n) // (every or {}).get(gk, 1)) // page_size)
+            need = -(-((s.pos_start + n) // per_entry) // page_size)
             if len(t) < need:
                 raise BatchError(f"request {s.req!r}: block table covers {len(t)} blocks, {need} needed")
             bt[i, :len(t)] = t
-            sm[r:r + n] = ts
-            r += n
+            slots += ts
+        sm = np.asarray(slots, dtype=np.int32)
         paged_host[gk] = (len(parts), bt.shape, page_size)
         parts.append(bt.reshape(-1))
         parts.append(sm)

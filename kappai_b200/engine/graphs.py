@@ -132,15 +132,17 @@ class _DecodeGraph:
         a[o["seg_slot"]:o["seg_slot"] + n] = [rc.slot for rc in rcs]
         for gk, ps in runner.group_page_size.items():
             pool = cache.pools[gk]
-            bt, sm, keys = self.host_bt[gk], self.host_sm[gk], self.row_key[gk]
-            for j, r in enumerate(reqs):
+            bt, keys = self.host_bt[gk], self.row_key[gk]
+            slots = []
+            for j, (r, n_before) in enumerate(zip(reqs, lens)):
                 t = pool.table(r)
                 key = (r, pool.version(r))
                 if keys[j] != key:
                     bt[j, :len(t)] = t
                     bt[j, len(t):] = 0
                     keys[j] = key
-                sm[j] = t[lens[j] // ps] * ps + lens[j] % ps if pool.every == 1 else pool.slot(r, lens[j])
+                slots.append(t[n_before // ps] * ps + n_before % ps if pool.every == 1 else pool.slot(r, n_before))
+            self.host_sm[gk][:] = slots
         if self.part_layout:
             self._fill_part_tables(lens)
         np.copyto(self.pinned_np[i], a)
@@ -207,17 +209,20 @@ class DecodeGraphs:
 
     @staticmethod
     def eligible(entries) -> bool:
-        return all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries)
+        for e in entries:
+            if len(e.tokens) != 1 or list(e.want) != [0]:
+                return False
+        return True
 
     def wants(self, entries) -> bool:
         """Should this decode step run from a captured graph (one that exists, or one that is due)?"""
         r = self.runner
-        blocks = 1
+        longest, requests = 0, r.cache.requests
         for e in entries:
-            rc = r.cache.requests.get(e.req)
-            need = (rc.length if rc is not None else 0) + 1
-            for ps in r.group_page_size.values():
-                blocks = max(blocks, -(-need // ps))
+            rc = requests.get(e.req)
+            if rc is not None and rc.length > longest:
+                longest = rc.length
+        blocks = max((-(-(longest + 1) // ps) for ps in r.group_page_size.values()), default=1)
         key = (len(entries), self.width_for(blocks))
         g = self.graphs.get(key)
         if g is not None and g.graph is not None:
@@ -237,8 +242,7 @@ class DecodeGraphs:
         r = self.runner
         reqs = [e.req for e in entries]
         n = len(reqs)
-        blocks = max(len(r.cache.block_table(q, gk)) for q in reqs for gk in r.group_page_size) \
-            if r.group_page_size else 1
+        blocks = max((max(map(len, map(r.cache.pools[gk].table, reqs))) for gk in r.group_page_size), default=1)
         key = (n, self.width_for(blocks))
         g = self.graphs.get(key)
         if g is None:

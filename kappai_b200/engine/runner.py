@@ -161,20 +161,22 @@ class ModelRunner:
             raise EngineError(f"a step of {n_rows} tokens exceeds the kernels' limit of {MAX_STEP_ROWS} rows a step")
         admitted = []
         try:
-            plan = []
+            plan, live, cache = [], self.cache.requests, self.cache
             for e in entries:
-                if len(e.tokens) < 1:
-                    raise EngineError(f"request {e.req!r}: no tokens in this step")
-                if e.req not in self.cache.requests:
-                    self.cache.admit(e.req)
-                    admitted.append(e.req)
-                rc = self.cache.requests[e.req]
-                new_len = rc.length + len(e.tokens)
+                req, n = e.req, len(e.tokens)
+                if n < 1:
+                    raise EngineError(f"request {req!r}: no tokens in this step")
+                rc = live.get(req)
+                if rc is None:
+                    rc = cache.admit(req)
+                    admitted.append(req)
+                new_len = rc.length + n
                 if new_len > self.max_model_len:
-                    raise EngineError(f"request {e.req!r}: {new_len} tokens exceed the limit of "
+                    raise EngineError(f"request {req!r}: {new_len} tokens exceed the limit of "
                                       f"{self.max_model_len} positions")
-                self.cache.extend(e.req, new_len)
-                plan.append((e.req, rc.length, new_len))
+                if not cache.try_extend(req, new_len):
+                    raise OutOfPages(f"request {req!r}: no pages for {new_len} tokens")
+                plan.append((req, rc.length, new_len))
             if len({p[0] for p in plan}) != len(plan):
                 raise EngineError("a request appears twice in one step")
             return plan
