@@ -12,10 +12,13 @@
 // before them: those come from earlier rows of the same segment or, at the
 // segment's head, from the request's state slot (nothing if the segment
 // starts at position 0, which is why a reused slot needs no clearing).
-// State layout: state[slot][K-1][d] float32.  The forward kernel only reads
-// the state; the update kernel, launched after it, writes the new history, one
+// State layout: state[slot][K-1][d] float32.  The forward kernels only read
+// the state; the update kernel, launched after them, writes the new history, one
 // thread per (segment, channel) so that a shift by fewer than K-1 rows reads
-// every old value before it is overwritten.
+// every old value before it is overwritten.  The kernel for K <= 4 can write it
+// itself: the thread that computes a segment's first K-1 rows, the only ones
+// that read the old history, writes the new one behind them (a launch less a
+// layer: 6.4 us of a prompt step with one request).
 #include "common.cuh"
 
 #define KP_CONV_MAX_K 16
@@ -200,20 +203,29 @@ shortconv_fwd_vec_kernel(const T* __restrict__ p, int ldp, const float* __restri
 // rows, keeping the last KK-1 products B*X and the channel weights in registers, so every input is read once
 // (the kernel above reads each row KK times).  The history of a chunk's first rows comes from the rows before
 // it or, at the head of a segment, from the state; the order of summation is that of the kernels above.
+// UPDATE: a segment's first KK-1 rows all belong to the chunk that its first row lies in (the next chunk leaves them
+// out), so that one thread a channel reads a segment's old history; behind them it writes the new one.
 #define CONV_ROWS 8
-template <typename T, int KK>
+template <typename T, int KK, bool UPDATE>
 __global__ void __launch_bounds__(128)
 shortconv_fwd_rows_kernel(const T* __restrict__ p, int ldp, const float* __restrict__ w,
-                          const float* __restrict__ bias, const float* __restrict__ state,
+                          const float* __restrict__ bias, float* state,
                           const int* __restrict__ row_seg, const int* __restrict__ cu_rows,
                           const int* __restrict__ seg_pos, const int* __restrict__ seg_slot,
                           T* __restrict__ out, int ldo, int n, int d) {
     kp_pdl_begin();
     constexpr int V = ConvVec<T>::N;
     const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
-    const int row_lo = blockIdx.y * CONV_ROWS;
-    if (c0 >= d || row_lo >= n) return;
-    const int row_hi = min(n, row_lo + CONV_ROWS);
+    const int chunk_lo = blockIdx.y * CONV_ROWS;
+    if (c0 >= d || chunk_lo >= n) return;
+    int row_lo = chunk_lo, row_hi = min(n, chunk_lo + CONV_ROWS);
+    if (UPDATE) {
+        const int first = row_seg[row_lo], head0 = cu_rows[first];        // its head lies before: rows t < KK-1 are the chunk's before
+        if (head0 < row_lo) row_lo = min(max(row_lo, head0 + KK - 1), max(row_lo, cu_rows[first + 1]));
+        const int last = row_seg[row_hi - 1], head1 = cu_rows[last];
+        if (head1 >= chunk_lo) row_hi = max(row_hi, min(cu_rows[last + 1], head1 + KK - 1));
+        if (row_lo >= row_hi) return;
+    }
     float wk[KK][V], bs[V];
 #pragma unroll
     for (int i = 0; i < V; i++) {
@@ -281,6 +293,31 @@ shortconv_fwd_rows_kernel(const T* __restrict__ p, int ldp, const float* __restr
             for (int i = 0; i < V; i++) hist[k][i] = hist[k + 1][i];
 #pragma unroll
         for (int i = 0; i < V; i++) hist[KK - 2][i] = bx[i];
+        if (UPDATE && t < KK - 1) {
+            const int nr = cu_rows[seg + 1] - (row - t);
+            if (t == min(nr, KK - 1) - 1) {
+                // the segment's last row that reads the old history: `hist` is the new one, or (a longer segment) it
+                // comes from the segment's last rows
+                float* st = state + (size_t)seg_slot[seg] * (KK - 1) * d;
+#pragma unroll
+                for (int k = 0; k < KK - 1; k++) {
+                    float h[V];
+                    if (nr > KK - 1) {
+                        float hb[V], hx[V];
+                        const T* ph = p + (size_t)(row - t + nr - (KK - 1) + k) * ldp;
+                        load_vec<T>(ph + c0, hb);
+                        load_vec<T>(ph + 2 * (size_t)d + c0, hx);
+#pragma unroll
+                        for (int i = 0; i < V; i++) h[i] = __fmul_rn(hb[i], hx[i]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < V; i++) h[i] = hist[k][i];
+                    }
+#pragma unroll
+                    for (int i = 0; i < V; i++) st[(size_t)k * d + c0 + i] = h[i];
+                }
+            }
+        }
     }
 }
 
@@ -326,10 +363,15 @@ int kp_shortconv_decode(const void* p, int ldp, const float* w, const float* bia
     return kp_launch_status();
 }
 
-int kp_shortconv_forward(const void* p, int ldp, const float* w, const float* bias, const float* state,
+int kp_shortconv_update_state(const void* p, int ldp, float* state, const int* cu_rows, const int* seg_pos,
+                              const int* seg_slot, int n_seg, int d, int K, int dtype, void* stream);
+
+// update != 0: the new history of the n_seg segments is written as well
+int kp_shortconv_forward(const void* p, int ldp, const float* w, const float* bias, float* state,
                          const int* row_seg, const int* cu_rows, const int* seg_pos, const int* seg_slot,
-                         void* out, int ldo, int n, int d, int K, int dtype, void* stream) {
+                         void* out, int ldo, int n, int d, int K, int dtype, int update, int n_seg, void* stream) {
     if (n <= 0) return 0;
+    if (update && n_seg > 65535) return KP_ERR_UNSUPPORTED;
     if (K < 2 || K > KP_CONV_MAX_K) return KP_ERR_UNSUPPORTED;
     if (n > 65535 * 32) return KP_ERR_UNSUPPORTED;
     if (n > 65535) return KP_ERR_UNSUPPORTED;
@@ -342,8 +384,9 @@ int kp_shortconv_forward(const void* p, int ldp, const float* w, const float* bi
                 // which kernel runs depends on the layer's sizes and alignment only, never on the batch
                 dim3 rgrid((d / vec + 127) / 128, (n + CONV_ROWS - 1) / CONV_ROWS);
 #define CONV_ROWS_LAUNCH(KK)                                                                                       \
-    KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(shortconv_fwd_rows_kernel<T, KK>, dim3(rgrid), dim3(128), 0,         \
-        (cudaStream_t)stream, (const T*)p, ldp, w, bias, state, row_seg, cu_rows, seg_pos, seg_slot, (T*)out, ldo, n, d)))
+    KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(update ? shortconv_fwd_rows_kernel<T, KK, true> : shortconv_fwd_rows_kernel<T, KK, false>,  \
+        dim3(rgrid), dim3(128), 0, (cudaStream_t)stream, (const T*)p, ldp, w, bias, state, row_seg, cu_rows, seg_pos, seg_slot,            \
+        (T*)out, ldo, n, d)))
                 if (K == 2) { CONV_ROWS_LAUNCH(2); } else if (K == 3) { CONV_ROWS_LAUNCH(3); } else { CONV_ROWS_LAUNCH(4); }
 #undef CONV_ROWS_LAUNCH
                 return kp_launch_status();
@@ -351,13 +394,13 @@ int kp_shortconv_forward(const void* p, int ldp, const float* w, const float* bi
             dim3 vgrid((d / vec + 127) / 128, n);
             KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(shortconv_fwd_vec_kernel<T>, dim3(vgrid), dim3(128), 0, (cudaStream_t)stream,
                 (const T*)p, ldp, w, bias, state, row_seg, cu_rows, seg_pos, seg_slot, (T*)out, ldo, n, d, K)));
-            return kp_launch_status();
+            return update ? kp_shortconv_update_state(p, ldp, state, cu_rows, seg_pos, seg_slot, n_seg, d, K, dtype, stream) : kp_launch_status();
         }
     }
     dim3 grid((d + 127) / 128, n);
     KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(shortconv_fwd_kernel<T>, dim3(grid), dim3(128), 0, (cudaStream_t)stream, 
         (const T*)p, ldp, w, bias, state, row_seg, cu_rows, seg_pos, seg_slot, (T*)out, ldo, n, d, K)));
-    return kp_launch_status();
+    return update ? kp_shortconv_update_state(p, ldp, state, cu_rows, seg_pos, seg_slot, n_seg, d, K, dtype, stream) : kp_launch_status();
 }
 
 int kp_shortconv_update_state(const void* p, int ldp, float* state, const int* cu_rows, const int* seg_pos,

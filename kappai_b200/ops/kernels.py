@@ -642,7 +642,8 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
 
 def shortconv_forward(p: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], state: torch.Tensor,
                       row_seg: torch.Tensor, cu_rows: torch.Tensor, seg_pos: torch.Tensor,
-                      seg_slot: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+                      seg_slot: torch.Tensor, out: torch.Tensor, update: bool = False) -> torch.Tensor:
+    """``update``: write the segments' new history into ``state`` as well (what :func:`shortconv_update_state` does)."""
     _need(p, "p", contiguous=False); _need(w, "w", torch.float32); _need(state, "state", torch.float32)
     _need(out, "out", p.dtype, contiguous=False)
     for t, nm in ((row_seg, "row_seg"), (cu_rows, "cu_rows"), (seg_pos, "seg_pos"), (seg_slot, "seg_slot")):
@@ -656,7 +657,7 @@ def shortconv_forward(p: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Ten
     lib = load_library("shortconv")
     _run("shortconv_forward", lib.kp_shortconv_forward, _ptr(p), _rows_2d(p, "p"), _ptr(w), _ptr(bias), _ptr(state), _ptr(row_seg),
                                     _ptr(cu_rows), _ptr(seg_pos), _ptr(seg_slot), _ptr(out), _rows_2d(out, "out"),
-                                    n, d, K, dtype_code(p.dtype), STREAM)
+                                    n, d, K, dtype_code(p.dtype), int(update), seg_pos.numel(), STREAM)
     return out
 
 

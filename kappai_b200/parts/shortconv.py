@@ -80,9 +80,7 @@ class ShortConv(Part):
             K.shortconv_decode(p, self.w_conv, self.b_conv, cache.tensor, ctx.seg_pos, ctx.seg_slot, y)
         else:
             K.shortconv_forward(p, self.w_conv, self.b_conv, cache.tensor, ctx.row_seg, ctx.cu_rows, ctx.seg_pos,
-                                ctx.seg_slot, y)
-            if cache.writes:
-                K.shortconv_update_state(p, cache.tensor, ctx.cu_rows, ctx.seg_pos, ctx.seg_slot, ctx.n_seg)
+                                ctx.seg_slot, y, update=cache.writes)
         linear(y, self.w_out, self.b_out, out=residual, accumulate=True)
 
 
