@@ -379,8 +379,10 @@ static int f32_rows(const F32Args& p, cudaStream_t s) {
     const int warps = n_jobs < most ? n_jobs : (n_jobs + (n_jobs + most - 1) / most - 1) / ((n_jobs + most - 1) / most);
     const size_t red = (size_t)n_jobs * 4 * MB * 8 * R * 4;
     const dim3 grid((p.N + 8 * R - 1) / (8 * R), (p.M + MB - 1) / MB);
-    // one CTA an SM: all the ring that pays (a job has 8 stages); more: a third of the SM's memory each
-    const size_t room = (int)(grid.x * grid.y) <= f32_n_sm() ? 200 * 1024 : 74 * 1024;
+    // one CTA an SM: all the ring that pays (a job has 8 stages); more: a third of the SM's memory each, or a sixth where a
+    // CTA is a single warp (8 rows by 9216 x 1024: 19.5 us with a third, 11.5 with a sixth; 65536 x 1024 95 and 52; one row by
+    // 6144 x 2048, two warps: 8.9 and 11.1)
+    const size_t room = (int)(grid.x * grid.y) <= f32_n_sm() ? 200 * 1024 : (warps == 1 ? 36 : 74) * 1024;
     int stages = red < room ? (int)((room - red) / ((size_t)warps * stage)) : 0;
     if (stages > 8) stages = 8;
     if (stages < 2) stages = 2;
