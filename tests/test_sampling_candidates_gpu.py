@@ -1,0 +1,49 @@
+"""Candidates of the sampler: the short way to the k largest (csrc/sampling.cu) against the definition, where it can go wrong --
+ties at the k-th value, k near the threads' number, zeros of both signs, infinities, short rows."""
+import numpy as np
+import pytest
+import torch
+
+import plain_sampler as PS
+
+pytestmark = pytest.mark.gpu
+
+
+def rows(kind, n, V, rng):
+    x = rng.standard_normal((n, V)).astype(np.float32)
+    if kind == "ties":
+        x = np.round(x * 2) / 2
+    elif kind == "equal":
+        x[:] = 1.25
+    elif kind == "zeros":
+        x = np.where(rng.random((n, V)) < 0.5, np.float32(-0.0), np.float32(0.0))
+    elif kind == "masked":
+        x[:, V // 3:] = np.finfo(np.float32).min
+        x[:, : V // 8] = -np.inf
+    elif kind == "few":
+        x[:] = -np.inf
+        x[:, [0, V // 2, V - 1]] = [1.0, 3.0, 2.0]
+    return x
+
+
+@pytest.mark.parametrize("kind", ["plain", "ties", "equal", "zeros", "masked", "few"])
+@pytest.mark.parametrize("V", [7, 331, 1024, 1025, 65536])
+def test_top_k_candidates(kind, V):
+    from kappai_b200 import SamplingParams
+    from kappai_b200.sampling import uniform
+    from kappai_b200.sampling.sampler import sample
+    n = 6
+    x = rows(kind, n, V, np.random.default_rng(V))
+    filters = [dict(top_p=1.0, min_p=0.0), dict(top_p=0.9, min_p=0.1), dict(top_p=0.5, min_p=0.0)] * 2
+    for k in (2, 3, 40, 200, 1000, 1024):
+        if k >= V:
+            continue
+        got = sample(torch.from_numpy(x).cuda(), [SamplingParams(temperature=0.7, top_k=k, **f) for f in filters],
+                     [i + 1 for i in range(n)], [3] * n).cpu().tolist()
+        for i, f in enumerate(filters):
+            if kind == "zeros":
+                # the selection's order puts 0 before -0, the plain sampler's takes them as equal
+                assert (np.signbit(x[i]) == 0).sum() < k or not np.signbit(x[i, got[i]])
+                continue
+            want, slack = PS.sample(x[i], uniform(i + 1, 3), temperature=0.7, top_k=k, **f)
+            assert got[i] == want or slack < 1e-5, (kind, V, k, f, got[i], want, slack)
