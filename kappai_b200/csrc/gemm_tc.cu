@@ -3,16 +3,16 @@
 // The product of prompt portions, and of few-row steps where it was measured faster than weight streaming.
 //
 // Persistent CTAs, one an SM; a CTA computes tiles of 128 x BN of C (tile b, b + grid, ...; m runs fastest so
-// that the CTAs that run together share W tiles in L2).  BN is 256 or 128 for products of many rows (chosen by
-// a cost model of rounds over the SMs), and for at most 128 rows the narrowest of 256..32 that still runs in
-// one round, so that as many CTAs as possible pull on the memory.  Roles by warp:
+// that the CTAs that run together share W tiles in L2).  BN is 256 to 32, chosen by a small cost model (tc_run).
+// Roles by warp:
 //   warp 0   : TMA producer.  For every k-block of 64 it waits for a free stage, arms the stage's "full"
 //              mbarrier with the byte count and issues the tiled loads of the A box (128 rows x 64, or only
 //              the rows there are, rounded up to 8, when M < 128) and the W box (BN rows x 64), both with
 //              the 128-byte swizzle, no multicast.  The ring has as many stages as fit shared memory.
 //   warp 1   : allocates 2 x BN columns of tensor memory (two accumulators: the epilogue of a tile runs under
-//              the main loop of the next), then one lane issues the MMAs: four tcgen05.mma (128 x BN x 16) per
-//              stage, descriptors advanced by 32 bytes inside the swizzled rows; tcgen05.commit frees the
+//              the main loop of the next), then an elected lane of the warp issues the MMAs: four tcgen05.mma (128 x BN x 16)
+//              per stage, descriptors advanced by 32 bytes inside the swizzled rows (from inside a branch that one lane
+//              took, a k-block cost about 0.3 us whatever its width: 128 rows by 2048 x 5632, 17.0 us against 12.4); tcgen05.commit frees the
 //              stage ("empty" mbarrier) and, after the last k-block, signals "accumulator full".
 //   the rest : epilogue, two warps for each quarter of the 128 lanes of tensor memory (a warp may only read
 //              the lanes 32 * (warp % 4) ...), taking the 32-column pieces in turn so that more loads and
@@ -220,82 +220,80 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const uint32_t tmem_base = *tmem_slot;
     bool parts_ok = false;                                                // (epilogue warps) this CTA's sums are in shared memory
 
+    // (the producer's and the MMA warp's lanes stay in step; one elected lane issues what they issue)
     if (warp == 0) {
-        if (lane == 0) {
-            auto load_w = [&](int s, int kb, int n0) {
-                unsigned char* b_dst = tiles + (size_t)s * (A_BYTES + B_BYTES) + A_BYTES;
-                if TC_GATED(EPI) {
-                    kp_tma_load_2d(b_dst, &tmW, kb * TC_BK, n0, &full[s]);                       // gate rows
-                    kp_tma_load_2d(b_dst + B_BYTES / 2, &tmW, kb * TC_BK, p.ff + n0, &full[s]);  // up rows
-                } else {
-                    kp_tma_load_2d(b_dst, &tmW, kb * TC_BK, n0, &full[s]);
-                }
-            };
-            // The weights depend on no earlier kernel: the W tiles of the first unit's first k-blocks (as many as
-            // the ring has stages) are on their way before the wait on the kernel before; their A tiles follow it.
-            int pre = 0;
-            if ((int)blockIdx.x < n_units) {
-                const int tile = blockIdx.x / S, part = blockIdx.x - tile * S;
-                const int n0 = (tile / tiles_m) * N_OUT_TILE;
-                const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
-                pre = min(STAGES, kb_hi - kb_lo);
-                for (int i = 0; i < pre; i++) {
-                    kp_mbar_expect_tx(&full[i], A_BYTES + B_BYTES);
-                    load_w(i, kb_lo + i, n0);
-                }
+        auto load_w = [&](int s, int kb, int n0) {
+            unsigned char* b_dst = tiles + (size_t)s * (A_BYTES + B_BYTES) + A_BYTES;
+            if TC_GATED(EPI) {
+                kp_tma_load_2d_warp(b_dst, &tmW, kb * TC_BK, n0, &full[s]);                       // gate rows
+                kp_tma_load_2d_warp(b_dst + B_BYTES / 2, &tmW, kb * TC_BK, p.ff + n0, &full[s]);  // up rows
+            } else {
+                kp_tma_load_2d_warp(b_dst, &tmW, kb * TC_BK, n0, &full[s]);
             }
-            KP_TRACE_MARK_LANE(0);
-            pdl_wait();
-            KP_TRACE_MARK_LANE(1);
-            pdl_launch_dependents();
-            int s = 0;                                                    // stage, and the parity of its round
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
-                const int tile = unit / S, part = unit - tile * S;
-                const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-                const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
-                for (int kb = kb_lo; kb < kb_hi; kb++) {
-                    unsigned char* a_dst = tiles + (size_t)s * (A_BYTES + B_BYTES);
-                    if (pre > 0) {
-                        pre--;                                            // armed, W on its way: only A is missing
-                    } else {
-                        if (*abort_flag || !kp_mbar_wait_bounded(&empty[s], ph ^ 1)) { *abort_flag = 1; ok = false; break; }
-                        kp_mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
-                        load_w(s, kb, n0);
-                    }
-                    kp_tma_load_2d(a_dst, &tmA, kb * TC_BK, m0, &full[s]);
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+        };
+        // The weights depend on no earlier kernel: the W tiles of the first unit's first k-blocks (as many as
+        // the ring has stages) are on their way before the wait on the kernel before; their A tiles follow it.
+        int pre = 0;
+        if ((int)blockIdx.x < n_units) {
+            const int tile = blockIdx.x / S, part = blockIdx.x - tile * S;
+            const int n0 = (tile / tiles_m) * N_OUT_TILE;
+            const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
+            pre = min(STAGES, kb_hi - kb_lo);
+            for (int i = 0; i < pre; i++) {
+                kp_mbar_expect_tx_warp(&full[i], A_BYTES + B_BYTES);
+                load_w(i, kb_lo + i, n0);
+            }
+        }
+        if (lane == 0) KP_TRACE_MARK_LANE(0);
+        pdl_wait();
+        if (lane == 0) KP_TRACE_MARK_LANE(1);
+        pdl_launch_dependents();
+        int s = 0;                                                    // stage, and the parity of its round
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+            const int tile = unit / S, part = unit - tile * S;
+            const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
+            const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
+            for (int kb = kb_lo; kb < kb_hi; kb++) {
+                unsigned char* a_dst = tiles + (size_t)s * (A_BYTES + B_BYTES);
+                if (pre > 0) {
+                    pre--;                                            // armed, W on its way: only A is missing
+                } else {
+                    ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&empty[s], ph ^ 1));
+                    if (!ok) { *abort_flag = 1; break; }
+                    kp_mbar_expect_tx_warp(&full[s], A_BYTES + B_BYTES);
+                    load_w(s, kb, n0);
                 }
+                kp_tma_load_2d_warp(a_dst, &tmA, kb * TC_BK, m0, &full[s]);
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
         kp_pdl_begin();
-        if (lane == 0) {
-            constexpr uint32_t idesc = kp_umma_idesc(TC_BM, BN);
-            int s = 0, ti = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ti++) {
-                const int b2 = ti & 1;                                    // accumulator of this unit
-                if (*abort_flag || !kp_mbar_wait_bounded(&acc_empty[b2], ((ti >> 1) & 1) ^ 1)) { *abort_flag = 1; break; }
+        constexpr uint32_t idesc = kp_umma_idesc(TC_BM, BN);
+        int s = 0, ti = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ti++) {
+            const int b2 = ti & 1;                                        // accumulator of this unit
+            ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], ((ti >> 1) & 1) ^ 1));
+            if (!ok) { *abort_flag = 1; break; }
+            kp_tc_fence_after();
+            const uint32_t tmem_d = tmem_base + (uint32_t)(b2 * BN);
+            const int part = unit % S;
+            const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
+            for (int kb = kb_lo; kb < kb_hi; kb++) {
+                ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
+                if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)(b2 * BN);
-                const int part = unit % S;
-                const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
-                for (int kb = kb_lo; kb < kb_hi; kb++) {
-                    if (!kp_mbar_wait_bounded(&full[s], ph)) { *abort_flag = 1; ok = false; break; }
-                    kp_tc_fence_after();
-                    const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * (A_BYTES + B_BYTES));
-                    const uint64_t adesc = kp_umma_desc(a_addr), bdesc = kp_umma_desc(a_addr + A_BYTES);
-#pragma unroll
-                    for (int k = 0; k < TC_BK / 16; k++)      // 32 bytes along K inside the swizzled row: +2 in the address field
-                        kp_umma_bf16(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, ((kb - kb_lo) | k) ? 1u : 0u);
-                    kp_umma_commit(&empty[s]);                    // the stage is free when these MMAs have read it
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
-                }
-                if (ok) kp_umma_commit(&acc_full[b2]);            // arrives when every MMA of the tile has completed
+                const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * (A_BYTES + B_BYTES));
+                // four MMAs of 16 columns (32 bytes along K inside the swizzled row: +2 in the address field)
+                kp_umma_bf16_box(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, kb != kb_lo);
+                kp_umma_commit_warp(&empty[s]);                           // the stage is free when these MMAs have read it
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
+            if (ok) kp_umma_commit_warp(&acc_full[b2]);                   // arrives when every MMA of the tile has completed
         }
     } else {
         kp_pdl_begin();
@@ -480,41 +478,40 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            auto load_w = [&](int s, int kb, int n0) {
-                // this CTA's half of the W tile: gate rows or up rows, or the first or second BN / 2 rows
-                const int row = TC_GATED(EPI) ? rank * p.ff + n0 : n0 + rank * (BN / 2);
-                kp_tma_load_2d_pair(tiles + (size_t)s * STAGE + A_BYTES, &tmW, kb * TC_BK, row, kp_cluster_addr(&full[s], 0));
-            };
-            int pre = 0;
-            if (pair < n_tiles) {
-                const int n0 = (pair / tiles_m) * N_OUT_TILE;
-                pre = min(STAGES, n_kb);
-                for (int i = 0; i < pre; i++) {
-                    if (rank == 0) kp_mbar_expect_tx(&full[i], 2 * STAGE);
-                    load_w(i, i, n0);
-                }
+        auto load_w = [&](int s, int kb, int n0) {
+            // this CTA's half of the W tile: gate rows or up rows, or the first or second BN / 2 rows
+            const int row = TC_GATED(EPI) ? rank * p.ff + n0 : n0 + rank * (BN / 2);
+            kp_tma_load_2d_pair(tiles + (size_t)s * STAGE + A_BYTES, &tmW, kb * TC_BK, row, kp_cluster_addr(&full[s], 0));
+        };
+        int pre = 0;
+        if (pair < n_tiles) {
+            const int n0 = (pair / tiles_m) * N_OUT_TILE;
+            pre = min(STAGES, n_kb);
+            for (int i = 0; i < pre; i++) {
+                if (rank == 0) kp_mbar_expect_tx_warp(&full[i], 2 * STAGE);
+                load_w(i, i, n0);
             }
-            KP_TRACE_MARK_LANE(0);
-            pdl_wait();
-            KP_TRACE_MARK_LANE(1);
-            pdl_launch_dependents();
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-                for (int kb = 0; kb < n_kb; kb++) {
-                    if (pre > 0) {
-                        pre--;
-                    } else {
-                        if (*abort_flag || !kp_mbar_wait_bounded(&empty[s], ph ^ 1)) { *abort_flag = 1; ok = false; break; }
-                        if (rank == 0) kp_mbar_expect_tx(&full[s], 2 * STAGE);
-                        load_w(s, kb, n0);
-                    }
-                    kp_tma_load_2d_pair(tiles + (size_t)s * STAGE, &tmA, kb * TC_BK, m0, kp_cluster_addr(&full[s], 0));
-                    if (++s == STAGES) { s = 0; ph ^= 1; }
+        }
+        if (lane == 0) KP_TRACE_MARK_LANE(0);
+        pdl_wait();
+        if (lane == 0) KP_TRACE_MARK_LANE(1);
+        pdl_launch_dependents();
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+            const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
+            for (int kb = 0; kb < n_kb; kb++) {
+                if (pre > 0) {
+                    pre--;
+                } else {
+                    ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&empty[s], ph ^ 1));
+                    if (!ok) { *abort_flag = 1; break; }
+                    if (rank == 0) kp_mbar_expect_tx_warp(&full[s], 2 * STAGE);
+                    load_w(s, kb, n0);
                 }
+                kp_tma_load_2d_pair(tiles + (size_t)s * STAGE, &tmA, kb * TC_BK, m0, kp_cluster_addr(&full[s], 0));
+                if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
@@ -634,12 +631,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
 // ------------------------------------------------------------------------------------------ host side
 #define TC_SMEM_KB 208                       // shared memory for the ring
-#ifndef TC_SPLIT_MAX_M_TILES
 #define TC_SPLIT_MAX_M_TILES 8               // rows of tiles up to which a product may be cut along K
-#endif
-#ifndef TC_SPLIT_COST_KB
-#define TC_SPLIT_COST_KB 64                  // what a split over K costs beside the operand reads, as KB brought into an SM
-#endif
+// the choice of a tile (tc_run), in bytes brought into an SM
+#define TC_KB_MIN (22 * 1024)                // a k-block at least
+#define TC_SPLIT_COST (220 * 1024)           // a split over K
+#define TC_PAIR_COST (100 * 1024)            // a pair of CTAs
 
 // SMs of the current device (asked once)
 static int tc_n_sm() {
@@ -808,84 +804,64 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
         a.ff = N / 2;
     }
     const int n_out = epi == EPI_SWIGLU ? a.ff : N;
-    // Tile width.  Many rows: by a small cost model: a CTA's main loop is bound by the bytes that it brings
-    // into shared memory for each k-block (128 rows of A and BN rows of W), so a narrow tile costs about 2/3
-    // of a wide one and does half the work; the number of rounds over the SMs decides between them.
-    // At most 128 rows (one row of tiles, W streamed once): see below.
     const long long m_tiles = (M + TC_BM - 1) / TC_BM;
     const int sms = tc_n_sm();
-    const int lowest = epi == EPI_SWIGLU ? 64 : 32;                      // the narrowest tile
-    auto tiles_at = [&](int w) { const int cols = epi == EPI_SWIGLU ? w / 2 : w; return (n_out + cols - 1) / cols; };
-    int bn;
-    if (m_tiles > 1) {
-        const long long rounds_wide = (((n_out + 255) / 256) * m_tiles + sms - 1) / sms;
-        const long long rounds_narrow = (((n_out + 127) / 128) * m_tiles + sms - 1) / sms;
-        bn = (epi == EPI_SWIGLU || rounds_wide * 3 <= rounds_narrow * 2) ? 256 : 128;
-    } else {
-        // the narrowest tile that still runs in one round over the SMs (as many CTAs as possible pull on the
-        // memory, none waits for a second round); products too wide for that take the widest tile
-        bn = 256;
-        while (bn > lowest && tiles_at(bn / 2) <= sms) bn /= 2;
-    }
-    // 17 to 128 rows (one row of tiles; for more see below): what bounds the product is the bytes that the busiest SM brings in, about
-    // 45 GB/s an SM whatever the source -- its share of W and, for every tile, all the rows of A.  Unsplit, a
-    // narrow tile reads A once for a few rows of W (64 rows by 2048 x 5632 in 32-row tiles: 720 KB of A for 360 KB
-    // of W) and wide tiles leave SMs idle.  So the product is cut along K as well: (tile width, parts) is chosen
-    // so that the units fill one round over the SMs and a unit brings in the fewest bytes; the price of the split
-    // (partial sums out and in, the wait for the other parts) is counted as TC_SPLIT_COST_KB of traffic.
-    a.splits = 1;
-    a.kb_per_split = (K + TC_BK - 1) / TC_BK;
+    const bool gated = epi == EPI_SWIGLU;
+    const int lowest = gated ? 64 : 32;                                  // the narrowest tile
+    auto tiles_at = [&](int w) { const int cols = gated ? w / 2 : w; return (n_out + cols - 1) / cols; };
+    // Tile width, parts along K, and one CTA or a pair of them a tile: the choice that keeps the busiest SM busy for the
+    // shortest time, counted in bytes brought into it (about 100 a nanosecond, from L2 or, all SMs together, HBM):
+    //   a k-block: its rows of A and W, but no less than TC_KB_MIN (waiting, issuing, handing on);
+    //   an epilogue: 0.6 KB a column of the tile, 1.2 KB gated, under the main loop of the next tile if there is one;
+    //   a split (17 to 1024 rows; all units in one round, the parts of a tile a cluster): TC_SPLIT_COST for the clusters'
+    //   barriers, four times the sums that are exchanged, and more for clusters of other than 2 or 4 CTAs; beyond 512 rows
+    //   a quarter more, as the sums of many tiles meet;
+    //   a pair: TC_PAIR_COST for its barriers.
+    // It was fitted to all widths and parts at 24 to 512 rows of nine layer products; measured, us, the chosen | the best:
+    // 64 rows by 2048 x 5632 11.0 | 11.0, by 6144 x 2048 11.1 | 10.2, by gated 11264 x 2048 15.0 | 15.0, 101 rows 15.6 | 15.6,
+    // 24 rows 12.8 | 12.8, 128 rows by 2048 x 5632 12.4 | 12.4, 200 rows by 1024 x 4608 10.9 | 10.9.
+    const int n_kb = (K + TC_BK - 1) / TC_BK;
+    const auto kb_cost = [](long long rows) { const long long bytes = rows * TC_BK * 2; return bytes > TC_KB_MIN ? bytes : (long long)TC_KB_MIN; };
+    const auto epi_cost = [&](int w) { return (long long)w * (gated ? 1228 : 614); };
+    const auto run_cost = [&](long long rounds, long long main, int w) {
+        return rounds * (main > epi_cost(w) ? main : epi_cost(w)) + epi_cost(w);
+    };
     a.a_rows = M >= TC_BM ? TC_BM : (M + 7) / 8 * 8;
-    // what the choice so far brings into the busiest SM, and below what others would
-    const int n_kb_all = (K + TC_BK - 1) / TC_BK;
-    long long cost_now = ((long long)tiles_at(bn) * m_tiles + sms - 1) / sms * n_kb_all * (TC_BK * 2) * (bn + a.a_rows);
-    if (m_tiles <= TC_SPLIT_MAX_M_TILES && M > 16 && split) {
-        // (the same holds for a few rows of tiles -- a prompt portion or decoded tokens beside one, 129 to 1024
-        // rows -- where the product has few tiles and a long K: 264 rows by 2048 x 5632 are 48 tiles of 88 k-blocks)
+    int bn = 256, pair_bn = 0;
+    a.splits = 1;
+    long long best = -1;
+    for (int w = 256; w >= lowest; w /= 2) {
+        const long long tiles = (long long)tiles_at(w) * m_tiles;
+        const long long cost = run_cost((tiles + sms - 1) / sms, n_kb * kb_cost(w + a.a_rows), w);
+        if (best < 0 || cost < best) { best = cost; bn = w; }
+    }
+    if (split && M > 16 && m_tiles <= TC_SPLIT_MAX_M_TILES) {
         const int rows = M < TC_BM ? M : TC_BM;                          // rows of a tile
-        const int n_kb = (K + TC_BK - 1) / TC_BK;
-        long long best = -1;
-        int best_bn = bn, best_sp = 1;
-        for (int w = 256; w >= (lowest < 64 ? 64 : lowest); w /= 2) {
-            const int tiles = tiles_at(w) * (int)m_tiles;
-            const long long rounds = (tiles + sms - 1) / sms;
+        for (int w = 256; w >= 64; w /= 2) {
+            const long long tiles = (long long)tiles_at(w) * m_tiles;
             int stages = 0;
             const size_t ring = tc_smem(a.a_rows, w, &stages) - 2048;
-            for (int sp = 1; sp <= 8; sp++) {
-                if (sp > 1) {
-                    if (tiles * sp > sms || sp * 2 > n_kb || (size_t)rows * w * 4 > ring) break;
-                    if (tiles > tc_max_clusters(w, epi, sp, a.a_rows)) continue;  // the clusters would not all run at once
-                }
+            for (int sp = 2; sp <= 8; sp++) {
+                if (tiles * sp > sms || sp * 2 > n_kb || (size_t)rows * w * 4 > ring) break;
+                if (tiles > tc_max_clusters(w, epi, sp, a.a_rows)) continue;      // the clusters would not all run at once
                 const int kbs = (n_kb + sp - 1) / sp;
-                if (sp > 1 && (n_kb + kbs - 1) / kbs != sp) continue;            // a part would be empty
-                long long cost = (sp == 1 ? rounds * n_kb : kbs) * (long long)(TC_BK * 2) * (w + a.a_rows);
-                if (sp > 1) {
-                    // the sums that a CTA reads from the others come in over the same port
-                    cost += TC_SPLIT_COST_KB * 1024 + (long long)rows * w * 4 * (sp - 1) / sp;
-                }
-                if (best < 0 || cost < best) { best = cost; best_bn = w; best_sp = sp; }
+                if ((n_kb + kbs - 1) / kbs != sp) continue;                       // a part would be empty
+                long long cost = kbs * kb_cost(w + a.a_rows) + epi_cost(w) / sp + TC_SPLIT_COST + 4LL * rows * w * 4 * (sp - 1) / sp;
+                if (sp != 2 && sp != 4) cost += sp == 3 ? 32 * 1024 : 100 * 1024;
+                if (m_tiles > 4) cost += cost / 4;
+                if (cost < best) { best = cost; bn = w; a.splits = sp; }
             }
         }
-        if (best >= 0 && (best_sp > 1 || m_tiles > 1)) cost_now = best;
-        if (best_sp > 1) {
-            bn = best_bn;
-            a.splits = best_sp;
-            a.kb_per_split = (n_kb + best_sp - 1) / best_sp;
-        }
     }
-    // Pairs of CTAs for more than one row of tiles, where they bring in less.  A split's exchange of sums costs more than
-    // its bytes: 1.5 times its cost and 90 KB separate the two (measured, us, split | pairs: 200 rows by 1024 x 1024
-    // 8.6 | 9.7, 300 rows by 2048 x 2048 18.7 | 14.2, 512 rows by 2048 x 5632 22.7 | 29.1, 768 rows 34.3 | 29.9, 200 rows
-    // by 3072 x 2048 14.4 | 11.1).
-    int pair_bn = 0;
     if (m_tiles > 1) {
-        if (a.splits > 1) cost_now += cost_now / 2 + 90 * 1024;
         for (int w = 256; w >= 128; w /= 2) {
             const long long tiles = (long long)tiles_at(w) * ((M + 2 * TC_BM - 1) / (2 * TC_BM));
-            const long long cost = (tiles + sms / 2 - 1) / (sms / 2) * n_kb_all * (TC_BK * 2) * (w / 2 + TC_BM);
-            if (cost <= cost_now) { cost_now = cost; pair_bn = w; }
+            const long long cost = run_cost((tiles + sms / 2 - 1) / (sms / 2), n_kb * kb_cost(w / 2 + TC_BM), w) + TC_PAIR_COST;
+            if (cost < best) { best = cost; pair_bn = w; }
         }
     }
+    if (pair_bn) a.splits = 1;
+    a.kb_per_split = (n_kb + a.splits - 1) / a.splits;
     cudaStream_t s = (cudaStream_t)stream;
     alignas(64) CUtensorMap ta, tw;
     int st = kp_make_map_bf16_2d(&ta, A, (unsigned long long)M, K, lda, TC_BK, a.a_rows);

@@ -133,9 +133,10 @@ __device__ __forceinline__ uint32_t kp_cluster_addr(const void* p, int rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(kp_smem_u32(p)), "r"(rank));
     return ra;
 }
-// a box of the 2-D tensor to this CTA's shared memory, its bytes counted at a barrier of either CTA of the pair
+// a box of the 2-D tensor to this CTA's shared memory, its bytes counted at a barrier of either CTA of the pair (elected lane)
 __device__ __forceinline__ void kp_tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}"
                  ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ void kp_mbar_arrive_cluster(uint32_t cluster_bar) {

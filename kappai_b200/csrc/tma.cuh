@@ -74,6 +74,18 @@ __device__ __forceinline__ void kp_tma_load_2d(void* dst, const CUtensorMap* map
                  ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(kp_smem_u32(bar)) : "memory");
 }
 
+// The same for a whole warp in step, whose operands are the same in every lane: one elected lane asks for the box
+// (from inside a branch that one lane took, the operands pass through general registers).
+__device__ __forceinline__ void kp_tma_load_2d_warp(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}"
+                 ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(kp_smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void kp_mbar_expect_tx_warp(uint64_t* bar, uint32_t bytes) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(kp_smem_u32(bar)), "r"(bytes) : "memory");
+}
+
 // box of a 3-D tensor at (x, y, z)
 __device__ __forceinline__ void kp_tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
