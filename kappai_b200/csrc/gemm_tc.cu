@@ -36,6 +36,8 @@
 //
 // Every wait on an mbarrier is bounded.  A wait that gives up sets a status word (kp_tc_status), the CTA
 // stops issuing work, still frees its tensor memory and returns.
+#include <atomic>
+
 #include "tcgen05.cuh"
 
 #define EPI_STORE 0
@@ -727,11 +729,13 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaSt
 template <int BN, int EPI>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcArgs& a, cudaStream_t s) {
     auto kern = gemm_tc_pair_kernel<BN, EPI>;
-    static bool ready = false;
-    if (!ready) {
+    static std::atomic<unsigned long long> ready{0};           // devices (bits) that the attribute is set on
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev > 63 || !((ready.load(std::memory_order_relaxed) >> dev) & 1)) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_PAIR_SMEM(BN));
         if (e != cudaSuccess) return (int)e;
-        ready = true;
+        if (dev <= 63) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
     }
     const int n_out = TC_GATED(EPI) ? a.ff : a.N, n_tile = TC_GATED(EPI) ? BN / 2 : BN;
     const int n_tiles = ((n_out + n_tile - 1) / n_tile) * ((a.M + 2 * TC_BM - 1) / (2 * TC_BM));
