@@ -9,8 +9,8 @@
 //              mbarrier with the byte count and issues the tiled loads of the A box (128 rows x 64, or only
 //              the rows there are, rounded up to 8, when M < 128) and the W box (BN rows x 64), both with
 //              the 128-byte swizzle, no multicast.  The ring has as many stages as fit shared memory.
-//   warp 1   : allocates 2 x BN columns of tensor memory (two accumulators: the epilogue of a tile runs under
-//              the main loop of the next), then an elected lane of the warp issues the MMAs: four tcgen05.mma (128 x BN x 16)
+//   warp 1   : allocates tensor memory (accumulators for two tiles, if there is room: the epilogue of a tile runs
+//              under the main loop of the next), then an elected lane of the warp issues the MMAs: four tcgen05.mma (128 x BN x 16)
 //              per stage, descriptors advanced by 32 bytes inside the swizzled rows (from inside a branch that one lane
 //              took, a k-block cost about 0.3 us whatever its width: 128 rows by 2048 x 5632, 17.0 us against 12.4); tcgen05.commit frees the
 //              stage ("empty" mbarrier) and, after the last k-block, signals "accumulator full".
@@ -20,16 +20,17 @@
 //              bias / residual accumulation / SwiGLU, writes its rows of C and hands the accumulator back.
 // Rows of A beyond M and rows of W beyond N are zero-filled by TMA (out-of-bounds fill) and masked at the
 // store; K needs no padding (the tail of the last k-block is zero-filled too) but K % 8 == 0 (16-byte rows).
-// Each output row sums its k-blocks in order, so a row's result does not depend on M.
+// Each output sums its k-blocks in order, within its part of K where the product is cut along K (tc_parts).
 //
 // SwiGLU epilogue: W holds gate rows then up rows (ff apart).  The CTA's W tile is BN/2 gate rows and the
 // matching BN/2 up rows (two TMA boxes into one tile), so accumulator columns c and BN/2 + c are the gate and
 // up of one output column: the epilogue writes silu(gate) * up.
 //
-// Split over K (17 to 1024 rows: up to eight rows of tiles, where that brings fewer bytes into the busiest SM): the
-// product is cut along K into `splits` parts, the unit of
-// work being (tile, part), all units in one round over the SMs and the parts of a tile one thread-block cluster.
-// Every CTA leaves the float32 sums of its unit in its own shared memory (the ring is free by then); after the
+// Split over K (17 to 1024 rows: up to eight rows of tiles; tc_parts): the product is cut along K into parts, whose sums
+// are added in the order of the parts.  A CTA runs the parts of its tile one after the other, each into an accumulator of
+// its own, and the epilogue adds them up (one commit a tile: a commit a part cost 0.25 us a part, the reading 0.05); or the
+// unit of work is (tile, part), all units in one round over the SMs and the parts of a tile one thread-block cluster.
+// Then every CTA leaves the float32 sums of its unit in its own shared memory (the ring is free by then); after the
 // cluster's barrier each adds up its share of the tile, reading the other CTAs' sums over the cluster's shared
 // memory, the parts in order of their number -- so the result does not depend on timing -- then the epilogue.
 // With it every SM brings in a part of A only, and wide tiles still keep all SMs streaming.
@@ -65,8 +66,11 @@ struct TcArgs {
     int vec_ok;                             // rows of C are 16-byte aligned: whole pieces go out in 16-byte stores
     int a_rows;                             // rows of the A box: 128, fewer (a multiple of 8) when M < 128
     int n_stages;                           // stages of the ring
-    int splits;                             // parts along K (1: none); only with one row of tiles; the cluster's size
-    int kb_per_split;                       // k-blocks a part
+    int splits;                             // CTAs that share a tile's parts along K, one each (1: no cluster)
+    int inner;                              // parts along K that a CTA (or a pair) runs itself, one after the other (1 beside splits > 1)
+    int kb_per_part;                        // k-blocks a part
+    int n_sets;                             // sets of `inner` accumulators of BN columns in tensor memory: two, or the one there is room for
+    int tmem_cols;                          // columns allocated
 };
 
 // all threads of all CTAs of the cluster; what they wrote to shared memory before is visible to the others after
@@ -175,6 +179,41 @@ __device__ __forceinline__ void tc_finish(const TcArgs& p, int n_lim, const floa
     }
 }
 
+// The 32 sums of a lane's row at a place of the unit's accumulators, g (and u: the up half, gated): one part's as they are,
+// several parts' added from zero in the order of the parts, as the split over a cluster adds them.
+// (PARTS false: there is one, which saves the pairs' gated epilogue the registers that the adding needs.)
+template <int EPI, int BN, bool PARTS>
+__device__ __forceinline__ void tc_sums(const TcArgs& p, uint32_t at, float (&g)[32], float (&up)[32]) {
+    uint32_t r[32];
+    {
+        uint32_t u[32];
+        kp_tmem_ld32_issue(at, r);
+        if TC_GATED(EPI) kp_tmem_ld32_issue(at + BN / 2, u);
+        kp_tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            g[j] = __uint_as_float(r[j]);
+            up[j] = TC_GATED(EPI) ? __uint_as_float(u[j]) : 0.f;
+        }
+    }
+    if (PARTS && p.inner > 1) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) { g[j] = 0.f + g[j]; if TC_GATED(EPI) up[j] = 0.f + up[j]; }
+#pragma unroll 1
+        for (int i = 1; i < p.inner; i++) {
+            at += BN;
+            kp_tmem_ld32(at, r);
+#pragma unroll
+            for (int j = 0; j < 32; j++) g[j] += __uint_as_float(r[j]);
+            if TC_GATED(EPI) {
+                kp_tmem_ld32(at + BN / 2, r);
+#pragma unroll
+                for (int j = 0; j < 32; j++) up[j] += __uint_as_float(r[j]);
+            }
+        }
+    }
+}
+
 template <int BN, int EPI>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const TcArgs p) {
@@ -190,8 +229,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * (A_BYTES + B_BYTES) + (TC_BM * TC_BK * 2 - A_BYTES));
     uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;                                  // [2]: accumulator b holds a finished tile
-    uint64_t* acc_empty = acc_full + 2;                                   // [2]: accumulator b has been read out
+    uint64_t* acc_full = empty + STAGES;                                  // [2]: set b holds a finished unit
+    uint64_t* acc_empty = acc_full + 2;                                   // [2]: set b has been read out
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -215,7 +254,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         *abort_flag = 0;
         kp_mbar_init_fence();
     }
-    if (warp == 1) kp_tmem_alloc(tmem_slot, 2 * BN);                         // two accumulators of BN columns
+    if (warp == 1) kp_tmem_alloc(tmem_slot, p.tmem_cols);
     kp_tc_fence_before();
     __syncthreads();
     kp_tc_fence_after();
@@ -239,7 +278,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if ((int)blockIdx.x < n_units) {
             const int tile = blockIdx.x / S, part = blockIdx.x - tile * S;
             const int n0 = (tile / tiles_m) * N_OUT_TILE;
-            const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
+            const int kb_lo = part * p.kb_per_part, kb_hi = S > 1 ? min(n_kb, kb_lo + p.kb_per_part) : n_kb;
             pre = min(STAGES, kb_hi - kb_lo);
             for (int i = 0; i < pre; i++) {
                 kp_mbar_expect_tx_warp(&full[i], A_BYTES + B_BYTES);
@@ -256,7 +295,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             const int tile = unit / S, part = unit - tile * S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-            const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
+            const int kb_lo = part * p.kb_per_part, kb_hi = S > 1 ? min(n_kb, kb_lo + p.kb_per_part) : n_kb;
             for (int kb = kb_lo; kb < kb_hi; kb++) {
                 unsigned char* a_dst = tiles + (size_t)s * (A_BYTES + B_BYTES);
                 if (pre > 0) {
@@ -274,28 +313,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     } else if (warp == 1) {
         kp_pdl_begin();
         constexpr uint32_t idesc = kp_umma_idesc(TC_BM, BN);
-        int s = 0, ti = 0;
-        uint32_t ph = 0;
+        int s = 0, b2 = 0;                                                // stage; set of accumulators of this unit
+        uint32_t ph = 0, set_ph = 1;                                      // (both sets are empty at first)
         bool ok = true;
-        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ti++) {
-            const int b2 = ti & 1;                                        // accumulator of this unit
-            ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], ((ti >> 1) & 1) ^ 1));
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+            ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph));
             if (!ok) { *abort_flag = 1; break; }
             kp_tc_fence_after();
-            const uint32_t tmem_d = tmem_base + (uint32_t)(b2 * BN);
+            uint32_t tmem_d = tmem_base + (uint32_t)(b2 * p.inner * BN);
             const int part = unit % S;
-            const int kb_lo = part * p.kb_per_split, kb_hi = min(n_kb, kb_lo + p.kb_per_split);
+            const int kb_lo = part * p.kb_per_part, kb_hi = S > 1 ? min(n_kb, kb_lo + p.kb_per_part) : n_kb;
+            int part_kb = 0;                                              // k-blocks in the accumulator so far
             for (int kb = kb_lo; kb < kb_hi; kb++) {
+                if (part_kb == p.kb_per_part) { part_kb = 0; tmem_d += BN; }
                 ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
                 if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
                 const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * (A_BYTES + B_BYTES));
                 // four MMAs of 16 columns (32 bytes along K inside the swizzled row: +2 in the address field)
-                kp_umma_bf16_box(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, kb != kb_lo);
+                kp_umma_bf16_box(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, part_kb++ != 0);
                 kp_umma_commit_warp(&empty[s]);                           // the stage is free when these MMAs have read it
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
-            if (ok) kp_umma_commit_warp(&acc_full[b2]);                   // arrives when every MMA of the tile has completed
+            if (ok) kp_umma_commit_warp(&acc_full[b2]);                   // arrives when every MMA of the unit has completed
+            if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
         }
     } else {
         kp_pdl_begin();
@@ -303,36 +344,29 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // MMA warp already fills the other accumulator with unit i + 1
         const int q = warp & 3;
         const int half = (warp - 2) >> 2;                                 // which of the quarter's warps
-        int ti = 0;
+        int b2 = 0;
+        uint32_t set_ph = 0;
         bool ok = true;
-        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ti++) {
-            const int b2 = ti & 1;
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             const int tile = unit / S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-            if (!kp_mbar_wait_bounded(&acc_full[b2], (ti >> 1) & 1) || *abort_flag) { ok = false; break; }
+            if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) { ok = false; break; }
             kp_tc_fence_after();
             const int m = m0 + q * 32 + lane;
-            const uint32_t lane_base = tmem_base + (uint32_t)(b2 * BN) + ((uint32_t)(q * 32) << 16);
+            const uint32_t lane_base = tmem_base + (uint32_t)(b2 * p.inner * BN) + ((uint32_t)(q * 32) << 16);
+            uint64_t* const read_out = &acc_empty[b2];
+            if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
             if (S == 1) {
 #pragma unroll 1
                 for (int c = half * 32; c < N_OUT_TILE; c += 32 * TC_EPI_PER_Q) {
-                    uint32_t r[32], u[32];
-                    kp_tmem_ld32(lane_base + c, r);
-                    if TC_GATED(EPI) kp_tmem_ld32(lane_base + BN / 2 + c, u);
-                    if (m < p.M) {
-                        float g[32], up[32];
-#pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            g[j] = __uint_as_float(r[j]);
-                            up[j] = TC_GATED(EPI) ? __uint_as_float(u[j]) : 0.f;
-                        }
-                        tc_finish<EPI, 32>(p, n_out, g, up, m, n0 + c);
-                    }
+                    float g[32], up[32];
+                    tc_sums<EPI, BN, true>(p, lane_base + c, g, up);
+                    if (m < p.M) tc_finish<EPI, 32>(p, n_out, g, up, m, n0 + c);
                 }
-                // this warp has read the accumulator out: hand it back to the MMA warp
+                // this warp has read the accumulators out: hand them back to the MMA warp
                 kp_tc_fence_before();
                 __syncwarp();
-                if (lane == 0) kp_mbar_arrive(&acc_empty[b2]);
+                if (lane == 0) kp_mbar_arrive(read_out);
                 continue;
             }
             // split over K: this part's sums of the whole accumulator (BN columns) go to this CTA's shared memory
@@ -355,7 +389,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             kp_tc_fence_before();
             __syncwarp();
-            if (lane == 0) kp_mbar_arrive(&acc_empty[b2]);
+            if (lane == 0) kp_mbar_arrive(read_out);
             parts_ok = true;
         }
         if (!ok && lane == 0) atomicExch(&g_tc_status, 1);
@@ -422,7 +456,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         kp_cluster_sync();
     }
     if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
-    if (warp == 1) kp_tmem_dealloc(tmem_base, 2 * BN);
+    if (warp == 1) kp_tmem_dealloc(tmem_base, p.tmem_cols);
 }
 
 // ------------------------------------------------------------------------------------------ pairs of CTAs
@@ -431,7 +465,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // reads 48 KB a k-block, about 770 cycles' worth from L2 for 512 cycles of MMAs.  A pair reads A once a CTA and each half
 // of W once a pair: 32 KB an SM.  The roles are those of gemm_tc_kernel; the first CTA's MMA warp issues for both, both
 // CTAs' loads count at its "full" barriers, and its commits free the stages and hand over the accumulators in both.
-// The sums run in the same order as in gemm_tc_kernel (the same bits).  Measured, us, one CTA a tile | pairs: 2,048 rows by
+// The sums run in the same order as in gemm_tc_kernel, parts included (the same bits).  Measured, us, one CTA a tile | pairs: 2,048 rows by
 // 11264 x 2048 (gated) 77.0 | 67.0, 1.41 PFLOP/s; 2048 x 5632 44.8 | 37.2; 6144 x 2048 46.8 | 37.7; 2048 x 2048 25.3 | 19.3;
 // 512 rows by 65536 x 1024 92.8 | 65.1.
 //
@@ -441,7 +475,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #define TC_PAIR_STAGES(BN) ((BN) == 256 ? 5 : 7)
 #define TC_PAIR_SMEM(BN) ((size_t)TC_PAIR_STAGES(BN) * (128 + (BN) / 2) * TC_BK * 2 + TC_EPI_PER_Q * 4 * 4096 + (2 * TC_PAIR_STAGES(BN) + 4) * 8 + 16 + 1024)
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const TcArgs p) {
     constexpr int STAGES = TC_PAIR_STAGES(BN);
@@ -472,7 +506,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         *abort_flag = 0;
         kp_mbar_init_fence();
     }
-    if (warp == 1) kp_tmem_alloc_pair(tmem_slot, 2 * BN);
+    if (warp == 1) kp_tmem_alloc_pair(tmem_slot, p.tmem_cols);
     kp_tc_fence_before();
     __syncthreads();
     kp_cluster_sync();                                                    // both CTAs' barriers and tensor memory are there
@@ -520,26 +554,28 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         kp_pdl_begin();
         if (rank == 0) {                                                  // (the whole warp in step: one elected lane issues)
             constexpr uint32_t idesc = kp_umma_idesc(2 * TC_BM, BN);
-            int s = 0, ti = 0;
-            uint32_t ph = 0;
+            int s = 0, b2 = 0;
+            uint32_t ph = 0, set_ph = 1;
             bool ok = true;
-            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ti++) {
-                const int b2 = ti & 1;
-                ok = !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], ((ti >> 1) & 1) ^ 1);
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+                ok = !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
-                const uint32_t tmem_d = tmem_base + (uint32_t)(b2 * BN);
+                uint32_t tmem_d = tmem_base + (uint32_t)(b2 * p.inner * BN);
+                int part_kb = 0;
                 for (int kb = 0; kb < n_kb; kb++) {
+                    if (part_kb == p.kb_per_part) { part_kb = 0; tmem_d += BN; }
                     ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
                     if (!ok) { *abort_flag = 1; break; }
                     kp_tc_fence_after();
                     const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * STAGE);
-                    kp_umma_bf16_box_pair(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, kb != 0);
+                    kp_umma_bf16_box_pair(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, part_kb++ != 0);
                     kp_umma_commit_pair(&empty[s]);
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
                 if (ok) kp_umma_commit_pair(&acc_full[b2]);
+                if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
             }
         }
     } else {
@@ -548,14 +584,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         unsigned char* piece = pieces + (size_t)(warp - 2) * 4096;
         constexpr bool NARROW = EPI == EPI_STORE || EPI == EPI_ACT || TC_GATED(EPI);   // 16-bit outputs: a piece is 64 columns
         constexpr int PW = NARROW ? 64 : 32;
-        int ti = 0;
+        int b2 = 0;
+        uint32_t set_ph = 0;
         bool ok = true;
-        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ti++) {
-            const int b2 = ti & 1;
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM + q * 32, n0 = (tile / tiles_m) * N_OUT_TILE;
-            if (!kp_mbar_wait_bounded(&acc_full[b2], (ti >> 1) & 1) || *abort_flag) { ok = false; break; }
+            if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) { ok = false; break; }
             kp_tc_fence_after();
-            const uint32_t lane_base = tmem_base + (uint32_t)(b2 * BN) + ((uint32_t)(q * 32) << 16);
+            const uint32_t lane_base = tmem_base + (uint32_t)(b2 * p.inner * BN) + ((uint32_t)(q * 32) << 16);
             const int m = m0 + lane;
 #pragma unroll 1
             for (int c = half * PW; c < N_OUT_TILE && m0 < p.M; c += PW * TC_EPI_PER_Q) {
@@ -572,13 +608,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 }
 #pragma unroll
                 for (int h = 0; h < PW / 32; h++) {
-                    uint32_t r[32], u[32];
-                    kp_tmem_ld32(lane_base + c + h * 32, r);
-                    if TC_GATED(EPI) kp_tmem_ld32(lane_base + BN / 2 + c + h * 32, u);
                     const int n_base = n0 + c + h * 32;
                     float v[32], up[32];
-#pragma unroll
-                    for (int j = 0; j < 32; j++) { v[j] = __uint_as_float(r[j]); up[j] = TC_GATED(EPI) ? __uint_as_float(u[j]) : 0.f; }
+                    tc_sums<EPI, BN, PARTS>(p, lane_base + c + h * 32, v, up);
                     if (!staged) {
                         if (m < p.M) tc_finish<EPI, 32>(p, n_out, v, up, m, n_base);
                         continue;
@@ -620,6 +652,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             kp_tc_fence_before();
             __syncwarp();
             if (lane == 0) kp_mbar_arrive_cluster(kp_cluster_addr(&acc_empty[b2], 0));
+            if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
         }
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(&g_tc_status, 1); }
     }
@@ -628,15 +661,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (*abort_flag) kp_linger_after_failure();
     if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
     kp_cluster_sync();                                                    // the other CTA may still signal barriers here
-    if (warp == 1) kp_tmem_dealloc_pair(tmem_base, 2 * BN);
+    if (warp == 1) kp_tmem_dealloc_pair(tmem_base, p.tmem_cols);
 }
 
 // ------------------------------------------------------------------------------------------ host side
 #define TC_SMEM_KB 208                       // shared memory for the ring
 #define TC_SPLIT_MAX_M_TILES 8               // rows of tiles up to which a product may be cut along K
-// the choice of a tile (tc_run), in bytes brought into an SM
+#define TC_SPLIT_COST (64 * 1024)            // a split over K, in bytes brought into an SM (tc_parts)
+// the choice of a tile (tc_choose), in bytes brought into an SM
 #define TC_KB_MIN (22 * 1024)                // a k-block at least
-#define TC_SPLIT_COST (220 * 1024)           // a split over K
 #define TC_PAIR_COST (100 * 1024)            // a pair of CTAs
 
 // SMs of the current device (asked once)
@@ -726,9 +759,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaSt
     return kp_launch_status();
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool PARTS>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcArgs& a, cudaStream_t s) {
-    auto kern = gemm_tc_pair_kernel<BN, EPI>;
+    auto kern = gemm_tc_pair_kernel<BN, EPI, PARTS>;
     static std::atomic<unsigned long long> ready{0};           // devices (bits) that the attribute is set on
     int dev = 0;
     cudaGetDevice(&dev);
@@ -767,6 +800,115 @@ static int tc_max_clusters(int bn, int epi, int cluster, int a_rows) {
 #undef TC_MC
 }
 
+// How a product runs: the width of its tiles, its parts along K, and whether the parts of a tile are shared by the CTAs of a
+// cluster or run one after the other, by one CTA or a pair of them.
+struct TcChoice { int bn, parts; bool cluster, pair; };
+
+// Sets of accumulators (one a part) that tensor memory's 512 columns have room for: two, so that the epilogue of a tile runs
+// under the main loop of the next, one, or none.
+static int tc_sets(int bn, int inner) { return 2 * inner * bn <= 512 ? 2 : (inner * bn <= 512 ? 1 : 0); }
+
+static int tc_a_rows(int M) { return M >= TC_BM ? TC_BM : (M + 7) / 8 * 8; }
+
+// Can parts along K of a tile `w` wide run at all: all units in one round, no part under two k-blocks, and the sums of a unit
+// fit where the ring was (false for more parts, too) ...
+static bool tc_split_starts(int M, int K, int w, int sp, int tiles) {
+    int stages = 0;
+    const size_t ring = tc_smem(tc_a_rows(M), w, &stages) - 2048;
+    const int rows = M < TC_BM ? M : TC_BM;
+    return tiles * sp <= tc_n_sm() && sp * 2 <= (K + TC_BK - 1) / TC_BK && (size_t)rows * w * 4 <= ring;
+}
+// ... the clusters all run at once, and no part is empty?
+static bool tc_split_runs(int M, int K, int epi, int w, int sp, int tiles) {
+    if (tiles > tc_max_clusters(w, epi, sp, tc_a_rows(M))) return false;
+    const int n_kb = (K + TC_BK - 1) / TC_BK, kbs = (n_kb + sp - 1) / sp;
+    return (n_kb + kbs - 1) / kbs == sp;
+}
+
+// Parts along K.  They alone decide an output's bits: its k-blocks are added in order within a part, the parts in order,
+// whatever the tile's width and whoever runs it.  And the tensor core cuts the sum off at every addition, so the error of
+// a sum grows with the length of its part (float32 sums against 64 bits, 2-norm: 2048 k's in one part 2.1e-6, in two
+// 1.0e-6, in four 4.7e-7).  So this rule is not a matter of speed alone: it is kept as it is, and tc_choose looks for the
+// fastest way to run what it gives.
+//
+// It counts the bytes that the busiest SM brings in, about 45 GB/s an SM whatever the source -- its share of W and, for
+// every tile, all the rows of A.  Unsplit, a narrow tile reads A once for a few rows of W (64 rows by 2048 x 5632 in
+// 32-row tiles: 720 KB of A for 360 KB of W) and wide tiles leave SMs idle.  So products of 17 to 1024 rows are cut where
+// the units (tile, part) fill one round over the SMs and a unit brings in fewer bytes; the price of the split (partial
+// sums out and in, the wait for the other parts) is counted as TC_SPLIT_COST of traffic.
+static int tc_parts(int M, int N, int K, int epi) {
+    const bool gated = epi == EPI_SWIGLU;
+    const int n_out = gated ? N / 2 : N, sms = tc_n_sm(), n_kb = (K + TC_BK - 1) / TC_BK;
+    const int m_tiles = (M + TC_BM - 1) / TC_BM, rows = M < TC_BM ? M : TC_BM, a_rows = tc_a_rows(M);
+    if (M <= 16 || m_tiles > TC_SPLIT_MAX_M_TILES) return 1;
+    long long best = -1;
+    int parts = 1;
+    for (int w = 256; w >= 64; w /= 2) {
+        const int cols = gated ? w / 2 : w, tiles = (n_out + cols - 1) / cols * m_tiles;
+        for (int sp = 1; sp <= 8; sp++) {
+            if (sp > 1 && !tc_split_starts(M, K, w, sp, tiles)) break;
+            if (sp > 1 && !tc_split_runs(M, K, epi, w, sp, tiles)) continue;
+            const int kbs = (n_kb + sp - 1) / sp;
+            long long cost = (sp == 1 ? (long long)((tiles + sms - 1) / sms) * n_kb : kbs) * (TC_BK * 2) * (w + a_rows);
+            if (sp > 1) cost += TC_SPLIT_COST + (long long)rows * w * 4 * (sp - 1) / sp;   // (the sums come in over the same port)
+            if (best < 0 || cost < best) { best = cost; parts = sp; }
+        }
+    }
+    return parts;
+}
+
+// The fastest way to run the parts that tc_parts gives: the choice that keeps the busiest SM busy for the shortest time,
+// counted in bytes brought into it (about 100 a nanosecond, from L2 or, all SMs together, HBM):
+//   a k-block: its rows of A and W, but no less than TC_KB_MIN (waiting, issuing, handing on);
+//   an epilogue: 0.6 KB a column of the tile, 1.2 KB gated, under the main loop of the next tile if there is one;
+//   parts one after the other: 6 KB a part more and 64 columns, for reading its sums;
+//   parts by a cluster (all units in one round): 100 KB and 5 KB a cluster (up to 24) for the barriers, four times the sums
+//   that are exchanged, more for clusters of other than 2 or 4 CTAs; beyond 512 rows a tenth more, as the sums of many tiles
+//   meet;
+//   a pair: TC_PAIR_COST for its barriers, and more for parts behind a gated epilogue, which is short of registers.
+// It was fitted to all that can run at 17 to 1000 rows of thirteen layer products: within 1 % of the best on average, 23 %
+// at worst (gated 700 rows by 9216 x 1024, where three kinds of tile tie).  Measured, us, a cluster always | the choice | the
+// choice were the parts free: 64 rows by 6144 x 2048 11.1 | 9.6 | 9.2, 200 by 3072 x 2048 14.1 | 10.2 | 9.9, 512 by 3072 x 1024
+// 14.5 | 7.5 | 7.2, 101 by 2048 x 5632 10.6 | 10.6 | 10.2.
+static TcChoice tc_choose(int M, int N, int K, int epi, int split) {
+    const bool gated = epi == EPI_SWIGLU;
+    const int n_out = gated ? N / 2 : N, sms = tc_n_sm(), n_kb = (K + TC_BK - 1) / TC_BK;
+    const int m_tiles = (M + TC_BM - 1) / TC_BM, rows = M < TC_BM ? M : TC_BM, a_rows = tc_a_rows(M);
+    const auto tiles_at = [&](int w) { const int cols = gated ? w / 2 : w; return (long long)((n_out + cols - 1) / cols); };
+    const auto kb_cost = [](long long r) { const long long bytes = r * TC_BK * 2; return bytes > TC_KB_MIN ? bytes : (long long)TC_KB_MIN; };
+    const auto epi_cost = [&](int w) { return (long long)w * (gated ? 1228 : 614); };
+    const auto run_cost = [&](long long rounds, long long main, int w) {
+        return rounds * (main > epi_cost(w) ? main : epi_cost(w)) + epi_cost(w);
+    };
+    const int parts = split ? tc_parts(M, N, K, epi) : 1;
+    const auto parts_cost = [&](int w) { return (parts - 1LL) * 6 * 1024 * (w > 64 ? w / 64 : 1); };
+    TcChoice ch = {0, parts, false, false};
+    long long best = -1;
+    for (int w = 256; w >= (gated ? 64 : 32); w /= 2) {
+        if (!tc_sets(w, parts)) continue;
+        const long long tiles = tiles_at(w) * m_tiles;
+        const long long cost = run_cost((tiles + sms - 1) / sms, n_kb * kb_cost(w + a_rows), w) + parts_cost(w);
+        if (best < 0 || cost < best) { best = cost; ch = {w, parts, false, false}; }
+    }
+    for (int w = 256; parts > 1 && w >= 64; w /= 2) {
+        const int tiles = (int)(tiles_at(w) * m_tiles), kbs = (n_kb + parts - 1) / parts;
+        if (!tc_split_starts(M, K, w, parts, tiles) || !tc_split_runs(M, K, epi, w, parts, tiles)) continue;
+        long long cost = kbs * kb_cost(w + a_rows) + epi_cost(w) / parts + 100 * 1024 + (tiles < 24 ? tiles : 24) * 5 * 1024 +
+                         4LL * rows * w * 4 * (parts - 1) / parts;
+        if (parts != 2 && parts != 4) cost += parts == 3 ? 32 * 1024 : 100 * 1024;
+        if (m_tiles > 4) cost += cost / 10;
+        if (cost < best) { best = cost; ch = {w, parts, true, false}; }
+    }
+    for (int w = 256; m_tiles > 1 && w >= 128; w /= 2) {
+        if (!tc_sets(w, parts)) continue;
+        const long long tiles = tiles_at(w) * ((M + 2 * TC_BM - 1) / (2 * TC_BM));
+        const long long cost = run_cost((tiles + sms / 2 - 1) / (sms / 2), n_kb * kb_cost(w / 2 + TC_BM), w) + TC_PAIR_COST +
+                               parts_cost(w) + (gated && parts > 1 ? 150 * 1024 : 0);
+        if (cost < best) { best = cost; ch = {w, parts, false, true}; }
+    }
+    return ch;
+}
+
 extern "C" {
 
 // epi: 0 store bf16, 1 store f32, 2 accumulate into f32, 3 SwiGLU (W = [gate; up], N = 2*ff, output [M, ff] bf16),
@@ -774,21 +916,52 @@ extern "C" {
 // split: products of 17 to 1024 rows may be cut along K (0: never).
 // glu: limit, alpha and shift of the gated unit with limits (activation code 3 in epi), else null.
 static int tc_run(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N,
-                  int K, int epi, int split, const float* glu, void* stream);
+                  int K, int epi, int split, const float* glu, const TcChoice* as, void* stream);
 
 int kp_gemm_tc_split(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N,
                      int K, int epi, int split, void* stream) {
-    return tc_run(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, split, nullptr, stream);
+    return tc_run(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, split, nullptr, nullptr, stream);
 }
 
 int kp_gemm_tc_split_glu(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N,
                          int K, int epi, int split, float limit, float alpha, float shift, void* stream) {
     const float glu[3] = {limit, alpha, shift};
-    return tc_run(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, split, glu, stream);
+    return tc_run(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, split, glu, nullptr, stream);
+}
+
+// out[0..3]: the tile width, the parts along K, whether a cluster shares them and whether pairs of CTAs run a product (epi:
+// its kind, without an activation)
+int kp_gemm_tc_choice(int M, int N, int K, int epi, int split, int* out) {
+    if (M <= 0 || N <= 0 || K < 8 || (K & 7)) return KP_ERR_BAD_ARG;
+    const TcChoice ch = tc_choose(M, N, K, epi, split);
+    out[0] = ch.bn; out[1] = ch.parts; out[2] = ch.cluster ? 1 : 0; out[3] = ch.pair ? 1 : 0;
+    return 0;
+}
+
+// kp_gemm_tc_split_glu (limit 0: the activation of epi) with all that given, where it can run
+int kp_gemm_tc_as(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K,
+                  int epi, int bn, int parts, int cluster, int pair, float limit, float alpha, float shift, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    const int kind = KP_EPI_KIND(epi), n_kb = (K + TC_BK - 1) / TC_BK;
+    const bool gated = kind == EPI_SWIGLU;
+    const int cols = gated ? bn / 2 : bn, n_out = gated ? N / 2 : N, m_tiles = (M + TC_BM - 1) / TC_BM;
+    if (bn != 256 && bn != 128 && bn != 64 && !(bn == 32 && !gated)) return KP_ERR_BAD_ARG;
+    if (parts < 1 || parts > 8 || (cluster && (pair || parts == 1 || bn < 64))) return KP_ERR_BAD_ARG;
+    if (pair && (bn < 128 || m_tiles < 2)) return KP_ERR_UNSUPPORTED;
+    if (cluster) {
+        const long long tiles = (long long)((n_out + cols - 1) / cols) * m_tiles;
+        if (tiles > 65535 || !tc_split_starts(M, K, bn, parts, (int)tiles) || !tc_split_runs(M, K, kind, bn, parts, (int)tiles)) return KP_ERR_UNSUPPORTED;
+    } else {
+        const int kbs = (n_kb + parts - 1) / parts;
+        if (!tc_sets(bn, parts) || (n_kb + kbs - 1) / kbs != parts) return KP_ERR_UNSUPPORTED;
+    }
+    const TcChoice ch = {bn, parts, cluster != 0, pair != 0};
+    const float glu[3] = {limit, alpha, shift};
+    return tc_run(A, lda, W, ldw, bias, C, ldc, M, N, K, epi, 1, limit > 0.f ? glu : nullptr, &ch, stream);
 }
 
 static int tc_run(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N,
-                  int K, int epi, int split, const float* glu, void* stream) {
+                  int K, int epi, int split, const float* glu, const TcChoice* as, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     const int act = KP_EPI_ACT(epi);
     epi = KP_EPI_KIND(epi);
@@ -807,65 +980,14 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
         if (N & 1) return KP_ERR_BAD_ARG;
         a.ff = N / 2;
     }
-    const int n_out = epi == EPI_SWIGLU ? a.ff : N;
-    const long long m_tiles = (M + TC_BM - 1) / TC_BM;
-    const int sms = tc_n_sm();
-    const bool gated = epi == EPI_SWIGLU;
-    const int lowest = gated ? 64 : 32;                                  // the narrowest tile
-    auto tiles_at = [&](int w) { const int cols = gated ? w / 2 : w; return (n_out + cols - 1) / cols; };
-    // Tile width, parts along K, and one CTA or a pair of them a tile: the choice that keeps the busiest SM busy for the
-    // shortest time, counted in bytes brought into it (about 100 a nanosecond, from L2 or, all SMs together, HBM):
-    //   a k-block: its rows of A and W, but no less than TC_KB_MIN (waiting, issuing, handing on);
-    //   an epilogue: 0.6 KB a column of the tile, 1.2 KB gated, under the main loop of the next tile if there is one;
-    //   a split (17 to 1024 rows; all units in one round, the parts of a tile a cluster): TC_SPLIT_COST for the clusters'
-    //   barriers, four times the sums that are exchanged, and more for clusters of other than 2 or 4 CTAs; beyond 512 rows
-    //   a quarter more, as the sums of many tiles meet;
-    //   a pair: TC_PAIR_COST for its barriers.
-    // It was fitted to all widths and parts at 24 to 512 rows of nine layer products; measured, us, the chosen | the best:
-    // 64 rows by 2048 x 5632 11.0 | 11.0, by 6144 x 2048 11.1 | 10.2, by gated 11264 x 2048 15.0 | 15.0, 101 rows 15.6 | 15.6,
-    // 24 rows 12.8 | 12.8, 128 rows by 2048 x 5632 12.4 | 12.4, 200 rows by 1024 x 4608 10.9 | 10.9.
-    const int n_kb = (K + TC_BK - 1) / TC_BK;
-    const auto kb_cost = [](long long rows) { const long long bytes = rows * TC_BK * 2; return bytes > TC_KB_MIN ? bytes : (long long)TC_KB_MIN; };
-    const auto epi_cost = [&](int w) { return (long long)w * (gated ? 1228 : 614); };
-    const auto run_cost = [&](long long rounds, long long main, int w) {
-        return rounds * (main > epi_cost(w) ? main : epi_cost(w)) + epi_cost(w);
-    };
-    a.a_rows = M >= TC_BM ? TC_BM : (M + 7) / 8 * 8;
-    int bn = 256, pair_bn = 0;
-    a.splits = 1;
-    long long best = -1;
-    for (int w = 256; w >= lowest; w /= 2) {
-        const long long tiles = (long long)tiles_at(w) * m_tiles;
-        const long long cost = run_cost((tiles + sms - 1) / sms, n_kb * kb_cost(w + a.a_rows), w);
-        if (best < 0 || cost < best) { best = cost; bn = w; }
-    }
-    if (split && M > 16 && m_tiles <= TC_SPLIT_MAX_M_TILES) {
-        const int rows = M < TC_BM ? M : TC_BM;                          // rows of a tile
-        for (int w = 256; w >= 64; w /= 2) {
-            const long long tiles = (long long)tiles_at(w) * m_tiles;
-            int stages = 0;
-            const size_t ring = tc_smem(a.a_rows, w, &stages) - 2048;
-            for (int sp = 2; sp <= 8; sp++) {
-                if (tiles * sp > sms || sp * 2 > n_kb || (size_t)rows * w * 4 > ring) break;
-                if (tiles > tc_max_clusters(w, epi, sp, a.a_rows)) continue;      // the clusters would not all run at once
-                const int kbs = (n_kb + sp - 1) / sp;
-                if ((n_kb + kbs - 1) / kbs != sp) continue;                       // a part would be empty
-                long long cost = kbs * kb_cost(w + a.a_rows) + epi_cost(w) / sp + TC_SPLIT_COST + 4LL * rows * w * 4 * (sp - 1) / sp;
-                if (sp != 2 && sp != 4) cost += sp == 3 ? 32 * 1024 : 100 * 1024;
-                if (m_tiles > 4) cost += cost / 4;
-                if (cost < best) { best = cost; bn = w; a.splits = sp; }
-            }
-        }
-    }
-    if (m_tiles > 1) {
-        for (int w = 256; w >= 128; w /= 2) {
-            const long long tiles = (long long)tiles_at(w) * ((M + 2 * TC_BM - 1) / (2 * TC_BM));
-            const long long cost = run_cost((tiles + sms / 2 - 1) / (sms / 2), n_kb * kb_cost(w / 2 + TC_BM), w) + TC_PAIR_COST;
-            if (cost < best) { best = cost; pair_bn = w; }
-        }
-    }
-    if (pair_bn) a.splits = 1;
-    a.kb_per_split = (n_kb + a.splits - 1) / a.splits;
+    const TcChoice ch = as ? *as : tc_choose(M, N, K, epi, split);
+    const int bn = ch.bn, pair_bn = ch.pair ? ch.bn : 0, n_kb = (K + TC_BK - 1) / TC_BK;
+    a.splits = ch.cluster ? ch.parts : 1;
+    a.inner = ch.cluster ? 1 : ch.parts;
+    a.kb_per_part = (n_kb + ch.parts - 1) / ch.parts;
+    a.n_sets = tc_sets(bn, a.inner);
+    for (a.tmem_cols = 32; a.tmem_cols < a.n_sets * a.inner * bn;) a.tmem_cols *= 2;
+    a.a_rows = tc_a_rows(M);
     cudaStream_t s = (cudaStream_t)stream;
     alignas(64) CUtensorMap ta, tw;
     int st = kp_make_map_bf16_2d(&ta, A, (unsigned long long)M, K, lda, TC_BK, a.a_rows);
@@ -873,7 +995,8 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
     st = kp_make_map_bf16_2d(&tw, W, (unsigned long long)N, K, ldw, TC_BK, pair_bn ? pair_bn / 2 : (epi == EPI_SWIGLU ? bn / 2 : bn));
     if (st) return st;
     if (pair_bn) {
-#define TC_PAIR(EPI) return pair_bn == 256 ? launch_pair<256, EPI>(ta, tw, a, s) : launch_pair<128, EPI>(ta, tw, a, s)
+#define TC_PAIR_BN(EPI, PARTS) return pair_bn == 256 ? launch_pair<256, EPI, PARTS>(ta, tw, a, s) : launch_pair<128, EPI, PARTS>(ta, tw, a, s)
+#define TC_PAIR(EPI) do { if (a.inner > 1) TC_PAIR_BN(EPI, true); TC_PAIR_BN(EPI, false); } while (0)
         switch (epi) {
             case EPI_STORE: TC_PAIR(EPI_STORE);
             case EPI_STORE_F32: TC_PAIR(EPI_STORE_F32);
@@ -886,6 +1009,7 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
             default: return KP_ERR_BAD_ARG;
         }
 #undef TC_PAIR
+#undef TC_PAIR_BN
     }
 #define TC_PICK(EPI)                                               \
     switch (bn) {                                                  \

@@ -1617,12 +1617,14 @@ def tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
             accumulate: bool = False, swiglu: bool = False, split: bool = True, activation: str = "silu",
-            glu: Optional[Tuple[float, float, float]] = None, plain_activation: Optional[str] = None) -> torch.Tensor:
+            glu: Optional[Tuple[float, float, float]] = None, plain_activation: Optional[str] = None,
+            choice: Optional[Tuple[int, int, bool, bool]] = None) -> torch.Tensor:
     """out = a @ w.T (+ bias) on the tcgen05 tensor cores (TMA-fed, accumulator in tensor memory); with
     ``swiglu`` ``w`` holds gate rows then up rows and out = silu(gate) * up (or ``activation``; with ``glu`` =
     (limit, alpha, shift) the gated unit with limits of :func:`glu_clamped`).  With ``split`` a product of 17 to
-    1024 rows is cut along K where that brings fewer bytes into the busiest SM (the parts of a tile are a
-    thread-block cluster and are added in a fixed order)."""
+    1024 rows is cut along K into parts that are added in a fixed order, run by a thread-block cluster or one after the
+    other.  ``choice`` runs it so instead
+    of as :func:`gemm_tc_choice` says, if that can be."""
     _need(a, "a", torch.bfloat16, contiguous=False); _need(w, "w", torch.bfloat16, contiguous=False)
     _need(out, "out", contiguous=False)
     M, K = a.shape
@@ -1635,6 +1637,16 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[
         if bias.numel() != N:
             raise KernelError("gemm_tc: bias size")
     lib = load_library("gemm_tc")
+    if choice is not None:
+        epi = _skinny_epilogue(out, accumulate, swiglu)
+        if swiglu:
+            epi |= (ACT_GLU_CLAMPED if glu is not None else _fused_activation(activation)) << 8
+        if plain_activation is not None:
+            epi = _plain_epilogue(epi, plain_activation)
+        width, parts, cluster, pair = choice
+        _run_gemm("gemm_tc", lib.kp_gemm_tc_as, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
+             _rows_2d(out, "out"), M, N, K, epi, width, parts, int(cluster), int(pair), *(_NO_LIMITS if glu is None else _glu_floats(glu)), STREAM)
+        return out
     if swiglu and glu is not None:
         epi = _skinny_epilogue(out, accumulate, swiglu) | (ACT_GLU_CLAMPED << 8)
         _run_gemm("gemm_tc", lib.kp_gemm_tc_split_glu, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
@@ -1646,6 +1658,16 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[
     _run_gemm("gemm_tc", lib.kp_gemm_tc_split, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
          _rows_2d(out, "out"), M, N, K, epi, 1 if split else 0, STREAM)
     return out
+
+
+def gemm_tc_choice(M: int, N: int, K: int, swiglu: bool = False, split: bool = True, out_dtype=torch.bfloat16) -> Tuple[int, int, bool, bool]:
+    """(tile width, parts along K, parts shared by a cluster, pairs of CTAs) of a :func:`gemm_tc` product.  The parts decide
+    its bits, the rest does not."""
+    out = (ctypes.c_int * 4)()
+    epi = EPI_SWIGLU if swiglu else (EPI_STORE if out_dtype == torch.bfloat16 else EPI_STORE_F32)
+    if load_library("gemm_tc").kp_gemm_tc_choice(M, N, K, epi, 1 if split else 0, out) != 0:
+        raise KernelError(f"gemm_tc_choice: no product of {M} x {N} x {K}")
+    return out[0], out[1], bool(out[2]), bool(out[3])
 
 
 STREAM_MAX_M = 64          # rows up to which the bulk-copy kernel is preferred
