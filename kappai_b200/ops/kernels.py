@@ -1591,15 +1591,16 @@ def skinny_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
 USE_TC = True              # bfloat16 products of more than 64 rows (and some of fewer) run on tcgen05 tensor cores
 
 
-TC_HEAD_FROM_M = 1         # rows from which a 65536-row head goes to the tcgen05 kernel (a step of one row 509 -> 501 us, of
-                           # the 350M shape 344 -> 334: its first weights are on their way before the wait on the norm)
+TC_HEAD_FROM_M = 2         # rows from which a 65536-row head goes to the tcgen05 kernel.  One row runs on csrc/gemm_rows.cu: as
+                           # fast (65536 x 1024 24.7 us against 25.0, x 2048 43.6 against 44.5), and its sums, cut along K
+                           # over eight warps, are closer to 64 bits (2.4e-7 against 2.2e-6 at 2048)
 TC_SPLIT_FROM_M = 17       # rows from which every product goes to the tcgen05 kernel (cut along K where that pays)
 
 
 def tc_pays_for_few_rows(M: int, N: int, swiglu: bool) -> bool:
     """Few-row products that the tcgen05 kernel runs faster than the weight-streaming
     kernels (measured on B200, K = 2048, inside a decode step): the 65536-row head from
-    1 row on (a step of 2 rows 638 -> 602 us, of 4 rows 661 -> 624, of one 509 -> 501), every
+    2 rows on (a step of 2 rows 638 -> 602 us, of 4 rows 661 -> 624), every
     product from 17 rows on (there the kernel cuts the product along K: a step of 64 rows
     1600 -> 1320 us), and below that wide products from 32 rows on."""
     if M >= TC_SPLIT_FROM_M:
@@ -1687,6 +1688,13 @@ def stream_pays(N: int, K: int) -> bool:
     fills the ring before it waits for the kernel before it, overlaps that kernel's tail inside a model step.
     It loses on the huge grid of a 65536-row head (65 against 48 us)."""
     return N <= 16384
+
+
+def rows_pays(M: int, N: int) -> bool:
+    """Up to 8 rows go to csrc/gemm_rows.cu, the same sums in the same order: of the layer products all, of a 65536-row head
+    one row (x 1024 29.3 -> 24.7 us, x 2048 42.6 -> 43.6, and it brings its first weights in before the wait on the norm; at
+    8 rows 30.9 | 31.0 and 48.6 | 51.6)."""
+    return M <= ROWS_MAX_M and (N <= 16384 or M == 1)
 
 
 CONV_STEP_MAX_M = 16       # rows up to which the conv step runs in in_proj's epilogue (measured: batch 8 703 -> 672 us a
@@ -1804,7 +1812,7 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optio
     if plain_activation is not None:
         epi = _plain_epilogue(epi, plain_activation)
     consts = _glu_floats(glu) if swiglu and glu is not None else ()
-    if USE_STREAM and stream_fits(K, swiglu) and stream_pays(N, K) and M <= ROWS_MAX_M:
+    if USE_STREAM and stream_fits(K, swiglu) and rows_pays(M, N):
         lib = load_library("gemm_rows")
         _run_gemm("gemm_stream", lib.kp_gemm_rows, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
              _rows_2d(out, "out"), M, N, K, epi, *(consts or _NO_LIMITS), STREAM)

@@ -39,6 +39,19 @@ def test_same_bits_as_the_streaming_kernel(monkeypatch, M, N, K):
     assert Kn.stream_status() == 0
 
 
+@pytest.mark.parametrize("N,K", [(65536, 1024), (40003, 512), (16385, 2048)])
+def test_one_row_of_a_head_has_the_sums_of_the_register_kernel(monkeypatch, N, K):
+    from kappai_b200.ops import kernels as Kn
+    from kappai_b200.ops.linear import linear
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a = torch.randn(1, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) / K ** 0.5).bfloat16()
+    one = linear(a, w, out_dtype=torch.float32)
+    monkeypatch.setattr(Kn, "USE_STREAM", False)
+    two = Kn.gemm_skinny(a, w, torch.empty(1, N, device="cuda"))
+    assert torch.equal(one, two)
+
+
 @pytest.mark.parametrize("M,d,K,taps", [(1, 512, 512, 3), (8, 1000, 1024, 2), (3, 2048, 512, 4), (7, 72, 1536, 7)])
 def test_conv_step_same_bits_and_state(monkeypatch, M, d, K, taps):
     from kappai_b200.ops import kernels as Kn
