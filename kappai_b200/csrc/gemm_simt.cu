@@ -105,6 +105,7 @@ constexpr int F32_GROUP = 256;                       // k's of one chain of FMAs
 struct F32Args {
     const float* A; const float* W; const float* bias; float* C;
     int M, N, K, lda, ldw, ldc;
+    int w_settled;                                   // W is written by nothing that may still run: it may be read before the wait
 };
 
 // 16 bytes to shared memory without a register between; `ok` false: zeros, nothing is read
@@ -132,8 +133,8 @@ template <int EPI> __device__ __forceinline__ void f32_store(const F32Args& p, i
 // Few rows.  A CTA owns 8 R rows of W; its warps cut K into jobs of 1024 columns = 4 stretches, and a lane (r, q) of a job
 // sums stretch q of the rows r, r + 8, ... for MB rows of A, so that every chain stays in one lane.  A warp brings its
 // job's W (and A) through a ring of its own in stages of 32 columns, by cp.async; nothing in the main loop waits for
-// another warp.  The stages of W that the ring holds are on their way before the wait on the kernel before (weights
-// depend on no kernel), those of A behind it.  In shared memory the eight 16-byte chunks of a row's stage are permuted
+// another warp.  The stages of a settled W that the ring holds are on their way before the wait on the kernel before
+// (a decode step of the 350M shape: 2 % of its time), those of A behind it.  In shared memory the eight 16-byte chunks of a row's stage are permuted
 // by the row (chunk c of row r at c ^ r), so the eight rows of a quarter warp read all banks once.
 //
 // More rows than MB take the grid's y; W then comes from L2.  Measured (W from HBM): 8 rows by 2048 x 5632 in 13.3 us
@@ -184,6 +185,7 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
 
     const int ahead = n_stages - 1;
     KP_TRACE_MARK(0);
+    if (!p.w_settled) pdl_wait();
     for (int it = 0; it < ahead && it < total; it++) load_w(it);
     pdl_wait();
     KP_TRACE_MARK(1);
@@ -289,6 +291,7 @@ gemm_f32_tile_kernel(const F32Args p) {
         }
     };
     KP_TRACE_MARK(0);
+    if (!p.w_settled) pdl_wait();
     for (int it = 0; it < F32T_STAGES - 1 && it < n_st; it++) load(it, false, true);
     pdl_wait();
     KP_TRACE_MARK(1);
@@ -418,13 +421,14 @@ static int f32_run(const F32Args& p, cudaStream_t s) {
     return f32_launch(gemm_f32_tile_kernel<EPI>, dim3((p.N + 63) / 64, (p.M + 63) / 64), 256, F32T_SMEM, s, p);
 }
 
+// w_settled: see F32Args (the general kernel waits first in any case)
 extern "C" int kp_gemm_nt_simt(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int lda,
-                               int ldw, int ldc, int epi, int dtype, void* stream) {
+                               int ldw, int ldc, int epi, int dtype, int w_settled, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return KP_ERR_BAD_ARG;
     if ((long long)((M + BM - 1) / BM) > 65535) return KP_ERR_UNSUPPORTED;
     if (dtype == KP_DTYPE_F32 && !((K | lda | ldw) & 3) && !(((uintptr_t)A | (uintptr_t)W) & 15)) {
-        const F32Args p = {(const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc};
+        const F32Args p = {(const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, w_settled};
         if (epi == EPI_STORE || epi == EPI_STORE_F32) return f32_run<EPI_STORE>(p, (cudaStream_t)stream);
         if (epi == EPI_ACCUM_F32) return f32_run<EPI_ACCUM_F32>(p, (cudaStream_t)stream);
         return KP_ERR_BAD_ARG;

@@ -610,8 +610,9 @@ def cast(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
 # ----------------------------------------------------------------------- gemm
 
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                 accumulate: bool = False) -> torch.Tensor:
-    """out = a @ w.T (+ bias); with ``accumulate`` out (float32) += that."""
+                 accumulate: bool = False, w_settled: bool = False) -> torch.Tensor:
+    """out = a @ w.T (+ bias); with ``accumulate`` out (float32) += that.  ``w_settled``: nothing that may still run writes
+    ``w`` (a weight), so a float32 product may read it before the launch in front of it has finished."""
     _need(a, "a", contiguous=False); _need(w, "w", a.dtype, contiguous=False); _need(out, "out", contiguous=False)
     lda, ldw, ldc = _rows_2d(a, "a"), _rows_2d(w, "w"), _rows_2d(out, "out")
     M, K = a.shape
@@ -634,7 +635,7 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Opti
         raise KernelError("gemm: output dtype must be the operand dtype or float32")
     lib = load_library("gemm_simt")
     _run_gemm("gemm_nt_simt", lib.kp_gemm_nt_simt, a, w, out, _ptr(a), _ptr(w), _ptr(bias), _ptr(out), M, N, K, lda, ldw, ldc, epi,
-         dtype_code(a.dtype), STREAM)
+         dtype_code(a.dtype), int(w_settled), STREAM)
     return out
 
 

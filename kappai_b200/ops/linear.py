@@ -8,9 +8,15 @@ kernels (decode steps) except where the tcgen05 kernel was measured faster
 (decode steps of 17 rows and more, where it cuts the product along K, and
 prompt portions).  The product is this package's own kernel in every case;
 no library matrix product is called.
+
+``w`` of a bfloat16 product is a weight: its first rows are read before the launch in front of the product has finished, so
+no launch that may still run may write it.  A float32 ``w`` may be anything, and is read early only where the caller says
+that it is such a weight: :func:`linear` with ``w_settled``, or the functions at the end of this module, which the model's
+parts call.
 """
 from __future__ import annotations
 
+from functools import partial
 from typing import Optional, Tuple
 
 import torch
@@ -20,7 +26,7 @@ from . import kernels as K
 
 def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
-           accumulate: bool = False) -> torch.Tensor:
+           accumulate: bool = False, w_settled: bool = False) -> torch.Tensor:
     """``out_dtype`` defaults to the operand dtype; ``accumulate`` adds into the
     float32 ``out`` (the residual sum stays in 32-bit)."""
     M, N = a.shape[0], w.shape[0]
@@ -34,8 +40,8 @@ def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         if w.dtype == torch.float32 and a.dtype == torch.bfloat16:
             a32 = K.cast(a.contiguous(), torch.empty(a.shape, dtype=torch.float32, device=a.device))
             if out.dtype == torch.float32:
-                return K.gemm_nt_simt(a32, w, out, bias, accumulate)
-            tmp = K.gemm_nt_simt(a32, w, torch.empty((M, N), dtype=torch.float32, device=a.device), bias)
+                return K.gemm_nt_simt(a32, w, out, bias, accumulate, w_settled)
+            tmp = K.gemm_nt_simt(a32, w, torch.empty((M, N), dtype=torch.float32, device=a.device), bias, w_settled=w_settled)
             return K.cast(tmp, out)
         raise K.KernelError(f"linear: operand dtypes {a.dtype} and {w.dtype} do not go together")
     tc = K.tc_ok(a, w) and out.stride(1) == 1
@@ -43,10 +49,11 @@ def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         return K.gemm_skinny(a, w, out, bias, accumulate)
     if tc:
         return K.gemm_tc(a, w, out, bias, accumulate)
-    return K.gemm_nt_simt(a, w, out, bias, accumulate)
+    return K.gemm_nt_simt(a, w, out, bias, accumulate, w_settled)
 
 
-def linear_act(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], activation: str) -> torch.Tensor:
+def linear_act(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], activation: str,
+               w_settled: bool = False) -> torch.Tensor:
     """``act(a @ w.T + bias)``, ungated, the activation taken of the float32 sums: in the product's epilogue where a kernel
     fits the shape, else by a row-wise kernel behind a float32 product."""
     M, N = a.shape[0], w.shape[0]
@@ -57,11 +64,12 @@ def linear_act(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], a
             return K.gemm_skinny(a, w, out, bias, plain_activation=activation)
         if tc:
             return K.gemm_tc(a, w, out, bias, plain_activation=activation)
-    return K.activate(linear(a, w, bias, out_dtype=torch.float32), out, activation)
+    return K.activate(linear(a, w, bias, out_dtype=torch.float32, w_settled=w_settled), out, activation)
 
 
 def linear_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, bias: Optional[torch.Tensor] = None,
-                  activation: str = "silu", glu: Optional[Tuple[float, float, float]] = None) -> torch.Tensor:
+                  activation: str = "silu", glu: Optional[Tuple[float, float, float]] = None,
+                  w_settled: bool = False) -> torch.Tensor:
     """``act(a @ Wg.T) * (a @ Wu.T)`` with ``w_gate_up = [Wg; Wu]`` and act = silu (or ``activation``); with
     ``glu`` = (limit, alpha, shift) the gated unit with limits instead, ``g sigmoid(alpha g) (u + shift)`` with
     ``g = min(gate, limit)`` and ``u = clamp(up, -limit, limit)``.  One fused kernel where there is one for the
@@ -75,7 +83,13 @@ def linear_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, bias: Optional[torch
         return K.gemm_skinny(a, w_gate_up, act, bias, swiglu=True, activation=activation, glu=glu)
     if tc:
         return K.gemm_tc(a, w_gate_up, act, bias, swiglu=True, activation=activation, glu=glu)
-    gu = linear(a, w_gate_up, bias)
+    gu = linear(a, w_gate_up, bias, w_settled=w_settled)
     if glu is not None:
         return K.glu_clamped(gu, act, *glu)
     return K.swiglu(gu, act, activation)
+
+
+# the products with a model's weights
+linear_weights = partial(linear, w_settled=True)
+linear_weights_act = partial(linear_act, w_settled=True)
+linear_weights_swiglu = partial(linear_swiglu, w_settled=True)

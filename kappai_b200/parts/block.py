@@ -50,7 +50,7 @@ import torch
 
 from ..config.schema import ConfigError
 from ..ops import kernels as K
-from ..ops.linear import linear
+from ..ops.linear import linear_weights as linear
 from .base import Part, WeightSpec, register_part
 from .streams import stream_norm
 

@@ -19,7 +19,7 @@ from typing import Dict
 import torch
 
 from ..ops import kernels as K
-from ..ops.linear import linear
+from ..ops.linear import linear_weights as linear
 from .base import Part, WeightSpec, register_part
 
 

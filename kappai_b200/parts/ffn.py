@@ -48,7 +48,7 @@ from typing import Dict
 import torch
 
 from ..ops import kernels as K
-from ..ops.linear import linear, linear_act, linear_swiglu
+from ..ops.linear import linear_weights as linear, linear_weights_act as linear_act, linear_weights_swiglu as linear_swiglu
 from ..config.schema import ConfigError
 from .base import Part, WeightSpec, register_part
 

@@ -41,7 +41,7 @@ import torch
 from ..cache.spec import StateSpec
 from ..config.schema import ConfigError, PartSpec
 from ..ops import kernels as K
-from ..ops.linear import linear
+from ..ops.linear import linear_weights as linear
 from .base import Part, WeightSpec, make_part, register_part
 
 

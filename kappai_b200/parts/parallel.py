@@ -17,7 +17,7 @@ import torch
 
 from ..cache.spec import CompositeSpec
 from ..config.schema import ConfigError, PartSpec
-from ..ops.linear import linear
+from ..ops.linear import linear_weights as linear
 from .base import Part, WeightSpec, make_part, register_part
 
 

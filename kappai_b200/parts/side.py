@@ -24,7 +24,7 @@ import torch
 
 from ..config.schema import ConfigError
 from ..ops import kernels as K
-from ..ops.linear import linear
+from ..ops.linear import linear_weights as linear
 from .base import Part, WeightSpec, register_part
 
 

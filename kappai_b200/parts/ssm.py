@@ -30,7 +30,7 @@ import torch
 from ..cache.spec import StateSpec
 from ..config.schema import ConfigError
 from ..ops import kernels as K
-from ..ops.linear import linear
+from ..ops.linear import linear_weights as linear
 from .base import Part, WeightSpec, register_part
 from .lightning import lightning_chunks
 

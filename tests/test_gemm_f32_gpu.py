@@ -42,3 +42,20 @@ def test_rows_that_are_not_16_byte_aligned_take_the_general_kernel():
         exact = a_.double() @ w[:, :k].double().T
         bound = (k + 2) * 2.0 ** -24 * (a_.double().abs() @ w[:, :k].double().abs().T)
         assert bool(((out.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8192, 2048), (8, 4096, 4096), (40, 4096, 2048), (300, 2048, 4096)])
+def test_second_operand_written_by_the_launch_in_front(M, N, K):
+    """(The cast lets the launch behind it in at its start.)"""
+    from kappai_b200.ops import kernels as Kn
+    from kappai_b200.ops.linear import linear
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(M, K, device="cuda", generator=g)
+    sources = [torch.randn(N, K, device="cuda", generator=g).bfloat16() for _ in range(3)]
+    want = [Kn.gemm_nt_simt(a, s.float(), torch.empty(M, N, device="cuda"), w_settled=True) for s in sources]
+    w = torch.zeros(N, K, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(12):
+        Kn.cast(sources[i % 3], w)
+        out = Kn.gemm_nt_simt(a, w, torch.empty(M, N, device="cuda")) if i % 2 else linear(a, w)
+        assert torch.equal(out, want[i % 3]), i
