@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define KP_DTYPE_F32 0
 #define KP_DTYPE_BF16 1
 
@@ -200,6 +202,20 @@ static inline cudaError_t kp_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+// Lets `kern` have up to `bytes` of dynamic shared memory a CTA, once a device (`ready`: a bit for each that it is done on).
+// The limit belongs to the function, not to a launch: `bytes` is the most that any launch of it may ask for, so that
+// launches of different sizes from several threads cannot lower it for one another.
+template <typename Kern>
+static inline int kp_smem_limit(Kern kern, size_t bytes, std::atomic<unsigned long long>& ready) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev <= 63 && ((ready.load(std::memory_order_relaxed) >> dev) & 1)) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && dev <= 63) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
+    return (int)e;
+}
+#define KP_SMEM_MAX (227 * 1024)              // shared memory a CTA can have
 
 static inline int kp_launch_status() {
     cudaError_t e = cudaGetLastError();

@@ -23,8 +23,6 @@
 // on others, and a step takes 613 us.  Rings of 122 KB 524, 155 KB 506, 190 KB 511, 210 KB 542.
 //
 // Epilogues as in gemm_stream.cu.  K a multiple of 512.
-#include <atomic>
-
 #include "mma.cuh"
 
 #define EPI_STORE 0
@@ -246,14 +244,9 @@ static int rows_launch(const RowsArgs& a, cudaStream_t s) {
     constexpr int S = RW_SMEM / (RW_WARPS * STAGE) > RW_MAX_STAGES ? RW_MAX_STAGES : RW_SMEM / (RW_WARPS * STAGE);
     constexpr size_t smem = (size_t)RW_WARPS * S * STAGE + sizeof(float) * 2 * RW_WARPS * MT * 128;
     auto kern = gemm_rows_kernel<WR, EPI>;
-    static std::atomic<unsigned long long> ready{0};                     // devices (bits) that the attribute is set on
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev > 63 || !((ready.load(std::memory_order_relaxed) >> dev) & 1)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        if (dev <= 63) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-    }
+    static std::atomic<unsigned long long> ready{0};
+    const int st = kp_smem_limit(kern, smem, ready);
+    if (st) return st;
     const int n_out = JOINS > 1 ? a.ff : a.N, n_tiles = (n_out + WR / JOINS - 1) / (WR / JOINS);
     return (int)kp_launch_pdl(kern, dim3(n_tiles < rw_n_sm() ? n_tiles : rw_n_sm()), dim3(RW_WARPS * 32), smem, s, a);
 }

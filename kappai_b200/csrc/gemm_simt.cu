@@ -365,15 +365,6 @@ static int f32_n_sm() {
     return n;
 }
 
-template <typename Kern, typename... Args>
-static int f32_launch(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
-    return (int)kp_launch_pdl(kern, grid, dim3(threads), smem, s, args...);
-}
-
 template <int R, int MB, int EPI>
 static int f32_rows(const F32Args& p, cudaStream_t s) {
     const int n_jobs = (p.K + F32R_JOB - 1) / F32R_JOB;
@@ -391,7 +382,9 @@ static int f32_rows(const F32Args& p, cudaStream_t s) {
     if (stages < 2) stages = 2;
     const size_t smem = (size_t)warps * stages * stage + red;
     if (smem > 220 * 1024) return KP_ERR_UNSUPPORTED;
-    return f32_launch(gemm_f32_rows_kernel<R, MB, EPI>, grid, warps * 32, smem, s, p, stages);
+    static std::atomic<unsigned long long> ready{0};
+    const int st = kp_smem_limit(gemm_f32_rows_kernel<R, MB, EPI>, KP_SMEM_MAX, ready);
+    return st ? st : (int)kp_launch_pdl(gemm_f32_rows_kernel<R, MB, EPI>, grid, dim3(warps * 32), smem, s, p, stages);
 }
 
 // Which kernel (K counts in every kernel alike, so the rule compares rounds over the SMs; measured at widths of 1024 to
@@ -418,7 +411,9 @@ static int f32_run(const F32Args& p, cudaStream_t s) {
         st = f32_rows<4, 16, EPI>(p, s);
     }
     if (st != KP_ERR_UNSUPPORTED) return st;
-    return f32_launch(gemm_f32_tile_kernel<EPI>, dim3((p.N + 63) / 64, (p.M + 63) / 64), 256, F32T_SMEM, s, p);
+    static std::atomic<unsigned long long> ready{0};
+    st = kp_smem_limit(gemm_f32_tile_kernel<EPI>, F32T_SMEM, ready);
+    return st ? st : (int)kp_launch_pdl(gemm_f32_tile_kernel<EPI>, dim3((p.N + 63) / 64, (p.M + 63) / 64), dim3(256), F32T_SMEM, s, p);
 }
 
 // w_settled: see F32Args (the general kernel waits first in any case)

@@ -37,8 +37,6 @@
 //
 // Every wait on an mbarrier is bounded.  A wait that gives up sets a status word (kp_tc_status), the CTA
 // stops issuing work, still frees its tensor memory and returns.
-#include <atomic>
-
 #include "tcgen05.cuh"
 
 #define EPI_STORE 0
@@ -695,15 +693,9 @@ static size_t tc_smem(int a_rows, int bn, int* stages_out) {
 }
 
 template <int BN, int EPI>
-static int prepare(size_t smem) {
-    auto kern = gemm_tc_kernel<BN, EPI>;
-    static size_t attr_smem = 0;
-    if (smem > attr_smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        attr_smem = smem;
-    }
-    return 0;
+static int prepare() {
+    static std::atomic<unsigned long long> ready{0};
+    return kp_smem_limit(gemm_tc_kernel<BN, EPI>, KP_SMEM_MAX, ready);
 }
 
 // Clusters of `cluster` CTAs of this kernel that the device runs at once (asked once for each size; 0 if it cannot
@@ -714,7 +706,7 @@ static int max_clusters(int cluster, size_t smem) {
     if (cluster < 2 || cluster > 8) return 0;
     if (known[cluster] == 0) {
         known[cluster] = -1;
-        if (prepare<BN, EPI>(smem) == 0) {
+        if (prepare<BN, EPI>() == 0) {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(cluster * 64); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = smem;
             cudaLaunchAttribute attr[1];
@@ -734,7 +726,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaSt
     int stages = 0;
     const size_t smem = tc_smem(a.a_rows, BN, &stages);
     a.n_stages = stages;
-    int st = prepare<BN, EPI>(smem);
+    int st = prepare<BN, EPI>();
     if (st) return st;
     const int n_out = TC_GATED(EPI) ? a.ff : a.N;
     const int n_tile = TC_GATED(EPI) ? BN / 2 : BN;
@@ -762,14 +754,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaSt
 template <int BN, int EPI, bool PARTS>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcArgs& a, cudaStream_t s) {
     auto kern = gemm_tc_pair_kernel<BN, EPI, PARTS>;
-    static std::atomic<unsigned long long> ready{0};           // devices (bits) that the attribute is set on
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev > 63 || !((ready.load(std::memory_order_relaxed) >> dev) & 1)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_PAIR_SMEM(BN));
-        if (e != cudaSuccess) return (int)e;
-        if (dev <= 63) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-    }
+    static std::atomic<unsigned long long> ready{0};
+    const int st = kp_smem_limit(kern, TC_PAIR_SMEM(BN), ready);
+    if (st) return st;
     const int n_out = TC_GATED(EPI) ? a.ff : a.N, n_tile = TC_GATED(EPI) ? BN / 2 : BN;
     const int n_tiles = ((n_out + n_tile - 1) / n_tile) * ((a.M + 2 * TC_BM - 1) / (2 * TC_BM));
     const int pairs = tc_n_sm() / 2;

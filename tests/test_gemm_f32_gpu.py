@@ -59,3 +59,33 @@ def test_second_operand_written_by_the_launch_in_front(M, N, K):
         Kn.cast(sources[i % 3], w)
         out = Kn.gemm_nt_simt(a, w, torch.empty(M, N, device="cuda")) if i % 2 else linear(a, w)
         assert torch.equal(out, want[i % 3]), i
+
+
+def test_launches_of_different_sizes_from_several_threads():
+    """The kernels' limit on shared memory belongs to the function: one thread's small launch must not lower it for another's
+    (of 20,000 launches a thread 970 to 2,973 failed where each set its own)."""
+    import ctypes
+    import threading
+    from kappai_b200.ops import kernels as Kn
+    from kappai_b200.ops.build import load_library
+    launch = load_library("gemm_simt").kp_gemm_nt_simt
+    failed, keep = [0] * 4, []
+    shapes = [(8, 64, 5632), (8, 64, 1024), (8, 64, 2048), (8, 64, 4608)]                # one instantiation, 70 to 200 KB
+
+    def work(i, args, stream):
+        for _ in range(5000):
+            failed[i] += launch(*args) != 0
+        stream.synchronize()
+
+    threads = []
+    for i, (M, N, K) in enumerate(shapes):
+        a, w, out, s = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda"), torch.empty(M, N, device="cuda"), torch.cuda.Stream()
+        keep.append((a, w, out))
+        args = [Kn._ptr(a), Kn._ptr(w), Kn._ptr(None), Kn._ptr(out)] + [ctypes.c_int(v) for v in (M, N, K, K, K, N, 0, 0, 0)]
+        threads.append(threading.Thread(target=work, args=(i, args + [ctypes.c_void_p(s.cuda_stream)], s)))
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert failed == [0] * 4
