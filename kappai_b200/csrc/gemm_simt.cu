@@ -365,55 +365,84 @@ static int f32_n_sm() {
     return n;
 }
 
-template <int R, int MB, int EPI>
-static int f32_rows(const F32Args& p, cudaStream_t s) {
-    const int n_jobs = (p.K + F32R_JOB - 1) / F32R_JOB;
-    const int stage = (8 * R + MB) * 4 * F32R_COLS * 4;
+// Which kernel runs, and how: R, MB, warps and ring stages of the few-row kernel, or tiles (R 0).
+struct F32Choice { int R, MB, warps, stages; size_t smem; };
+
+// The few-row kernel's warps and ring; `fits` false: not even one warp's ring and the stretches' sums have room.
+static bool f32_rows_fit(int M, int N, int K, int R, int MB, F32Choice* c) {
+    const int n_jobs = (K + F32R_JOB - 1) / F32R_JOB, stage = (8 * R + MB) * 4 * F32R_COLS * 4;
     const int most = R == 4 ? 4 : F32R_MAX_WARPS;
-    const int warps = n_jobs < most ? n_jobs : (n_jobs + (n_jobs + most - 1) / most - 1) / ((n_jobs + most - 1) / most);
     const size_t red = (size_t)n_jobs * 4 * MB * 8 * R * 4;
-    const dim3 grid((p.N + 8 * R - 1) / (8 * R), (p.M + MB - 1) / MB);
+    int warps = n_jobs < most ? n_jobs : (n_jobs + (n_jobs + most - 1) / most - 1) / ((n_jobs + most - 1) / most);
+    while (warps > 1 && (size_t)warps * 2 * stage + red > KP_SMEM_MAX) warps--;      // (the order of the sums is the same)
+    const long long ctas = (long long)((N + 8 * R - 1) / (8 * R)) * ((M + MB - 1) / MB);
     // one CTA an SM: all the ring that pays (a job has 8 stages); more: a third of the SM's memory each, or a sixth where a
     // CTA is a single warp (8 rows by 9216 x 1024: 19.5 us with a third, 11.5 with a sixth; 65536 x 1024 95 and 52; one row by
     // 6144 x 2048, two warps: 8.9 and 11.1)
-    const size_t room = (int)(grid.x * grid.y) <= f32_n_sm() ? 200 * 1024 : (warps == 1 ? 36 : 74) * 1024;
+    const size_t room = ctas <= f32_n_sm() ? 200 * 1024 : (warps == 1 ? 36 : 74) * 1024;
     int stages = red < room ? (int)((room - red) / ((size_t)warps * stage)) : 0;
     if (stages > 8) stages = 8;
     if (stages < 2) stages = 2;
-    const size_t smem = (size_t)warps * stages * stage + red;
-    if (smem > 220 * 1024) return KP_ERR_UNSUPPORTED;
-    static std::atomic<unsigned long long> ready{0};
-    const int st = kp_smem_limit(gemm_f32_rows_kernel<R, MB, EPI>, KP_SMEM_MAX, ready);
-    return st ? st : (int)kp_launch_pdl(gemm_f32_rows_kernel<R, MB, EPI>, grid, dim3(warps * 32), smem, s, p, stages);
+    *c = {R, MB, warps, stages, (size_t)warps * stages * stage + red};
+    return c->smem <= KP_SMEM_MAX;
 }
 
-// Which kernel (K counts in every kernel alike, so the rule compares rounds over the SMs; measured at widths of 1024 to
-// 11264, us, with rows of 8 | rows of 16 | tiles):
+// K counts in every kernel alike, so the rule compares rounds over the SMs; measured at widths of 1024 to 11264, us, with
+// rows of 8 | rows of 16 | tiles:
 //   up to 24 rows: rows of 8 (16 rows by 2048 x 5632: 25 | 38 | 172; by 1024 x 1024: 8 | 19 | 32), but not for a wide W
 //   with one job of K, whose CTAs are single warps (16 rows by 9216 x 1024: 30 | 21 | 40);
 //   a round of rows of 16 takes 7.2 us for 1,000 k, one of tiles 30.5 (128 rows by 2048 x 5632: 165 | 152 | 172; 160 rows:
-//   - | 190 | 173; 96 rows by 6144 x 2048: 98 | 82 | 121; 256 rows by 1024 x 1024: - | 22 | 33; 400 rows: - | 42 | 33).
-template <int EPI>
-static int f32_run(const F32Args& p, cudaStream_t s) {
+//   - | 190 | 173; 96 rows by 6144 x 2048: 98 | 82 | 121; 256 rows by 1024 x 1024: - | 22 | 33; 400 rows: - | 42 | 33);
+//   where the sums leave room for fewer than four warps, a round of rows of 16 takes 18 us a turn of them (32 rows by
+//   4096 x 4096, four warps: - | 41 | 127; x 7168, three: - | 111 | 219; 128 rows by 2048 x 12288, two: - | 422 | 375).
+// A K whose stretches' sums leave no room for a ring (some 100,000 at 8 rows, 20,000 at rows of 16) goes to tiles.
+static F32Choice f32_choose(int M, int N, int K) {
     const int sms = f32_n_sm();
     const auto rounds = [&](long long ctas) { return (ctas + sms - 1) / sms; };
     const auto cuts = [](int n, int size) { return (long long)((n + size - 1) / size); };
-    int st = KP_ERR_UNSUPPORTED;                                         // (a K too long for the sums of its stretches: tiles)
-    if (p.M <= 8 || (p.M <= 24 && (p.K > F32R_JOB || p.N <= 32 * sms))) {
-        const bool narrow = cuts(p.N, 16) < sms;                         // 8 rows of W a CTA where 16 leave SMs idle
-#define F32_ROWS(MB_) st = narrow ? f32_rows<1, MB_, EPI>(p, s) : f32_rows<2, MB_, EPI>(p, s)
-        if (p.M == 1) F32_ROWS(1);
-        else if (p.M == 2) F32_ROWS(2);
-        else if (p.M <= 4) F32_ROWS(4);
-        else F32_ROWS(8);
-#undef F32_ROWS
-    } else if (rounds(cuts(p.M, 16) * cuts(p.N, 32)) * 72 < rounds(cuts(p.M, 64) * cuts(p.N, 64)) * 305) {
-        st = f32_rows<4, 16, EPI>(p, s);
+    F32Choice c;
+    if (M <= 8 || (M <= 24 && (K > F32R_JOB || N <= 32 * sms))) {
+        const int R = cuts(N, 16) < sms ? 1 : 2;                                     // 8 rows of W a CTA where 16 leave SMs idle
+        if (f32_rows_fit(M, N, K, R, M == 1 ? 1 : M == 2 ? 2 : M <= 4 ? 4 : 8, &c)) return c;
+    } else if (f32_rows_fit(M, N, K, 4, 16, &c)) {
+        const long long jobs = (K + F32R_JOB - 1) / F32R_JOB, turns = (jobs + c.warps - 1) / c.warps;
+        const long long row = turns > (jobs + 3) / 4 && 180000 * turns > 72LL * K ? 180000 * turns : 72LL * K;
+        if (rounds(cuts(M, 16) * cuts(N, 32)) * row < rounds(cuts(M, 64) * cuts(N, 64)) * 305 * K) return c;
     }
-    if (st != KP_ERR_UNSUPPORTED) return st;
+    return {0, 0, 0, 0, 0};
+}
+
+template <int R, int MB, int EPI>
+static int f32_rows(const F32Args& p, const F32Choice& c, cudaStream_t s) {
     static std::atomic<unsigned long long> ready{0};
-    st = kp_smem_limit(gemm_f32_tile_kernel<EPI>, F32T_SMEM, ready);
+    const int st = kp_smem_limit(gemm_f32_rows_kernel<R, MB, EPI>, KP_SMEM_MAX, ready);
+    if (st) return st;
+    const dim3 grid((p.N + 8 * R - 1) / (8 * R), (p.M + MB - 1) / MB);
+    return (int)kp_launch_pdl(gemm_f32_rows_kernel<R, MB, EPI>, grid, dim3(c.warps * 32), c.smem, s, p, c.stages);
+}
+
+template <int EPI>
+static int f32_run(const F32Args& p, cudaStream_t s) {
+    const F32Choice c = f32_choose(p.M, p.N, p.K);
+    if (c.R == 4) return f32_rows<4, 16, EPI>(p, c, s);
+#define F32_ROWS(MB_) return c.R == 1 ? f32_rows<1, MB_, EPI>(p, c, s) : f32_rows<2, MB_, EPI>(p, c, s)
+    switch (c.MB) {
+        case 1: F32_ROWS(1);
+        case 2: F32_ROWS(2);
+        case 4: F32_ROWS(4);
+        case 8: F32_ROWS(8);
+    }
+#undef F32_ROWS
+    static std::atomic<unsigned long long> ready{0};
+    const int st = kp_smem_limit(gemm_f32_tile_kernel<EPI>, F32T_SMEM, ready);
     return st ? st : (int)kp_launch_pdl(gemm_f32_tile_kernel<EPI>, dim3((p.N + 63) / 64, (p.M + 63) / 64), dim3(256), F32T_SMEM, s, p);
+}
+
+// out[0..3]: R, MB, warps and stages of the few-row kernel that runs a float32 product with 16-byte rows; R 0: tiles
+extern "C" int kp_gemm_f32_choice(int M, int N, int K, int* out) {
+    const F32Choice c = f32_choose(M, N, K);
+    out[0] = c.R; out[1] = c.MB; out[2] = c.warps; out[3] = c.stages;
+    return 0;
 }
 
 // w_settled: see F32Args (the general kernel waits first in any case)

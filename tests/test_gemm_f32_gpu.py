@@ -89,3 +89,14 @@ def test_launches_of_different_sizes_from_several_threads():
     for t in threads:
         t.join()
     assert failed == [0] * 4
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 300, 16384), (8, 2400, 4096), (8, 2500, 36864), (33, 1100, 3076), (40, 1100, 4096), (17, 700, 7168),
+                                   (64, 1100, 8192), (25, 100, 20480)])
+def test_long_sums(M, N, K):
+    """Where the stretches' sums leave the few-row kernels fewer warps, or none: the bits of the tiles."""
+    from kappai_b200.ops import kernels as Kn
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, w = torch.randn(2048, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    tiles = Kn.gemm_nt_simt(a, w, torch.empty(2048, N, device="cuda"))
+    assert torch.equal(Kn.gemm_nt_simt(a[:M], w, torch.empty(M, N, device="cuda")), tiles[:M])
