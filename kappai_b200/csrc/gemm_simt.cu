@@ -384,7 +384,7 @@ static bool f32_rows_fit(int M, int N, int K, int R, int MB, F32Choice* c) {
     if (stages > 8) stages = 8;
     if (stages < 2) stages = 2;
     *c = {R, MB, warps, stages, (size_t)warps * stages * stage + red};
-    return c->smem <= KP_SMEM_MAX;
+    return c->smem <= KP_SMEM_MAX && (M + MB - 1) / MB <= 65535;                     // (more rows of A than a grid has)
 }
 
 // K counts in every kernel alike, so the rule compares rounds over the SMs; measured at widths of 1024 to 11264, us, with

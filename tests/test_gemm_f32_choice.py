@@ -24,3 +24,7 @@ def test_rows_kernels_take_every_k_their_sums_leave_room_for(M, N, K, R, MB):
 @pytest.mark.parametrize("M,N,K", [(2048, 2048, 2048), (128, 2048, 12288), (96, 1024, 20480), (400, 1024, 1024), (8, 4096, 400000)])
 def test_tiles(M, N, K):
     assert choice(M, N, K)[0] == 0
+
+
+def test_rows_beyond_a_grid_take_tiles():
+    assert choice(16 * 65535, 8, 64)[0] == 4 and choice(16 * 65535 + 1, 8, 64)[0] == 0

@@ -100,3 +100,12 @@ def test_long_sums(M, N, K):
     a, w = torch.randn(2048, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
     tiles = Kn.gemm_nt_simt(a, w, torch.empty(2048, N, device="cuda"))
     assert torch.equal(Kn.gemm_nt_simt(a[:M], w, torch.empty(M, N, device="cuda")), tiles[:M])
+
+
+def test_more_rows_than_a_grid_has():
+    from kappai_b200.ops import kernels as Kn
+    M = 16 * 65535 + 40
+    a, w = torch.randn(M, 8, device="cuda"), torch.randn(8, 8, device="cuda")
+    out = Kn.gemm_nt_simt(a, w, torch.empty(M, 8, device="cuda"))
+    for lo in (0, M - 130):
+        assert torch.equal(out[lo:lo + 130], Kn.gemm_nt_simt(a[lo:lo + 130], w, torch.empty(130, 8, device="cuda")))
