@@ -17,6 +17,7 @@
 
 #define SAMPLE_THREADS 1024
 #define SAMPLE_MAX_CAND 1024
+#define SAMPLE_SHORT_K 600                   // the largest k of a long row whose candidates are looked for the short way first
 
 __device__ __forceinline__ unsigned int order_key(float f) {
     unsigned int u = __float_as_uint(f);
@@ -154,11 +155,14 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
     // First without a selection over the whole row: every thread's largest key; at least k keys are as large as the k-th
     // of these 1024, so the row's k largest are among the keys that are, and for a k like 40 those are hardly more than k.
     // The row is read once, and again by the threads whose largest key passes.  What bounds it is the one SM that reads
-    // a row.  Where more than 1024 pass (a large k, many equal values), and for rows with NaN or a -0 among the
-    // candidates, whose order the selection below defines, that runs instead.
-    // Measured at 8 rows of 65536, k = 40, between two events: 175 us with the selection, 36 so.
-    int n_cand = 0;
-    {
+    // a row.  Where more than 1024 pass (many equal values), and for rows with NaN or a -0 among the candidates, whose order
+    // the selection below defines, that runs instead.  It runs at once for a k above SAMPLE_SHORT_K in a row longer than the
+    // threads are many: of a long row some -1024 ln(1 - k/1024) keys pass, 710 at 512 and more than 1024 from 650 on.
+    // Measured at 8 rows of 65536, us, with the selection | so: normal values, k = 40 168 | 27, 512 184 | 50, 600 187 | 53;
+    // above the line the attempt would add 9 to 19 us to the selection (top-p alone, k = 1024: 201 | 210 before that line was
+    // drawn, 161 now that the selection's counts read eight values at a time); a row masked but for 20 values 162 | 147.
+    int n_cand = SAMPLE_MAX_CAND + 1;
+    if (k <= SAMPLE_SHORT_K || V <= SAMPLE_THREADS) {
         unsigned int best = 0;
         bool odd = false;
 #pragma unroll 8
@@ -174,7 +178,11 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
             if (__syncthreads_count(best >= c) >= k) t = c;
         }
         if (odd) s_kleft = 1;
-        if (best >= t) {
+        // (where the k-th value stands at many threads, as in a row that is masked but for fewer than k, too many keys pass)
+        const int passing = __syncthreads_count(best >= t);
+        if (passing > (k + SAMPLE_THREADS) / 2 && V > SAMPLE_THREADS) {
+            if (tid == 0) s_kleft = 1;
+        } else if (best >= t) {
 #pragma unroll 8
             for (int i = tid; i < V; i += SAMPLE_THREADS) {
                 const float v = l[i];
@@ -203,7 +211,8 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
         __syncthreads();
         const unsigned int prefix = s_prefix;
         const unsigned int mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
-        for (int i = tid; i < V; i += blockDim.x) {
+#pragma unroll 8
+        for (int i = tid; i < V; i += SAMPLE_THREADS) {                  // (eight reads under way: what the attempt cost, and more)
             const unsigned int key = order_key(l[i]);
             if ((key & mask) == prefix) atomicAdd(&s_hist[(key >> shift) & 255u], 1u);
         }

@@ -47,3 +47,22 @@ def test_top_k_candidates(kind, V):
                 continue
             want, slack = PS.sample(x[i], uniform(i + 1, 3), temperature=0.7, top_k=k, **f)
             assert got[i] == want or slack < 1e-5, (kind, V, k, f, got[i], want, slack)
+
+
+@pytest.mark.parametrize("V", [1024, 1025, 65536])
+@pytest.mark.parametrize("k", [512, 600, 601, 0])
+def test_rows_on_either_side_of_the_short_way(V, k):
+    """k at the line and no k at all (the 1024 largest), of rows that are masked but for fewer than k too."""
+    from kappai_b200 import SamplingParams
+    from kappai_b200.sampling import uniform
+    from kappai_b200.sampling.sampler import sample
+    if k >= V:
+        return
+    rng = np.random.default_rng(V + k)
+    x = np.stack([rows(kind, 1, V, rng)[0] for kind in ("plain", "ties", "equal", "masked", "few")])
+    f = dict(top_p=0.9, min_p=0.0)
+    got = sample(torch.from_numpy(x).cuda(), [SamplingParams(temperature=0.7, top_k=k, **f)] * len(x), [i + 1 for i in range(len(x))],
+                 [3] * len(x)).cpu().tolist()
+    for i in range(len(x)):
+        want, slack = PS.sample(x[i], uniform(i + 1, 3), temperature=0.7, top_k=k, **f)
+        assert got[i] == want or slack < 1e-5, (V, k, i, got[i], want, slack)
