@@ -19,10 +19,18 @@
 #define SAMPLE_MAX_CAND 1024
 #define SAMPLE_SHORT_K 600                   // the largest k of a long row whose candidates are looked for the short way first
 
+// Ascending in the float order, -0 below 0, and a NaN (of either sign) below everything: it is never a candidate while there
+// are k others, and counts as -inf where it is one, as argmax passes it over too.  By an exclusive or: of "u | sign" a
+// compiler may make -|f|, an operation on floats that need not keep a NaN's bits.  Written so, a NaN's key was 0xffc00000 by
+// itself and yet not the maximum of the loop below, and a row with a NaN could have one threshold by its counts, another by its
+// comparisons and candidates that nobody had written.
 __device__ __forceinline__ unsigned int order_key(float f) {
-    unsigned int u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);   // ascending in the float order
+    const int u = __float_as_int(f);
+    const unsigned int key = (unsigned int)(u ^ ((u >> 31) | (int)0x80000000));
+    return key > 0xff800000u ? 0u : key;                 // (0xff800000: +inf; a NaN with its sign set lies below -inf already)
 }
+// what stands for a candidate in the sort
+__device__ __forceinline__ float cand_value(float f) { return f != f ? -INFINITY : f; }
 
 // ---- repeat penalty: each occurrence of a token among `recent` divides a
 // positive logit by the penalty or multiplies a non-positive one (:205-216)
@@ -155,21 +163,18 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
     // First without a selection over the whole row: every thread's largest key; at least k keys are as large as the k-th
     // of these 1024, so the row's k largest are among the keys that are, and for a k like 40 those are hardly more than k.
     // The row is read once, and again by the threads whose largest key passes.  What bounds it is the one SM that reads
-    // a row.  Where more than 1024 pass (many equal values), and for rows with NaN or a -0 among the candidates, whose order
-    // the selection below defines, that runs instead.  It runs at once for a k above SAMPLE_SHORT_K in a row longer than the
+    // a row.  Where more than 1024 pass (many equal values), and where a NaN or a -0 is among them, whose order the selection
+    // below defines, that runs instead.  It runs at once for a k above SAMPLE_SHORT_K in a row longer than the
     // threads are many: of a long row some -1024 ln(1 - k/1024) keys pass, 710 at 512 and more than 1024 from 650 on.
     // Measured at 8 rows of 65536, us, with the selection | so: normal values, k = 40 168 | 27, 512 184 | 50, 600 187 | 53;
     // above the line the attempt would add 9 to 19 us to the selection (top-p alone, k = 1024: 201 | 210 before that line was
-    // drawn, 161 now that the selection's counts read eight values at a time); a row masked but for 20 values 162 | 147.
+    // drawn, 171 now that the selection's counts read eight values at a time); a row masked but for 20 values 162 | 155.
     int n_cand = SAMPLE_MAX_CAND + 1;
     if (k <= SAMPLE_SHORT_K || V <= SAMPLE_THREADS) {
         unsigned int best = 0;
-        bool odd = false;
 #pragma unroll 8
         for (int i = tid; i < V; i += SAMPLE_THREADS) {
-            const float v = l[i];
-            odd |= v != v;
-            best = max(best, order_key(v));
+            best = max(best, order_key(l[i]));
         }
         unsigned int t = 0;
         if (tid == 0) { s_result = 0; s_kleft = 0; }
@@ -177,7 +182,6 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
             const unsigned int c = t | (1u << bit);
             if (__syncthreads_count(best >= c) >= k) t = c;
         }
-        if (odd) s_kleft = 1;
         // (where the k-th value stands at many threads, as in a row that is masked but for fewer than k, too many keys pass)
         const int passing = __syncthreads_count(best >= t);
         if (passing > (k + SAMPLE_THREADS) / 2 && V > SAMPLE_THREADS) {
@@ -189,7 +193,7 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
                 if (order_key(v) >= t) {
                     const int at = atomicAdd(&s_result, 1);
                     if (at < SAMPLE_MAX_CAND) { c_val[at] = v; c_idx[at] = i; }
-                    if (__float_as_uint(v) == 0x80000000u) s_kleft = 1;
+                    if (v != v || __float_as_uint(v) == 0x80000000u) s_kleft = 1;
                 }
             }
         }
@@ -259,9 +263,9 @@ sample_rows_kernel(const float* __restrict__ logits, int V, const float* __restr
         for (int i = b; i < e; i++) {
             const float v = l[i];
             const unsigned int key = order_key(v);
-            if (key > thr) { c_val[pg] = v; c_idx[pg] = i; pg++; }
+            if (key > thr) { c_val[pg] = v; c_idx[pg] = i; pg++; }           // (no NaN is above anything)
             else if (key == thr) {
-                if (pe < n_eq_keep) { c_val[n_gt + pe] = v; c_idx[n_gt + pe] = i; }
+                if (pe < n_eq_keep) { c_val[n_gt + pe] = cand_value(v); c_idx[n_gt + pe] = i; }
                 pe++;
             }
         }

@@ -66,3 +66,21 @@ def test_rows_on_either_side_of_the_short_way(V, k):
     for i in range(len(x)):
         want, slack = PS.sample(x[i], uniform(i + 1, 3), temperature=0.7, top_k=k, **f)
         assert got[i] == want or slack < 1e-5, (V, k, i, got[i], want, slack)
+
+
+@pytest.mark.parametrize("V,k", [(65536, 4), (65536, 40), (65536, 601), (65536, 0), (1025, 200), (1000, 0), (500, 3)])
+@pytest.mark.parametrize("kind", ["one", "several", "negative", "most"])
+def test_a_nan_counts_as_minus_infinity(V, k, kind):
+    """... in every row alike: 64 rows of the same values, a uniform number each."""
+    from kappai_b200 import SamplingParams
+    from kappai_b200.sampling import uniform
+    from kappai_b200.sampling.sampler import sample
+    x = np.random.default_rng(V).standard_normal(V).astype(np.float32)
+    at = {"one": [V // 3], "several": [1, V // 3, int(np.argmax(x)), V - 2], "negative": [V // 3], "most": list(range(2, V))}[kind]
+    x[at] = np.array([0xffc00001 if kind == "negative" else 0x7fc00000], np.uint32).view(np.float32)[0]
+    plain = np.where(np.isnan(x), np.float32(-np.inf), x)
+    for f in (dict(top_p=1.0, min_p=0.01), dict(top_p=0.9, min_p=0.0)):
+        got = sample(torch.from_numpy(np.tile(x, (64, 1))).cuda(), [SamplingParams(temperature=0.7, top_k=k, **f)] * 64, list(range(64)), [3] * 64)
+        for i, tok in enumerate(got.cpu().tolist()):
+            want, slack = PS.sample(plain, uniform(i, 3), temperature=0.7, top_k=k, **f)
+            assert tok == want or slack < 1e-5, (i, tok, want, slack)
