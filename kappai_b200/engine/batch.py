@@ -167,8 +167,20 @@ def lay_out_step(segments: Sequence[Segment], groups: Dict[Hashable, int], vocab
                 raise BatchError(f"request {s.req!r}: wanted index {w} outside its {n} tokens")
     n_rows = sum(seg_len)
 
-    # rows by arrays over all segments (a step may have hundreds of one row)
-    ids = np.asarray([t for s in segments for t in s.tokens], dtype=np.int64)
+    # rows by arrays over all segments (a step may have hundreds of one row), long segments by themselves: of 2,048 tokens an
+    # array takes 1 us so and 165 element by element, a list 60 and 78
+    pieces, few = [], []
+    for s, n in zip(segments, seg_len):
+        if n <= 32:
+            few.extend(s.tokens)
+            continue
+        if few:
+            pieces.append(np.asarray(few, dtype=np.int64))
+            few = []
+        pieces.append(np.asarray(s.tokens, dtype=np.int64))
+    if few:
+        pieces.append(np.asarray(few, dtype=np.int64))
+    ids = pieces[0] if len(pieces) == 1 else np.concatenate(pieces)
     lens = np.asarray(seg_len, dtype=np.int64)
     cu_rows = np.zeros(n_seg + 1, np.int32)
     np.cumsum(lens, out=cu_rows[1:])

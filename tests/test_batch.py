@@ -111,3 +111,26 @@ def test_refusals():
         build_step_context([seg("a", 5, 0, 0, want=[5])], {"g": 16}, CPU, 10, 64)
     with pytest.raises(BatchError):                                   # two segments, one state slot
         build_step_context([seg("a", 2, 0, 0), seg("b", 2, 0, 0)], {"g": 16}, CPU, 10, 64)
+
+
+def test_tokens_of_any_kind_of_sequence_and_long_arrays_at_once():
+    class Whole(np.ndarray):
+        def __iter__(self):
+            raise AssertionError("a long array is taken whole")
+
+    kinds = [lambda t: t, tuple, np.asarray, lambda t: np.asarray(t, dtype=np.int32), torch.tensor, lambda t: range(t[0], t[-1] + 1)]
+    lens = [1, 33, 1, 2, 32, 40, 1, 1, 700]
+    segs, want = [], []
+    for i, n in enumerate(lens):
+        tokens = list(range(7 * i, 7 * i + n))
+        want += tokens
+        s = seg(i, n, 0, i)
+        s.tokens = kinds[i % len(kinds)](tokens)
+        segs.append(s)
+    assert build_step_context(segs, {"g": 16}, CPU, 1000, 4096).token_ids.tolist() == want
+    s = seg("a", 2048, 0, 0)
+    s.tokens = np.arange(2048).view(Whole)
+    assert build_step_context([s], {"g": 16}, CPU, 4096, 4096).token_ids.tolist() == list(range(2048))
+    s.tokens = np.arange(2048) + 2000
+    with pytest.raises(BatchError, match="token id 3000 outside the vocabulary of 3000"):
+        build_step_context([s], {"g": 16}, CPU, 3000, 4096)
