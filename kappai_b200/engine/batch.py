@@ -226,7 +226,7 @@ def lay_out_step(segments: Sequence[Segment], groups: Dict[Hashable, int], vocab
             if len(t) < need:
                 raise BatchError(f"request {s.req!r}: block table covers {len(t)} blocks, {need} needed")
             bt[i, :len(t)] = t
-            slots += ts
+            slots.extend(ts)                   # (an array added to a list would be a sum)
         sm = np.asarray(slots, dtype=np.int32)
         paged_host[gk] = (len(parts), bt.shape, page_size)
         parts.append(bt.reshape(-1))

@@ -134,3 +134,12 @@ def test_tokens_of_any_kind_of_sequence_and_long_arrays_at_once():
     s.tokens = np.arange(2048) + 2000
     with pytest.raises(BatchError, match="token id 3000 outside the vocabulary of 3000"):
         build_step_context([s], {"g": 16}, CPU, 3000, 4096)
+
+
+@pytest.mark.parametrize("kind", [list, tuple, np.asarray])
+def test_token_slots_of_any_kind_of_sequence(kind):
+    segs = [seg("a", 1, 20, 0), seg("b", 5, 3, 1), seg("c", 1, 0, 2), seg("d", 40, 16, 3)]
+    want = [x for s in segs for x in s.token_slots["g"]]
+    for s in segs:
+        s.token_slots = {"g": kind(s.token_slots["g"])}
+    assert build_step_context(segs, {"g": 16}, CPU, 1000, 4096).paged["g"].slot_map.tolist() == want
