@@ -1577,16 +1577,15 @@ EPI_ACT = 6
 
 
 def _rows_16_bytes(t: torch.Tensor) -> bool:
-    """Is every row of a 2-D bfloat16 tensor contiguous and 16-byte aligned?"""
-    ld, one = t.stride()
-    return one == 1 and ld % 8 == 0 and t.data_ptr() % 16 == 0
+    """Is it a 2-D tensor of bfloat16 whose every row is contiguous and 16-byte aligned?"""
+    s = t.stride()
+    return t.dtype == torch.bfloat16 and len(s) == 2 and s[1] == 1 and s[0] % 8 == 0 and t.data_ptr() % 16 == 0
 
 
 def skinny_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Can the weight-streaming kernel take this product?"""
-    M, K = a.shape
-    return (M <= SKINNY_MAX_M and K % 32 == 0 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-            and _rows_16_bytes(a) and _rows_16_bytes(w))
+    s = a.shape
+    return len(s) == 2 and s[0] <= SKINNY_MAX_M and s[1] % 32 == 0 and _rows_16_bytes(a) and _rows_16_bytes(w)
 
 
 USE_TC = True              # bfloat16 products of more than 64 rows (and some of fewer) run on tcgen05 tensor cores
@@ -1613,8 +1612,7 @@ def tc_pays_for_few_rows(M: int, N: int, swiglu: bool) -> bool:
 
 def tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Can the tcgen05 kernel take this product (bfloat16, 16-byte aligned rows, K a multiple of 8)?"""
-    return (USE_TC and a.shape[1] % 8 == 0 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-            and _rows_16_bytes(a) and _rows_16_bytes(w))
+    return USE_TC and _rows_16_bytes(a) and _rows_16_bytes(w) and a.shape[1] % 8 == 0
 
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
