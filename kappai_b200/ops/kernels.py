@@ -1692,8 +1692,8 @@ def stream_pays(N: int, K: int) -> bool:
 def rows_pays(M: int, N: int) -> bool:
     """Up to 8 rows go to csrc/gemm_rows.cu, the same sums in the same order: of the layer products all, of a 65536-row head
     one row (x 1024 29.3 -> 24.7 us, x 2048 42.6 -> 43.6, and it brings its first weights in before the wait on the norm; at
-    8 rows 30.9 | 31.0 and 48.6 | 51.6)."""
-    return M <= ROWS_MAX_M and (N <= 16384 or M == 1)
+    8 rows 30.9 | 31.0 and 48.6 | 51.6).  In between (24576 x 2048, one row 17.9 | 20.1) the register-streaming kernel stays."""
+    return M <= ROWS_MAX_M and (N <= 16384 or (M == 1 and N >= 32768))
 
 
 CONV_STEP_MAX_M = 16       # rows up to which the conv step runs in in_proj's epilogue (measured: batch 8 703 -> 672 us a
