@@ -99,7 +99,7 @@ struct StreamArgs {
 // shared memory: [ring: n_stages x NW*8 rows x ST_ROW_BYTES][full[n_stages]][empty[n_stages]][red]
 // WIDE (more than 16 batch rows, no SwiGLU): a tile is 16 rows of W, so that an activation fragment, whose
 // loads weigh more than the weights' once there are several m-tiles, serves two n-tiles.
-template <int MT, bool HALF, int EPI, bool WIDE>
+template <int MT, int EPI, bool WIDE>
 __global__ void __launch_bounds__(ST_THREADS)
 gemm_stream_kernel(const StreamArgs p) {
     constexpr int NW = EPI == EPI_CONV_STEP ? 3 : ((EPI == EPI_SWIGLU || WIDE) ? 2 : 1);
@@ -175,9 +175,8 @@ gemm_stream_kernel(const StreamArgs p) {
     auto load_acts = [&](uint4 (&lo)[MT], uint4 (&hi)[MT], int kb) {
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
-            hi[mt] = make_uint4(0, 0, 0, 0);
             lo[mt] = __ldg(reinterpret_cast<const uint4*>(p.A + (size_t)r0[mt] * p.lda) + kb * 4 + t);
-            if (!HALF) hi[mt] = __ldg(reinterpret_cast<const uint4*>(p.A + (size_t)r1[mt] * p.lda) + kb * 4 + t);
+            hi[mt] = __ldg(reinterpret_cast<const uint4*>(p.A + (size_t)r1[mt] * p.lda) + kb * 4 + t);
         }
     };
 
@@ -365,7 +364,7 @@ static int launch_pdl(Kern kern, dim3 grid, size_t smem, cudaStream_t s, const S
     return (int)kp_launch_pdl(kern, grid, dim3(ST_THREADS), smem, s, a);
 }
 
-template <int MT, bool HALF>
+template <int MT>
 static int launch_epi(StreamArgs a, int epi, cudaStream_t s) {
     // tiles of 16 rows of W from three m-tiles on (see the kernel; measured at 64 batch rows: 2048 x 5632 15.5 us
     // against 23.7, 2048 x 2048 8.0 against 12.2; at 32 rows the narrow tile is as fast or faster)
@@ -387,25 +386,24 @@ static int launch_epi(StreamArgs a, int epi, cudaStream_t s) {
     dim3 grid(g);
     const size_t sm = smem_bytes(NW, MT, a.n_stages);
     switch (epi) {
-        case EPI_STORE: return launch_pdl(gemm_stream_kernel<MT, HALF, EPI_STORE, WIDE>, grid, sm, s, a);
-        case EPI_STORE_F32: return launch_pdl(gemm_stream_kernel<MT, HALF, EPI_STORE_F32, WIDE>, grid, sm, s, a);
-        case EPI_ACCUM_F32: return launch_pdl(gemm_stream_kernel<MT, HALF, EPI_ACCUM_F32, WIDE>, grid, sm, s, a);
-        case EPI_SWIGLU: return launch_pdl(gemm_stream_kernel<MT, HALF, EPI_SWIGLU, false>, grid, sm, s, a);
-        case EPI_ACT: return launch_pdl(gemm_stream_kernel<MT, HALF, EPI_ACT, WIDE>, grid, sm, s, a);
+        case EPI_STORE: return launch_pdl(gemm_stream_kernel<MT, EPI_STORE, WIDE>, grid, sm, s, a);
+        case EPI_STORE_F32: return launch_pdl(gemm_stream_kernel<MT, EPI_STORE_F32, WIDE>, grid, sm, s, a);
+        case EPI_ACCUM_F32: return launch_pdl(gemm_stream_kernel<MT, EPI_ACCUM_F32, WIDE>, grid, sm, s, a);
+        case EPI_SWIGLU: return launch_pdl(gemm_stream_kernel<MT, EPI_SWIGLU, false>, grid, sm, s, a);
+        case EPI_ACT: return launch_pdl(gemm_stream_kernel<MT, EPI_ACT, WIDE>, grid, sm, s, a);
         case EPI_CONV_STEP:
             // at most 16 rows: from 32 rows on the tensor-core kernel and the separate conv kernel are faster (measured)
-            if constexpr (MT == 1) return launch_pdl(gemm_stream_kernel<MT, HALF, EPI_CONV_STEP, false>, grid, sm, s, a);
+            if constexpr (MT == 1) return launch_pdl(gemm_stream_kernel<MT, EPI_CONV_STEP, false>, grid, sm, s, a);
             else return KP_ERR_UNSUPPORTED;
         default: return KP_ERR_BAD_ARG;
     }
 }
 
 static int launch_m(const StreamArgs& a, int epi, cudaStream_t s) {
-    if (a.M <= 8) return launch_epi<1, true>(a, epi, s);
-    if (a.M <= 16) return launch_epi<1, false>(a, epi, s);
-    if (a.M <= 32) return launch_epi<2, false>(a, epi, s);
-    if (a.M <= 48) return launch_epi<3, false>(a, epi, s);
-    return launch_epi<4, false>(a, epi, s);
+    if (a.M <= 16) return launch_epi<1>(a, epi, s);          // (up to 8 rows run on gemm_rows.cu: kernels.rows_pays)
+    if (a.M <= 32) return launch_epi<2>(a, epi, s);
+    if (a.M <= 48) return launch_epi<3>(a, epi, s);
+    return launch_epi<4>(a, epi, s);
 }
 
 static int check_common(StreamArgs& a, int M, int N, int K, int ldw, const void* W, int epi) {

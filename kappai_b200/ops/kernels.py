@@ -1681,11 +1681,10 @@ def stream_fits(K: int, swiglu: bool) -> bool:
 
 
 def stream_pays(N: int, K: int) -> bool:
-    """Measured on B200 (8 rows, back to back in a graph): the bulk-copy kernel wins or ties with the
-    register-streaming kernel for the layer products (6144 x 2048: 8.0 against 8.1 us; gate/up 11264 x 2048:
-    9.5 against 16.0; 2048 x 5632: 10.2 against 8.9; 2048 x 2048: 4.6 against 4.4) and, because its producer
-    fills the ring before it waits for the kernel before it, overlaps that kernel's tail inside a model step.
-    It loses on the huge grid of a 65536-row head (65 against 48 us)."""
+    """For the layer products of 9 to 16 rows (fewer: :func:`rows_pays`; more run on tcgen05).  Measured on B200 (16 rows, back to
+    back in a graph) against the register-streaming kernel: 6144 x 2048 7.4 us against 9.2, 2048 x 5632 8.4 against 8.8, 2048 x 2048
+    4.1 each, 1024 x 4608 5.9 against 6.7; gated 6144 x 2048 5.8 against 8.6.  Its producer also fills the ring before it waits for
+    the kernel before it, and overlaps that kernel's tail inside a model step.  Wider products are a head's, which runs on tcgen05."""
     return N <= 16384
 
 
@@ -1729,7 +1728,7 @@ def gemm_stream_conv_step(a: torch.Tensor, w_in: torch.Tensor, bias: Optional[to
                 raise KernelError(f"gemm_stream_conv_step: {nm} size")
     few = M <= ROWS_MAX_M
     lib = load_library("gemm_rows" if few else "gemm_stream")
-    _run_gemm("gemm_stream_conv_step", lib.kp_gemm_rows_conv_step if few else lib.kp_gemm_stream_conv_step, a, w_in, out, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
+    _run_gemm("gemm_rows_conv_step" if few else "gemm_stream_conv_step", lib.kp_gemm_rows_conv_step if few else lib.kp_gemm_stream_conv_step, a, w_in, out, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
          _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, _ptr(conv_w), _ptr(conv_bias), _ptr(state), _ptr(seg_pos),
          _ptr(seg_slot), conv_k, STREAM)
     return out
@@ -1813,7 +1812,7 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optio
     consts = _glu_floats(glu) if swiglu and glu is not None else ()
     if USE_STREAM and stream_fits(K, swiglu) and rows_pays(M, N):
         lib = load_library("gemm_rows")
-        _run_gemm("gemm_stream", lib.kp_gemm_rows, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
+        _run_gemm("gemm_rows", lib.kp_gemm_rows, a, w, out, _ptr(a), _rows_2d(a, "a"), _ptr(w), _rows_2d(w, "w"), _ptr(bias), _ptr(out),
              _rows_2d(out, "out"), M, N, K, epi, *(consts or _NO_LIMITS), STREAM)
         return out
     if USE_STREAM and stream_fits(K, swiglu) and stream_pays(N, K) and M <= STREAM_MAX_M:
