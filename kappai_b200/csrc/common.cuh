@@ -206,12 +206,15 @@ static inline cudaError_t kp_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim
 // Lets `kern` have up to `bytes` of dynamic shared memory a CTA, once a device (`ready`: a bit for each that it is done on).
 // The limit belongs to the function, not to a launch: `bytes` is the most that any launch of it may ask for, so that
 // launches of different sizes from several threads cannot lower it for one another.
+// `beside`: the SM is to give all it can to shared memory, not just what this kernel's own CTAs need, so that another kernel's
+// CTA fits beside one of this.
 template <typename Kern>
-static inline int kp_smem_limit(Kern kern, size_t bytes, std::atomic<unsigned long long>& ready) {
+static inline int kp_smem_limit(Kern kern, size_t bytes, std::atomic<unsigned long long>& ready, bool beside = false) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev <= 63 && ((ready.load(std::memory_order_relaxed) >> dev) & 1)) return 0;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess && beside) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess && dev <= 63) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
     return (int)e;
 }

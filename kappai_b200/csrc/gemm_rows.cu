@@ -15,12 +15,21 @@
 //    lanes of a quarter warp read all banks once.
 //  * At a tile's end the warps' partial sums are added in warp order from zero.  The order of every sum is that of
 //    gemm_stream.cu, so a row's result does not depend on which of the two ran.
+//  * Behind an RMS norm (the normed form) a CTA brings the float32 rows in itself: a warp its own columns, times the norm's
+//    weight, rounded to bfloat16 and held beside the rings for all the CTA's tiles; the sums are multiplied by 1 / rms where
+//    they leave.  So no launch stands between the product in front and this one.  (Left to the product in front -- it
+//    writes the weighted rows and sums of squares, this one reads both -- a step took 3 % longer.)
 //
 // Measured back to back, us, gemm_stream | this, one row and 8: 2048 x 5632 7.8 | 6.5, 7.9 | 7.1; 6144 x 2048 6.8 | 5.2,
-// 6.9 | 5.7; 2048 x 2048 3.8 | 2.6, 3.8 | 2.8; at 16 rows it loses (8.2 | 9.0), as A then weighs as much as W.  A decode
-// step of the 1.2B shape: one request 601 -> 506 us, eight 607 -> 550; of the 350M shape 376 -> 343.  One CTA must have an
-// SM to itself: with rings of 100 KB two fit, the next product's CTAs come in early and unevenly, two on some SMs and none
-// on others, and a step takes 613 us.  Rings of 122 KB 524, 155 KB 506, 190 KB 511, 210 KB 542.
+// 6.9 | 5.7; 2048 x 2048 3.8 | 2.6, 3.8 | 2.8; at 16 rows it loses (8.2 | 9.0), as A then weighs as much as W.
+//
+// Two CTAs an SM, of two products that follow one another: the next product's rings fill while this one still streams.  That
+// pays only if every SM gets one of each, so accumulating products have small CTAs and the others, between which they
+// stand, big ones of more than half an SM; and only if the SM's split between cache and shared memory allows it (it is
+// set for the kernel that comes first: without the preference asked for in kp_smem_limit the second never came in).
+// A decode step of one request, us, norms apart | norms inside | and two CTAs an SM: 1.2B shape 511 | 475 | 459, 350M 341 |
+// 335 | 312; of eight requests (see rows_run) 555 | 539 | 567 and 369 | 378 | 366.
+// Big and small, KB, 64 steps of one request, 1.2B shape, ms: 148 + 78 32.1, 128 + 96 31.9, 116 + 110 32.2, 164 + 62 33.2.
 //
 // Epilogues as in gemm_stream.cu.  K a multiple of 512.
 #include "mma.cuh"
@@ -33,8 +42,12 @@
 #define EPI_ACT 6
 
 #define RW_WARPS 8
-#define RW_SMEM (155 * 1024)                 // shared memory of the rings: more than half an SM's, see above
-#define RW_MAX_STAGES 8
+#define RW_NORM_MAX_K 4096                   // columns up to which the normed form holds A (8 rows: 64 KB)
+// Shared memory of a CTA: with a big ring, with a small ring, and of one that has the SM to itself.
+#define RW_BIG (128 * 1024)
+#define RW_SMALL (96 * 1024)
+#define RW_ALONE (155 * 1024)
+#define RW_MAX_STAGES 12
 
 struct RowsArgs {
     const bf16* A; int lda;
@@ -47,17 +60,32 @@ struct RowsArgs {
     const float* conv_w; const float* conv_bias; float* conv_state;
     const int* seg_pos; const int* seg_slot;
     int conv_k;
+    const float* X; int ldx;                 // the normed form: float32 rows, the norm's weight and eps
+    const float* gamma; float eps;
 };
 
-// WR: rows of W a tile (8, 16, or 24: the conv step).
-template <int WR, int EPI>
+// How a launch runs.  WR: rows of W a tile (8, 16, or 24: the conv step).  R: rows of A that are kept, at least M (1, 4 or 8).
+// NORM: A is normed by the kernel and held beside the rings, which are of W alone.  ROOM: a size of the three above.
+template <int WR, int R, bool NORM, int ROOM> struct RowsShape {
+    static constexpr int MT = (WR + 15) / 16;                            // m16 tiles (of a 24-row tile's second one half is empty)
+    static constexpr int W_BYTES = WR * 128, STAGE = W_BYTES + (NORM ? 0 : R * 128);
+    static constexpr int SUMS = 2 * RW_WARPS * MT * 128 * 4 + RW_WARPS * 8 * 4;
+    static constexpr int FIT = (ROOM - SUMS - (NORM ? 2048 * 2 * R : 0)) / (RW_WARPS * STAGE);
+    static constexpr int S = FIT > RW_MAX_STAGES ? RW_MAX_STAGES : FIT;  // ring stages of a warp
+    static_assert(S >= 2, "a ring of two stages at least");
+    static constexpr size_t bytes(int K) {
+        const size_t need = (size_t)RW_WARPS * S * STAGE + SUMS + (NORM ? (size_t)K * 2 * R : 0);
+        return ROOM != RW_SMALL && need < ROOM ? (size_t)ROOM : need;   // (more than half an SM: two of one product never share one)
+    }
+};
+
+template <int WR, int EPI, int R, bool NORM, int ROOM>
 __global__ void __launch_bounds__(RW_WARPS * 32, 1)
 gemm_rows_kernel(const RowsArgs p) {
-    constexpr int MT = (WR + 15) / 16;                                   // m16 tiles (of a 24-row tile's second one half is empty)
+    using Shape = RowsShape<WR, R, NORM, ROOM>;
+    constexpr int MT = Shape::MT, W_BYTES = Shape::W_BYTES, STAGE = Shape::STAGE, S = Shape::S;
     constexpr int JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
     constexpr int TROWS = WR / JOINS;                                    // output columns a tile
-    constexpr int W_BYTES = WR * 128, STAGE = W_BYTES + 8 * 128;
-    constexpr int S = RW_SMEM / (RW_WARPS * STAGE) > RW_MAX_STAGES ? RW_MAX_STAGES : RW_SMEM / (RW_WARPS * STAGE);
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
@@ -65,6 +93,10 @@ gemm_rows_kernel(const RowsArgs p) {
     const int n_tiles = (n_out + TROWS - 1) / TROWS, n_ch = p.K / 512;   // chunks of 64 columns a warp and tile
     unsigned char* ring = smem + (size_t)warp * S * STAGE;
     float* red = reinterpret_cast<float*>(smem + (size_t)RW_WARPS * S * STAGE);   // [2][warp][MT][4][32]
+    // (NORM) the squares' sums [warp][8], then for every warp its columns of A [chunk][row][64], laid out as a stage's
+    float* squares = red + 2 * RW_WARPS * MT * 128;
+    unsigned char* held = reinterpret_cast<unsigned char*>(squares + RW_WARPS * 8) + (size_t)warp * n_ch * (R * 128);
+    const int ga = g < R ? g : R - 1;                                    // the row of A this lane's fragments are of
     const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - blockIdx.x - 1) / gridDim.x + 1 : 0;
     const int total = my_tiles * n_ch;
 
@@ -84,7 +116,7 @@ gemm_rows_kernel(const RowsArgs p) {
     auto load_a = [&](int c, int s) {
         unsigned char* dst = ring + (size_t)s * STAGE + W_BYTES;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < (R + 3) / 4; i++) {
             const int row = i * 4 + cr;
             if (row < M) cp_async16(dst + row * 128 + ((cc ^ ((row & 1) << 2)) * 16), p.A + (size_t)row * p.lda + c * 512 + col0, true);
         }
@@ -100,14 +132,63 @@ gemm_rows_kernel(const RowsArgs p) {
         if (i < total) { load_w(ld_tile, ld_c, ld_s); advance(); }
         cp_async_commit();
     }
-    pdl_wait();
-    KP_TRACE_MARK(1);
-    for (int i = 0; i < S; i++) {
-        if (i < total) load_a(i % n_ch, i);
-        cp_async_commit();
+    if constexpr (NORM) {
+        // Half a warp a chunk: lane j of it has columns 4 j ... of the chunk's 64 (columns of A as load_a has them).
+        constexpr int CU = R >= 8 ? 2 : 4;                               // chunks a lane has in flight for each of R rows
+        const int half = lane >> 4, j = lane & 15;
+        const int colx = warp * 32 + (j >> 3) * 256 + (j & 7) * 4;
+        float4 gm[CU];
+#pragma unroll
+        for (int k = 0; k < CU; k++)
+            gm[k] = 2 * k + half < n_ch ? __ldg(reinterpret_cast<const float4*>(p.gamma + (2 * k + half) * 512 + colx)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float ss[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) ss[r] = 0.f;
+        pdl_wait();
+        KP_TRACE_MARK(1);
+        for (int c0 = 0; c0 < n_ch; c0 += 2 * CU) {
+            float4 v[R][CU];
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int k = 0; k < CU; k++) {
+                    const int c = c0 + 2 * k + half;
+                    v[r][k] = r < M && c < n_ch ? *reinterpret_cast<const float4*>(p.X + (size_t)r * p.ldx + c * 512 + colx) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            if (c0 > 0) {
+#pragma unroll
+                for (int k = 0; k < CU; k++)
+                    gm[k] = c0 + 2 * k + half < n_ch ? __ldg(reinterpret_cast<const float4*>(p.gamma + (c0 + 2 * k + half) * 512 + colx)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int k = 0; k < CU; k++) {
+                    const int c = c0 + 2 * k + half;
+                    const float4 x = v[r][k], g4 = gm[k];
+                    ss[r] = fmaf(x.x, x.x, ss[r]); ss[r] = fmaf(x.y, x.y, ss[r]); ss[r] = fmaf(x.z, x.z, ss[r]); ss[r] = fmaf(x.w, x.w, ss[r]);
+                    if (r < M && c < n_ch)
+                        *reinterpret_cast<uint2*>(held + (size_t)c * (R * 128) + r * 128 + (((j >> 1) ^ ((r & 1) << 2)) * 16) + (j & 1) * 8) =
+                            make_uint2(pack_bf16(x.x * g4.x, x.y * g4.y), pack_bf16(x.z * g4.z, x.w * g4.w));
+                }
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const float q = warp_sum(ss[r]);
+            if (lane == r) squares[warp * 8 + r] = q;
+        }
+        __syncwarp();
+    } else {
+        pdl_wait();
+        KP_TRACE_MARK(1);
+        for (int i = 0; i < S; i++) {
+            if (i < total) load_a(i % n_ch, i);
+            cp_async_commit();
+        }
     }
 
     int s = 0, buf = 0;
+    float scale = 1.f;                                                   // (NORM) 1 / root mean square of this thread's row
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
         const int n0 = tile * TROWS;
         // what the epilogue needs beside the sums is asked for now: its trips to L2 run under the main loop
@@ -143,7 +224,7 @@ gemm_rows_kernel(const RowsArgs p) {
                 uint4 w[2 * MT];
 #pragma unroll
                 for (int i = 0; i < 2 * MT; i++) w[i] = i * 8 < WR ? *reinterpret_cast<const uint4*>(st + (i * 8 + g) * 128 + at) : make_uint4(0, 0, 0, 0);
-                const uint4 x = *reinterpret_cast<const uint4*>(st + W_BYTES + g * 128 + at);   // (rows beyond M: any values, nobody reads their sums)
+                const uint4 x = *reinterpret_cast<const uint4*>((NORM ? held + (size_t)c * (R * 128) : st + W_BYTES) + ga * 128 + ((b * 4 + t) ^ ((ga & 1) << 2)) * 16);   // (rows beyond M: any values, nobody reads their sums)
 #pragma unroll
                 for (int a = 0; a < MT; a++) {
                     mma_bf16(acc[a], w[2 * a].x, w[2 * a + 1].x, w[2 * a].y, w[2 * a + 1].y, x.x, x.y);
@@ -151,7 +232,11 @@ gemm_rows_kernel(const RowsArgs p) {
                 }
             }
             __syncwarp();                                                // the stage has been read
-            if (ld_tile < n_tiles) { load_w(ld_tile, ld_c, ld_s); load_a(ld_c, ld_s); advance(); }
+            if (ld_tile < n_tiles) {
+                load_w(ld_tile, ld_c, ld_s);
+                if (!NORM) load_a(ld_c, ld_s);
+                advance();
+            }
             cp_async_commit();
             if (++s == S) s = 0;
         }
@@ -162,6 +247,12 @@ gemm_rows_kernel(const RowsArgs p) {
 #pragma unroll
             for (int i = 0; i < 4; i++) r[(warp * MT + a) * 128 + i * 32 + lane] = acc[a][i];
         __syncthreads();                                                 // (the other half of `red` is free: its readers were here)
+        if (NORM && tile == (int)blockIdx.x && om < M) {
+            float q = 0.f;
+#pragma unroll
+            for (int w8 = 0; w8 < RW_WARPS; w8++) q += squares[w8 * 8 + om];
+            scale = 1.0f / sqrtf(q / (float)p.K + p.eps);
+        }
         if (mine) {
             // the sum of W row `row` of the tile for this thread's batch row, over the warps in order
             auto sum_of = [&](int row) {
@@ -169,7 +260,7 @@ gemm_rows_kernel(const RowsArgs p) {
                 float v = 0.f;
 #pragma unroll
                 for (int w8 = 0; w8 < RW_WARPS; w8++) v += r[(w8 * MT + a) * 128 + i * 32 + l];
-                return v;
+                return NORM ? v * scale : v;
             };
             const int m = om, n = on, lr = on - n0;
             float v = sum_of(lr);
@@ -237,52 +328,63 @@ static int rw_n_sm() {
     return n;
 }
 
-template <int WR, int EPI>
+template <int WR, int EPI, int R, bool NORM, int ROOM>
 static int rows_launch(const RowsArgs& a, cudaStream_t s) {
-    constexpr int MT = (WR + 15) / 16, JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
-    constexpr int STAGE = WR * 128 + 8 * 128;
-    constexpr int S = RW_SMEM / (RW_WARPS * STAGE) > RW_MAX_STAGES ? RW_MAX_STAGES : RW_SMEM / (RW_WARPS * STAGE);
-    constexpr size_t smem = (size_t)RW_WARPS * S * STAGE + sizeof(float) * 2 * RW_WARPS * MT * 128;
-    auto kern = gemm_rows_kernel<WR, EPI>;
+    using Shape = RowsShape<WR, R, NORM, ROOM>;
+    constexpr int JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
+    auto kern = gemm_rows_kernel<WR, EPI, R, NORM, ROOM>;
     static std::atomic<unsigned long long> ready{0};
-    const int st = kp_smem_limit(kern, smem, ready);
+    const int st = kp_smem_limit(kern, Shape::bytes(RW_NORM_MAX_K), ready, true);
     if (st) return st;
     const int n_out = JOINS > 1 ? a.ff : a.N, n_tiles = (n_out + WR / JOINS - 1) / (WR / JOINS);
-    return (int)kp_launch_pdl(kern, dim3(n_tiles < rw_n_sm() ? n_tiles : rw_n_sm()), dim3(RW_WARPS * 32), smem, s, a);
+    return (int)kp_launch_pdl(kern, dim3(n_tiles < rw_n_sm() ? n_tiles : rw_n_sm()), dim3(RW_WARPS * 32), Shape::bytes(a.K), s, a);
 }
 
-static int rows_run(const RowsArgs& a, int epi, cudaStream_t s) {
+template <int R, bool NORM, int BIG, int SMALL>
+static int rows_run_r(const RowsArgs& a, int epi, cudaStream_t s) {
     // tiles of 8 rows where the busiest SM then has fewer rows of W (3072 rows: 24 against 32; 1024 rows: 8 against 16)
     const int sms = rw_n_sm();
     const auto busiest = [&](int rows) { return ((a.N + rows - 1) / rows + sms - 1) / sms * rows; };
     const bool narrow = busiest(8) < busiest(16);
-#define RW_PICK(EPI) return narrow ? rows_launch<8, EPI>(a, s) : rows_launch<16, EPI>(a, s)
+#define RW_PICK(EPI, ROOM) return narrow ? rows_launch<8, EPI, R, NORM, ROOM>(a, s) : rows_launch<16, EPI, R, NORM, ROOM>(a, s)
     switch (epi) {
-        case EPI_STORE: RW_PICK(EPI_STORE);
-        case EPI_STORE_F32: RW_PICK(EPI_STORE_F32);
-        case EPI_ACCUM_F32: RW_PICK(EPI_ACCUM_F32);
-        case EPI_ACT: RW_PICK(EPI_ACT);
-        case EPI_SWIGLU: return rows_launch<16, EPI_SWIGLU>(a, s);
-        case EPI_CONV_STEP: return rows_launch<24, EPI_CONV_STEP>(a, s);
+        case EPI_STORE: RW_PICK(EPI_STORE, BIG);
+        case EPI_STORE_F32: RW_PICK(EPI_STORE_F32, BIG);
+        case EPI_ACCUM_F32:
+            if constexpr (!NORM) RW_PICK(EPI_ACCUM_F32, SMALL);
+            return KP_ERR_BAD_ARG;
+        case EPI_ACT: RW_PICK(EPI_ACT, BIG);
+        case EPI_SWIGLU: return rows_launch<16, EPI_SWIGLU, R, NORM, BIG>(a, s);
+        case EPI_CONV_STEP: return rows_launch<24, EPI_CONV_STEP, R, NORM, BIG>(a, s);
         default: return KP_ERR_BAD_ARG;
     }
 #undef RW_PICK
 }
 
+// Two CTAs an SM or one (see the top).  With more than four rows A weighs as much as half of W, and two CTAs pay up to a residual of
+// 1024 columns only: a step of eight requests, us, two | one: 350M shape (1024 columns) 366 | 378, 1.2B shape (2048) 567 | 539;
+// of four requests 343 | 364 and 508 | 503.
+template <bool NORM>
+static int rows_run(const RowsArgs& a, int epi, cudaStream_t s) {
+    if (a.M == 1) return rows_run_r<1, NORM, RW_BIG, RW_SMALL>(a, epi, s);
+    if (a.M <= 4) return rows_run_r<4, NORM, RW_BIG, RW_SMALL>(a, epi, s);
+    const int residual = epi == EPI_ACCUM_F32 ? a.N : a.K;
+    return residual <= 1024 ? rows_run_r<8, NORM, RW_BIG, RW_SMALL>(a, epi, s) : rows_run_r<8, NORM, RW_ALONE, RW_ALONE>(a, epi, s);
+}
+
 static int rows_check(const RowsArgs& a) {
     if (a.M > 8 || a.K < 512 || (a.K % 512) || (a.lda & 7) || (a.ldw & 7) || ((uintptr_t)a.A & 15) || ((uintptr_t)a.W & 15))
         return KP_ERR_UNSUPPORTED;
+    if (a.gamma && (a.K > RW_NORM_MAX_K || (a.ldx & 3) || ((uintptr_t)a.X & 15) || ((uintptr_t)a.gamma & 15))) return KP_ERR_UNSUPPORTED;
     return 0;
 }
 
 extern "C" {
 
 // epi and glu as in gemm_stream.cu
-int kp_gemm_rows(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K,
-                 int epi, float limit, float alpha, float shift, void* stream) {
-    if (M <= 0 || N <= 0) return 0;
-    RowsArgs a = {};
-    a.A = (const bf16*)A; a.lda = lda; a.W = (const bf16*)W; a.ldw = ldw; a.bias = bias; a.C = C; a.ldc = ldc;
+static int rows_args(RowsArgs& a, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K, int& epi,
+                     float limit, float alpha, float shift) {
+    a.W = (const bf16*)W; a.ldw = ldw; a.bias = bias; a.C = C; a.ldc = ldc;
     a.M = M; a.N = N; a.K = K;
     a.act = KP_EPI_ACT(epi);
     epi = KP_EPI_KIND(epi);
@@ -294,9 +396,40 @@ int kp_gemm_rows(const void* A, int lda, const void* W, int ldw, const float* bi
         if (N & 1) return KP_ERR_BAD_ARG;
         a.ff = N / 2;
     }
-    int st = rows_check(a);
+    return rows_check(a);
+}
+
+int kp_gemm_rows(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K,
+                 int epi, float limit, float alpha, float shift, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    RowsArgs a = {};
+    a.A = (const bf16*)A; a.lda = lda;
+    const int st = rows_args(a, W, ldw, bias, C, ldc, M, N, K, epi, limit, alpha, shift);
+    return st ? st : rows_run<false>(a, epi, (cudaStream_t)stream);
+}
+
+// The product with A = the RMS norm of the float32 rows X (weight gamma): see the top.  Not with an accumulated output.
+int kp_gemm_rows_normed(const float* X, int ldx, const float* gamma, float eps, const void* W, int ldw, const float* bias, void* C,
+                        int ldc, int M, int N, int K, int epi, float limit, float alpha, float shift, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    RowsArgs a = {};
+    a.X = X; a.ldx = ldx; a.gamma = gamma; a.eps = eps;
+    if (!gamma) return KP_ERR_BAD_ARG;
+    const int st = rows_args(a, W, ldw, bias, C, ldc, M, N, K, epi, limit, alpha, shift);
+    return st ? st : rows_run<true>(a, epi, (cudaStream_t)stream);
+}
+
+static int conv_step_args(RowsArgs& a, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K, const float* conv_w,
+                          const float* conv_bias, float* conv_state, const int* seg_pos, const int* seg_slot, int conv_k) {
+    a.W = (const bf16*)W; a.ldw = ldw; a.bias = bias; a.C = C; a.ldc = ldc;
+    a.M = M; a.N = N; a.K = K; a.ff = N / 3;
+    if (N % 3) return KP_ERR_BAD_ARG;
+    const int st = rows_check(a);
     if (st) return st;
-    return rows_run(a, epi, (cudaStream_t)stream);
+    if (conv_k < 2 || conv_k > 16 || !conv_w || !conv_state || !seg_pos || !seg_slot) return KP_ERR_UNSUPPORTED;
+    a.conv_w = conv_w; a.conv_bias = conv_bias; a.conv_state = conv_state; a.seg_pos = seg_pos; a.seg_slot = seg_slot;
+    a.conv_k = conv_k;
+    return 0;
 }
 
 // The in_proj of the gated short convolution with the conv step of a decode step in its epilogue: W = [B; C; X]
@@ -307,15 +440,21 @@ int kp_gemm_rows_conv_step(const void* A, int lda, const void* W, int ldw, const
                            const int* seg_slot, int conv_k, void* stream) {
     if (M <= 0 || N <= 0) return 0;
     RowsArgs a = {};
-    a.A = (const bf16*)A; a.lda = lda; a.W = (const bf16*)W; a.ldw = ldw; a.bias = bias; a.C = C; a.ldc = ldc;
-    a.M = M; a.N = N; a.K = K; a.ff = N / 3;
-    if (N % 3) return KP_ERR_BAD_ARG;
-    int st = rows_check(a);
-    if (st) return st;
-    if (conv_k < 2 || conv_k > 16 || !conv_w || !conv_state || !seg_pos || !seg_slot) return KP_ERR_UNSUPPORTED;
-    a.conv_w = conv_w; a.conv_bias = conv_bias; a.conv_state = conv_state; a.seg_pos = seg_pos; a.seg_slot = seg_slot;
-    a.conv_k = conv_k;
-    return rows_run(a, EPI_CONV_STEP, (cudaStream_t)stream);
+    a.A = (const bf16*)A; a.lda = lda;
+    const int st = conv_step_args(a, W, ldw, bias, C, ldc, M, N, K, conv_w, conv_bias, conv_state, seg_pos, seg_slot, conv_k);
+    return st ? st : rows_run<false>(a, EPI_CONV_STEP, (cudaStream_t)stream);
+}
+
+// The same behind an RMS norm of the float32 rows X (see kp_gemm_rows_normed).
+int kp_gemm_rows_conv_step_normed(const float* X, int ldx, const float* gamma, float eps, const void* W, int ldw, const float* bias,
+                                  void* C, int ldc, int M, int N, int K, const float* conv_w, const float* conv_bias, float* conv_state,
+                                  const int* seg_pos, const int* seg_slot, int conv_k, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    RowsArgs a = {};
+    a.X = X; a.ldx = ldx; a.gamma = gamma; a.eps = eps;
+    if (!gamma) return KP_ERR_BAD_ARG;
+    const int st = conv_step_args(a, W, ldw, bias, C, ldc, M, N, K, conv_w, conv_bias, conv_state, seg_pos, seg_slot, conv_k);
+    return st ? st : rows_run<true>(a, EPI_CONV_STEP, (cudaStream_t)stream);
 }
 
 }  // extern "C"

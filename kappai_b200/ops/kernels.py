@@ -1702,16 +1702,21 @@ CONV_STEP_MAX_M = 16       # rows up to which the conv step runs in in_proj's ep
 def conv_step_fusable(a: torch.Tensor, w_in: torch.Tensor, conv_k: int) -> bool:
     """Can the weight-streaming kernel run the conv step of a decode step in in_proj's epilogue?"""
     return (USE_STREAM and skinny_ok(a, w_in) and a.shape[0] <= CONV_STEP_MAX_M and stream_fits(a.shape[1], False)
-            and w_in.shape[0] % 3 == 0 and 2 <= conv_k <= 16)
+            and conv_step_sizes(w_in, conv_k))
+
+
+def conv_step_sizes(w_in: torch.Tensor, conv_k: int) -> bool:
+    return w_in.shape[0] % 3 == 0 and 2 <= conv_k <= 16
 
 
 def gemm_stream_conv_step(a: torch.Tensor, w_in: torch.Tensor, bias: Optional[torch.Tensor], conv_w: torch.Tensor,
                           conv_bias: Optional[torch.Tensor], state: torch.Tensor, seg_pos: torch.Tensor,
-                          seg_slot: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+                          seg_slot: torch.Tensor, out: torch.Tensor, norm: Optional[Tuple[torch.Tensor, float]] = None) -> torch.Tensor:
     """``out = C * conv(B * X)`` for one-row segments, with ``[B | C | X] = a @ w_in.T (+ bias)`` never written
     out: the product's tile holds the matching rows of B, C and X and its epilogue runs the conv step and the
-    state update of :func:`shortconv_decode` (same arithmetic, same bits)."""
-    _need(a, "a", torch.bfloat16, contiguous=False); _need(w_in, "w_in", torch.bfloat16, contiguous=False)
+    state update of :func:`shortconv_decode` (same arithmetic, same bits).  With ``norm`` = (weight, eps) ``a`` holds float32
+    rows whose RMS norm is meant (see :func:`gemm_rows_normed`; at most 8 rows)."""
+    _need(a, "a", torch.bfloat16 if norm is None else torch.float32, contiguous=False); _need(w_in, "w_in", torch.bfloat16, contiguous=False)
     _need(out, "out", torch.bfloat16, contiguous=False)
     _need(conv_w, "conv_w", torch.float32); _need(state, "state", torch.float32)
     _need(seg_pos, "seg_pos", torch.int32); _need(seg_slot, "seg_slot", torch.int32)
@@ -1726,11 +1731,59 @@ def gemm_stream_conv_step(a: torch.Tensor, w_in: torch.Tensor, bias: Optional[to
             _need(t, nm, torch.float32)
             if t.numel() != n:
                 raise KernelError(f"gemm_stream_conv_step: {nm} size")
-    few = M <= ROWS_MAX_M
-    lib = load_library("gemm_rows" if few else "gemm_stream")
-    _run_gemm("gemm_rows_conv_step" if few else "gemm_stream_conv_step", lib.kp_gemm_rows_conv_step if few else lib.kp_gemm_stream_conv_step, a, w_in, out, _ptr(a), _rows_2d(a, "a"), _ptr(w_in), _rows_2d(w_in, "w_in"),
+    if norm is not None:
+        what, fn, rows = "gemm_rows_conv_step_normed", load_library("gemm_rows").kp_gemm_rows_conv_step_normed, _normed_args(a, *norm)
+    elif M <= ROWS_MAX_M:
+        what, fn, rows = "gemm_rows_conv_step", load_library("gemm_rows").kp_gemm_rows_conv_step, (_ptr(a), _rows_2d(a, "a"))
+    else:
+        what, fn, rows = "gemm_stream_conv_step", load_library("gemm_stream").kp_gemm_stream_conv_step, (_ptr(a), _rows_2d(a, "a"))
+    _run_gemm(what, fn, a, w_in, out, *rows, _ptr(w_in), _rows_2d(w_in, "w_in"),
          _ptr(bias), _ptr(out), _rows_2d(out, "out"), M, N, K, _ptr(conv_w), _ptr(conv_bias), _ptr(state), _ptr(seg_pos),
          _ptr(seg_slot), conv_k, STREAM)
+    return out
+
+
+ROWS_NORM_MAX_K = 4096     # columns up to which csrc/gemm_rows.cu norms its rows itself
+
+
+def rows_norm_fusable(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Can the product of the RMS norm of ``x`` (float32 rows, to bfloat16) with ``w`` norm the rows itself?  Up to 8 rows, where the
+    product would run on csrc/gemm_rows.cu: the norm in front of it is a launch of 2 us whose work is a load and two multiplications
+    a value."""
+    M, d = x.shape
+    return (USE_STREAM and 0 < M <= ROWS_MAX_M and d <= ROWS_NORM_MAX_K and stream_fits(d, False) and w.shape[0] <= 16384
+            and w.shape[1] == d and _rows_16_bytes(w) and x.is_contiguous() and x.data_ptr() % 16 == 0)
+
+
+def _normed_args(x: torch.Tensor, gamma: torch.Tensor, eps: float):
+    _need(x, "x", torch.float32, contiguous=False); _need(gamma, "norm weight", torch.float32)
+    if gamma.numel() != x.shape[1]:
+        raise KernelError("norm weight: size")
+    return _ptr(x), _rows_2d(x, "x"), _ptr(gamma), ctypes.c_float(eps)
+
+
+def gemm_rows_normed(x: torch.Tensor, gamma: torch.Tensor, eps: float, w: torch.Tensor, out: torch.Tensor,
+                     bias: Optional[torch.Tensor] = None, swiglu: bool = False, activation: str = "silu",
+                     glu: Optional[Tuple[float, float, float]] = None, plain_activation: Optional[str] = None) -> torch.Tensor:
+    """:func:`gemm_skinny` of the RMS norm of up to 8 float32 rows ``x`` (weight ``gamma``): the product takes ``x gamma`` rounded to
+    bfloat16 and multiplies the sums by ``1 / rms``."""
+    norm = _normed_args(x, gamma, eps)
+    _need(w, "w", torch.bfloat16, contiguous=False); _need(out, "out", contiguous=False)
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K or out.shape != (M, N // 2 if swiglu else N):
+        raise KernelError(f"gemm_rows_normed: shapes x{tuple(x.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
+    if bias is not None:
+        _need(bias, "bias", torch.float32)
+        if bias.numel() != N:
+            raise KernelError("gemm_rows_normed: bias size")
+    epi = _skinny_epilogue(out, False, swiglu)
+    if swiglu:
+        epi |= (ACT_GLU_CLAMPED if glu is not None else _fused_activation(activation)) << 8
+    if plain_activation is not None:
+        epi = _plain_epilogue(epi, plain_activation)
+    _run_gemm("gemm_rows_normed", load_library("gemm_rows").kp_gemm_rows_normed, x, w, out, *norm, _ptr(w), _rows_2d(w, "w"), _ptr(bias),
+              _ptr(out), _rows_2d(out, "out"), M, N, K, epi, *(_NO_LIMITS if glu is None else _glu_floats(glu)), STREAM)
     return out
 
 

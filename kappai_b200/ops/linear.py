@@ -13,6 +13,9 @@ no library matrix product is called.
 no launch that may still run may write it.  A float32 ``w`` may be anything, and is read early only where the caller says
 that it is such a weight: :func:`linear` with ``w_settled``, or the functions at the end of this module, which the model's
 parts call.
+
+The left operand of a weight's product may also be :class:`NormedRows`, rows whose RMS norm is still to be taken: the kernel
+for up to 8 rows takes it itself, for every other one the rows are normed first.
 """
 from __future__ import annotations
 
@@ -24,6 +27,34 @@ import torch
 from . import kernels as K
 
 
+class NormedRows:
+    """The RMS norm of the float32 rows ``x`` in bfloat16, for the one product that reads it.  ``x`` must stay as it is until
+    then.  (Not a tensor: a part is handed one only if its forward is marked ``takes_normed_rows``.)"""
+
+    def __init__(self, x: torch.Tensor, weight: torch.Tensor, eps: float):
+        self.x, self.weight, self.eps = x, weight, eps
+
+    dtype = torch.bfloat16
+
+    @property
+    def shape(self):
+        return self.x.shape
+
+    @property
+    def device(self):
+        return self.x.device
+
+    @property
+    def norm(self) -> Tuple[torch.Tensor, float]:
+        return self.weight, self.eps
+
+    def fusable(self, w: torch.Tensor) -> bool:
+        return K.rows_norm_fusable(self.x, w)
+
+    def rows(self) -> torch.Tensor:
+        return K.rmsnorm_rows(self.x, self.weight, self.eps, torch.empty(self.x.shape, dtype=self.dtype, device=self.x.device))
+
+
 def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
            accumulate: bool = False, w_settled: bool = False) -> torch.Tensor:
@@ -31,6 +62,11 @@ def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     float32 ``out`` (the residual sum stays in 32-bit)."""
     M, N = a.shape[0], w.shape[0]
     a_dtype = a.dtype
+    if isinstance(a, NormedRows):
+        if w_settled and not accumulate and a.fusable(w):
+            out = torch.empty((M, N), dtype=out_dtype or a_dtype, device=a.device) if out is None else out
+            return K.gemm_rows_normed(a.x, *a.norm, w, out, bias)
+        a = a.rows()
     if out is None:
         if accumulate:
             raise K.KernelError("linear: accumulate needs an output")
@@ -58,6 +94,10 @@ def linear_act(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], a
     fits the shape, else by a row-wise kernel behind a float32 product."""
     M, N = a.shape[0], w.shape[0]
     out = torch.empty((M, N), dtype=a.dtype, device=a.device)
+    if isinstance(a, NormedRows):
+        if w_settled and a.fusable(w):
+            return K.gemm_rows_normed(a.x, *a.norm, w, out, bias, plain_activation=activation)
+        a = a.rows()
     if a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
         tc = K.tc_ok(a, w)
         if K.skinny_ok(a, w) and not (tc and K.tc_pays_for_few_rows(M, N, False)):
@@ -78,6 +118,10 @@ def linear_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, bias: Optional[torch
     ff = w_gate_up.shape[0] // 2
     act = torch.empty((a.shape[0], ff), dtype=a.dtype, device=a.device)
     fused = glu is not None or activation in K.FUSED_ACTIVATIONS
+    if isinstance(a, NormedRows):
+        if fused and w_settled and a.fusable(w_gate_up):
+            return K.gemm_rows_normed(a.x, *a.norm, w_gate_up, act, bias, swiglu=True, activation=activation, glu=glu)
+        a = a.rows()
     tc = fused and K.tc_ok(a, w_gate_up)
     if fused and K.skinny_ok(a, w_gate_up) and not (tc and K.tc_pays_for_few_rows(a.shape[0], w_gate_up.shape[0], True)):
         return K.gemm_skinny(a, w_gate_up, act, bias, swiglu=True, activation=activation, glu=glu)

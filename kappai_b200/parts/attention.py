@@ -443,6 +443,8 @@ class Attention(PagedAttentionKernels, Part):
         a convolution of two taps or more, also the :class:`~kappai_b200.cache.storage.StateView` of its kept inputs)."""
         self.forward_projected(linear(h, self.w_qkv, self.b_qkv), residual, ctx, cache)
 
+    forward.takes_normed_rows = True
+
     def _convolve(self, qkv, ctx, kept, keep):
         """q, k and v behind their convolutions; the columns behind them (a gate) stay where they are."""
         out = torch.empty((ctx.n_rows, (self.H + 2 * self.G) * self.hd), dtype=qkv.dtype, device=qkv.device)

@@ -63,10 +63,17 @@ class PreNormResidualBlock(Part):
         self.mixer, self.ffn, self.mixer_norm, self.ffn_norm, self.side = mixer, ffn, mixer_norm, ffn_norm, side
         return self
 
+    @staticmethod
+    def _normed(norm, part, x):
+        if norm is None:
+            return x
+        # (a norm registered from outside need not know that a part may take its rows before the norm)
+        return norm.forward_for(part, x) if hasattr(norm, "forward_for") else norm.forward(x)
+
     def forward(self, x, ctx, cache):
-        self.mixer.forward(self.mixer_norm.forward(x) if self.mixer_norm is not None else x, x, ctx, cache)
+        self.mixer.forward(self._normed(self.mixer_norm, self.mixer, x), x, ctx, cache)
         if self.ffn is not None:
-            self.ffn.forward(self.ffn_norm.forward(x) if self.ffn_norm is not None else x, x, ctx)
+            self.ffn.forward(self._normed(self.ffn_norm, self.ffn, x), x, ctx)
         if self.side is not None:
             self.side.forward(x, ctx)
 

@@ -86,6 +86,8 @@ class SwiGLU(Part):
         act = linear_swiglu(h, self.w_gu, self.b_gu, self.activation)
         linear(act, self.w_down, self.b_down, out=residual, accumulate=True)
 
+    forward.takes_normed_rows = True
+
 
 class UngatedUnit(Part):
     """``mlp``: see the module's text.  The activation runs in the first product's epilogue, on its float32 sums."""
@@ -109,6 +111,8 @@ class UngatedUnit(Part):
     def forward(self, h, residual, ctx):
         linear(linear_act(h, self.w_up, None, self.activation), self.w_down, out=residual, accumulate=True)
 
+    forward.takes_normed_rows = True
+
 
 class ClampedGLU(SwiGLU):
     """``glu_clamped``: see the module's text.  Gate and up run as one product whose epilogue computes the unit, in
@@ -129,6 +133,8 @@ class ClampedGLU(SwiGLU):
     def forward(self, h, residual, ctx):
         act = linear_swiglu(h, self.w_gu, self.b_gu, glu=(self.limit, self.alpha, self.shift))
         linear(act, self.w_down, self.b_down, out=residual, accumulate=True)
+
+    forward.takes_normed_rows = True
 
 
 class MixtureOfExperts(Part):

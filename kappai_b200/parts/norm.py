@@ -15,6 +15,7 @@ from typing import Dict, Optional
 import torch
 
 from ..ops import kernels as K
+from ..ops.linear import NormedRows
 from .base import Part, WeightSpec, register_part
 
 
@@ -39,6 +40,13 @@ class RMSNorm(Part):
         out = torch.empty((n, self.size), dtype=self.env.dtype, device=x.device)
         return K.rmsnorm_rows(x, self.weight, self.eps, out, rows)
 
+    def forward_for(self, part, x: torch.Tensor):
+        """The norm as ``part``'s input: in a bfloat16 step of few rows left to the part's first product, if the part's forward is
+        marked as one that takes :class:`NormedRows` (a subclass with a forward of its own is not)."""
+        if x.shape[0] <= K.ROWS_MAX_M and self.env.dtype == torch.bfloat16 and getattr(part.forward, "takes_normed_rows", False):
+            return NormedRows(x, self.weight, self.eps)
+        return self.forward(x)
+
 
 class LayerNorm(RMSNorm):
     """Same sizes, weight and interface as :class:`RMSNorm`; the rows are centred first."""
@@ -47,6 +55,9 @@ class LayerNorm(RMSNorm):
         n = x.shape[0] if rows is None else rows.numel()
         out = torch.empty((n, self.size), dtype=self.env.dtype, device=x.device)
         return K.layernorm_rows(x, self.weight, self.eps, out, rows)
+
+    def forward_for(self, part, x: torch.Tensor):
+        return self.forward(x)
 
 
 register_part("norm", "rmsnorm", RMSNorm)

@@ -21,7 +21,7 @@ import torch
 from ..cache.spec import StateSpec
 from ..config.schema import ConfigError
 from ..ops import kernels as K
-from ..ops.linear import linear_weights as linear
+from ..ops.linear import NormedRows, linear_weights as linear
 from .base import Part, WeightSpec, register_part
 
 MAX_KERNEL = 16
@@ -66,14 +66,20 @@ class ShortConv(Part):
     def forward(self, h, residual, ctx, cache):
         """``cache``: a :class:`~kappai_b200.cache.storage.StateView` with tensor
         [n_slots, kernel_size - 1, hidden_size] float32."""
-        if (ctx.decode_only and cache.writes and h.dtype == torch.bfloat16 and self.fuse_step
-                and K.conv_step_fusable(h, self.w_in, self.K)):
+        if ctx.decode_only and cache.writes and h.dtype == torch.bfloat16 and self.fuse_step:
             # a decode step of few rows: the conv step runs in in_proj's epilogue (one launch less a layer)
-            y = torch.empty((ctx.n_rows, self.d), dtype=h.dtype, device=h.device)
-            K.gemm_stream_conv_step(h, self.w_in, self.b_in, self.w_conv, self.b_conv, cache.tensor, ctx.seg_pos,
-                                    ctx.seg_slot, y)
-            linear(y, self.w_out, self.b_out, out=residual, accumulate=True)
-            return
+            norm = None
+            if isinstance(h, NormedRows):
+                if h.fusable(self.w_in) and K.conv_step_sizes(self.w_in, self.K):
+                    h, norm = h.x, h.norm
+                else:
+                    h = h.rows()
+            if norm is not None or K.conv_step_fusable(h, self.w_in, self.K):
+                y = torch.empty((ctx.n_rows, self.d), dtype=torch.bfloat16, device=h.device)
+                K.gemm_stream_conv_step(h, self.w_in, self.b_in, self.w_conv, self.b_conv, cache.tensor, ctx.seg_pos,
+                                        ctx.seg_slot, y, norm)
+                linear(y, self.w_out, self.b_out, out=residual, accumulate=True)
+                return
         p = linear(h, self.w_in, self.b_in)
         y = torch.empty((ctx.n_rows, self.d), dtype=p.dtype, device=p.device)
         if ctx.decode_only and cache.writes:
@@ -82,6 +88,8 @@ class ShortConv(Part):
             K.shortconv_forward(p, self.w_conv, self.b_conv, cache.tensor, ctx.row_seg, ctx.cu_rows, ctx.seg_pos,
                                 ctx.seg_slot, y, update=cache.writes)
         linear(y, self.w_out, self.b_out, out=residual, accumulate=True)
+
+    forward.takes_normed_rows = True
 
 
 register_part("mixer", "shortconv", ShortConv)
