@@ -30,9 +30,13 @@
 // are added in the order of the parts.  A CTA runs the parts of its tile one after the other, each into an accumulator of
 // its own, and the epilogue adds them up (one commit a tile: a commit a part cost 0.25 us a part, the reading 0.05); or the
 // unit of work is (tile, part), all units in one round over the SMs and the parts of a tile one thread-block cluster.
-// Then every CTA leaves the float32 sums of its unit in its own shared memory (the ring is free by then); after the
-// cluster's barrier each adds up its share of the tile, reading the other CTAs' sums over the cluster's shared
-// memory, the parts in order of their number -- so the result does not depend on timing -- then the epilogue.
+// Then every CTA owns some of the tile's output columns: when its sums are done it sends the other CTAs theirs
+// (a bulk copy between the CTAs' rings, counted at a barrier of the owner), and adds up its own, the parts in order of their number -- so the result
+// does not depend on timing -- then the epilogue.  The old values of an accumulated output come in under the exchange.
+// (Sums left in shared memory and read by the others between two barriers of the cluster took 4.5 us from the last MMA to the
+// end, of products of 8 to 16: 128 rows by 2048 x 5632 16.0 us, this 12.0; 17 rows by 2048 x 2048 6.0 and 5.7.  Sent by single
+// stores that count at the barrier, st.async, 13.0 and 7.7; added by the threads that read tensor memory, a few lanes of few
+// warps at few rows, 12.9 and 6.7.)
 // With it every SM brings in a part of A only, and wide tiles still keep all SMs streaming.
 //
 // Every wait on an mbarrier is bounded.  A wait that gives up sets a status word (kp_tc_status), the CTA
@@ -69,22 +73,21 @@ struct TcArgs {
     int kb_per_part;                        // k-blocks a part
     int n_sets;                             // sets of `inner` accumulators of BN columns in tensor memory: two, or the one there is room for
     int tmem_cols;                          // columns allocated
+    int area;                               // bytes of the ring with its slack, or of what lies there later
+    int recv_apart;                         // a split over a cluster: other CTAs' sums have a place of their own behind the barriers
 };
 
 // all threads of all CTAs of the cluster; what they wrote to shared memory before is visible to the others after
-__device__ __forceinline__ void kp_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void kp_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void kp_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void kp_cluster_sync() { kp_cluster_arrive(); kp_cluster_wait(); }
+__device__ __forceinline__ void kp_cluster_sync_arrive() { kp_cluster_wait(); kp_cluster_arrive(); }   // the end of one round, the next one's start
+// `bytes` (16 or a multiple) of this CTA's shared memory to a CTA of the cluster, counted there at a barrier (addresses in
+// the cluster's window)
+__device__ __forceinline__ void kp_copy_to_cluster(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "r"(kp_smem_u32(src)), "r"(bytes), "r"(bar) : "memory");
 }
-// 16 bytes of the shared memory of the cluster's CTA `rank`, at the place that `addr` has in this CTA's
-__device__ __forceinline__ float4 kp_ld_cluster_f4(uint32_t addr, int rank) {
-    uint32_t ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
-    return v;
-}
-
 // the epilogue warps (threads 64 ...) among themselves
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(TC_EPI_PER_Q * 128) : "memory"); }
 
@@ -225,12 +228,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // stage's start (on into the W tile and beyond: the host leaves room after the last stage), and what it
     // makes of the rest lands in accumulator rows that nobody reads.
     unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * (A_BYTES + B_BYTES) + (TC_BM * TC_BK * 2 - A_BYTES));
+    uint64_t* full = reinterpret_cast<uint64_t*>(tiles + p.area);
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;                                  // [2]: set b holds a finished unit
     uint64_t* acc_empty = acc_full + 2;                                   // [2]: set b has been read out
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* recv_full = acc_empty + 2;                                  // (split over a cluster) the other parts' sums are here
+    uint64_t* rings_free = recv_full + 1;                                 // ... the other CTAs' rings are free
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rings_free + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    unsigned char* recv = p.recv_apart ? tiles + p.area + ((2 * STAGES + 6) * 8 + 8 + 15) / 16 * 16 : tiles + (size_t)min(p.M, TC_BM) * BN * 4;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_kb = (p.K + TC_BK - 1) / TC_BK;
@@ -239,6 +245,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int n_tiles = tiles_m * tiles_n;
     const int S = p.splits;                                              // parts along K; a unit of work is (tile, part)
     const int n_units = n_tiles * S;
+    // (split over a cluster) the tile's output columns in eights, in which is counted what a CTA owns, and the bytes of a row's
+    // sums that an eight takes
+    constexpr int U = N_OUT_TILE / 8, EIGHT = TC_GATED(EPI) ? 64 : 32;
     // the CTA is persistent: it takes tiles blockIdx.x, blockIdx.x + gridDim.x, ... ; consecutive tiles
     // share the W tile (m runs fastest), so the CTAs that run together read the same few W tiles from L2
 
@@ -249,15 +258,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
         for (int s = 0; s < STAGES; s++) { kp_mbar_init(&full[s], 1); kp_mbar_init(&empty[s], 1); }
         for (int b2 = 0; b2 < 2; b2++) { kp_mbar_init(&acc_full[b2], 1); kp_mbar_init(&acc_empty[b2], 4 * TC_EPI_PER_Q); }
+        kp_mbar_init(recv_full, 1);
+        if (S > 1) kp_mbar_init(rings_free, S - 1);
         *abort_flag = 0;
         kp_mbar_init_fence();
+        if (S > 1) {                                                      // (the bytes that the cluster's other CTAs will send)
+            const int rank = blockIdx.x % S, R = min(TC_BM, p.M - (int)((blockIdx.x / S) % tiles_m) * TC_BM);
+            kp_mbar_expect_tx(recv_full, (S - 1) * (U * (rank + 1) / S - U * rank / S) * EIGHT * R);
+        }
     }
     if (warp == 1) kp_tmem_alloc(tmem_slot, p.tmem_cols);
     kp_tc_fence_before();
     __syncthreads();
     kp_tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    bool parts_ok = false;                                                // (epilogue warps) this CTA's sums are in shared memory
+    if (S > 1) kp_cluster_arrive();                                       // (waited for in front of the first use of another CTA's memory)
 
     // (the producer's and the MMA warp's lanes stay in step; one elected lane issues what they issue)
     if (warp == 0) {
@@ -308,6 +323,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
+        if (S > 1) { __syncwarp(); kp_cluster_sync_arrive(); }
     } else if (warp == 1) {
         kp_pdl_begin();
         constexpr uint32_t idesc = kp_umma_idesc(TC_BM, BN);
@@ -336,6 +352,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (ok) kp_umma_commit_warp(&acc_full[b2]);                   // arrives when every MMA of the unit has completed
             if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
         }
+        if (S > 1) { __syncwarp(); kp_cluster_sync_arrive(); }
     } else {
         kp_pdl_begin();
         // epilogue: warp w reads the 32 lanes (w % 4) * 32 ... of tensor memory; it works on unit i while the
@@ -348,7 +365,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             const int tile = unit / S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-            if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) { ok = false; break; }
+            if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) {
+                ok = false;
+                if (S > 1) { __syncwarp(); kp_cluster_wait(); epi_sync(); }   // (where the other warps may be waiting for this one)
+                break;
+            }
             kp_tc_fence_after();
             const int m = m0 + q * 32 + lane;
             const uint32_t lane_base = tmem_base + (uint32_t)(b2 * p.inner * BN) + ((uint32_t)(q * 32) << 16);
@@ -367,92 +388,98 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (lane == 0) kp_mbar_arrive(read_out);
                 continue;
             }
-            // split over K: this part's sums of the whole accumulator (BN columns) go to this CTA's shared memory
-            // (the ring is free: every MMA of the unit has completed), laid out [piece of 32 columns][float4 of
-            // the piece][row of the tile][4] so that a warp's rows lie one behind the other; the tile's CTAs -- a cluster --
-            // add them up below
-            float4* mine = reinterpret_cast<float4*>(tiles);
-            const int R = min(TC_BM, p.M - m0);                          // rows of this tile
+            // Split over K: every CTA of the cluster owns some of the tile's output columns, in eights.  A CTA writes its sums to
+            // its ring, which is free, an eight behind the other, each [gate, up][half][row][4]; sends every other owner its
+            // eights -- into the owner's ring, behind its sums, once that is free as well, or apart from it -- and adds up its own.
+            const int rank = unit - tile * S, R = min(TC_BM, p.M - m0);   // (rows of this tile)
+            const int lo = U * rank / S, own = U * (rank + 1) / S - lo;
+            kp_cluster_wait();
+            if (!p.recv_apart && threadIdx.x < 64 + S && (int)threadIdx.x - 64 != rank) kp_mbar_arrive_cluster(kp_cluster_addr(rings_free, threadIdx.x - 64));
 #pragma unroll 1
-            for (int c = half * 32; c < BN; c += 32 * TC_EPI_PER_Q) {
+            for (int c = half * 32; c < BN && q * 32 < R; c += 32 * TC_EPI_PER_Q) {
                 uint32_t r[32];
                 kp_tmem_ld32(lane_base + c, r);
+                const int cu = c / 8, up = cu >= U ? 1 : 0;
                 if (m < p.M) {
-                    float4* dst = mine + (size_t)(c >> 5) * 8 * R + (m - m0);
+                    uint4* dst = reinterpret_cast<uint4*>(tiles + ((cu - up * U) * EIGHT + up * 32) * R) + (m - m0);
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        dst[(size_t)j * R] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                                           __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+                    for (int k = 0; k < 4; k++, dst += EIGHT / 16 * R) {
+                        dst[0] = make_uint4(r[8 * k], r[8 * k + 1], r[8 * k + 2], r[8 * k + 3]);
+                        dst[R] = make_uint4(r[8 * k + 4], r[8 * k + 5], r[8 * k + 6], r[8 * k + 7]);
+                    }
                 }
             }
-            kp_tc_fence_before();
-            __syncwarp();
-            if (lane == 0) kp_mbar_arrive(read_out);
-            parts_ok = true;
-        }
-        if (!ok && lane == 0) atomicExch(&g_tc_status, 1);
-    }
-    kp_tc_fence_before();
-    __syncthreads();
-    if (S > 1) {
-        // Split over K: the CTAs of a tile are a cluster (rank = part).  When all of them have their sums in
-        // shared memory, each adds up its share of the tile, reading the others' over the cluster's shared
-        // memory: the parts in the order of their numbers, so the result does not depend on timing; then the
-        // epilogue.  Every thread of every CTA comes here, also after a wait that gave up, so the cluster's
-        // barriers always complete; no CTA leaves before the others have read its sums.
-        kp_cluster_sync();
-        if (warp >= 2 && parts_ok) {
-            const int tile = blockIdx.x / S, part = blockIdx.x - tile * S;
-            const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-            const int R = min(TC_BM, p.M - m0);                           // rows of this tile
-            const int n_vec = N_OUT_TILE / 32 * R * 8;                    // float4s of the tile's output
-            const int lo = (int)((long long)n_vec * part / S), hi = (int)((long long)n_vec * (part + 1) / S);
-            const uint32_t mine = kp_smem_u32(tiles);
-            const uint32_t up_off = (uint32_t)(BN / 64) * 8 * R * 16;     // bytes from a gate piece to its up piece
-            constexpr int NT = TC_EPI_PER_Q * 128;
-            // VI float4s a thread at a time, the parts four by four: the loads of a round are all in flight
-            // together (each is a trip to another SM), the sums still run in the order of the parts
-            constexpr int VI = TC_GATED(EPI) ? 2 : 4;
-            for (int i0 = lo + (int)threadIdx.x - 64; i0 < hi; i0 += VI * NT) {
-                float4 g[VI], up[VI];
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            epi_sync();
+            if (warp == 2) {
+                if (!p.recv_apart && !kp_mbar_wait_bounded(rings_free, 0)) ok = false;
+                const int olo = U * lane / S, bytes = (U * (lane + 1) / S - olo) * EIGHT * R;
+                if (ok && lane < S && lane != rank && bytes > 0)
+                    kp_copy_to_cluster(kp_cluster_addr(recv, lane) + (rank < lane ? rank : rank - 1) * bytes, tiles + olo * EIGHT * R, bytes,
+                                       kp_cluster_addr(recv_full, lane));
+                __syncwarp();
+            }
+            // Its own, by all epilogue threads: VI pieces of four columns of a row at a time; the old values of an accumulated
+            // output are asked for before the wait.
+            constexpr int VI = TC_GATED(EPI) ? 2 : 4, NT = TC_EPI_PER_Q * 128;
+            const int n_vec = own * 2 * R;
+            const bool old_apart = EPI == EPI_ACCUM_F32 && p.vec_ok;
+            bool here = false;
+#pragma unroll 1
+            for (int i0 = (int)threadIdx.x - 64; i0 - lane - (warp - 2) * 32 < n_vec || !here; i0 += VI * NT) {
+                int at[VI], col[VI], row[VI];                             // where in an owner's eights; the output's column and row, -1: none
+                float4 old[VI];
 #pragma unroll
-                for (int v = 0; v < VI; v++) g[v] = up[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int sp0 = 0; sp0 < S; sp0 += 4) {
-                    float4 t[VI][4], t2[VI][4];
+                for (int v = 0; v < VI; v++) {
+                    const int idx = i0 + v * NT, piece = idx / R;
+                    row[v] = idx < n_vec ? idx - piece * R : -1;
+                    col[v] = n0 + lo * 8 + piece * 4;
+                    at[v] = ((piece >> 1) * EIGHT + (piece & 1) * 16) * R + row[v] * 16;
+                    if (old_apart && row[v] >= 0 && col[v] + 4 <= n_out) old[v] = *reinterpret_cast<const float4*>((const float*)p.C + (size_t)(m0 + row[v]) * p.ldc + col[v]);
+                }
+                if (!here) {
+                    here = true;
+                    ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(recv_full, 0) && ok);
+                    if (!ok) break;
+                }
+                float g[VI][4], up[VI][4];
 #pragma unroll
-                    for (int v = 0; v < VI; v++)
+                for (int v = 0; v < VI; v++)
 #pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const int idx = i0 + v * NT;
-                            t[v][u] = t2[v][u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (idx < hi && sp0 + u < S) {
-                                t[v][u] = kp_ld_cluster_f4(mine + (uint32_t)idx * 16, sp0 + u);
-                                if TC_GATED(EPI) t2[v][u] = kp_ld_cluster_f4(mine + (uint32_t)idx * 16 + up_off, sp0 + u);
-                            }
+                    for (int j = 0; j < 4; j++) g[v][j] = up[v][j] = 0.f;
+#pragma unroll 2
+                for (int part = 0; part < S; part++) {
+                    const unsigned char* src = part == rank ? tiles + lo * EIGHT * R : recv + (part < rank ? part : part - 1) * own * EIGHT * R;
+#pragma unroll
+                    for (int v = 0; v < VI; v++) {
+                        if (row[v] < 0) continue;
+                        const float4 a = *reinterpret_cast<const float4*>(src + at[v]);
+                        g[v][0] += a.x; g[v][1] += a.y; g[v][2] += a.z; g[v][3] += a.w;
+                        if TC_GATED(EPI) {
+                            const float4 b = *reinterpret_cast<const float4*>(src + at[v] + 32 * R);
+                            up[v][0] += b.x; up[v][1] += b.y; up[v][2] += b.z; up[v][3] += b.w;
                         }
-#pragma unroll
-                    for (int v = 0; v < VI; v++)
-#pragma unroll
-                        for (int u = 0; u < 4; u++)
-                            if (sp0 + u < S) {
-                                g[v].x += t[v][u].x; g[v].y += t[v][u].y; g[v].z += t[v][u].z; g[v].w += t[v][u].w;
-                                up[v].x += t2[v][u].x; up[v].y += t2[v][u].y; up[v].z += t2[v][u].z; up[v].w += t2[v][u].w;
-                            }
+                    }
                 }
 #pragma unroll
                 for (int v = 0; v < VI; v++) {
-                    const int idx = i0 + v * NT;
-                    if (idx < hi) {
-                        const float g4[4] = {g[v].x, g[v].y, g[v].z, g[v].w}, u4[4] = {up[v].x, up[v].y, up[v].z, up[v].w};
-                        const int piece = idx / (R * 8), rem = idx - piece * (R * 8);
-                        const int j4 = rem / R, row = rem - j4 * R;
-                        tc_finish<EPI, 4>(p, n_out, g4, u4, m0 + row, n0 + piece * 32 + j4 * 4);
+                    if (row[v] < 0) continue;
+                    if (old_apart && col[v] + 4 <= n_out) {
+                        tc_bias<EPI, 4>(p, n_out, g[v], up[v], col[v]);
+                        *reinterpret_cast<float4*>((float*)p.C + (size_t)(m0 + row[v]) * p.ldc + col[v]) =
+                            make_float4(g[v][0] + old[v].x, g[v][1] + old[v].y, g[v][2] + old[v].z, g[v][3] + old[v].w);
+                    } else {
+                        tc_finish<EPI, 4>(p, n_out, g[v], up[v], m0 + row[v], col[v]);
                     }
                 }
             }
         }
-        kp_cluster_sync();
+        if (!ok && lane == 0) atomicExch(&g_tc_status, 1);
+        if (S > 1) { __syncwarp(); kp_cluster_arrive(); }
     }
+    kp_tc_fence_before();
+    __syncthreads();
+    if (S > 1) kp_cluster_wait();                                         // no CTA leaves before all have what they were sent, or have given up
     if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
     if (warp == 1) kp_tmem_dealloc(tmem_base, p.tmem_cols);
 }
@@ -681,15 +708,25 @@ static int tc_n_sm() {
     return sms;
 }
 
-// Shared memory of a launch: `stages` ring stages, the slack behind a short last stage, barriers, alignment.
-static size_t tc_smem(int a_rows, int bn, int* stages_out) {
-    const int stage = a_rows * TC_BK * 2 + bn * TC_BK * 2;
+#define TC_RECV_APART (24 * 1024)            // up to this much has a place of its own, and no CTA has to know that another's ring is free
+// Shared memory of a launch: `stages` ring stages with the slack behind a short last stage, or a cluster's exchange of sums if
+// that is more (`area`); barriers, alignment, and what other CTAs send apart from that (`apart`).
+struct TcSmem { int stages, area, apart; size_t bytes; };
+static TcSmem tc_smem(int M, int a_rows, int bn, bool gated, int splits) {
+    TcSmem t = {};
+    const int rows = M < TC_BM ? M : TC_BM, stage = a_rows * TC_BK * 2 + bn * TC_BK * 2;
     const int slack = (TC_BM - a_rows) * TC_BK * 2;            // the MMA's reads past a short last stage
-    int stages = (TC_SMEM_KB * 1024 - slack) / stage;
-    if (stages > 24) stages = 24;
-    if (stages < 2) stages = 2;
-    *stages_out = stages;
-    return (size_t)stages * stage + slack + (size_t)(2 * stages + 4) * 8 + 16 + 1024;
+    // the most that a CTA of a cluster is sent: the others' sums of its output columns, which are counted in eights
+    const int eights = bn / (gated ? 16 : 8), recv = (splits - 1) * ((eights + splits - 1) / splits) * (gated ? 64 : 32) * rows;
+    t.apart = recv <= TC_RECV_APART ? recv : 0;
+    t.stages = (TC_SMEM_KB * 1024 - slack - t.apart) / stage;
+    if (t.stages > 24) t.stages = 24;
+    if (t.stages < 2) t.stages = 2;
+    t.area = t.stages * stage + slack;
+    const int exchange = splits > 1 ? rows * bn * 4 + recv - t.apart : 0;
+    if (t.area < exchange) t.area = (exchange + 1023) / 1024 * 1024;
+    t.bytes = (size_t)t.area + (size_t)(2 * t.stages + 6) * 8 + 8 + 16 + t.apart + 1024;
+    return t;
 }
 
 template <int BN, int EPI>
@@ -723,9 +760,10 @@ static int max_clusters(int cluster, size_t smem) {
 
 template <int BN, int EPI>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaStream_t s) {
-    int stages = 0;
-    const size_t smem = tc_smem(a.a_rows, BN, &stages);
-    a.n_stages = stages;
+    const TcSmem sm = tc_smem(a.M, a.a_rows, BN, TC_GATED(EPI), a.splits);
+    if (sm.bytes > KP_SMEM_MAX) return KP_ERR_UNSUPPORTED;
+    a.n_stages = sm.stages; a.area = sm.area; a.recv_apart = sm.apart > 0;
+    const size_t smem = sm.bytes;
     int st = prepare<BN, EPI>();
     if (st) return st;
     const int n_out = TC_GATED(EPI) ? a.ff : a.N;
@@ -765,8 +803,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcArg
 
 // Clusters of `cluster` CTAs that run at once, for the tile width and epilogue of a launch.
 static int tc_max_clusters(int bn, int epi, int cluster, int a_rows) {
-    int stages = 0;
-    const size_t smem = tc_smem(a_rows, bn, &stages);
+    const size_t smem = tc_smem(TC_BM, a_rows, bn, false, 1).bytes;
 #define TC_MC(BN_, EPI_) return max_clusters<BN_, EPI_>(cluster, smem);
 #define TC_MC_BN(EPI_)                                             \
     switch (bn) {                                                  \
@@ -797,13 +834,10 @@ static int tc_sets(int bn, int inner) { return 2 * inner * bn <= 512 ? 2 : (inne
 
 static int tc_a_rows(int M) { return M >= TC_BM ? TC_BM : (M + 7) / 8 * 8; }
 
-// Can parts along K of a tile `w` wide run at all: all units in one round, no part under two k-blocks, and the sums of a unit
-// fit where the ring was (false for more parts, too) ...
-static bool tc_split_starts(int M, int K, int w, int sp, int tiles) {
-    int stages = 0;
-    const size_t ring = tc_smem(tc_a_rows(M), w, &stages) - 2048;
-    const int rows = M < TC_BM ? M : TC_BM;
-    return tiles * sp <= tc_n_sm() && sp * 2 <= (K + TC_BK - 1) / TC_BK && (size_t)rows * w * 4 <= ring;
+// Can parts along K of a tile `w` wide run at all: all units in one round, no part under two k-blocks (false for more parts,
+// too) ...
+static bool tc_split_starts(int K, int sp, int tiles) {
+    return tiles * sp <= tc_n_sm() && sp * 2 <= (K + TC_BK - 1) / TC_BK;
 }
 // ... the clusters all run at once, and no part is empty?
 static bool tc_split_runs(int M, int K, int epi, int w, int sp, int tiles) {
@@ -833,7 +867,7 @@ static int tc_parts(int M, int N, int K, int epi) {
     for (int w = 256; w >= 64; w /= 2) {
         const int cols = gated ? w / 2 : w, tiles = (n_out + cols - 1) / cols * m_tiles;
         for (int sp = 1; sp <= 8; sp++) {
-            if (sp > 1 && !tc_split_starts(M, K, w, sp, tiles)) break;
+            if (sp > 1 && !tc_split_starts(K, sp, tiles)) break;
             if (sp > 1 && !tc_split_runs(M, K, epi, w, sp, tiles)) continue;
             const int kbs = (n_kb + sp - 1) / sp;
             long long cost = (sp == 1 ? (long long)((tiles + sms - 1) / sms) * n_kb : kbs) * (TC_BK * 2) * (w + a_rows);
@@ -849,14 +883,12 @@ static int tc_parts(int M, int N, int K, int epi) {
 //   a k-block: its rows of A and W, but no less than TC_KB_MIN (waiting, issuing, handing on);
 //   an epilogue: 0.6 KB a column of the tile, 1.2 KB gated, under the main loop of the next tile if there is one;
 //   parts one after the other: 6 KB a part more and 64 columns, for reading its sums;
-//   parts by a cluster (all units in one round): 100 KB and 5 KB a cluster (up to 24) for the barriers, four times the sums
-//   that are exchanged, more for clusters of other than 2 or 4 CTAs; beyond 512 rows a tenth more, as the sums of many tiles
-//   meet;
+//   parts by a cluster (all units in one round): 20 KB and 1.4 KB a CTA for the exchange, five times the sums that are
+//   exchanged, a little more for clusters of other than 2 or 4 CTAs;
 //   a pair: TC_PAIR_COST for its barriers, and more for parts behind a gated epilogue, which is short of registers.
-// It was fitted to all that can run at 17 to 1000 rows of thirteen layer products: within 1 % of the best on average, 23 %
-// at worst (gated 700 rows by 9216 x 1024, where three kinds of tile tie).  Measured, us, a cluster always | the choice | the
-// choice were the parts free: 64 rows by 6144 x 2048 11.1 | 9.6 | 9.2, 200 by 3072 x 2048 14.1 | 10.2 | 9.9, 512 by 3072 x 1024
-// 14.5 | 7.5 | 7.2, 101 by 2048 x 5632 10.6 | 10.6 | 10.2.
+// It was fitted to all that can run at 17 to 1000 rows of twelve layer products (860 timings): within 0.7 % of the best on average,
+// 24 % at worst (gated 600 rows by 9216 x 1024, where a pair's third row of tiles holds 88 rows).  Measured, us, the choice before
+// the exchange by copies | now: 64 rows by 2048 x 2048 7.6 | 6.5, 128 by 2048 x 5632 16.0 | 12.0, 200 by 1024 x 4608 13.4 | 10.1.
 static TcChoice tc_choose(int M, int N, int K, int epi, int split) {
     const bool gated = epi == EPI_SWIGLU;
     const int n_out = gated ? N / 2 : N, sms = tc_n_sm(), n_kb = (K + TC_BK - 1) / TC_BK;
@@ -879,11 +911,9 @@ static TcChoice tc_choose(int M, int N, int K, int epi, int split) {
     }
     for (int w = 256; parts > 1 && w >= 64; w /= 2) {
         const int tiles = (int)(tiles_at(w) * m_tiles), kbs = (n_kb + parts - 1) / parts;
-        if (!tc_split_starts(M, K, w, parts, tiles) || !tc_split_runs(M, K, epi, w, parts, tiles)) continue;
-        long long cost = kbs * kb_cost(w + a_rows) + epi_cost(w) / parts + 100 * 1024 + (tiles < 24 ? tiles : 24) * 5 * 1024 +
-                         4LL * rows * w * 4 * (parts - 1) / parts;
-        if (parts != 2 && parts != 4) cost += parts == 3 ? 32 * 1024 : 100 * 1024;
-        if (m_tiles > 4) cost += cost / 10;
+        if (!tc_split_starts(K, parts, tiles) || !tc_split_runs(M, K, epi, w, parts, tiles) || tc_smem(M, a_rows, w, gated, parts).bytes > KP_SMEM_MAX) continue;
+        const long long cost = kbs * kb_cost(w + a_rows) + epi_cost(w) / parts + 20 * 1024 + tiles * parts * 1434LL +
+                               5LL * rows * w * 4 * (parts - 1) / parts + (parts != 2 && parts != 4 ? 20 * 1024 : 0);
         if (cost < best) { best = cost; ch = {w, parts, true, false}; }
     }
     for (int w = 256; m_tiles > 1 && w >= 128; w /= 2) {
@@ -937,7 +967,7 @@ int kp_gemm_tc_as(const void* A, int lda, const void* W, int ldw, const float* b
     if (pair && (bn < 128 || m_tiles < 2)) return KP_ERR_UNSUPPORTED;
     if (cluster) {
         const long long tiles = (long long)((n_out + cols - 1) / cols) * m_tiles;
-        if (tiles > 65535 || !tc_split_starts(M, K, bn, parts, (int)tiles) || !tc_split_runs(M, K, kind, bn, parts, (int)tiles)) return KP_ERR_UNSUPPORTED;
+        if (tiles > 65535 || !tc_split_starts(K, parts, (int)tiles) || !tc_split_runs(M, K, kind, bn, parts, (int)tiles)) return KP_ERR_UNSUPPORTED;
     } else {
         const int kbs = (n_kb + parts - 1) / parts;
         if (!tc_sets(bn, parts) || (n_kb + kbs - 1) / kbs != parts) return KP_ERR_UNSUPPORTED;
