@@ -18,6 +18,16 @@
 //              the lanes 32 * (warp % 4) ...), taking the 32-column pieces in turn so that more loads and
 //              stores are in flight.  Each reads its lanes with tcgen05.ld (32 columns at a time), applies
 //              bias / residual accumulation / SwiGLU, writes its rows of C and hands the accumulator back.
+// A k-block costs the producer and the MMA warp about 0.1 us of waits, arming and commits beside its copies and MMAs, so a
+// stage holds two k-blocks where that is at most 64 KB: one copy an operand, of a tensor map with the k-blocks as a
+// dimension of its own (gate and up another), where K is a multiple of 64.  64 rows by 6144 x 2048 10.2 us with one, 9.4
+// with two; 17 by 2048 x 5632 10.1 and 9.6.
+//
+// The kernels of a decode step follow one another through the SMs' instruction caches, and what a kernel does not find
+// there it waits for, at every launch.  Hence loops that are not unrolled, the long part of a wait out of line, an epilogue
+// of 16 columns at a time: 43 to 69 KB of code a kernel became 42 to 59, those of one k-block a stage half of that.  A step
+// of 17 requests of the 1.2B shape 803 -> 770 us, of 100 of the 350M shape 729 -> 669; back to back the products hardly differ.
+//
 // Rows of A beyond M and rows of W beyond N are zero-filled by TMA (out-of-bounds fill) and masked at the
 // store; K needs no padding (the tail of the last k-block is zero-filled too) but K % 8 == 0 (16-byte rows).
 // Each output sums its k-blocks in order, within its part of K where the product is cut along K (tc_parts).
@@ -55,6 +65,8 @@
 #define TC_BM 128
 #define TC_BK 64
 #define TC_EPI_PER_Q 2                       // epilogue warps for each quarter of the tensor-memory lanes
+#define TC_VI 2
+#define TC_PIECE 16                          // columns that an epilogue warp of the one-CTA kernel takes at a time
 #define TC_THREADS (64 + TC_EPI_PER_Q * 128) // the producer warp, the MMA warp and the epilogue warps
 
 KP_STATUS_WORD(g_tc_status, tc)          // 0 ok; 1: a bounded wait gave up
@@ -68,6 +80,7 @@ struct TcArgs {
     int vec_ok;                             // rows of C are 16-byte aligned: whole pieces go out in 16-byte stores
     int a_rows;                             // rows of the A box: 128, fewer (a multiple of 8) when M < 128
     int n_stages;                           // stages of the ring
+    int kb_stage;                           // k-blocks a stage: 1, or more that one copy an operand brings
     int splits;                             // CTAs that share a tile's parts along K, one each (1: no cluster)
     int inner;                              // parts along K that a CTA (or a pair) runs itself, one after the other (1 beside splits > 1)
     int kb_per_part;                        // k-blocks a part
@@ -180,40 +193,41 @@ __device__ __forceinline__ void tc_finish(const TcArgs& p, int n_lim, const floa
     }
 }
 
-// The 32 sums of a lane's row at a place of the unit's accumulators, g (and u: the up half, gated): one part's as they are,
+// W columns of tensor memory, without the wait
+__device__ __forceinline__ void tc_ld_issue(uint32_t at, uint32_t (&r)[32]) { kp_tmem_ld32_issue(at, r); }
+__device__ __forceinline__ void tc_ld_issue(uint32_t at, uint32_t (&r)[16]) { kp_tmem_ld16_issue(at, r); }
+__device__ __forceinline__ void tc_ld_issue(uint32_t at, uint32_t (&r)[8]) { kp_tmem_ld8_issue(at, r); }
+
+// The W sums of a lane's row at a place of the unit's accumulators, g (and u: the up half, gated): one part's as they are,
 // several parts' added from zero in the order of the parts, as the split over a cluster adds them.
 // (PARTS false: there is one, which saves the pairs' gated epilogue the registers that the adding needs.)
-template <int EPI, int BN, bool PARTS>
-__device__ __forceinline__ void tc_sums(const TcArgs& p, uint32_t at, float (&g)[32], float (&up)[32]) {
-    uint32_t r[32];
-    {
-        uint32_t u[32];
-        kp_tmem_ld32_issue(at, r);
-        if TC_GATED(EPI) kp_tmem_ld32_issue(at + BN / 2, u);
-        kp_tmem_ld_wait();
+template <int EPI, int BN, bool PARTS, int W>
+__device__ __forceinline__ void tc_sums(const TcArgs& p, uint32_t at, float (&g)[W], float (&up)[W]) {
+    uint32_t r[W], u[W];
+    tc_ld_issue(at, r);
+    if TC_GATED(EPI) tc_ld_issue(at + BN / 2, u);
+    kp_tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-            g[j] = __uint_as_float(r[j]);
-            up[j] = TC_GATED(EPI) ? __uint_as_float(u[j]) : 0.f;
-        }
+    for (int j = 0; j < W; j++) {
+        g[j] = __uint_as_float(r[j]);
+        up[j] = TC_GATED(EPI) ? __uint_as_float(u[j]) : 0.f;
     }
     if (PARTS && p.inner > 1) {
 #pragma unroll
-        for (int j = 0; j < 32; j++) { g[j] = 0.f + g[j]; if TC_GATED(EPI) up[j] = 0.f + up[j]; }
+        for (int j = 0; j < W; j++) { g[j] = 0.f + g[j]; if TC_GATED(EPI) up[j] = 0.f + up[j]; }
 #pragma unroll 1
         for (int i = 1; i < p.inner; i++) {
             at += BN;
-            kp_tmem_ld32(at, r);
+            tc_ld_issue(at, r);
+            if TC_GATED(EPI) tc_ld_issue(at + BN / 2, u);
+            kp_tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 32; j++) g[j] += __uint_as_float(r[j]);
-            if TC_GATED(EPI) {
-                kp_tmem_ld32(at + BN / 2, r);
-#pragma unroll
-                for (int j = 0; j < 32; j++) up[j] += __uint_as_float(r[j]);
-            }
+            for (int j = 0; j < W; j++) { g[j] += __uint_as_float(r[j]); if TC_GATED(EPI) up[j] += __uint_as_float(u[j]); }
         }
     }
 }
+
+template <int N> struct TcInt { static constexpr int value = N; };
 
 template <int BN, int EPI>
 __global__ void __launch_bounds__(TC_THREADS)
@@ -221,6 +235,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr int B_BYTES = BN * TC_BK * 2;
     constexpr int N_OUT_TILE = TC_GATED(EPI) ? BN / 2 : BN;       // output columns of the tile
     const int A_BYTES = p.a_rows * TC_BK * 2;                            // the rows of A that are brought in
+    // (a stage: the A tiles of its kb_stage k-blocks, then their W tiles)
     const int STAGES = p.n_stages;
     extern __shared__ unsigned char smem[];
     // STAGES x (A tile | B tile); the swizzled tiles must start on 1024-byte boundaries.  With fewer than 128
@@ -256,6 +271,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // (the tensor maps are fetched now: the first TMA load through a map that has not been used waits for it)
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
+#pragma unroll 1
         for (int s = 0; s < STAGES; s++) { kp_mbar_init(&full[s], 1); kp_mbar_init(&empty[s], 1); }
         for (int b2 = 0; b2 < 2; b2++) { kp_mbar_init(&acc_full[b2], 1); kp_mbar_init(&acc_empty[b2], 4 * TC_EPI_PER_Q); }
         kp_mbar_init(recv_full, 1);
@@ -275,27 +291,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (S > 1) kp_cluster_arrive();                                       // (waited for in front of the first use of another CTA's memory)
 
     // (the producer's and the MMA warp's lanes stay in step; one elected lane issues what they issue)
-    if (warp == 0) {
+    // (their loops are compiled for each number of k-blocks a stage: they are what a narrow tile's k-blocks wait for)
+    const auto produce = [&](auto nb) {
+        constexpr int NB = decltype(nb)::value;
+        const int STAGE = NB * (A_BYTES + B_BYTES);
         auto load_w = [&](int s, int kb, int n0) {
-            unsigned char* b_dst = tiles + (size_t)s * (A_BYTES + B_BYTES) + A_BYTES;
-            if TC_GATED(EPI) {
+            unsigned char* b_dst = tiles + (size_t)s * STAGE + NB * A_BYTES;
+            if (NB > 1) {
+                if TC_GATED(EPI) kp_tma_load_4d_warp(b_dst, &tmW, 0, n0, 0, kb, &full[s]);
+                else kp_tma_load_3d_warp(b_dst, &tmW, 0, n0, kb, &full[s]);
+            } else if TC_GATED(EPI) {
                 kp_tma_load_2d_warp(b_dst, &tmW, kb * TC_BK, n0, &full[s]);                       // gate rows
                 kp_tma_load_2d_warp(b_dst + B_BYTES / 2, &tmW, kb * TC_BK, p.ff + n0, &full[s]);  // up rows
             } else {
                 kp_tma_load_2d_warp(b_dst, &tmW, kb * TC_BK, n0, &full[s]);
             }
         };
-        // The weights depend on no earlier kernel: the W tiles of the first unit's first k-blocks (as many as
-        // the ring has stages) are on their way before the wait on the kernel before; their A tiles follow it.
+        // The weights depend on no earlier kernel: the W tiles of the first unit's first stages (as many as
+        // the ring has) are on their way before the wait on the kernel before; their A tiles follow it.
         int pre = 0;
         if ((int)blockIdx.x < n_units) {
             const int tile = blockIdx.x / S, part = blockIdx.x - tile * S;
             const int n0 = (tile / tiles_m) * N_OUT_TILE;
             const int kb_lo = part * p.kb_per_part, kb_hi = S > 1 ? min(n_kb, kb_lo + p.kb_per_part) : n_kb;
-            pre = min(STAGES, kb_hi - kb_lo);
+            pre = min(STAGES, (kb_hi - kb_lo + NB - 1) / NB);
+#pragma unroll 1
             for (int i = 0; i < pre; i++) {
-                kp_mbar_expect_tx_warp(&full[i], A_BYTES + B_BYTES);
-                load_w(i, kb_lo + i, n0);
+                kp_mbar_expect_tx_warp(&full[i], STAGE);
+                load_w(i, kb_lo + i * NB, n0);
             }
         }
         if (lane == 0) KP_TRACE_MARK_LANE(0);
@@ -305,31 +328,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int s = 0;                                                    // stage, and the parity of its round
         uint32_t ph = 0;
         bool ok = true;
+#pragma unroll 1
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             const int tile = unit / S, part = unit - tile * S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
             const int kb_lo = part * p.kb_per_part, kb_hi = S > 1 ? min(n_kb, kb_lo + p.kb_per_part) : n_kb;
-            for (int kb = kb_lo; kb < kb_hi; kb++) {
-                unsigned char* a_dst = tiles + (size_t)s * (A_BYTES + B_BYTES);
+#pragma unroll 1
+            for (int kb = kb_lo; kb < kb_hi; kb += NB) {
+                unsigned char* a_dst = tiles + (size_t)s * STAGE;
                 if (pre > 0) {
                     pre--;                                            // armed, W on its way: only A is missing
                 } else {
                     ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&empty[s], ph ^ 1));
                     if (!ok) { *abort_flag = 1; break; }
-                    kp_mbar_expect_tx_warp(&full[s], A_BYTES + B_BYTES);
+                    kp_mbar_expect_tx_warp(&full[s], STAGE);
                     load_w(s, kb, n0);
                 }
-                kp_tma_load_2d_warp(a_dst, &tmA, kb * TC_BK, m0, &full[s]);
+                if (NB > 1) kp_tma_load_3d_warp(a_dst, &tmA, 0, m0, kb, &full[s]);
+                else kp_tma_load_2d_warp(a_dst, &tmA, kb * TC_BK, m0, &full[s]);
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
-        if (S > 1) { __syncwarp(); kp_cluster_sync_arrive(); }
-    } else if (warp == 1) {
-        kp_pdl_begin();
+    };
+    const auto multiply = [&](auto nb) {
+        constexpr int NB = decltype(nb)::value;
+        const int STAGE = NB * (A_BYTES + B_BYTES);
         constexpr uint32_t idesc = kp_umma_idesc(TC_BM, BN);
         int s = 0, b2 = 0;                                                // stage; set of accumulators of this unit
         uint32_t ph = 0, set_ph = 1;                                      // (both sets are empty at first)
         bool ok = true;
+#pragma unroll 1
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph));
             if (!ok) { *abort_flag = 1; break; }
@@ -338,20 +366,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int part = unit % S;
             const int kb_lo = part * p.kb_per_part, kb_hi = S > 1 ? min(n_kb, kb_lo + p.kb_per_part) : n_kb;
             int part_kb = 0;                                              // k-blocks in the accumulator so far
-            for (int kb = kb_lo; kb < kb_hi; kb++) {
-                if (part_kb == p.kb_per_part) { part_kb = 0; tmem_d += BN; }
+#pragma unroll 1
+            for (int kb = kb_lo; kb < kb_hi; kb += NB) {
                 ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
                 if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
-                const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * (A_BYTES + B_BYTES));
-                // four MMAs of 16 columns (32 bytes along K inside the swizzled row: +2 in the address field)
-                kp_umma_bf16_box(tmem_d, kp_umma_desc(a_addr), kp_umma_desc(a_addr + A_BYTES), idesc, part_kb++ != 0);
+                const uint32_t a_addr = kp_smem_u32(tiles + (size_t)s * STAGE);
+#pragma unroll
+                for (int j = 0; j < NB; j++) {
+                    if (j > 0 && kb + j >= kb_hi) break;
+                    if (part_kb == p.kb_per_part) { part_kb = 0; tmem_d += BN; }
+                    // four MMAs of 16 columns (32 bytes along K inside the swizzled row: +2 in the address field)
+                    kp_umma_bf16_box(tmem_d, kp_umma_desc(a_addr + j * A_BYTES), kp_umma_desc(a_addr + NB * A_BYTES + j * B_BYTES), idesc, part_kb++ != 0);
+                }
                 kp_umma_commit_warp(&empty[s]);                           // the stage is free when these MMAs have read it
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
             if (ok) kp_umma_commit_warp(&acc_full[b2]);                   // arrives when every MMA of the unit has completed
             if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
         }
+    };
+    if (warp == 0) {
+        if (p.kb_stage == 1) produce(TcInt<1>{}); else produce(TcInt<2>{});
+        if (S > 1) { __syncwarp(); kp_cluster_sync_arrive(); }
+    } else if (warp == 1) {
+        kp_pdl_begin();
+        if (p.kb_stage == 1) multiply(TcInt<1>{}); else multiply(TcInt<2>{});
         if (S > 1) { __syncwarp(); kp_cluster_sync_arrive(); }
     } else {
         kp_pdl_begin();
@@ -362,6 +402,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int b2 = 0;
         uint32_t set_ph = 0;
         bool ok = true;
+#pragma unroll 1
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             const int tile = unit / S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
@@ -377,10 +418,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (++b2 == p.n_sets) { b2 = 0; set_ph ^= 1; }
             if (S == 1) {
 #pragma unroll 1
-                for (int c = half * 32; c < N_OUT_TILE; c += 32 * TC_EPI_PER_Q) {
-                    float g[32], up[32];
+                for (int c = half * TC_PIECE; c < N_OUT_TILE; c += TC_PIECE * TC_EPI_PER_Q) {
+                    float g[TC_PIECE], up[TC_PIECE];
                     tc_sums<EPI, BN, true>(p, lane_base + c, g, up);
-                    if (m < p.M) tc_finish<EPI, 32>(p, n_out, g, up, m, n0 + c);
+                    if (m < p.M) tc_finish<EPI, TC_PIECE>(p, n_out, g, up, m, n0 + c);
                 }
                 // this warp has read the accumulators out: hand them back to the MMA warp
                 kp_tc_fence_before();
@@ -421,7 +462,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             // Its own, by all epilogue threads: VI pieces of four columns of a row at a time; the old values of an accumulated
             // output are asked for before the wait.
-            constexpr int VI = TC_GATED(EPI) ? 2 : 4, NT = TC_EPI_PER_Q * 128;
+            constexpr int VI = TC_VI, NT = TC_EPI_PER_Q * 128;
             const int n_vec = own * 2 * R;
             const bool old_apart = EPI == EPI_ACCUM_F32 && p.vec_ok;
             bool here = false;
@@ -447,7 +488,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int v = 0; v < VI; v++)
 #pragma unroll
                     for (int j = 0; j < 4; j++) g[v][j] = up[v][j] = 0.f;
-#pragma unroll 2
+#pragma unroll 1
                 for (int part = 0; part < S; part++) {
                     const unsigned char* src = part == rank ? tiles + lo * EIGHT * R : recv + (part < rank ? part : part - 1) * own * EIGHT * R;
 #pragma unroll
@@ -548,6 +589,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (pair < n_tiles) {
             const int n0 = (pair / tiles_m) * N_OUT_TILE;
             pre = min(STAGES, n_kb);
+#pragma unroll 1
             for (int i = 0; i < pre; i++) {
                 if (rank == 0) kp_mbar_expect_tx_warp(&full[i], 2 * STAGE);
                 load_w(i, i, n0);
@@ -560,8 +602,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         int s = 0;
         uint32_t ph = 0;
         bool ok = true;
+#pragma unroll 1
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
+#pragma unroll 1
             for (int kb = 0; kb < n_kb; kb++) {
                 if (pre > 0) {
                     pre--;
@@ -582,14 +626,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             int s = 0, b2 = 0;
             uint32_t ph = 0, set_ph = 1;
             bool ok = true;
-            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+    #pragma unroll 1
+        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
                 ok = !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
                 uint32_t tmem_d = tmem_base + (uint32_t)(b2 * p.inner * BN);
                 int part_kb = 0;
-                for (int kb = 0; kb < n_kb; kb++) {
+    #pragma unroll 1
+            for (int kb = 0; kb < n_kb; kb++) {
                     if (part_kb == p.kb_per_part) { part_kb = 0; tmem_d += BN; }
                     ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
                     if (!ok) { *abort_flag = 1; break; }
@@ -612,6 +658,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         int b2 = 0;
         uint32_t set_ph = 0;
         bool ok = true;
+#pragma unroll 1
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM + q * 32, n0 = (tile / tiles_m) * N_OUT_TILE;
             if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) { ok = false; break; }
@@ -712,9 +759,9 @@ static int tc_n_sm() {
 // Shared memory of a launch: `stages` ring stages with the slack behind a short last stage, or a cluster's exchange of sums if
 // that is more (`area`); barriers, alignment, and what other CTAs send apart from that (`apart`).
 struct TcSmem { int stages, area, apart; size_t bytes; };
-static TcSmem tc_smem(int M, int a_rows, int bn, bool gated, int splits) {
+static TcSmem tc_smem(int M, int a_rows, int bn, bool gated, int splits, int kb_stage = 1) {
     TcSmem t = {};
-    const int rows = M < TC_BM ? M : TC_BM, stage = a_rows * TC_BK * 2 + bn * TC_BK * 2;
+    const int rows = M < TC_BM ? M : TC_BM, stage = kb_stage * (a_rows + bn) * TC_BK * 2;
     const int slack = (TC_BM - a_rows) * TC_BK * 2;            // the MMA's reads past a short last stage
     // the most that a CTA of a cluster is sent: the others' sums of its output columns, which are counted in eights
     const int eights = bn / (gated ? 16 : 8), recv = (splits - 1) * ((eights + splits - 1) / splits) * (gated ? 64 : 32) * rows;
@@ -760,7 +807,7 @@ static int max_clusters(int cluster, size_t smem) {
 
 template <int BN, int EPI>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tw, TcArgs a, cudaStream_t s) {
-    const TcSmem sm = tc_smem(a.M, a.a_rows, BN, TC_GATED(EPI), a.splits);
+    const TcSmem sm = tc_smem(a.M, a.a_rows, BN, TC_GATED(EPI), a.splits, a.kb_stage);
     if (sm.bytes > KP_SMEM_MAX) return KP_ERR_UNSUPPORTED;
     a.n_stages = sm.stages; a.area = sm.area; a.recv_apart = sm.apart > 0;
     const size_t smem = sm.bytes;
@@ -827,6 +874,13 @@ static int tc_max_clusters(int bn, int epi, int cluster, int a_rows) {
 // How a product runs: the width of its tiles, its parts along K, and whether the parts of a tile are shared by the CTAs of a
 // cluster or run one after the other, by one CTA or a pair of them.
 struct TcChoice { int bn, parts; bool cluster, pair; };
+
+// K-blocks a stage (see the top)
+#define TC_KB_STAGE_BYTES (64 * 1024)
+static int tc_kb_stage(int a_rows, int bn) {
+    const int kb = (a_rows + bn) * TC_BK * 2;
+    return 2 * kb <= TC_KB_STAGE_BYTES ? 2 : 1;
+}
 
 // Sets of accumulators (one a part) that tensor memory's 512 columns have room for: two, so that the epilogue of a tile runs
 // under the main loop of the next, one, or none.
@@ -1006,10 +1060,17 @@ static int tc_run(const void* A, int lda, const void* W, int ldw, const float* b
     for (a.tmem_cols = 32; a.tmem_cols < a.n_sets * a.inner * bn;) a.tmem_cols *= 2;
     a.a_rows = tc_a_rows(M);
     cudaStream_t s = (cudaStream_t)stream;
+    a.kb_stage = !ch.pair && K % TC_BK == 0 && n_kb > 1 ? tc_kb_stage(a.a_rows, bn) : 1;
     alignas(64) CUtensorMap ta, tw;
-    int st = kp_make_map_bf16_2d(&ta, A, (unsigned long long)M, K, lda, TC_BK, a.a_rows);
-    if (st) return st;
-    st = kp_make_map_bf16_2d(&tw, W, (unsigned long long)N, K, ldw, TC_BK, pair_bn ? pair_bn / 2 : (epi == EPI_SWIGLU ? bn / 2 : bn));
+    int st;
+    if (a.kb_stage > 1) {
+        st = kp_make_map_bf16_groups(&ta, A, (unsigned long long)M, n_kb, lda, a.a_rows, a.kb_stage);
+        if (!st) st = epi == EPI_SWIGLU ? kp_make_map_bf16_halves(&tw, W, (unsigned long long)a.ff, n_kb, ldw, bn / 2, a.kb_stage)
+                                        : kp_make_map_bf16_groups(&tw, W, (unsigned long long)N, n_kb, ldw, bn, a.kb_stage);
+    } else {
+        st = kp_make_map_bf16_2d(&ta, A, (unsigned long long)M, K, lda, TC_BK, a.a_rows);
+        if (!st) st = kp_make_map_bf16_2d(&tw, W, (unsigned long long)N, K, ldw, TC_BK, pair_bn ? pair_bn / 2 : (epi == EPI_SWIGLU ? bn / 2 : bn));
+    }
     if (st) return st;
     if (pair_bn) {
 #define TC_PAIR_BN(EPI, PARTS) return pair_bn == 256 ? launch_pair<256, EPI, PARTS>(ta, tw, a, s) : launch_pair<128, EPI, PARTS>(ta, tw, a, s)

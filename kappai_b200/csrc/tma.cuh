@@ -33,17 +33,24 @@ __device__ __forceinline__ unsigned long long kp_now_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// false if the barrier did not flip within limit_ns
-__device__ __forceinline__ bool kp_mbar_wait_bounded(uint64_t* bar, uint32_t parity,
-                                                     unsigned long long limit_ns = KP_TMA_WAIT_NS) {
-    if (kp_mbar_try_wait(bar, parity)) return true;
+// (out of line: kernels wait in many places, and what a place does not find ready at once it can afford to call for)
+__device__ __noinline__ bool kp_mbar_wait_long(uint32_t bar, uint32_t parity, unsigned long long limit_ns) {
     const unsigned long long t0 = kp_now_ns();
     for (;;) {
 #pragma unroll 1
-        for (int i = 0; i < 64; i++)
-            if (kp_mbar_try_wait(bar, parity)) return true;
+        for (int i = 0; i < 64; i++) {
+            uint32_t ok;
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+            if (ok) return true;
+        }
         if (kp_now_ns() - t0 > limit_ns) return false;
     }
+}
+// false if the barrier did not flip within limit_ns
+__device__ __forceinline__ bool kp_mbar_wait_bounded(uint64_t* bar, uint32_t parity,
+                                                     unsigned long long limit_ns = KP_TMA_WAIT_NS) {
+    return kp_mbar_try_wait(bar, parity) || kp_mbar_wait_long(kp_smem_u32(bar), parity, limit_ns);
 }
 // A CTA that gave up a wait must not leave while bulk copies into its shared memory may still be under way
 // (the memory could be handed to the next CTA meanwhile): it lingers for a moment that is far longer than any
@@ -80,6 +87,16 @@ __device__ __forceinline__ void kp_tma_load_2d_warp(void* dst, const CUtensorMap
     asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
                  " @e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}"
                  ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(kp_smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void kp_tma_load_3d_warp(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n}"
+                 ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(kp_smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void kp_tma_load_4d_warp(void* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+    asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+                 " @e cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n}"
+                 ::"r"(kp_smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(kp_smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void kp_mbar_expect_tx_warp(uint64_t* bar, uint32_t bytes) {
     asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
@@ -136,6 +153,22 @@ static inline int kp_make_map_bf16_groups(CUtensorMap* map, const void* base, un
     cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)(box_groups ? box_groups : groups)};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : KP_ERR_UNSUPPORTED;
+}
+
+// The same of two blocks of rows, `half` rows apart (gate and up): (64 columns, rows of a block, two blocks, groups); a box takes
+// box_rows rows of both blocks and box_groups groups, and lies as box_groups tiles of 2 box_rows rows of 128 bytes
+static inline int kp_make_map_bf16_halves(CUtensorMap* map, const void* base, unsigned long long half, int groups, long long ld, int box_rows,
+                                          int box_groups) {
+    KpEncodeTiledFn fn = kp_encode_tiled_fn();
+    if (!fn) return KP_ERR_UNSUPPORTED;
+    cuuint64_t dims[4] = {64, (cuuint64_t)half, 2, (cuuint64_t)groups};
+    cuuint64_t strides[3] = {(cuuint64_t)ld * 2, (cuuint64_t)half * ld * 2, 128};
+    cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 2, (cuuint32_t)box_groups};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : KP_ERR_UNSUPPORTED;
