@@ -333,7 +333,7 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_acc, const floa
 // ...) chunk by chunk.  The arithmetic is that of the kernel above, so a row's result does not depend on which
 // of the two ran.  (With 64 rows the kernel above took 10.7 us for 2048 small CTAs of 256 threads.)
 #define MERGE_WARP_CHUNKS 64
-#define MERGE_WARP_BLOCK 16                               // chunks whose sums a warp fetches at a time
+#define MERGE_WARP_BLOCK 8                                // chunks whose sums a warp fetches at a time
 template <typename T>
 __global__ void attn_merge_warp_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                        const int* __restrict__ positions, T* __restrict__ out, int ldo, int n_chunks,
@@ -370,6 +370,7 @@ __global__ void attn_merge_warp_kernel(const float* __restrict__ part_acc, const
     if (sink) m = fmaxf(m, sink[h]);
     const float w0 = lane < n ? expf(m0 - m) : 0.f, w1 = lane + 32 < n ? expf(m1 - m) : 0.f;
     float l = sink ? expf(sink[h] - m) : 0.f, v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
     for (int c0 = 0; c0 < n; c0 += B) {
         if (c0) fetch(c0);
 #pragma unroll

@@ -340,6 +340,7 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
         const int box = min(page_size, AM_TILE), n_boxes = AR_CHUNK / box;   // keys a box; at most 32 boxes (pages of 8 keys)
         int k = 0;
         bool alive = true;
+#pragma unroll 1
         for (int it0 = blockIdx.x; it0 < n_items && alive; it0 += 32 * gridDim.x) {
             // 32 candidates at a time, one a lane: which of them have keys to read
             const int it = it0 + lane * gridDim.x;
@@ -360,6 +361,7 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
                 if (valid) c_seg = row_seg[c_row];
             }
             unsigned todo = __ballot_sync(0xffffffffu, valid);
+#pragma unroll 1
             while (todo && alive) {
                 const int src = __ffs(todo) - 1;
                 todo &= todo - 1;
@@ -401,6 +403,7 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
             }
         }
         // no more items: a mark for each group
+#pragma unroll 1
         for (int e = 0; e < AR_GROUPS && alive; e++, k++) {
             const int s = k % AR_STAGES;
             if (lane == 0) {
@@ -424,6 +427,7 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
     float* wl = wm + AR_NW * AM_RMAX;
     const int gtid = tid - grp * AR_NW * 32;                          // thread of the group
     auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(AR_NW * 32) : "memory"); };
+#pragma unroll 1
     for (int k = grp;; k += AR_GROUPS) {
         const int s = k % AR_STAGES;
         // The four warps of the group leave the loop together or not at all (the group's barriers below count all
@@ -455,6 +459,7 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
         // V rows of keys that this row does not read hold whatever was there: zero them (P is 0 there, but
         // 0 * NaN is not); K rows need nothing, their scores are masked
         if (t0 < k_lo || t0 + AM_TILE - 1 > k_hi) {
+#pragma unroll 1
             for (int idx = lane; idx < AM_TILE * (HD / 8); idx += 32) {
                 const int r = idx / (HD / 8), c = idx % (HD / 8);
                 if (t0 + r < k_lo || t0 + r > k_hi) *reinterpret_cast<uint4*>(tile_chunk<HD>(Vt, r, c)) = make_uint4(0, 0, 0, 0);

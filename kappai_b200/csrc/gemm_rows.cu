@@ -31,7 +31,9 @@
 // 335 | 312; of eight requests (see rows_run) 555 | 539 | 567 and 369 | 378 | 366.
 // Big and small, KB, 64 steps of one request, 1.2B shape, ms: 148 + 78 32.1, 128 + 96 31.9, 116 + 110 32.2, 164 + 62 33.2.
 //
-// Epilogues as in gemm_stream.cu.  K a multiple of 512.
+// Epilogues as in gemm_stream.cu.  K a multiple of 512.  Loops are not unrolled where that gains nothing back to back: in a step
+// the kernels' code is fetched anew at every launch (the conv step's 27 KB of it became 16; with the attention kernels', the
+// merge's 34 KB 19, a step of eight requests of the 1.2B shape took 515 us instead of 541).
 #include "mma.cuh"
 
 #define EPI_STORE 0
@@ -128,6 +130,7 @@ gemm_rows_kernel(const RowsArgs p) {
 
     KP_TRACE_MARK(0);
     pdl_launch_dependents();                                             // (what comes next reads nothing before its own wait)
+#pragma unroll 1
     for (int i = 0; i < S; i++) {
         if (i < total) { load_w(ld_tile, ld_c, ld_s); advance(); }
         cp_async_commit();
@@ -146,6 +149,7 @@ gemm_rows_kernel(const RowsArgs p) {
         for (int r = 0; r < R; r++) ss[r] = 0.f;
         pdl_wait();
         KP_TRACE_MARK(1);
+#pragma unroll 1
         for (int c0 = 0; c0 < n_ch; c0 += 2 * CU) {
             float4 v[R][CU];
 #pragma unroll
@@ -181,6 +185,7 @@ gemm_rows_kernel(const RowsArgs p) {
     } else {
         pdl_wait();
         KP_TRACE_MARK(1);
+#pragma unroll 1
         for (int i = 0; i < S; i++) {
             if (i < total) load_a(i % n_ch, i);
             cp_async_commit();
@@ -189,24 +194,23 @@ gemm_rows_kernel(const RowsArgs p) {
 
     int s = 0, buf = 0;
     float scale = 1.f;                                                   // (NORM) 1 / root mean square of this thread's row
+#pragma unroll 1
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
         const int n0 = tile * TROWS;
         // what the epilogue needs beside the sums is asked for now: its trips to L2 run under the main loop
-        float pre_c = 0.f, pre_hist[3] = {0.f, 0.f, 0.f}, pre_cw[4] = {0.f, 0.f, 0.f, 0.f};
+        float pre_c = 0.f, pre_hist[2] = {0.f, 0.f}, pre_cw[3] = {0.f, 0.f, 0.f};
         const int om = threadIdx.x / TROWS, on = n0 + threadIdx.x % TROWS;   // this thread's output (the first TROWS * M threads)
         const bool mine = om < M && on < n_out;
         if (mine) {
             if (EPI == EPI_ACCUM_F32) pre_c = ((const float*)p.C)[(size_t)om * p.ldc + on];
-            if (EPI == EPI_CONV_STEP && p.conv_k <= 4) {
+            if (EPI == EPI_CONV_STEP && p.conv_k == 3) {
                 const bool fresh = p.seg_pos[om] == 0;
-                const float* st = p.conv_state + (size_t)p.seg_slot[om] * (p.conv_k - 1) * p.ff;
-                const float* cw = p.conv_w + (size_t)on * p.conv_k;
+                const float* st = p.conv_state + (size_t)p.seg_slot[om] * 2 * p.ff;
+                const float* cw = p.conv_w + (size_t)on * 3;
 #pragma unroll
-                for (int k = 0; k < 3; k++)
-                    if (k < p.conv_k - 1) pre_hist[k] = fresh ? 0.f : st[(size_t)k * p.ff + on];
+                for (int k = 0; k < 2; k++) pre_hist[k] = fresh ? 0.f : st[(size_t)k * p.ff + on];
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (k < p.conv_k) pre_cw[k] = cw[k];
+                for (int k = 0; k < 3; k++) pre_cw[k] = cw[k];
             }
         }
         float acc[MT][4];
@@ -214,6 +218,7 @@ gemm_rows_kernel(const RowsArgs p) {
         for (int a = 0; a < MT; a++)
 #pragma unroll
             for (int i = 0; i < 4; i++) acc[a][i] = 0.f;
+#pragma unroll 1
         for (int c = 0; c < n_ch; c++) {
             cp_async_wait<S - 1>();                                      // this stage has come, all but the S - 1 behind it
             __syncwarp();
@@ -275,29 +280,25 @@ gemm_rows_kernel(const RowsArgs p) {
                 const int d = p.ff, Kc = p.conv_k;
                 float* st = p.conv_state + (size_t)p.seg_slot[m] * (Kc - 1) * d;
                 const float bx = __fmul_rn(b, xq);
-                float hist[15], tap[16];
-                if (Kc <= 4) {
-#pragma unroll
-                    for (int k = 0; k < 3; k++) hist[k] = pre_hist[k];
-#pragma unroll
-                    for (int k = 0; k < 4; k++) tap[k] = pre_cw[k];
+                float sum;
+                if (Kc == 3) {
+                    sum = __fadd_rn(__fadd_rn(__fmul_rn(pre_hist[0], pre_cw[0]), __fmul_rn(pre_hist[1], pre_cw[1])), __fmul_rn(bx, pre_cw[2]));
+                    st[n] = pre_hist[1];
+                    st[(size_t)d + n] = bx;
                 } else {
                     const bool fresh = p.seg_pos[m] == 0;
                     const float* cw = p.conv_w + (size_t)n * Kc;
-                    for (int k = 0; k < Kc - 1; k++) hist[k] = fresh ? 0.f : st[(size_t)k * d + n];
-                    for (int k = 0; k < Kc; k++) tap[k] = cw[k];
-                }
-                float sum;
-                if (Kc == 3) {
-                    sum = __fadd_rn(__fadd_rn(__fmul_rn(hist[0], tap[0]), __fmul_rn(hist[1], tap[1])), __fmul_rn(bx, tap[2]));
-                } else {
-                    sum = __fmul_rn(bx, tap[Kc - 1]);
-                    for (int k = 0; k < Kc - 1; k++) sum = __fadd_rn(sum, __fmul_rn(hist[k], tap[k]));
+                    sum = __fmul_rn(bx, cw[Kc - 1]);
+#pragma unroll 1
+                    for (int k = 0; k < Kc - 1; k++) {
+                        const float h = fresh ? 0.f : st[(size_t)k * d + n];
+                        sum = __fadd_rn(sum, __fmul_rn(h, cw[k]));
+                        if (k > 0) st[(size_t)(k - 1) * d + n] = h;
+                    }
+                    st[(size_t)(Kc - 2) * d + n] = bx;
                 }
                 if (p.conv_bias) sum = __fadd_rn(sum, p.conv_bias[n]);
                 ((bf16*)p.C)[o] = from_f32<bf16>(__fmul_rn(cq, sum));
-                for (int k = 0; k + 1 < Kc - 1; k++) st[(size_t)k * d + n] = hist[k + 1];
-                st[(size_t)(Kc - 2) * d + n] = bx;
             } else if (EPI == EPI_SWIGLU) {
                 float u = sum_of(8 + lr);
                 if (p.bias) u += p.bias[p.ff + n];

@@ -186,17 +186,20 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
     const int ahead = n_stages - 1;
     KP_TRACE_MARK(0);
     if (!p.w_settled) pdl_wait();
+#pragma unroll 1
     for (int it = 0; it < ahead && it < total; it++) load_w(it);
     pdl_wait();
     KP_TRACE_MARK(1);
     pdl_launch_dependents();
     // (the first stages' W is part of the first stage's group: it was asked for first and comes first)
+#pragma unroll 1
     for (int it = 0; it < ahead; it++) {
         if (it < total) load_a(it);
         f32_cp_commit();
     }
 
     f32x2 acc[R][MB];
+#pragma unroll 1
     for (int it = 0; it < total; it++) {
         if (it % PER_JOB == 0) {
 #pragma unroll
@@ -242,6 +245,7 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
     }
     __syncthreads();
     const int n_groups = (K + F32_GROUP - 1) / F32_GROUP;
+#pragma unroll 1
     for (int e = threadIdx.x; e < MB * 8 * R; e += blockDim.x) {
         const int m = m0 + e / (8 * R), n = n0 + e % (8 * R);
         if (m >= p.M || n >= p.N) continue;

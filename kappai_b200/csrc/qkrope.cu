@@ -50,6 +50,7 @@ qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
     float* x = buf[warp];
 
     float ss = 0.f;
+#pragma unroll 2
     for (int i = lane; i < hd; i += 32) {
         const float v = to_f32(src[i]);
         x[i] = v;
@@ -59,12 +60,14 @@ qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
     if (w) {
         ss = warp_sum(ss);
         const float scale = 1.0f / sqrtf(ss / (float)norm_dim + eps);
+#pragma unroll 2
         for (int i = lane; i < hd; i += 32) x[i] = (x[i] * scale) * w[i];
     }
     __syncwarp();
     if (kind != 2 && cos_tab) {
         const int half = rot >> 1;
         const size_t tb = (size_t)positions[row] * half;
+#pragma unroll 1
         for (int j = lane; j < half; j += 32) {
             const int ia = interleaved ? 2 * j : j;
             const int ib = interleaved ? 2 * j + 1 : j + half;
@@ -77,13 +80,16 @@ qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
     }
     if (norm_after && kind != 2) {
         float sq = 0.f;
+#pragma unroll 1
         for (int i = lane; i < hd; i += 32) sq = fmaf(x[i], x[i], sq);
         sq = warp_sum(sq);
         const float scale = 1.0f / sqrtf(sq / (float)norm_dim + eps);
+#pragma unroll 1
         for (int i = lane; i < hd; i += 32) x[i] *= scale;
     }
     if (kind == 0 && temp_every > 0.f) {
         const float tq = kp_query_temperature(positions[row], temp_coef, temp_every);
+#pragma unroll 1
         for (int i = lane; i < hd; i += 32) x[i] *= tq;
     }
     T* dst;
@@ -98,6 +104,7 @@ qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
         const int g = kind == 1 ? head - H : head - H - G;
         dst = cache + ((((size_t)page * 2 + (kind - 1)) * G + g) * page_size + off) * hd;
     }
+#pragma unroll 2
     for (int i = lane; i < hd; i += 32) dst[i] = from_f32<T>(x[i]);
 }
 

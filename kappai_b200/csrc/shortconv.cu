@@ -336,17 +336,23 @@ __global__ void shortconv_decode_kernel(const T* __restrict__ p, int ldp, const 
     float* st = state + (size_t)seg_slot[row] * (K - 1) * d;
     const float* wc = w + (size_t)c * K;
     const float bx = bx_of(p, row, ldp, d, c);
-    float hist[KP_CONV_MAX_K - 1];
-    for (int k = 0; k < K - 1; k++) hist[k] = fresh ? 0.f : st[(size_t)k * d + c];
-    float sum;
+    const float cg = to_f32(p[(size_t)row * ldp + d + c]);
     if (K == 3) {
-        sum = conv_sum3(hist[0], hist[1], bx, wc[0], wc[1], wc[2]);
-    } else {
-        sum = tap(bx, wc[K - 1]);
-        for (int k = 0; k < K - 1; k++) sum = add_tap(sum, hist[k], wc[k]);
+        const float h0 = fresh ? 0.f : st[c], h1 = fresh ? 0.f : st[(size_t)d + c];
+        const float sum = conv_sum3(h0, h1, bx, wc[0], wc[1], wc[2]);
+        out[(size_t)row * ldo + c] = from_f32<T>(gate_out(cg, sum, bias != nullptr, bias ? bias[c] : 0.f));
+        st[c] = h1;
+        st[(size_t)d + c] = bx;
+        return;
     }
-    out[(size_t)row * ldo + c] = from_f32<T>(gate_out(to_f32(p[(size_t)row * ldp + d + c]), sum, bias != nullptr,
-                                                      bias ? bias[c] : 0.f));
+    float hist[KP_CONV_MAX_K - 1];
+#pragma unroll 1
+    for (int k = 0; k < K - 1; k++) hist[k] = fresh ? 0.f : st[(size_t)k * d + c];
+    float sum = tap(bx, wc[K - 1]);
+#pragma unroll 1
+    for (int k = 0; k < K - 1; k++) sum = add_tap(sum, hist[k], wc[k]);
+    out[(size_t)row * ldo + c] = from_f32<T>(gate_out(cg, sum, bias != nullptr, bias ? bias[c] : 0.f));
+#pragma unroll 1
     for (int k = 0; k + 1 < K - 1; k++) st[(size_t)k * d + c] = hist[k + 1];
     st[(size_t)(K - 2) * d + c] = bx;
 }
