@@ -72,6 +72,8 @@ __device__ __forceinline__ int merge_front(int first_hi, int chunk_keys, int c_l
     return front_slot0 >= 0 ? (first_hi + AD_CHUNK_KEYS - 1) / AD_CHUNK_KEYS : front_chunks(first_hi, chunk_keys, c_lo);
 }
 
+// `out`: null, or where the rows go at once because every row has this one chunk and nothing else enters (what the merge makes of
+// one chunk: the same bits).
 // HD, RR: head size and query heads per kv head fixed at compile time (loops unroll, loads overlap);
 // 0 means "taken from the arguments".
 template <typename T, int HD, int RR>
@@ -79,7 +81,8 @@ __global__ void __launch_bounds__(AD_THREADS)
 attn_split_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache, const int* __restrict__ block_table,
                   int max_blocks, const int* __restrict__ row_seg, const int* __restrict__ positions,
                   float* __restrict__ part_acc, float* __restrict__ part_ml, int n_chunks, float scale, int window,
-                  int page_size, int H, int G, int hd_rt, int block, int keep_first, int slot0, int front, float cap, int pool) {
+                  int page_size, int H, int G, int hd_rt, int block, int keep_first, int slot0, int front, float cap, int pool,
+                  T* __restrict__ out, int ldo, float out_scale) {
     kp_pdl_begin();
     extern __shared__ float smem[];
     const int hd = HD ? HD : hd_rt;
@@ -107,20 +110,29 @@ attn_split_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache,
         qs[i] = to_f32(q[(size_t)row * ldq + (size_t)(g * R) * hd + i]);
     __syncthreads();
 
-    // (head size 64, 16-bit cache) the values this thread multiplies later are fetched now, so that their
-    // latency passes under the scores and the softmax: thread = (pair of dims, slice of 32 keys)
-    constexpr bool PREFETCH_V = (HD == 64) && (sizeof(T) == 2);
-    uint32_t vpre[PREFETCH_V ? 32 : 1];
+    // (head size 64) the values this thread multiplies later are fetched now, so that their latency passes under the scores
+    // and the softmax: thread = (pair of dims, slice of 32 keys); of a float32 cache where the heads that share it are known
+    // (a step of 8 float32 requests of the 350M shape with 60 keys each 1036 -> 902 us, with the instance for two heads a kv
+    // head, which has the code of two and not of eight; one request of the 1.2B shape 970 -> 869)
+    constexpr bool PREFETCH_V = HD == 64 && (sizeof(T) == 2 || RR > 0);
+    constexpr int VW = sizeof(T) == 2 ? 1 : 2;
+    uint32_t vpre[PREFETCH_V ? 32 : 1][VW];
     if (PREFETCH_V) {
         const int pair_p = tid & 31, slice_p = tid >> 5;
+        int page = (c0 + slice_p * 32) / page_size, in_page = c0 + slice_p * 32 - page * page_size;
+        const T* base = cache + v_off + 2 * pair_p;
 #pragma unroll
         for (int j = 0; j < 32; j++) {
             const int key2 = c0 + slice_p * 32 + j;
-            uint32_t v = 0;
-            if (key2 <= k_hi && (key2 >= k_lo || key2 < first_hi))
-                v = *reinterpret_cast<const uint32_t*>(cache + (size_t)bt[key2 / page_size] * page_stride + v_off +
-                                                       (size_t)(key2 % page_size) * hd + 2 * pair_p);
-            vpre[j] = v;
+            uint2 v = make_uint2(0, 0);
+            if (key2 <= k_hi && (key2 >= k_lo || key2 < first_hi)) {
+                const T* src = base + (size_t)bt[page] * page_stride + (size_t)in_page * hd;
+                if (VW == 1) v.x = *reinterpret_cast<const uint32_t*>(src);
+                else v = *reinterpret_cast<const uint2*>(src);
+            }
+            vpre[j][0] = v.x;
+            if (VW == 2) vpre[j][VW - 1] = v.y;
+            if (++in_page == page_size) { in_page = 0; page++; }
         }
     }
 
@@ -191,7 +203,7 @@ attn_split_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache,
 #pragma unroll
         for (int j = 0; j < 32; j++) {
             const int kk = slice * 32 + j;                       // keys outside the row's range have p = 0
-            const float v0 = __uint_as_float(vpre[j] << 16), v1 = __uint_as_float(vpre[j] & 0xffff0000u);
+            const float v0 = __uint_as_float(VW == 2 ? vpre[j][0] : vpre[j][0] << 16), v1 = __uint_as_float(VW == 2 ? vpre[j][VW - 1] : vpre[j][0] & 0xffff0000u);
 #pragma unroll
             for (int r = 0; r < AD_RMAX; r++) {
                 if (r < R) {
@@ -235,13 +247,19 @@ attn_split_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache,
         }
     }
     __syncthreads();
+#pragma unroll 1
     for (int e = tid; e < R * hd; e += AD_THREADS) {
         const int r = e / hd, d = e % hd;
         float v = 0.f;
         for (int sl = 0; sl < n_slices; sl++) v += red[((size_t)sl * R + r) * hd + d];
-        part_acc[(((size_t)row * H + g * R + r) * n_chunks + slot0 + chunk) * hd + d] = v;
+        if (out) {
+            const float l = stat_l[r], inv = l > 0.f ? out_scale / l : 0.f;
+            out[(size_t)row * ldo + (size_t)(g * R + r) * hd + d] = from_f32<T>(v * inv);
+        } else {
+            part_acc[(((size_t)row * H + g * R + r) * n_chunks + slot0 + chunk) * hd + d] = v;
+        }
     }
-    if (tid < R) {
+    if (tid < R && !out) {
         float* ml = part_ml + (((size_t)row * H + g * R + tid) * n_chunks + slot0 + chunk) * 2;
         ml[0] = stat_m[tid];
         ml[1] = stat_l[tid];
@@ -459,21 +477,25 @@ int kp_attention_split_pooled(const void* q, int ldq, const void* cache, const i
     float* part_ml = scratch + (size_t)n * H * n_slots * hd;
     cudaStream_t s = (cudaStream_t)stream;
     constexpr int SLOT0 = 0, FRONT = 0;
+    const bool whole = n_slots == 1 && keep_first == 0 && !sink;               // the chunk pass writes the rows itself
 #define AD_LAUNCH(T, HD, RR)                                                                                      \
     kp_launch_pdl(attn_split_kernel<T, HD, RR>, dim3(n_chunks, G, n), dim3(AD_THREADS), smem, s, (const T*)q, ldq, (const T*)cache, block_table,       \
                                                                 max_blocks, row_seg, positions, part_acc, part_ml,    \
-                                                                n_slots, scale, window, page_size, H, G, hd, block, keep_first, SLOT0, FRONT, cap, 0)
+                                                                n_slots, scale, window, page_size, H, G, hd, block, keep_first, SLOT0, FRONT, cap, 0, \
+                                                                whole ? (T*)out : (T*)nullptr, ldo, out_scale)
     KP_DISPATCH_DTYPE(dtype, T, {
         cudaError_t e0;
         if (hd == 64 && R == 4) e0 = AD_LAUNCH(T, 64, 4);
+        else if (hd == 64 && R == 2) e0 = AD_LAUNCH(T, 64, 2);
         else if (hd == 64) e0 = AD_LAUNCH(T, 64, 0);
         else if (hd == 128) e0 = AD_LAUNCH(T, 128, 0);
         else e0 = AD_LAUNCH(T, 0, 0);
         if (e0 != cudaSuccess) { cudaGetLastError(); return (int)e0; }      // the first launch that failed
+        if (whole) return kp_launch_status();
         if (pool > 0) {
             kp_launch_pdl(attn_split_kernel<T, 0, 0>, dim3(n_pool_chunks, G, n), dim3(AD_THREADS), smem, s, (const T*)q, ldq, (const T*)pool_cache,
                           pool_table, max_pool_blocks, row_seg, positions, part_acc, part_ml, n_slots, scale, window, page_size, H, G,
-                          hd, 0, 0, n_chunks, 2, cap, pool);
+                          hd, 0, 0, n_chunks, 2, cap, pool, (T*)nullptr, 0, 1.f);
         }
         return launch_merge<T>(part_acc, part_ml, positions, out, ldo, n_slots, AD_CHUNK, window, block, keep_first, sink, n, H, hd, s,
                                pool > 0 ? n_chunks : -1, out_scale, pool);
@@ -523,7 +545,8 @@ int kp_attention_front_chunks(const void* q, int ldq, const void* cache, const i
     float* part_ml = scratch + (size_t)n * H * n_chunks * hd;
     KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(attn_split_kernel<T, 0, 0>, dim3(n_front, G, n), dim3(AD_THREADS), smem, (cudaStream_t)stream,
                                                (const T*)q, ldq, (const T*)cache, block_table, max_blocks, row_seg, positions, part_acc,
-                                               part_ml, n_chunks, scale, window, page_size, H, G, hd, 0, keep_first, front_slot0, 1, 0.f, 0)));
+                                               part_ml, n_chunks, scale, window, page_size, H, G, hd, 0, keep_first, front_slot0, 1, 0.f, 0,
+                                               (T*)nullptr, 0, 1.f)));
     return kp_launch_status();
 }
 

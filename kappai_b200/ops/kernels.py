@@ -1340,7 +1340,8 @@ def attention_split(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Ten
          n_chunks, ctypes.c_float(scale), int(window or 0), int(block or 0), keep_first, _ptr(sink), ctypes.c_float(cap),
          ctypes.c_float(out_scale), *_pool_args(pooled), pooled.chunks(n_chunks) if pooled is not None else 0, page_size, n, H, G, hd,
          dtype_code(q.dtype), STREAM)
-    LAUNCHES[0] += 1 if pooled is None else 2
+    # (one chunk a row and nothing else: the chunk pass writes the rows itself)
+    LAUNCHES[0] += 2 if pooled is not None else int(n_chunks > 1 or keep_first > 0 or sink is not None)
     return out
 
 
