@@ -137,6 +137,8 @@ template <int EPI> __device__ __forceinline__ void f32_store(const F32Args& p, i
 // (a decode step of the 350M shape: 2 % of its time), those of A behind it.  In shared memory the eight 16-byte chunks of a row's stage are permuted
 // by the row (chunk c of row r at c ^ r), so the eight rows of a quarter warp read all banks once.
 //
+// SHARE: warps that share a job, each for MB / SHARE of the rows (see f32_rows).
+//
 // More rows than MB take the grid's y; W then comes from L2.  Measured (W from HBM): 8 rows by 2048 x 5632 in 13.3 us
 // (3.5 TB/s; 608 us with tiles of 64 x 64 and a chain of K), 11264 x 2048 in 23 us, 65536 x 2048 in 93 us (5.8 TB/s); one
 // row 10.6, 15.7 and 78 us (6.9 TB/s).  R = 4, MB = 16 reads shared memory least for its FMAs: 64 rows by 2048 x 5632 in
@@ -145,14 +147,20 @@ template <int EPI> __device__ __forceinline__ void f32_store(const F32Args& p, i
 #define F32R_JOB (4 * F32_GROUP)                      // columns of a job
 #define F32R_MAX_WARPS 8
 
-template <int R, int MB, int EPI>
-__global__ void __launch_bounds__(F32R_MAX_WARPS * 32)
+template <int R, int MB, int EPI, int SHARE>
+__global__ void __launch_bounds__(F32R_MAX_WARPS * SHARE * 32)
 gemm_f32_rows_kernel(const F32Args p, int n_stages) {
     constexpr int W_BYTES = 8 * R * 4 * F32R_COLS * 4, A_BYTES = MB * 4 * F32R_COLS * 4, STAGE = W_BYTES + A_BYTES;
     constexpr int PER_JOB = F32_GROUP / F32R_COLS;    // stages of a job
     extern __shared__ __align__(128) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    constexpr int MS = MB / SHARE;                    // rows of A that a warp sums
+    const int part = (threadIdx.x >> 5) % SHARE, warp = (threadIdx.x >> 5) / SHARE;       // part: which of the warps that share a job
+    const int lane = threadIdx.x & 31, n_warps = (blockDim.x >> 5) / SHARE;
     const int r = lane & 7, q = lane >> 3;
+    const auto job_sync = [&]() {
+        if (SHARE == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + warp), "n"(SHARE * 32) : "memory");
+    };
     const int n0 = blockIdx.x * 8 * R, m0 = blockIdx.y * MB;
     const int K = p.K, n_jobs = (K + F32R_JOB - 1) / F32R_JOB;
     unsigned char* ring = smem + (size_t)warp * n_stages * STAGE;
@@ -170,6 +178,7 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
         for (int g = 0; g < 4; g++)
 #pragma unroll
             for (int i = 0; i < 2 * R; i++) {
+                if ((g * 2 * R + i) % SHARE != part) continue;
                 const int row = i * 4 + cr, k = k0 + g * F32_GROUP;                       // row of the CTA's 8 R
                 const float* src = p.W + (size_t)min(n0 + row, p.N - 1) * p.ldw + k;
                 f32_cp16(dst + ((((row >> 3) * 4 + g) * 8 + (row & 7)) * 8 + (cc ^ (row & 7))) * 16, src, k < K);
@@ -179,8 +188,10 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
         unsigned char* dst = ring + (size_t)(it % n_stages) * STAGE + W_BYTES;
         const int k = col_of(it) + cc * 4 + cr * F32_GROUP;                               // stretch cr, chunk cc
 #pragma unroll
-        for (int m = 0; m < MB; m++)
+        for (int i = 0; i < MS; i++) {
+            const int m = part * MS + i;
             f32_cp16(dst + ((m * 4 + cr) * 8 + ((cc + 2 * cr) & 7)) * 16, p.A + (size_t)min(m0 + m, p.M - 1) * p.lda + k, k < K);
+        }
     };
 
     const int ahead = n_stages - 1;
@@ -198,14 +209,14 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
         f32_cp_commit();
     }
 
-    f32x2 acc[R][MB];
+    f32x2 acc[R][MS];
 #pragma unroll 1
     for (int it = 0; it < total; it++) {
         if (it % PER_JOB == 0) {
 #pragma unroll
             for (int i = 0; i < R; i++)
 #pragma unroll
-                for (int m = 0; m < MB; m++) acc[i][m] = 0;
+                for (int m = 0; m < MS; m++) acc[i][m] = 0;
         }
         // stage `it` has come: all but the ahead - 1 groups behind it
         switch (ahead) {
@@ -217,19 +228,19 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
             case 6: f32_cp_wait<5>(); break;
             default: f32_cp_wait<6>(); break;
         }
-        __syncwarp();
+        job_sync();
         if (it + ahead < total) { load_w(it + ahead); load_a(it + ahead); }
         f32_cp_commit();
         const unsigned char* st = ring + (size_t)(it % n_stages) * STAGE;
         const ulonglong2* wr = reinterpret_cast<const ulonglong2*>(st) + (q * 8 + r) * 8;
-        const ulonglong2* ar = reinterpret_cast<const ulonglong2*>(st + W_BYTES) + q * 8;
+        const ulonglong2* ar = reinterpret_cast<const ulonglong2*>(st + W_BYTES) + part * MS * 32 + q * 8;
 #pragma unroll
         for (int c = 0; c < F32R_COLS / 4; c++) {
             ulonglong2 w[R];
 #pragma unroll
             for (int i = 0; i < R; i++) w[i] = wr[i * 256 + (c ^ r)];
 #pragma unroll
-            for (int m = 0; m < MB; m++) {
+            for (int m = 0; m < MS; m++) {
                 const ulonglong2 a = ar[m * 32 + ((c + 2 * q) & 7)];
 #pragma unroll
                 for (int i = 0; i < R; i++) { f32_fma2(acc[i][m], a.x, w[i].x); f32_fma2(acc[i][m], a.y, w[i].y); }
@@ -240,7 +251,7 @@ gemm_f32_rows_kernel(const F32Args p, int n_stages) {
 #pragma unroll
             for (int i = 0; i < R; i++)
 #pragma unroll
-                for (int m = 0; m < MB; m++) red[((size_t)g * MB + m) * 8 * R + i * 8 + r] = f32_halves(acc[i][m]);
+                for (int m = 0; m < MS; m++) red[((size_t)g * MB + part * MS + m) * 8 * R + i * 8 + r] = f32_halves(acc[i][m]);
         }
     }
     __syncthreads();
@@ -416,13 +427,26 @@ static F32Choice f32_choose(int M, int N, int K) {
     return {0, 0, 0, 0, 0};
 }
 
-template <int R, int MB, int EPI>
-static int f32_rows(const F32Args& p, const F32Choice& c, cudaStream_t s) {
+template <int R, int MB, int EPI, int SHARE>
+static int f32_rows_shared(const F32Args& p, const F32Choice& c, cudaStream_t s) {
     static std::atomic<unsigned long long> ready{0};
-    const int st = kp_smem_limit(gemm_f32_rows_kernel<R, MB, EPI>, KP_SMEM_MAX, ready);
+    const int st = kp_smem_limit(gemm_f32_rows_kernel<R, MB, EPI, SHARE>, KP_SMEM_MAX, ready);
     if (st) return st;
     const dim3 grid((p.N + 8 * R - 1) / (8 * R), (p.M + MB - 1) / MB);
-    return (int)kp_launch_pdl(gemm_f32_rows_kernel<R, MB, EPI>, grid, dim3(c.warps * 32), c.smem, s, p, c.stages);
+    return (int)kp_launch_pdl(gemm_f32_rows_kernel<R, MB, EPI, SHARE>, grid, dim3(c.warps * SHARE * 32), c.smem, s, p, c.stages);
+}
+
+// Where K is one job, a CTA of up to 8 rows is a single warp, and few CTAs leave an SM with few warps: two warps then share the
+// job (half of the rows each).  8 rows, us, one warp | two: 1024 x 1024 7.6 | 6.5, 3072 x 1024 10.0 | 9.2, 9216 x 1024 11.5 | 11.0;
+// but 65536 x 1024 51.6 | 70.5, as W is then read twice from shared memory, which is what bounds many CTAs, and with several
+// jobs as well: 2048 x 5632 13.1 | 16.0.
+template <int R, int MB, int EPI>
+static int f32_rows(const F32Args& p, const F32Choice& c, cudaStream_t s) {
+    if constexpr (MB == 4 || MB == 8) {
+        const long long ctas = (long long)((p.N + 8 * R - 1) / (8 * R)) * ((p.M + MB - 1) / MB);
+        if (p.K <= F32R_JOB && ctas <= 4LL * f32_n_sm()) return f32_rows_shared<R, MB, EPI, 2>(p, c, s);
+    }
+    return f32_rows_shared<R, MB, EPI, 1>(p, c, s);
 }
 
 template <int EPI>
