@@ -936,21 +936,22 @@ static int tc_parts(int M, int N, int K, int epi) {
 // The fastest way to run the parts that tc_parts gives: the choice that keeps the busiest SM busy for the shortest time,
 // counted in bytes brought into it (about 100 a nanosecond, from L2 or, all SMs together, HBM):
 //   a k-block: its rows of A and W, but no less than TC_KB_MIN (waiting, issuing, handing on);
-//   an epilogue: 0.6 KB a column of the tile, 1.2 KB gated, under the main loop of the next tile if there is one;
+//   an epilogue: 0.6 KB a column of the tile, 1 KB gated, under the main loop of the next tile if there is one;
 //   parts one after the other: 6 KB a part more and 64 columns, for reading its sums;
 //   parts by a cluster (all units in one round): 20 KB and 1.4 KB a CTA for the exchange, five times the sums that are
 //   exchanged, a little more for clusters of other than 2 or 4 CTAs;
 //   a pair: TC_PAIR_COST for its barriers, and more for parts behind a gated epilogue, which is short of registers.
-// It was fitted to all that can run at 17 to 1000 rows of twelve layer products (860 timings): within 0.7 % of the best on average,
-// 24 % at worst (gated 600 rows by 9216 x 1024, where a pair's third row of tiles holds 88 rows).  Measured, us, the choice before
-// the exchange by copies | now: 64 rows by 2048 x 2048 7.6 | 6.5, 128 by 2048 x 5632 16.0 | 12.0, 200 by 1024 x 4608 13.4 | 10.1.
+// It was fitted to all that can run at 17 to 1000 rows of twelve layer products (1,087 timings): within 1 % of the best on average,
+// 23 % at worst (128 rows by 3072 x 2048, five parts by a cluster or by one CTA of 32 columns).  Measured, us, the
+// choice before the exchange by copies | now: 64 rows by 2048 x 2048 7.6 | 6.5, 128 by 2048 x 5632 16.0 | 12.0, 200 by
+// 1024 x 4608 13.4 | 10.1; gated 600 rows by 9216 x 1024 25.1 | 20.5.
 static TcChoice tc_choose(int M, int N, int K, int epi, int split) {
     const bool gated = epi == EPI_SWIGLU;
     const int n_out = gated ? N / 2 : N, sms = tc_n_sm(), n_kb = (K + TC_BK - 1) / TC_BK;
     const int m_tiles = (M + TC_BM - 1) / TC_BM, rows = M < TC_BM ? M : TC_BM, a_rows = tc_a_rows(M);
     const auto tiles_at = [&](int w) { const int cols = gated ? w / 2 : w; return (long long)((n_out + cols - 1) / cols); };
     const auto kb_cost = [](long long r) { const long long bytes = r * TC_BK * 2; return bytes > TC_KB_MIN ? bytes : (long long)TC_KB_MIN; };
-    const auto epi_cost = [&](int w) { return (long long)w * (gated ? 1228 : 614); };
+    const auto epi_cost = [&](int w) { return (long long)w * (gated ? 1000 : 614); };
     const auto run_cost = [&](long long rounds, long long main, int w) {
         return rounds * (main > epi_cost(w) ? main : epi_cost(w)) + epi_cost(w);
     };
