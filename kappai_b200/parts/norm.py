@@ -42,10 +42,15 @@ class RMSNorm(Part):
 
     def forward_for(self, part, x: torch.Tensor):
         """The norm as ``part``'s input: in a bfloat16 step of few rows left to the part's first product, if the part's forward is
-        marked as one that takes :class:`NormedRows` (a subclass with a forward of its own is not)."""
-        if x.shape[0] <= K.ROWS_MAX_M and self.env.dtype == torch.bfloat16 and getattr(part.forward, "takes_normed_rows", False):
+        marked as one that takes :class:`NormedRows` (a subclass with a forward of its own is not) and the norm is this one (and
+        not a subclass's, with a forward of its own)."""
+        if (x.shape[0] <= K.ROWS_MAX_M and self.env.dtype == torch.bfloat16 and getattr(part.forward, "takes_normed_rows", False)
+                and getattr(self.forward, "__func__", None) is _RMS_FORWARD):
             return NormedRows(x, self.weight, self.eps)
         return self.forward(x)
+
+
+_RMS_FORWARD = RMSNorm.forward
 
 
 class LayerNorm(RMSNorm):
@@ -55,9 +60,6 @@ class LayerNorm(RMSNorm):
         n = x.shape[0] if rows is None else rows.numel()
         out = torch.empty((n, self.size), dtype=self.env.dtype, device=x.device)
         return K.layernorm_rows(x, self.weight, self.eps, out, rows)
-
-    def forward_for(self, part, x: torch.Tensor):
-        return self.forward(x)
 
 
 register_part("norm", "rmsnorm", RMSNorm)

@@ -1,0 +1,48 @@
+"""Which norms are left to the product behind them: an RMS norm's own, for a part whose forward is marked as one that takes the rows
+before the norm, in bfloat16 steps of up to 8 rows; nobody else's."""
+import pytest
+import torch
+
+from kappai_b200.ops.linear import NormedRows
+from kappai_b200.parts.base import BuildEnv
+from kappai_b200.parts.norm import LayerNorm, RMSNorm
+
+
+class Marked:
+    def forward(self, h):
+        pass
+
+    forward.takes_normed_rows = True
+
+
+class Overridden(Marked):
+    def forward(self, h):
+        pass
+
+
+class OtherNorm(RMSNorm):
+    def forward(self, x, rows=None):
+        return "its own"
+
+
+def norm(cls, dtype=torch.bfloat16):
+    n = cls({"size": 512, "eps": 1e-5}, BuildEnv(torch.device("cpu"), dtype, 16))
+    n.weight = torch.ones(512)
+    return n
+
+
+def test_left_to_the_product():
+    x = torch.zeros(8, 512)
+    h = norm(RMSNorm).forward_for(Marked(), x)
+    assert isinstance(h, NormedRows) and h.x is x and h.shape == x.shape
+
+
+@pytest.mark.parametrize("cls,part,rows,dtype", [(RMSNorm, Overridden, 8, torch.bfloat16), (RMSNorm, Marked, 9, torch.bfloat16),
+                                                 (RMSNorm, Marked, 8, torch.float32), (LayerNorm, Marked, 8, torch.bfloat16),
+                                                 (OtherNorm, Marked, 8, torch.bfloat16)])
+def test_taken_by_the_norm(monkeypatch, cls, part, rows, dtype):
+    from kappai_b200.parts import norm as module
+    for name in ("rmsnorm_rows", "layernorm_rows"):
+        monkeypatch.setattr(module.K, name, lambda *a: "normed")
+    got = norm(cls, dtype).forward_for(part(), torch.zeros(rows, 512))
+    assert got == ("its own" if cls is OtherNorm else "normed")
