@@ -15,10 +15,14 @@
 //    lanes of a quarter warp read all banks once.
 //  * At a tile's end the warps' partial sums are added in warp order from zero.  The order of every sum is that of
 //    gemm_stream.cu, so a row's result does not depend on which of the two ran.
-//  * Behind an RMS norm (the normed form) a CTA brings the float32 rows in itself: a warp its own columns, times the norm's
-//    weight, rounded to bfloat16 and held beside the rings for all the CTA's tiles; the sums are multiplied by 1 / rms where
-//    they leave.  So no launch stands between the product in front and this one.  (Left to the product in front -- it
-//    writes the weighted rows and sums of squares, this one reads both -- a step took 3 % longer.)
+//  * Behind an RMS norm (the normed form) a CTA brings the float32 rows in itself, norms them with the arithmetic of the norm
+//    kernel for that many columns (rowwise.cu: the same order of the squares' sum, x times the scale times the weight, rounded
+//    to bfloat16) and holds them beside the rings for all its tiles: the bits of the norm kernel and the product, without a
+//    launch between the product in front and this one.  (The weighted rows rounded before the scale, which then goes to the sums,
+//    saves two barriers a CTA but rounds a row elsewhere than with nine rows and more, and makes NaN of rows whose squares
+//    overflow; and with a warp's own columns read by itself, 128 bytes at a time, it was slower: rounds of one request of the
+//    1.2B shape 31.33 ms, this 31.06, of a short chat 8.02 and 7.88, of eight requests 44.10 and 43.77.  Left to the product in
+//    front -- it writes the weighted rows and sums of squares, this one reads both -- a step took 3 % longer.)
 //
 // Measured back to back, us, gemm_stream | this, one row and 8: 2048 x 5632 7.8 | 6.5, 7.9 | 7.1; 6144 x 2048 6.8 | 5.2,
 // 6.9 | 5.7; 2048 x 2048 3.8 | 2.6, 3.8 | 2.8; at 16 rows it loses (8.2 | 9.0), as A then weighs as much as W.
@@ -71,7 +75,7 @@ struct RowsArgs {
 template <int WR, int R, bool NORM, int ROOM> struct RowsShape {
     static constexpr int MT = (WR + 15) / 16;                            // m16 tiles (of a 24-row tile's second one half is empty)
     static constexpr int W_BYTES = WR * 128, STAGE = W_BYTES + (NORM ? 0 : R * 128);
-    static constexpr int SUMS = 2 * RW_WARPS * MT * 128 * 4 + RW_WARPS * 8 * 4;
+    static constexpr int SUMS = 2 * RW_WARPS * MT * 128 * 4 + 128;
     static constexpr int FIT = (ROOM - SUMS - (NORM ? 2048 * 2 * R : 0)) / (RW_WARPS * STAGE);
     static constexpr int S = FIT > RW_MAX_STAGES ? RW_MAX_STAGES : FIT;  // ring stages of a warp
     static_assert(S >= 2, "a ring of two stages at least");
@@ -95,9 +99,10 @@ gemm_rows_kernel(const RowsArgs p) {
     const int n_tiles = (n_out + TROWS - 1) / TROWS, n_ch = p.K / 512;   // chunks of 64 columns a warp and tile
     unsigned char* ring = smem + (size_t)warp * S * STAGE;
     float* red = reinterpret_cast<float*>(smem + (size_t)RW_WARPS * S * STAGE);   // [2][warp][MT][4][32]
-    // (NORM) the squares' sums [warp][8], then for every warp its columns of A [chunk][row][64], laid out as a stage's
-    float* squares = red + 2 * RW_WARPS * MT * 128;
-    unsigned char* held = reinterpret_cast<unsigned char*>(squares + RW_WARPS * 8) + (size_t)warp * n_ch * (R * 128);
+    // (NORM) the rows' 1 / root mean square, then for every warp its columns of A [chunk][row][64], laid out as a stage's
+    float* scales = red + 2 * RW_WARPS * MT * 128;
+    unsigned char* held0 = reinterpret_cast<unsigned char*>(scales + 32);
+    const unsigned char* held = held0 + (size_t)warp * n_ch * (R * 128);
     const int ga = g < R ? g : R - 1;                                    // the row of A this lane's fragments are of
     const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - blockIdx.x - 1) / gridDim.x + 1 : 0;
     const int total = my_tiles * n_ch;
@@ -136,52 +141,81 @@ gemm_rows_kernel(const RowsArgs p) {
         cp_async_commit();
     }
     if constexpr (NORM) {
-        // Half a warp a chunk: lane j of it has columns 4 j ... of the chunk's 64 (columns of A as load_a has them).
-        constexpr int CU = R >= 8 ? 2 : 4;                               // chunks a lane has in flight for each of R rows
-        const int half = lane >> 4, j = lane & 15;
-        const int colx = warp * 32 + (j >> 3) * 256 + (j & 7) * 4;
-        float4 gm[CU];
-#pragma unroll
-        for (int k = 0; k < CU; k++)
-            gm[k] = 2 * k + half < n_ch ? __ldg(reinterpret_cast<const float4*>(p.gamma + (2 * k + half) * 512 + colx)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float ss[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) ss[r] = 0.f;
+        // A thread has the float4s threadIdx.x, + 256, ... of every row; the first KEEP of each stay in registers.
+        constexpr int KEEP = 2;
+        const int tid = threadIdx.x, n4 = p.K >> 2;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const auto x_at = [&](int r, int i) { return r < M && i < n4 ? *reinterpret_cast<const float4*>(p.X + (size_t)r * p.ldx + i * 4) : zero; };
+        const auto gamma_at = [&](int i) { return i < n4 ? *reinterpret_cast<const float4*>(p.gamma + i * 4) : zero; };
+        const auto squares = [](const float4& x, float ss) { return fmaf(x.w, x.w, fmaf(x.z, x.z, fmaf(x.y, x.y, fmaf(x.x, x.x, ss)))); };
         pdl_wait();
         KP_TRACE_MARK(1);
-#pragma unroll 1
-        for (int c0 = 0; c0 < n_ch; c0 += 2 * CU) {
-            float4 v[R][CU];
+        float4 v[R][KEEP], gm[KEEP];
 #pragma unroll
-            for (int r = 0; r < R; r++)
+        for (int r = 0; r < R; r++)
 #pragma unroll
-                for (int k = 0; k < CU; k++) {
-                    const int c = c0 + 2 * k + half;
-                    v[r][k] = r < M && c < n_ch ? *reinterpret_cast<const float4*>(p.X + (size_t)r * p.ldx + c * 512 + colx) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            if (c0 > 0) {
+            for (int j = 0; j < KEEP; j++) v[r][j] = x_at(r, tid + j * 256);
 #pragma unroll
-                for (int k = 0; k < CU; k++)
-                    gm[k] = c0 + 2 * k + half < n_ch ? __ldg(reinterpret_cast<const float4*>(p.gamma + (c0 + 2 * k + half) * 512 + colx)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int r = 0; r < R; r++)
-#pragma unroll
-                for (int k = 0; k < CU; k++) {
-                    const int c = c0 + 2 * k + half;
-                    const float4 x = v[r][k], g4 = gm[k];
-                    ss[r] = fmaf(x.x, x.x, ss[r]); ss[r] = fmaf(x.y, x.y, ss[r]); ss[r] = fmaf(x.z, x.z, ss[r]); ss[r] = fmaf(x.w, x.w, ss[r]);
-                    if (r < M && c < n_ch)
-                        *reinterpret_cast<uint2*>(held + (size_t)c * (R * 128) + r * 128 + (((j >> 1) ^ ((r & 1) << 2)) * 16) + (j & 1) * 8) =
-                            make_uint2(pack_bf16(x.x * g4.x, x.y * g4.y), pack_bf16(x.z * g4.z, x.w * g4.w));
-                }
-        }
+        for (int j = 0; j < KEEP; j++) gm[j] = gamma_at(tid + j * 256);
+        float ss[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const float q = warp_sum(ss[r]);
-            if (lane == r) squares[warp * 8 + r] = q;
+            ss[r] = 0.f;
+#pragma unroll
+            for (int j = 0; j < KEEP; j++) ss[r] = squares(v[r][j], ss[r]);
         }
-        __syncwarp();
+#pragma unroll 1
+        for (int j = KEEP; j * 256 < n4; j++)
+#pragma unroll
+            for (int r = 0; r < R; r++) ss[r] = squares(x_at(r, tid + j * 256), ss[r]);
+        // the sum over the threads, as the norm kernel of that size has it: up to 2048 columns the warps' values lane by lane, in
+        // the order of the warps, then the lanes; beyond, the lanes of a warp, then the warps
+        const bool by_lane = n4 <= 512;
+        float* part = red;                                               // [row][warp][lane], or [row][256] by warp
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const float q = by_lane ? ss[r] : warp_sum(ss[r]);
+            if (by_lane || lane == 0) part[r * 256 + (by_lane ? tid : warp)] = q;
+        }
+        __syncthreads();
+        const auto scale_of = [&](int r) {
+            float q;
+            if (by_lane) {
+                q = part[r * 256 + lane];
+#pragma unroll
+                for (int w8 = 1; w8 < RW_WARPS; w8++) q += part[r * 256 + w8 * 32 + lane];
+            } else {
+                q = lane < RW_WARPS ? part[r * 256 + lane] : 0.f;
+            }
+            return 1.0f / sqrtf(warp_sum(q) / (float)p.K + p.eps);
+        };
+        float scale[R];
+        if (R == 1) {
+            scale[0] = scale_of(0);                                      // (every warp: that saves a barrier)
+        } else {
+            if (warp < R) scales[warp] = scale_of(warp);
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < R; r++) scale[r] = scales[r];
+        }
+        // column 4 i is of chunk i / 128, there of half i / 64 % 2, there of warp i / 8 % 8 (see load_a)
+        const auto hold = [&](int r, int i, const float4& x, const float4& g4) {
+            if (r >= M || i >= n4) return;
+            const int j = (i >> 6 & 1) * 8 + (i & 7);
+            *reinterpret_cast<uint2*>(held0 + (size_t)((i >> 3 & 7) * n_ch + (i >> 7)) * (R * 128) + r * 128 + (((j >> 1) ^ ((r & 1) << 2)) * 16) + (j & 1) * 8) =
+                make_uint2(pack_bf16((x.x * scale[r]) * g4.x, (x.y * scale[r]) * g4.y), pack_bf16((x.z * scale[r]) * g4.z, (x.w * scale[r]) * g4.w));
+        };
+#pragma unroll
+        for (int r = 0; r < R; r++)
+#pragma unroll
+            for (int j = 0; j < KEEP; j++) hold(r, tid + j * 256, v[r][j], gm[j]);
+#pragma unroll 1
+        for (int j = KEEP; j * 256 < n4; j++) {
+            const float4 g4 = gamma_at(tid + j * 256);
+#pragma unroll
+            for (int r = 0; r < R; r++) hold(r, tid + j * 256, x_at(r, tid + j * 256), g4);
+        }
+        __syncthreads();
     } else {
         pdl_wait();
         KP_TRACE_MARK(1);
@@ -193,7 +227,6 @@ gemm_rows_kernel(const RowsArgs p) {
     }
 
     int s = 0, buf = 0;
-    float scale = 1.f;                                                   // (NORM) 1 / root mean square of this thread's row
 #pragma unroll 1
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
         const int n0 = tile * TROWS;
@@ -252,12 +285,6 @@ gemm_rows_kernel(const RowsArgs p) {
 #pragma unroll
             for (int i = 0; i < 4; i++) r[(warp * MT + a) * 128 + i * 32 + lane] = acc[a][i];
         __syncthreads();                                                 // (the other half of `red` is free: its readers were here)
-        if (NORM && tile == (int)blockIdx.x && om < M) {
-            float q = 0.f;
-#pragma unroll
-            for (int w8 = 0; w8 < RW_WARPS; w8++) q += squares[w8 * 8 + om];
-            scale = 1.0f / sqrtf(q / (float)p.K + p.eps);
-        }
         if (mine) {
             // the sum of W row `row` of the tile for this thread's batch row, over the warps in order
             auto sum_of = [&](int row) {
@@ -265,7 +292,7 @@ gemm_rows_kernel(const RowsArgs p) {
                 float v = 0.f;
 #pragma unroll
                 for (int w8 = 0; w8 < RW_WARPS; w8++) v += r[(w8 * MT + a) * 128 + i * 32 + l];
-                return NORM ? v * scale : v;
+                return v;
             };
             const int m = om, n = on, lr = on - n0;
             float v = sum_of(lr);
@@ -409,7 +436,8 @@ int kp_gemm_rows(const void* A, int lda, const void* W, int ldw, const float* bi
     return st ? st : rows_run<false>(a, epi, (cudaStream_t)stream);
 }
 
-// The product with A = the RMS norm of the float32 rows X (weight gamma): see the top.  Not with an accumulated output.
+// The product with A = the RMS norm of the float32 rows X (weight gamma), the bits of kp_rmsnorm_rows and kp_gemm_rows: see the top.
+// Not with an accumulated output.
 int kp_gemm_rows_normed(const float* X, int ldx, const float* gamma, float eps, const void* W, int ldw, const float* bias, void* C,
                         int ldc, int M, int N, int K, int epi, float limit, float alpha, float shift, void* stream) {
     if (M <= 0 || N <= 0) return 0;

@@ -1766,8 +1766,8 @@ def _normed_args(x: torch.Tensor, gamma: torch.Tensor, eps: float):
 def gemm_rows_normed(x: torch.Tensor, gamma: torch.Tensor, eps: float, w: torch.Tensor, out: torch.Tensor,
                      bias: Optional[torch.Tensor] = None, swiglu: bool = False, activation: str = "silu",
                      glu: Optional[Tuple[float, float, float]] = None, plain_activation: Optional[str] = None) -> torch.Tensor:
-    """:func:`gemm_skinny` of the RMS norm of up to 8 float32 rows ``x`` (weight ``gamma``): the product takes ``x gamma`` rounded to
-    bfloat16 and multiplies the sums by ``1 / rms``."""
+    """:func:`gemm_skinny` of the RMS norm of up to 8 float32 rows ``x`` (weight ``gamma``), which the product takes itself: the bits
+    of :func:`rmsnorm_rows` and the product behind it."""
     norm = _normed_args(x, gamma, eps)
     _need(w, "w", torch.bfloat16, contiguous=False); _need(out, "out", contiguous=False)
     M, K = x.shape
