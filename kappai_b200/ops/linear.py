@@ -62,7 +62,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     float32 ``out`` (the residual sum stays in 32-bit)."""
     M, N = a.shape[0], w.shape[0]
     a_dtype = a.dtype
-    if isinstance(a, NormedRows):
+    if type(a) is NormedRows:
         if w_settled and not accumulate and a.fusable(w):
             out = torch.empty((M, N), dtype=out_dtype or a_dtype, device=a.device) if out is None else out
             return K.gemm_rows_normed(a.x, *a.norm, w, out, bias)
@@ -94,7 +94,7 @@ def linear_act(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], a
     fits the shape, else by a row-wise kernel behind a float32 product."""
     M, N = a.shape[0], w.shape[0]
     out = torch.empty((M, N), dtype=a.dtype, device=a.device)
-    if isinstance(a, NormedRows):
+    if type(a) is NormedRows:
         if w_settled and a.fusable(w):
             return K.gemm_rows_normed(a.x, *a.norm, w, out, bias, plain_activation=activation)
         a = a.rows()
@@ -118,7 +118,7 @@ def linear_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, bias: Optional[torch
     ff = w_gate_up.shape[0] // 2
     act = torch.empty((a.shape[0], ff), dtype=a.dtype, device=a.device)
     fused = glu is not None or activation in K.FUSED_ACTIVATIONS
-    if isinstance(a, NormedRows):
+    if type(a) is NormedRows:
         if fused and w_settled and a.fusable(w_gate_up):
             return K.gemm_rows_normed(a.x, *a.norm, w_gate_up, act, bias, swiglu=True, activation=activation, glu=glu)
         a = a.rows()

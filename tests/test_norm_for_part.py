@@ -46,3 +46,28 @@ def test_taken_by_the_norm(monkeypatch, cls, part, rows, dtype):
         monkeypatch.setattr(module.K, name, lambda *a: "normed")
     got = norm(cls, dtype).forward_for(part(), torch.zeros(rows, 512))
     assert got == ("its own" if cls is OtherNorm else "normed")
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 999])
+def test_asked_in_steps_of_few_rows_only(rows):
+    """A step of more rows launches from Python and waits for it: nothing is asked there whose answer is always no."""
+    from types import SimpleNamespace
+    from kappai_b200.parts.block import PreNormResidualBlock
+    calls = []
+
+    class Norm:
+        def forward(self, x):
+            calls.append("norm")
+            return "normed"
+
+        def forward_for(self, part, x):
+            calls.append("asked")
+            return "left"
+
+    class Sublayer:
+        def forward(self, h, *args):
+            calls.append(h)
+
+    block = PreNormResidualBlock({}, BuildEnv(torch.device("cpu"), torch.bfloat16, 16)).assemble(Sublayer(), Sublayer(), Norm(), Norm())
+    block.forward(torch.zeros(rows, 4), SimpleNamespace(n_rows=rows), None)
+    assert calls == (["asked", "left"] if rows <= 8 else ["norm", "normed"]) * 2
