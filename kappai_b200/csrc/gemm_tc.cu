@@ -537,8 +537,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 //
 // The epilogue warps pass their pieces (128 bytes of 32 rows) through shared memory, so that a warp writes, and for an
 // accumulated output reads, four whole rows' stretches of 128 bytes at a time instead of 16 bytes of 32 rows; the old
-// values of an accumulated output are asked for before the piece is read from tensor memory.  16 columns of sums at a time:
-// with 32 the gated kernels were 98 KB of code for 41, and a prompt of 2,048 tokens of the 1.2B shape took 3.33 ms for 3.28.
+// values of an accumulated output are asked for before the piece is read from tensor memory.  Accumulating and gated kernels take
+// 16 columns of sums at a time, the others 32.  us, 16 | 32 at a time: accumulating 2,048 rows by 2048 x 2048 18.9 | 20.1 (the old
+// values need the registers); stored 999 rows by 3072 x 2048 15.5 | 15.3, by 65536 x 1024 in 32 bits 120.0 | 119.0, 2,048 rows by
+// 3072 x 2048 25.8 | 25.0; gated 999 rows by 9216 x 1024 22.2 | 21.8, but 41 KB of code against 98, and in a prompt, where the
+// code comes anew at every launch, the gain is gone (2,048 tokens of the 1.2B shape 3.249 | 3.253 ms, 999 rows of the 350M shape
+// 1.730 | 1.732).
 #define TC_PAIR_STAGES(BN) ((BN) == 256 ? 5 : 7)
 #define TC_PAIR_SMEM(BN) ((size_t)TC_PAIR_STAGES(BN) * (128 + (BN) / 2) * TC_BK * 2 + TC_EPI_PER_Q * 4 * 4096 + (2 * TC_PAIR_STAGES(BN) + 4) * 8 + 16 + 1024)
 
@@ -656,6 +660,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         unsigned char* piece = pieces + (size_t)(warp - 2) * 4096;
         constexpr bool NARROW = EPI == EPI_STORE || EPI == EPI_ACT || TC_GATED(EPI);   // 16-bit outputs: a piece is 64 columns
         constexpr int PW = NARROW ? 64 : 32;
+        constexpr int PC = EPI == EPI_ACCUM_F32 || TC_GATED(EPI) ? 16 : 32;            // columns of sums at a time (see above)
         int b2 = 0;
         uint32_t set_ph = 0;
         bool ok = true;
@@ -679,30 +684,30 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         if (row < p.M) old[i] = *reinterpret_cast<const float4*>((const float*)p.C + (size_t)row * p.ldc + n0 + c + pch * 4);
                     }
                 }
-#pragma unroll 1
-                for (int h = 0; h < PW / 16; h++) {
-                    const int n_base = n0 + c + h * 16;
-                    float v[16], up[16];
-                    tc_sums<EPI, BN, PARTS>(p, lane_base + c + h * 16, v, up);
+#pragma unroll (PC == 32 ? 2 : 1)
+                for (int h = 0; h < PW / PC; h++) {
+                    const int n_base = n0 + c + h * PC;
+                    float v[PC], up[PC];
+                    tc_sums<EPI, BN, PARTS>(p, lane_base + c + h * PC, v, up);
                     if (!staged) {
-                        if (m < p.M) tc_finish<EPI, 16>(p, n_out, v, up, m, n_base);
+                        if (m < p.M) tc_finish<EPI, PC>(p, n_out, v, up, m, n_base);
                         continue;
                     }
                     // (rows beyond the last hold zeros, on which the activation's division is slow: they are left alone)
                     if (m < p.M) {
-                        tc_bias<EPI, 16>(p, n_out, v, up, n_base);
+                        tc_bias<EPI, PC>(p, n_out, v, up, n_base);
 #pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = tc_value<EPI>(p, v[j], up[j]);
+                        for (int j = 0; j < PC; j++) v[j] = tc_value<EPI>(p, v[j], up[j]);
                     }
                     if (NARROW) {
 #pragma unroll
-                        for (int j = 0; j < 2; j++)
-                            *reinterpret_cast<uint4*>(piece + lane * 128 + (((h * 2 + j) ^ (lane & 7)) * 16)) =
+                        for (int j = 0; j < PC / 8; j++)
+                            *reinterpret_cast<uint4*>(piece + lane * 128 + (((h * (PC / 8) + j) ^ (lane & 7)) * 16)) =
                                 make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]), pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            *reinterpret_cast<float4*>(piece + lane * 128 + (((h * 4 + j) ^ (lane & 7)) * 16)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                        for (int j = 0; j < PC / 4; j++)
+                            *reinterpret_cast<float4*>(piece + lane * 128 + (((h * (PC / 4) + j) ^ (lane & 7)) * 16)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
                     }
                 }
                 if (!staged) continue;
