@@ -26,7 +26,9 @@ __device__ __forceinline__ float kp_query_temperature(int pos, float coef, float
     return 1.0f + coef * logf(floorf((float)(pos + 1) / every) + 1.0f);
 }
 
-template <typename T>
+// V: values of a head a lane has, at least hd / 32: 2, 4 or 8, so that all of a head's loads are under way together and a kernel
+// has the code of its own head size only.
+template <typename T, int V>
 __global__ void __launch_bounds__(128)
 qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
                        const float* __restrict__ k_w, float eps, const float* __restrict__ cos_tab,
@@ -49,48 +51,66 @@ qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
     const T* src = qkv + (size_t)row * ld + (kind == 2 ? (size_t)v_col + (size_t)(head - H - G) * hd : (size_t)head * hd);
     float* x = buf[warp];
 
-    float ss = 0.f;
-#pragma unroll 2
-    for (int i = lane; i < hd; i += 32) {
-        const float v = to_f32(src[i]);
-        x[i] = v;
-        ss = fmaf(v, v, ss);
+    // (a lane's values, lane, lane + 32, ..., pass through shared memory for the rotation only)
+    float val[V], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+        val[i] = lane + 32 * i < hd ? to_f32(src[lane + 32 * i]) : 0.f;
+        ss = fmaf(val[i], val[i], ss);
     }
     const float* w = kind == 0 ? q_w : (kind == 1 ? k_w : nullptr);
     if (w) {
+        float wv[V];
+#pragma unroll
+        for (int i = 0; i < V; i++) wv[i] = lane + 32 * i < hd ? w[lane + 32 * i] : 0.f;
         ss = warp_sum(ss);
         const float scale = 1.0f / sqrtf(ss / (float)norm_dim + eps);
-#pragma unroll 2
-        for (int i = lane; i < hd; i += 32) x[i] = (x[i] * scale) * w[i];
+#pragma unroll
+        for (int i = 0; i < V; i++) val[i] = (val[i] * scale) * wv[i];
     }
-    __syncwarp();
     if (kind != 2 && cos_tab) {
         const int half = rot >> 1;
         const size_t tb = (size_t)positions[row] * half;
-#pragma unroll 1
-        for (int j = lane; j < half; j += 32) {
-            const int ia = interleaved ? 2 * j : j;
-            const int ib = interleaved ? 2 * j + 1 : j + half;
-            const float c = cos_tab[tb + j], s = sin_tab[tb + j];
-            const float a = x[ia], b = x[ib];
-            x[ia] = a * c - b * s;
-            x[ib] = a * s + b * c;
+        float c[V / 2], s[V / 2];
+#pragma unroll
+        for (int i = 0; i < V / 2; i++) {
+            const int j = lane + 32 * i;
+            c[i] = j < half ? cos_tab[tb + j] : 0.f;
+            s[i] = j < half ? sin_tab[tb + j] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < V; i++)
+            if (lane + 32 * i < hd) x[lane + 32 * i] = val[i];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < V / 2; i++) {
+            const int j = lane + 32 * i;
+            if (j < half) {
+                const int ia = interleaved ? 2 * j : j;
+                const int ib = interleaved ? 2 * j + 1 : j + half;
+                const float a = x[ia], b = x[ib];
+                x[ia] = a * c[i] - b * s[i];
+                x[ib] = a * s[i] + b * c[i];
+            }
         }
         __syncwarp();
+#pragma unroll
+        for (int i = 0; i < V; i++)
+            if (lane + 32 * i < hd) val[i] = x[lane + 32 * i];
     }
     if (norm_after && kind != 2) {
         float sq = 0.f;
-#pragma unroll 1
-        for (int i = lane; i < hd; i += 32) sq = fmaf(x[i], x[i], sq);
+#pragma unroll
+        for (int i = 0; i < V; i++) sq = fmaf(val[i], val[i], sq);
         sq = warp_sum(sq);
         const float scale = 1.0f / sqrtf(sq / (float)norm_dim + eps);
-#pragma unroll 1
-        for (int i = lane; i < hd; i += 32) x[i] *= scale;
+#pragma unroll
+        for (int i = 0; i < V; i++) val[i] *= scale;
     }
     if (kind == 0 && temp_every > 0.f) {
         const float tq = kp_query_temperature(positions[row], temp_coef, temp_every);
-#pragma unroll 1
-        for (int i = lane; i < hd; i += 32) x[i] *= tq;
+#pragma unroll
+        for (int i = 0; i < V; i++) val[i] *= tq;
     }
     T* dst;
     if (in_place) {
@@ -104,8 +124,9 @@ qk_norm_rope_kv_kernel(const T* qkv, int ld, const float* __restrict__ q_w,
         const int g = kind == 1 ? head - H : head - H - G;
         dst = cache + ((((size_t)page * 2 + (kind - 1)) * G + g) * page_size + off) * hd;
     }
-#pragma unroll 2
-    for (int i = lane; i < hd; i += 32) dst[i] = from_f32<T>(x[i]);
+#pragma unroll
+    for (int i = 0; i < V; i++)
+        if (lane + 32 * i < hd) dst[lane + 32 * i] = from_f32<T>(val[i]);
 }
 
 // The same for bfloat16 with head size 64 or 128, NeoX rotation of the first `rot` dimensions (rot / 16 a power
@@ -237,9 +258,12 @@ extern "C" int kp_qk_norm_rope_kv_after(const void* qkv, int ld, const float* q_
         return kp_launch_status();
     }
     dim3 grid((H + 2 * G + 3) / 4, n);
-    KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(qk_norm_rope_kv_kernel<T>, dim3(grid), dim3(128), 0, (cudaStream_t)stream, 
-        (const T*)qkv, ld, q_w, k_w, eps, cos_tab, sin_tab, rot, interleaved, positions, slot_map, (T*)q_out, ldq,
-        (T*)cache, page_size, H, G, hd, write_kv, v_col, norm_dim, temp_coef, temp_every, norm_after)));
+#define QK_LAUNCH(T, V)                                                                                                                  \
+    kp_launch_pdl(qk_norm_rope_kv_kernel<T, V>, dim3(grid), dim3(128), 0, (cudaStream_t)stream, (const T*)qkv, ld, q_w, k_w, eps,        \
+                  cos_tab, sin_tab, rot, interleaved, positions, slot_map, (T*)q_out, ldq, (T*)cache, page_size, H, G, hd, write_kv,     \
+                  v_col, norm_dim, temp_coef, temp_every, norm_after)
+    KP_DISPATCH_DTYPE(dtype, T, { if (hd <= 64) QK_LAUNCH(T, 2); else if (hd <= 128) QK_LAUNCH(T, 4); else QK_LAUNCH(T, 8); });
+#undef QK_LAUNCH
     return kp_launch_status();
 }
 
