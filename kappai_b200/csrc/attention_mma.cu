@@ -459,7 +459,7 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
         // V rows of keys that this row does not read hold whatever was there: zero them (P is 0 there, but
         // 0 * NaN is not); K rows need nothing, their scores are masked
         if (t0 < k_lo || t0 + AM_TILE - 1 > k_hi) {
-#pragma unroll 1
+#pragma unroll 4
             for (int idx = lane; idx < AM_TILE * (HD / 8); idx += 32) {
                 const int r = idx / (HD / 8), c = idx % (HD / 8);
                 if (t0 + r < k_lo || t0 + r > k_hi) *reinterpret_cast<uint4*>(tile_chunk<HD>(Vt, r, c)) = make_uint4(0, 0, 0, 0);
