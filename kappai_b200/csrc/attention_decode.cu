@@ -72,11 +72,12 @@ __device__ __forceinline__ int merge_front(int first_hi, int chunk_keys, int c_l
     return front_slot0 >= 0 ? (first_hi + AD_CHUNK_KEYS - 1) / AD_CHUNK_KEYS : front_chunks(first_hi, chunk_keys, c_lo);
 }
 
-// `out`: null, or where the rows go at once because every row has this one chunk and nothing else enters (what the merge makes of
-// one chunk: the same bits).
+// WHOLE: the rows go to `out` at once because every row has this one chunk and nothing else enters (what the merge makes of one
+// chunk: the same bits).  An instance of its own: as an argument it cost the others registers (float32, 16 heads on 16 kv heads, 8
+// rows of 16,000 keys: 381 -> 403 us).
 // HD, RR: head size and query heads per kv head fixed at compile time (loops unroll, loads overlap);
 // 0 means "taken from the arguments".
-template <typename T, int HD, int RR>
+template <typename T, int HD, int RR, bool WHOLE>
 __global__ void __launch_bounds__(AD_THREADS)
 attn_split_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache, const int* __restrict__ block_table,
                   int max_blocks, const int* __restrict__ row_seg, const int* __restrict__ positions,
@@ -252,14 +253,14 @@ attn_split_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ cache,
         const int r = e / hd, d = e % hd;
         float v = 0.f;
         for (int sl = 0; sl < n_slices; sl++) v += red[((size_t)sl * R + r) * hd + d];
-        if (out) {
+        if (WHOLE) {
             const float l = stat_l[r], inv = l > 0.f ? out_scale / l : 0.f;
             out[(size_t)row * ldo + (size_t)(g * R + r) * hd + d] = from_f32<T>(v * inv);
         } else {
             part_acc[(((size_t)row * H + g * R + r) * n_chunks + slot0 + chunk) * hd + d] = v;
         }
     }
-    if (tid < R && !out) {
+    if (tid < R && !WHOLE) {
         float* ml = part_ml + (((size_t)row * H + g * R + tid) * n_chunks + slot0 + chunk) * 2;
         ml[0] = stat_m[tid];
         ml[1] = stat_l[tid];
@@ -478,11 +479,12 @@ int kp_attention_split_pooled(const void* q, int ldq, const void* cache, const i
     cudaStream_t s = (cudaStream_t)stream;
     constexpr int SLOT0 = 0, FRONT = 0;
     const bool whole = n_slots == 1 && keep_first == 0 && !sink;               // the chunk pass writes the rows itself
-#define AD_LAUNCH(T, HD, RR)                                                                                      \
-    kp_launch_pdl(attn_split_kernel<T, HD, RR>, dim3(n_chunks, G, n), dim3(AD_THREADS), smem, s, (const T*)q, ldq, (const T*)cache, block_table,       \
+#define AD_LAUNCH_AS(T, HD, RR, WHOLE)                                                                            \
+    kp_launch_pdl(attn_split_kernel<T, HD, RR, WHOLE>, dim3(n_chunks, G, n), dim3(AD_THREADS), smem, s, (const T*)q, ldq, (const T*)cache, block_table,       \
                                                                 max_blocks, row_seg, positions, part_acc, part_ml,    \
                                                                 n_slots, scale, window, page_size, H, G, hd, block, keep_first, SLOT0, FRONT, cap, 0, \
-                                                                whole ? (T*)out : (T*)nullptr, ldo, out_scale)
+                                                                (T*)out, ldo, out_scale)
+#define AD_LAUNCH(T, HD, RR) (whole ? AD_LAUNCH_AS(T, HD, RR, true) : AD_LAUNCH_AS(T, HD, RR, false))
     KP_DISPATCH_DTYPE(dtype, T, {
         cudaError_t e0;
         if (hd == 64 && R == 4) e0 = AD_LAUNCH(T, 64, 4);
@@ -493,7 +495,7 @@ int kp_attention_split_pooled(const void* q, int ldq, const void* cache, const i
         if (e0 != cudaSuccess) { cudaGetLastError(); return (int)e0; }      // the first launch that failed
         if (whole) return kp_launch_status();
         if (pool > 0) {
-            kp_launch_pdl(attn_split_kernel<T, 0, 0>, dim3(n_pool_chunks, G, n), dim3(AD_THREADS), smem, s, (const T*)q, ldq, (const T*)pool_cache,
+            kp_launch_pdl(attn_split_kernel<T, 0, 0, false>, dim3(n_pool_chunks, G, n), dim3(AD_THREADS), smem, s, (const T*)q, ldq, (const T*)pool_cache,
                           pool_table, max_pool_blocks, row_seg, positions, part_acc, part_ml, n_slots, scale, window, page_size, H, G,
                           hd, 0, 0, n_chunks, 2, cap, pool, (T*)nullptr, 0, 1.f);
         }
@@ -543,7 +545,7 @@ int kp_attention_front_chunks(const void* q, int ldq, const void* cache, const i
     const size_t smem = split_smem_bytes(H / G, hd);
     float* part_acc = scratch;
     float* part_ml = scratch + (size_t)n * H * n_chunks * hd;
-    KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(attn_split_kernel<T, 0, 0>, dim3(n_front, G, n), dim3(AD_THREADS), smem, (cudaStream_t)stream,
+    KP_DISPATCH_DTYPE(dtype, T, (kp_launch_pdl(attn_split_kernel<T, 0, 0, false>, dim3(n_front, G, n), dim3(AD_THREADS), smem, (cudaStream_t)stream,
                                                (const T*)q, ldq, (const T*)cache, block_table, max_blocks, row_seg, positions, part_acc,
                                                part_ml, n_chunks, scale, window, page_size, H, G, hd, 0, keep_first, front_slot0, 1, 0.f, 0,
                                                (T*)nullptr, 0, 1.f)));
