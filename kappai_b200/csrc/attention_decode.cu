@@ -351,9 +351,12 @@ __global__ void attn_merge_kernel(const float* __restrict__ part_acc, const floa
 // hold the chunks' statistics and weights and pass them round, every lane sums its dimensions (lane, lane + 32,
 // ...) chunk by chunk.  The arithmetic is that of the kernel above, so a row's result does not depend on which
 // of the two ran.  (With 64 rows the kernel above took 10.7 us for 2048 small CTAs of 256 threads.)
+// B: chunks whose sums a warp fetches at a time; D: values of a head a lane has (hd <= 32 D).  The kernel's code is fetched at every
+// launch, so a step of short contexts wants little of it, and long contexts want their sums in few trips: 8 at a time up to 8 chunks,
+// 16 up to 16, beyond 32 (heads of more than 64 values: 16).  us with the chunk pass, 8 at a time always | this: bfloat16, 16
+// heads on 4, one row of 4,000 keys 8.8 | 8.4, of 16,000 17.7 | 13.5; 8 rows of 16,000 41.5 | 34.6.
 #define MERGE_WARP_CHUNKS 64
-#define MERGE_WARP_BLOCK 8                                // chunks whose sums a warp fetches at a time
-template <typename T>
+template <typename T, int B, int D>
 __global__ void attn_merge_warp_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                        const int* __restrict__ positions, T* __restrict__ out, int ldo, int n_chunks,
                                        int chunk_keys, int window, int H, int hd, int n_rows, int block, int keep_first,
@@ -369,14 +372,13 @@ __global__ void attn_merge_warp_kernel(const float* __restrict__ part_acc, const
     const int n_front = merge_front(min(keep_first, k_lo), chunk_keys, c_lo, front_slot0, k_hi, window, pool), n = n_front + c_hi - c_lo + 1;
     const float* pa = part_acc + ((size_t)row * H + h) * n_chunks * hd;
     const float* ml = part_ml + ((size_t)row * H + h) * n_chunks * 2;
-    // the sums of the first MERGE_WARP_BLOCK chunks are on their way while the statistics are worked out
-    constexpr int B = MERGE_WARP_BLOCK;
-    float a[B][4];
+    // the sums of the first B chunks are on their way while the statistics are worked out
+    float a[B][D];
     auto fetch = [&](int c0) {
 #pragma unroll
         for (int j = 0; j < B; j++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
+            for (int i = 0; i < D; i++) {
                 const int d = lane + 32 * i;
                 a[j][i] = (c0 + j < n && d < hd) ? pa[(size_t)chunk_at(c0 + j, n_front, c_lo, front_slot0) * hd + d] : 0.f;
             }
@@ -388,7 +390,9 @@ __global__ void attn_merge_warp_kernel(const float* __restrict__ part_acc, const
     float m = warp_max(fmaxf(m0, m1));
     if (sink) m = fmaxf(m, sink[h]);
     const float w0 = lane < n ? expf(m0 - m) : 0.f, w1 = lane + 32 < n ? expf(m1 - m) : 0.f;
-    float l = sink ? expf(sink[h] - m) : 0.f, v[4] = {0.f, 0.f, 0.f, 0.f};
+    float l = sink ? expf(sink[h] - m) : 0.f, v[D];
+#pragma unroll
+    for (int i = 0; i < D; i++) v[i] = 0.f;
 #pragma unroll 1
     for (int c0 = 0; c0 < n; c0 += B) {
         if (c0) fetch(c0);
@@ -400,13 +404,13 @@ __global__ void attn_merge_warp_kernel(const float* __restrict__ part_acc, const
                 const float lc = __shfl_sync(0xffffffffu, c < 32 ? l0 : l1, c & 31);
                 l = __fmaf_rn(lc, wc, l);
 #pragma unroll
-                for (int i = 0; i < 4; i++) v[i] = fmaf(a[j][i], wc, v[i]);
+                for (int i = 0; i < D; i++) v[i] = fmaf(a[j][i], wc, v[i]);
             }
         }
     }
     const float inv = l > 0.f ? out_scale / l : 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < D; i++) {
         const int d = lane + 32 * i;
         if (d < hd) out[(size_t)row * ldo + (size_t)h * hd + d] = from_f32<T>(v[i] * inv);
     }
@@ -422,8 +426,13 @@ static int launch_merge(const float* part_acc, const float* part_ml, const int* 
     if (keep_first == 0 && pool == 0) front_slot0 = -1;
     if (n_chunks <= MERGE_WARP_CHUNKS && hd <= 128) {
         const int warps = 8;
-        kp_launch_pdl(attn_merge_warp_kernel<T>, dim3((n * H + warps - 1) / warps), dim3(warps * 32), 0, s, part_acc, part_ml,
-                      positions, (T*)out, ldo, n_chunks, chunk_keys, window, H, hd, n, block, keep_first, sink, front_slot0, out_scale, pool);
+#define MERGE_LAUNCH(B, D)                                                                                                               \
+    kp_launch_pdl(attn_merge_warp_kernel<T, B, D>, dim3((n * H + warps - 1) / warps), dim3(warps * 32), 0, s, part_acc, part_ml,          \
+                  positions, (T*)out, ldo, n_chunks, chunk_keys, window, H, hd, n, block, keep_first, sink, front_slot0, out_scale, pool)
+        if (n_chunks <= 8) MERGE_LAUNCH(8, 4);
+        else if (n_chunks <= 16 || hd > 64) MERGE_LAUNCH(16, 4);
+        else MERGE_LAUNCH(32, 2);
+#undef MERGE_LAUNCH
         return kp_launch_status();
     }
     const size_t smem = merge_smem_bytes(n_chunks);

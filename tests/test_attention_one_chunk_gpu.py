@@ -24,3 +24,18 @@ def test_the_bits_of_the_merge(dtype, H, G, hd, page, window):
     one = run_split(q, cache, bt, seg, pos, 1.0 / math.sqrt(hd), window, page, H, G, hd, dtype, n_chunks=1)
     assert bool(torch.isfinite(one.float()).all())
     assert torch.equal(one, run_split(q, cache, bt, seg, pos, 1.0 / math.sqrt(hd), window, page, H, G, hd, dtype, n_chunks=3))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,hd,longest,chunks", [(4, 2, 64, 2000, (8, 9, 40, 64)), (3, 1, 48, 2048, (8, 9, 33)), (4, 1, 80, 1999, (8, 9, 17)),
+                                                   (4, 2, 128, 2048, (8, 16, 64)), (2, 2, 64, 8500, (34, 64)), (2, 1, 128, 8500, (34, 64))])
+def test_how_many_chunks_the_merge_fetches_at_a_time_changes_no_bit(dtype, H, G, hd, longest, chunks):
+    rng = np.random.default_rng(8)
+    seq_lens = [1, 256, 257, longest]
+    cache, bt, _, _ = paged_setup(rng, seq_lens, 64, G, hd, dtype)
+    pos, seg = [n - 1 for n in seq_lens], list(range(len(seq_lens)))
+    q = rt(rng.standard_normal((len(pos), H * hd)), dtype)
+    outs = [run_split(q, cache, bt, seg, pos, 1.0 / math.sqrt(hd), None, 64, H, G, hd, dtype, n_chunks=n) for n in chunks]
+    assert bool(torch.isfinite(outs[0].float()).all())
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
