@@ -141,8 +141,9 @@ gemm_rows_kernel(const RowsArgs p) {
         cp_async_commit();
     }
     if constexpr (NORM) {
-        // A thread has the float4s threadIdx.x, + 256, ... of every row; the first KEEP of each stay in registers.
-        constexpr int KEEP = 2;
+        // A thread has the float4s threadIdx.x, + 256, ... of every row; the first KEEP of each stay in registers (all of them, but
+        // for more than 2048 columns of more than four rows: 128 registers).
+        constexpr int KEEP = R <= 4 ? 4 : 2;
         const int tid = threadIdx.x, n4 = p.K >> 2;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         const auto x_at = [&](int r, int i) { return r < M && i < n4 ? *reinterpret_cast<const float4*>(p.X + (size_t)r * p.ldx + i * 4) : zero; };
@@ -152,11 +153,11 @@ gemm_rows_kernel(const RowsArgs p) {
         KP_TRACE_MARK(1);
         float4 v[R][KEEP], gm[KEEP];
 #pragma unroll
-        for (int r = 0; r < R; r++)
+        for (int j = 0; j < KEEP; j++) {
 #pragma unroll
-            for (int j = 0; j < KEEP; j++) v[r][j] = x_at(r, tid + j * 256);
-#pragma unroll
-        for (int j = 0; j < KEEP; j++) gm[j] = gamma_at(tid + j * 256);
+            for (int r = 0; r < R; r++) v[r][j] = x_at(r, tid + j * 256);
+            gm[j] = gamma_at(tid + j * 256);
+        }
         float ss[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
