@@ -232,19 +232,23 @@ gemm_rows_kernel(const RowsArgs p) {
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
         const int n0 = tile * TROWS;
         // what the epilogue needs beside the sums is asked for now: its trips to L2 run under the main loop
-        float pre_c = 0.f, pre_hist[2] = {0.f, 0.f}, pre_cw[3] = {0.f, 0.f, 0.f};
+        float pre_c = 0.f, pre_hist[3] = {0.f, 0.f, 0.f}, pre_cw[3] = {0.f, 0.f, 0.f}, pre_last = 0.f;
+        bool pre_fresh = false;
         const int om = threadIdx.x / TROWS, on = n0 + threadIdx.x % TROWS;   // this thread's output (the first TROWS * M threads)
         const bool mine = om < M && on < n_out;
         if (mine) {
             if (EPI == EPI_ACCUM_F32) pre_c = ((const float*)p.C)[(size_t)om * p.ldc + on];
-            if (EPI == EPI_CONV_STEP && p.conv_k == 3) {
-                const bool fresh = p.seg_pos[om] == 0;
-                const float* st = p.conv_state + (size_t)p.seg_slot[om] * 2 * p.ff;
-                const float* cw = p.conv_w + (size_t)on * 3;
+            if (EPI == EPI_CONV_STEP) {                                  // (the first three of the kept inputs, the last tap; a new request's kept
+                pre_fresh = p.seg_pos[om] == 0;                          //  inputs count as zeros below, so that nothing here waits for its position)
+                const float* st = p.conv_state + (size_t)p.seg_slot[om] * (p.conv_k - 1) * p.ff + on;
+                const float* cw = p.conv_w + (size_t)on * p.conv_k;
 #pragma unroll
-                for (int k = 0; k < 2; k++) pre_hist[k] = fresh ? 0.f : st[(size_t)k * p.ff + on];
-#pragma unroll
-                for (int k = 0; k < 3; k++) pre_cw[k] = cw[k];
+                for (int k = 0; k < 3; k++) {
+                    const int kk = min(k, p.conv_k - 2);
+                    pre_hist[k] = st[(size_t)kk * p.ff];
+                    pre_cw[k] = cw[kk];
+                }
+                pre_last = cw[p.conv_k - 1];
             }
         }
         float acc[MT][4];
@@ -309,22 +313,36 @@ gemm_rows_kernel(const RowsArgs p) {
                 float* st = p.conv_state + (size_t)p.seg_slot[m] * (Kc - 1) * d;
                 const float bx = __fmul_rn(b, xq);
                 float sum;
+#pragma unroll
+                for (int k = 0; k < 3; k++) pre_hist[k] = pre_fresh ? 0.f : pre_hist[k];
                 if (Kc == 3) {
-                    sum = __fadd_rn(__fadd_rn(__fmul_rn(pre_hist[0], pre_cw[0]), __fmul_rn(pre_hist[1], pre_cw[1])), __fmul_rn(bx, pre_cw[2]));
-                    st[n] = pre_hist[1];
-                    st[(size_t)d + n] = bx;
+                    sum = __fadd_rn(__fadd_rn(__fmul_rn(pre_hist[0], pre_cw[0]), __fmul_rn(pre_hist[1], pre_cw[1])), __fmul_rn(bx, pre_last));
                 } else {
-                    const bool fresh = p.seg_pos[m] == 0;
-                    const float* cw = p.conv_w + (size_t)n * Kc;
-                    sum = __fmul_rn(bx, cw[Kc - 1]);
-#pragma unroll 1
-                    for (int k = 0; k < Kc - 1; k++) {
-                        const float h = fresh ? 0.f : st[(size_t)k * d + n];
-                        sum = __fadd_rn(sum, __fmul_rn(h, cw[k]));
-                        if (k > 0) st[(size_t)(k - 1) * d + n] = h;
-                    }
-                    st[(size_t)(Kc - 2) * d + n] = bx;
+                    sum = __fmul_rn(bx, pre_last);
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        if (k < Kc - 1) sum = __fadd_rn(sum, __fmul_rn(pre_hist[k], pre_cw[k]));
                 }
+#pragma unroll
+                for (int k = 1; k < 3; k++)
+                    if (k < Kc - 1) st[(size_t)(k - 1) * d + n] = pre_hist[k];
+                if (Kc > 4) {                                            // more taps: four at a time, their loads in front of the stores
+                    const float* cw = p.conv_w + (size_t)n * Kc;
+#pragma unroll 1
+                    for (int k0 = 3; k0 < Kc - 1; k0 += 4) {
+                        float h[4], t4[4];
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const bool in = k0 + k < Kc - 1;
+                            h[k] = in && !pre_fresh ? st[(size_t)(k0 + k) * d + n] : 0.f;
+                            t4[k] = in ? cw[k0 + k] : 0.f;
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            if (k0 + k < Kc - 1) { sum = __fadd_rn(sum, __fmul_rn(h[k], t4[k])); st[(size_t)(k0 + k - 1) * d + n] = h[k]; }
+                    }
+                }
+                st[(size_t)(Kc - 2) * d + n] = bx;
                 if (p.conv_bias) sum = __fadd_rn(sum, p.conv_bias[n]);
                 ((bf16*)p.C)[o] = from_f32<bf16>(__fmul_rn(cq, sum));
             } else if (EPI == EPI_SWIGLU) {

@@ -70,7 +70,8 @@ def test_a_row_keeps_its_bits_when_a_ninth_joins(K):
             assert torch.equal(f(NormedRows(x[:M], gamma, EPS), w), nine[:M])
 
 
-@pytest.mark.parametrize("M,d,K,taps", [(1, 512, 512, 3), (8, 1000, 1024, 2), (3, 2048, 4096, 4), (7, 72, 1536, 7)])
+@pytest.mark.parametrize("M,d,K,taps", [(1, 512, 512, 3), (8, 1000, 1024, 2), (3, 2048, 4096, 4), (7, 72, 1536, 7), (2, 40, 512, 5), (5, 24, 512, 8),
+                                        (4, 520, 512, 9), (8, 16, 512, 12), (1, 300, 1024, 16)])
 def test_conv_step(M, d, K, taps):
     from kappai_b200.ops import kernels as Kn
     g = torch.Generator(device="cuda").manual_seed(d)
