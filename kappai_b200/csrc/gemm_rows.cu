@@ -31,13 +31,13 @@
 // pays only if every SM gets one of each, so accumulating products have small CTAs and the others, between which they
 // stand, big ones of more than half an SM; and only if the SM's split between cache and shared memory allows it (it is
 // set for the kernel that comes first: without the preference asked for in kp_smem_limit the second never came in).
-// A decode step of one request, us, norms apart | norms inside | and two CTAs an SM: 1.2B shape 511 | 475 | 459, 350M 341 |
-// 335 | 312; of eight requests (see rows_run) 555 | 539 | 567 and 369 | 378 | 366.
+// A decode step through eight layers, us, norms apart and a CTA an SM | norms apart, two | norms inside, two (five to eight rows: see
+// rows_run): one request, 1024 columns 183 | 183 | 165, 2048 275 | 278 | 251, 2560 422 | 430 | 372; eight 193 | 188 | 177,
+// 299 | 288 | 276, 457 | 448 | 431.
 // Big and small, KB, 64 steps of one request, 1.2B shape, ms: 148 + 78 32.1, 128 + 96 31.9, 116 + 110 32.2, 164 + 62 33.2.
 //
 // Epilogues as in gemm_stream.cu.  K a multiple of 512.  Loops are not unrolled where that gains nothing back to back: in a step
-// the kernels' code is fetched anew at every launch (the conv step's 27 KB of it became 16; with the attention kernels', the
-// merge's 34 KB 19, a step of eight requests of the 1.2B shape took 515 us instead of 541).
+// the kernels' code is fetched anew at every launch.
 #include "mma.cuh"
 
 #define EPI_STORE 0
@@ -409,8 +409,8 @@ static int rows_run_r(const RowsArgs& a, int epi, cudaStream_t s) {
 }
 
 // Two CTAs an SM or one (see the top).  With more than four rows A weighs as much as half of W, and two CTAs pay up to a residual of
-// 1024 columns only: a step of eight requests, us, two | one: 350M shape (1024 columns) 366 | 378, 1.2B shape (2048) 567 | 539;
-// of four requests 343 | 364 and 508 | 503.
+// 1024 columns only: a step through eight layers, us, two | one, of five requests 1024 columns 177 | 186, 1536 225 | 218, 2048
+// 283 | 275, 2560 427 | 416; of eight 176 | 185, 227 | 220, 287 | 277, 437 | 427.
 template <bool NORM>
 static int rows_run(const RowsArgs& a, int epi, cudaStream_t s) {
     if (a.M == 1) return rows_run_r<1, NORM, RW_BIG, RW_SMALL>(a, epi, s);
