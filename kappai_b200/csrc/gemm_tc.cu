@@ -49,8 +49,9 @@
 // warps at few rows, 12.9 and 6.7.)
 // With it every SM brings in a part of A only, and wide tiles still keep all SMs streaming.
 //
-// Every wait on an mbarrier is bounded.  A wait that gives up sets a status word (kp_tc_status), the CTA
-// stops issuing work, still frees its tensor memory and returns.
+// Every wait on an mbarrier is bounded, and a warp goes on or gives up as one: instructions for a whole warp come next.  A wait
+// that gives up sets a status word (kp_tc_status), the CTA stops issuing work, tells the other CTAs of its cluster, and all of
+// them linger until what is under way must have come, still free their tensor memory and return.
 #include "tcgen05.cuh"
 
 #define EPI_STORE 0
@@ -101,6 +102,7 @@ __device__ __forceinline__ void kp_copy_to_cluster(uint32_t dst, const void* src
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "r"(kp_smem_u32(src)), "r"(bytes), "r"(bar) : "memory");
 }
+__device__ __forceinline__ void kp_st_cluster(uint32_t addr, int v) { asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 // the epilogue warps (threads 64 ...) among themselves
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(TC_EPI_PER_Q * 128) : "memory"); }
 
@@ -406,9 +408,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
             const int tile = unit / S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
-            if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) {
-                ok = false;
-                if (S > 1) { __syncwarp(); kp_cluster_wait(); epi_sync(); }   // (where the other warps may be waiting for this one)
+            ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&acc_full[b2], set_ph) && !*abort_flag);
+            if (!ok) {
+                if (S > 1) { kp_cluster_wait(); epi_sync(); }             // (where the other warps may be waiting for this one)
                 break;
             }
             kp_tc_fence_after();
@@ -453,7 +455,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             epi_sync();
             if (warp == 2) {
-                if (!p.recv_apart && !kp_mbar_wait_bounded(rings_free, 0)) ok = false;
+                if (!p.recv_apart) ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(rings_free, 0));
                 const int olo = U * lane / S, bytes = (U * (lane + 1) / S - olo) * EIGHT * R;
                 if (ok && lane < S && lane != rank && bytes > 0)
                     kp_copy_to_cluster(kp_cluster_addr(recv, lane) + (rank < lane ? rank : rank - 1) * bytes, tiles + olo * EIGHT * R, bytes,
@@ -515,12 +517,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             }
         }
-        if (!ok && lane == 0) atomicExch(&g_tc_status, 1);
+        if (!ok) {
+            if (lane == 0) { *abort_flag = 1; atomicExch(&g_tc_status, 1); }
+            // (all CTAs of the cluster are told, none of which has left yet: copies from them to here and from here to them may be on their way)
+            if (S > 1 && lane < S) kp_st_cluster(kp_cluster_addr(const_cast<const int*>(abort_flag), lane), 1);
+        }
         if (S > 1) { __syncwarp(); kp_cluster_arrive(); }
     }
     kp_tc_fence_before();
     __syncthreads();
     if (S > 1) kp_cluster_wait();                                         // no CTA leaves before all have what they were sent, or have given up
+    if (*abort_flag) kp_linger_after_failure();
     if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
     if (warp == 1) kp_tmem_dealloc(tmem_base, p.tmem_cols);
 }
@@ -633,8 +640,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             bool ok = true;
     #pragma unroll 1
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-                ok = !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph));
                 if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
                 uint32_t tmem_d = tmem_base + (uint32_t)(b2 * p.inner * BN);
@@ -667,7 +673,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll 1
         for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const int m0 = (tile % tiles_m) * 2 * TC_BM + rank * TC_BM + q * 32, n0 = (tile / tiles_m) * N_OUT_TILE;
-            if (!kp_mbar_wait_bounded(&acc_full[b2], set_ph) || *abort_flag) { ok = false; break; }
+            ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&acc_full[b2], set_ph) && !*abort_flag);
+            if (!ok) break;
             kp_tc_fence_after();
             const uint32_t lane_base = tmem_base + (uint32_t)(b2 * p.inner * BN) + ((uint32_t)(q * 32) << 16);
             const int m = m0 + lane;

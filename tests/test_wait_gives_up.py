@@ -1,0 +1,45 @@
+"""What a kernel does when a bounded wait runs out, read from its source (no GPU is made to wait here): csrc/gemm_tc.cu, whose warps
+execute instructions for a whole warp or a whole cluster behind their waits, and whose CTAs are sent copies by other CTAs."""
+import os
+import re
+
+import pytest
+
+from kappai_b200.ops.build import CSRC_DIR
+
+WAIT = re.compile(r"\bkp_mbar_wait_bounded\(")
+
+
+def kernels(name):
+    """The text of each kernel of a source file, comments taken out."""
+    with open(os.path.join(CSRC_DIR, name), encoding="utf-8") as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    out = {}
+    for m in re.finditer(r"\n(\w+)\((?:[^()]|\([^()]*\))*\) \{\n", text):
+        if "__global__" in text[text.rfind("template", 0, m.start()):m.start()]:
+            out[m.group(1)] = text[m.start():text.index("\n}\n", m.end())]
+    return out
+
+
+@pytest.mark.parametrize("kernel", ["gemm_tc_kernel", "gemm_tc_pair_kernel"])
+def test_a_warp_gives_up_as_one(kernel):
+    body = kernels("gemm_tc.cu")[kernel]
+    lines = [l for l in body.splitlines() if WAIT.search(l)]
+    assert len(lines) >= 4
+    for l in lines:
+        assert re.search(r"__all_sync\(0xffffffffu, .*kp_mbar_wait_bounded\(", l), l
+
+
+@pytest.mark.parametrize("kernel", ["gemm_tc_kernel", "gemm_tc_pair_kernel"])
+def test_a_cta_that_gave_up_lingers_before_it_leaves(kernel):
+    body = kernels("gemm_tc.cu")[kernel]
+    linger = body.index("if (*abort_flag) kp_linger_after_failure();")
+    assert linger < body.index("kp_tmem_dealloc")
+    # behind every place that sets the flag, and (where other CTAs copy into this one) behind the last barrier of the cluster
+    assert linger > body.rindex("*abort_flag = 1")
+    if kernel == "gemm_tc_kernel":
+        assert linger > body.rindex("kp_cluster_wait()")
+        tell = body.index("kp_st_cluster(kp_cluster_addr(const_cast<const int*>(abort_flag), lane), 1)")
+        assert tell < body.rindex("kp_cluster_arrive()") < linger
+    else:
+        assert linger < body.rindex("kp_cluster_sync()")
