@@ -1747,13 +1747,13 @@ def gemm_stream_conv_step(a: torch.Tensor, w_in: torch.Tensor, bias: Optional[to
 ROWS_NORM_MAX_K = 4096     # columns up to which csrc/gemm_rows.cu norms its rows itself
 
 
-def rows_norm_fusable(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Can the product of the RMS norm of ``x`` (float32 rows, to bfloat16) with ``w`` norm the rows itself?  Up to 8 rows, where the
+def rows_norm_fusable(x: torch.Tensor, gamma: torch.Tensor, w: torch.Tensor) -> bool:
+    """Can the product of the RMS norm of ``x`` (float32 rows, weight ``gamma``, to bfloat16) with ``w`` norm the rows itself?  Up to 8 rows, where the
     product would run on csrc/gemm_rows.cu: the norm in front of it is a launch of 2 us whose work is a load and two multiplications
     a value."""
     M, d = x.shape
     return (USE_STREAM and 0 < M <= ROWS_MAX_M and d <= ROWS_NORM_MAX_K and stream_fits(d, False) and w.shape[0] <= 16384
-            and w.shape[1] == d and _rows_16_bytes(w) and x.is_contiguous() and x.data_ptr() % 16 == 0)
+            and w.shape[1] == d and _rows_16_bytes(w) and x.is_contiguous() and x.data_ptr() % 16 == 0 and gamma.data_ptr() % 16 == 0)
 
 
 def _normed_args(x: torch.Tensor, gamma: torch.Tensor, eps: float):

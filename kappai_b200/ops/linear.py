@@ -49,7 +49,7 @@ class NormedRows:
         return self.weight, self.eps
 
     def fusable(self, w: torch.Tensor) -> bool:
-        return K.rows_norm_fusable(self.x, w)
+        return K.rows_norm_fusable(self.x, self.weight, w)
 
     def rows(self) -> torch.Tensor:
         return K.rmsnorm_rows(self.x, self.weight, self.eps, torch.empty(self.x.shape, dtype=self.dtype, device=self.x.device))

@@ -102,3 +102,13 @@ def test_one_door_norms_the_rows_where_the_kernel_does_not():
         assert torch.equal(linear_weights(NormedRows(x, gamma, EPS), w), linear(h, w))           # (768 is no multiple of 512)
         assert torch.equal(linear_weights(NormedRows(x, gamma, EPS), w.float()), linear(h, w.float()))
         assert torch.equal(linear_weights_swiglu(NormedRows(x, gamma, EPS), w), linear_weights_swiglu(h, w))
+
+
+@pytest.mark.parametrize("off", [0, 1, 2])
+def test_a_norm_weight_that_is_part_of_a_larger_one(off):
+    from kappai_b200.ops import kernels as Kn
+    from kappai_b200.ops.linear import NormedRows, linear_weights
+    g = torch.Generator(device="cuda").manual_seed(off)
+    x, gamma = torch.randn(3, 1024, device="cuda", generator=g), torch.rand(1026, device="cuda", generator=g)[off:off + 1024]
+    w = (torch.randn(72, 1024, device="cuda", generator=g) / 32).bfloat16()
+    assert torch.equal(linear_weights(NormedRows(x, gamma, EPS), w), linear_weights(normed(Kn, x, gamma), w))

@@ -71,3 +71,12 @@ def test_asked_in_steps_of_few_rows_only(rows):
     block = PreNormResidualBlock({}, BuildEnv(torch.device("cpu"), torch.bfloat16, 16)).assemble(Sublayer(), Sublayer(), Norm(), Norm())
     block.forward(torch.zeros(rows, 4), SimpleNamespace(n_rows=rows), None)
     assert calls == (["asked", "left"] if rows <= 8 else ["norm", "normed"]) * 2
+
+
+def test_a_weight_off_its_boundary_is_left_to_the_norm_kernel():
+    """The product reads the norm's weight 16 bytes at a time; the norm kernel takes any."""
+    x, w = torch.zeros(3, 512), torch.zeros(64, 512, dtype=torch.bfloat16)
+    whole = torch.ones(516)
+    assert NormedRows(x, whole[:512], 1e-5).fusable(w) and NormedRows(x, whole[4:], 1e-5).fusable(w)
+    for off in (1, 2, 3):
+        assert not NormedRows(x, whole[off:off + 512], 1e-5).fusable(w)
