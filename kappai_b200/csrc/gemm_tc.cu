@@ -544,12 +544,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 //
 // The epilogue warps pass their pieces (128 bytes of 32 rows) through shared memory, so that a warp writes, and for an
 // accumulated output reads, four whole rows' stretches of 128 bytes at a time instead of 16 bytes of 32 rows; the old
-// values of an accumulated output are asked for before the piece is read from tensor memory.  Accumulating and gated kernels take
-// 16 columns of sums at a time, the others 32.  us, 16 | 32 at a time: accumulating 2,048 rows by 2048 x 2048 18.9 | 20.1 (the old
-// values need the registers); stored 999 rows by 3072 x 2048 15.5 | 15.3, by 65536 x 1024 in 32 bits 120.0 | 119.0, 2,048 rows by
-// 3072 x 2048 25.8 | 25.0; gated 999 rows by 9216 x 1024 22.2 | 21.8, but 41 KB of code against 98, and in a prompt, where the
-// code comes anew at every launch, the gain is gone (2,048 tokens of the 1.2B shape 3.249 | 3.253 ms, 999 rows of the 350M shape
-// 1.730 | 1.732).
+// values of an accumulated output are asked for before the piece is read from tensor memory.  16 columns of
+// sums at a time, but for a float32 store (a head) 32.  us, 16 | 32 at a time: float32 999 rows by 65536 x 1024 120.0 | 119.0;
+// accumulating 2,048 rows by 2048 x 2048 18.9 | 20.1 (the old values need the registers); gated 999 rows by 9216 x 1024 22.2 | 21.8,
+// but 41 KB of code against 98, and in a prompt, where the code comes anew at every launch, the gain is gone (2,048 tokens of the 1.2B
+// shape 3.249 | 3.253 ms); stored 999 rows by 3072 x 2048 15.5 | 15.3, but the convolution behind such a product is then no longer resident
+// beside it, for the registers, and the product behind that takes the SMs in front of it: a step of 2,048 rows, some of them
+// decoded, 3.28 | 3.41 ms (350M shape 2.10 | 2.31).
 #define TC_PAIR_STAGES(BN) ((BN) == 256 ? 5 : 7)
 #define TC_PAIR_SMEM(BN) ((size_t)TC_PAIR_STAGES(BN) * (128 + (BN) / 2) * TC_BK * 2 + TC_EPI_PER_Q * 4 * 4096 + (2 * TC_PAIR_STAGES(BN) + 4) * 8 + 16 + 1024)
 
@@ -666,7 +667,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         unsigned char* piece = pieces + (size_t)(warp - 2) * 4096;
         constexpr bool NARROW = EPI == EPI_STORE || EPI == EPI_ACT || TC_GATED(EPI);   // 16-bit outputs: a piece is 64 columns
         constexpr int PW = NARROW ? 64 : 32;
-        constexpr int PC = EPI == EPI_ACCUM_F32 || TC_GATED(EPI) ? 16 : 32;            // columns of sums at a time (see above)
+        constexpr int PC = EPI == EPI_STORE_F32 ? 32 : 16;                // columns of sums at a time (see above)
         int b2 = 0;
         uint32_t set_ph = 0;
         bool ok = true;
@@ -691,7 +692,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         if (row < p.M) old[i] = *reinterpret_cast<const float4*>((const float*)p.C + (size_t)row * p.ldc + n0 + c + pch * 4);
                     }
                 }
-#pragma unroll (PC == 32 ? 2 : 1)
+#pragma unroll 1
                 for (int h = 0; h < PW / PC; h++) {
                     const int n_base = n0 + c + h * PC;
                     float v[PC], up[PC];
