@@ -1037,6 +1037,13 @@ int kp_gemm_tc_as(const void* A, int lda, const void* W, int ldw, const float* b
     if (cluster) {
         const long long tiles = (long long)((n_out + cols - 1) / cols) * m_tiles;
         if (tiles > 65535 || !tc_split_starts(K, parts, (int)tiles) || !tc_split_runs(M, K, kind, bn, parts, (int)tiles)) return KP_ERR_UNSUPPORTED;
+        // Five parts or more of 256 columns by 121 rows and more: the sums that go out and come in do not fit beside one another.
+        // The same parts, and so the same bits, by a cluster for each half of the columns, or one after the other.
+        if (tc_smem(M, tc_a_rows(M), bn, gated, parts).bytes > KP_SMEM_MAX) {
+            const long long halves = (long long)((n_out + cols / 2 - 1) / (cols / 2)) * m_tiles;
+            cluster = halves <= 65535 && tc_split_starts(K, parts, (int)halves) && tc_split_runs(M, K, kind, bn / 2, parts, (int)halves);
+            bn = cluster ? bn / 2 : 64;
+        }
     } else {
         const int kbs = (n_kb + parts - 1) / parts;
         if (!tc_sets(bn, parts) || (n_kb + kbs - 1) / kbs != parts) return KP_ERR_UNSUPPORTED;
