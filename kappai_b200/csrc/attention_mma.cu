@@ -181,8 +181,9 @@ attn_split_mma_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __res
     const int t0 = c0 + warp * AM_TILE;                           // first key of this warp's tile
     if (TMA) {
         __syncthreads();                                          // the barrier is initialised
-        if (!kp_mbar_wait_bounded(bar, 0)) {
+        if (!__all_sync(0xffffffffu, kp_mbar_wait_bounded(bar, 0))) {   // (a warp gives up as one)
             if (lane == 0) atomicExch(&g_attn_status, 1);
+            kp_linger_after_failure();
             return;                                                // (every thread sees the same barrier)
         }
         // V rows of keys that this row does not read hold whatever was there: zero them (P is 0 there, but
@@ -432,11 +433,11 @@ attn_split_ring_kernel(const __grid_constant__ CUtensorMap tmC, const bf16* __re
         const int s = k % AR_STAGES;
         // The four warps of the group leave the loop together or not at all (the group's barriers below count all
         // of them): a warp whose wait ran out says so, and all of them look after a barrier.
-        if (!kp_mbar_wait_bounded(&full[s], (k / AR_STAGES) & 1)) {
+        if (!__all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], (k / AR_STAGES) & 1))) {
             if (lane == 0) { atomicExch(&g_attn_status, 1); gave_up[grp] = 1; }
         }
         group_sync();
-        if (gave_up[grp]) break;
+        if (gave_up[grp]) { kp_linger_after_failure(); break; }
         const ArMeta me = metas[s];
         if (me.row < 0) break;
         unsigned char* st = base + (size_t)s * STAGE;

@@ -225,7 +225,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             for (int d = 0; d < AT_HD; d++) o[d] = 0.f;
             float m = -INFINITY, l = 0.f;
             for (int kt = it.kt_lo; kt <= it.kt_hi && ok; kt++, i++) {
-                if (!kp_mbar_wait_bounded(s_full, i & 1) || *abort_flag) { ok = false; break; }
+                ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(s_full, i & 1) && !*abort_flag);   // (a warp gives up as one)
+                if (!ok) break;
                 kp_tc_fence_after();
                 // Most tiles lie wholly inside every row's keys; only the tile on the diagonal, a window's edge
                 // and rows past the end of the segment need the mask.  Scores are taken in base 2:
@@ -295,7 +296,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P is read by the tensor core
                 kp_mbar_arrive(p_full);
                 // O = O * corr + P V
-                if (!kp_mbar_wait_bounded(pv_full, i & 1)) { ok = false; break; }
+                ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(pv_full, i & 1));
+                if (!ok) break;
                 kp_tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < AT_HD; c += 32) {
@@ -319,10 +321,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 }
             }
         }
-        if (!ok && lane == 0) atomicExch(&g_attn_tc_status, 1);
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(&g_attn_tc_status, 1); }
     }
     kp_tc_fence_before();
     __syncthreads();
+    if (*abort_flag) kp_linger_after_failure();
     if (warp == 1) kp_tmem_dealloc(tmem_base, 256);
 }
 
@@ -494,7 +497,7 @@ attn_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             const int lo_max = kp_key_lo(it.k_hi_all, p.window, p.block);
             float m = -INFINITY, l = 0.f;
             for (int kt = it.kt_lo; kt <= it.kt_hi; kt++, i++) {
-                if (ok && (*abort_flag || !kp_mbar_wait_bounded(&s_full[g], i & 1))) ok = false;
+                if (ok) ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&s_full[g], i & 1));   // (a warp gives up as one)
                 kp_tc_fence_after();
                 uint32_t s0[32], s1[32], s2[32], s3[32];
                 kp_tmem_ld32_issue(tmem_s, s0);
@@ -524,7 +527,7 @@ attn_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                 const float m_sub = (m_new == -INFINITY) ? 0.f : m_new;
                 if (kt > it.kt_lo) {
                     // the product of the tile before has read P and added to O
-                    if (ok && !kp_mbar_wait_bounded(&o_done[g], (i - 1) & 1)) ok = false;
+                    if (ok) ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&o_done[g], (i - 1) & 1));
                     if (__any_sync(0xffffffffu, corr != 1.0f)) {
                         kp_tc_fence_after();
 #pragma unroll 1
@@ -578,7 +581,7 @@ attn_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                 kp_mbar_arrive(&p_full[g]);
             }
             // the row is complete when the last product is
-            if (ok && !kp_mbar_wait_bounded(&o_done[g], (i - 1) & 1)) ok = false;
+            if (ok) ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&o_done[g], (i - 1) & 1));
             kp_tc_fence_after();
             const float inv = l > 0.f ? 1.0f / l : 0.f;
             bf16* dst = p.out + (size_t)(it.row0 + r) * p.ldo + (size_t)h * AT_HD;
@@ -600,10 +603,11 @@ attn_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             }
             kp_tc_fence_before();
         }
-        if (!ok && lane == 0) atomicExch(&g_attn_tc_status, 1);
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(&g_attn_tc_status, 1); }
     }
     kp_tc_fence_before();
     __syncthreads();
+    if (*abort_flag) kp_linger_after_failure();
     if (warp == 1) kp_tmem_dealloc(tmem_base, 512);
 }
 

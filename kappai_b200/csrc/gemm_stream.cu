@@ -228,7 +228,7 @@ gemm_stream_kernel(const StreamArgs p) {
         auto run_stage = [&](int c, auto slot0) {
             constexpr int SLOT0 = decltype(slot0)::value;
             const int s = it % S;
-            if (alive && !kp_mbar_wait_bounded(&full[s], (it / S) & 1, ST_WAIT_NS)) alive = false;
+            if (alive) alive = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], (it / S) & 1, ST_WAIT_NS));   // (a warp gives up as one)
             const unsigned char* stage = ring + (size_t)s * STAGE_BYTES + 16 * t;
 #pragma unroll
             for (int j = 0; j < 2; j++) {

@@ -409,7 +409,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int tile = unit / S;
             const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * N_OUT_TILE;
             ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&acc_full[b2], set_ph) && !*abort_flag);
-            if (!ok) {
+            if (__builtin_expect(!ok, 0)) {
                 if (S > 1) { kp_cluster_wait(); epi_sync(); }             // (where the other warps may be waiting for this one)
                 break;
             }
@@ -517,7 +517,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             }
         }
-        if (!ok) {
+        if (__builtin_expect(!ok, 0)) {
             if (lane == 0) { *abort_flag = 1; atomicExch(&g_tc_status, 1); }
             // (all CTAs of the cluster are told, none of which has left yet: copies from them to here and from here to them may be on their way)
             if (S > 1 && lane < S) kp_st_cluster(kp_cluster_addr(const_cast<const int*>(abort_flag), lane), 1);
@@ -527,9 +527,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     kp_tc_fence_before();
     __syncthreads();
     if (S > 1) kp_cluster_wait();                                         // no CTA leaves before all have what they were sent, or have given up
-    if (*abort_flag) kp_linger_after_failure();
     if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
-    if (warp == 1) kp_tmem_dealloc(tmem_base, p.tmem_cols);
+    if (warp == 1) {                                                      // (one warp that lingers keeps the CTA's memory)
+        if (*abort_flag) kp_linger_after_failure();
+        kp_tmem_dealloc(tmem_base, p.tmem_cols);
+    }
 }
 
 // ------------------------------------------------------------------------------------------ pairs of CTAs

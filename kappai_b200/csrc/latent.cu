@@ -487,7 +487,7 @@ latent_split_tc_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_con
         };
         auto softmax = [&](int it) {                               // false: the warps of the group leave
             const int b = it & 1, s = it % p.n_stages;
-            if (ok && (!kp_mbar_wait_bounded(&s_full[b], (it >> 1) & 1) || *abort_flag)) ok = false;
+            if (ok) ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&s_full[b], (it >> 1) & 1) && !*abort_flag);   // (a warp gives up as one)
             kp_tc_fence_after();
             const int valid = min(LT_TILE, n_keys - it * LT_TILE);
             float v[HQ];
@@ -556,7 +556,8 @@ latent_split_tc_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_con
             return true;
         };
         auto gather = [&](int it) {
-            if (!kp_mbar_wait_bounded(u_full, it & 1) || *abort_flag) { ok = false; return; }
+            ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(u_full, it & 1) && !*abort_flag);
+            if (!ok) return;
             kp_tc_fence_after();
             const float* corr = corr_s + (it & 3) * NH;
 #pragma unroll

@@ -635,7 +635,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
         }
     } else if (live) {
         const int q = warp & 3;                              // the quarter of the lanes this warp may read
-        const bool ok = kp_mbar_wait_bounded(acc_full, 0) && !*abort_flag;
+        const bool ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(acc_full, 0) && !*abort_flag);   // (a warp gives up as one)
         if (!ok) *abort_flag = 1;
         kp_tc_fence_after();
         const int m = row0 + q * 32 + lane;

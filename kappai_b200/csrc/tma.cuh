@@ -55,7 +55,7 @@ __device__ __forceinline__ bool kp_mbar_wait_bounded(uint64_t* bar, uint32_t par
 // A CTA that gave up a wait must not leave while bulk copies into its shared memory may still be under way
 // (the memory could be handed to the next CTA meanwhile): it lingers for a moment that is far longer than any
 // copy takes.  Only the failure path comes here.
-__device__ __forceinline__ void kp_linger_after_failure() {
+__device__ __noinline__ void kp_linger_after_failure() {
     const unsigned long long t0 = kp_now_ns();
     while (kp_now_ns() - t0 < 200000ull) __nanosleep(1000);
 }

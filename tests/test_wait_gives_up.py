@@ -43,3 +43,20 @@ def test_a_cta_that_gave_up_lingers_before_it_leaves(kernel):
         assert tell < body.rindex("kp_cluster_arrive()") < linger
     else:
         assert linger < body.rindex("kp_cluster_sync()")
+
+
+@pytest.mark.parametrize("name,barriers", [("attention_tc.cu", ["s_full", "pv_full", "&s_full[g]", "&o_done[g]"]), ("latent.cu", ["&s_full[b]", "u_full", "o_full"]),
+                                           ("moe.cu", ["acc_full"]), ("attention_mma.cu", ["bar", "&full[s]"]), ("gemm_stream.cu", ["&full[s]"])])
+def test_warps_of_other_kernels_give_up_as_one(name, barriers):
+    """The waits of whole warps, behind which instructions for a whole warp come (elsewhere one lane waits)."""
+    with open(os.path.join(CSRC_DIR, name), encoding="utf-8") as f:
+        lines = f.read().splitlines()
+    for b in barriers:
+        waits = [l for l in lines if f"kp_mbar_wait_bounded({b}," in l]
+        assert waits and all("__all_sync(0xffffffffu, " in l for l in waits), (b, waits)
+
+
+def test_no_attention_cta_leaves_with_copies_under_way():
+    for name, n in (("attention_tc.cu", 2), ("attention_mma.cu", 2)):
+        with open(os.path.join(CSRC_DIR, name), encoding="utf-8") as f:
+            assert f.read().count("kp_linger_after_failure()") == n
