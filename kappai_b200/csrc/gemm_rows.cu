@@ -46,6 +46,7 @@
 #define EPI_SWIGLU 3
 #define EPI_CONV_STEP 4
 #define EPI_ACT 6
+#define EPI_CONV_ANY 7                       // inside this file only: EPI_CONV_STEP with other than three taps
 
 #define RW_WARPS 8
 #define RW_NORM_MAX_K 4096                   // columns up to which the normed form holds A (8 rows: 64 KB)
@@ -85,12 +86,14 @@ template <int WR, int R, bool NORM, int ROOM> struct RowsShape {
     }
 };
 
-template <int WR, int EPI, int R, bool NORM, int ROOM>
+// LONG: the normed form of more than 2048 columns.  EPI_CONV_STEP has three taps, EPI_CONV_ANY any number.
+template <int WR, int EPI, int R, bool NORM, int ROOM, bool LONG>
 __global__ void __launch_bounds__(RW_WARPS * 32, 1)
 gemm_rows_kernel(const RowsArgs p) {
     using Shape = RowsShape<WR, R, NORM, ROOM>;
     constexpr int MT = Shape::MT, W_BYTES = Shape::W_BYTES, STAGE = Shape::STAGE, S = Shape::S;
-    constexpr int JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
+    constexpr bool CONV = EPI == EPI_CONV_STEP || EPI == EPI_CONV_ANY;
+    constexpr int JOINS = CONV ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
     constexpr int TROWS = WR / JOINS;                                    // output columns a tile
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -143,7 +146,7 @@ gemm_rows_kernel(const RowsArgs p) {
     if constexpr (NORM) {
         // A thread has the float4s threadIdx.x, + 256, ... of every row; the first KEEP of each stay in registers (all of them, but
         // for more than 2048 columns of more than four rows: 128 registers).
-        constexpr int KEEP = R <= 4 ? 4 : 2;
+        constexpr int KEEP = LONG && R <= 4 ? 4 : 2;
         const int tid = threadIdx.x, n4 = p.K >> 2;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         const auto x_at = [&](int r, int i) { return r < M && i < n4 ? *reinterpret_cast<const float4*>(p.X + (size_t)r * p.ldx + i * 4) : zero; };
@@ -165,13 +168,15 @@ gemm_rows_kernel(const RowsArgs p) {
 #pragma unroll
             for (int j = 0; j < KEEP; j++) ss[r] = squares(v[r][j], ss[r]);
         }
+        if (LONG && R > 4) {
 #pragma unroll 1
-        for (int j = KEEP; j * 256 < n4; j++)
+            for (int j = KEEP; j * 256 < n4; j++)
 #pragma unroll
-            for (int r = 0; r < R; r++) ss[r] = squares(x_at(r, tid + j * 256), ss[r]);
+                for (int r = 0; r < R; r++) ss[r] = squares(x_at(r, tid + j * 256), ss[r]);
+        }
         // the sum over the threads, as the norm kernel of that size has it: up to 2048 columns the warps' values lane by lane, in
         // the order of the warps, then the lanes; beyond, the lanes of a warp, then the warps
-        const bool by_lane = n4 <= 512;
+        constexpr bool by_lane = !LONG;
         float* part = red;                                               // [row][warp][lane], or [row][256] by warp
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -210,11 +215,13 @@ gemm_rows_kernel(const RowsArgs p) {
         for (int r = 0; r < R; r++)
 #pragma unroll
             for (int j = 0; j < KEEP; j++) hold(r, tid + j * 256, v[r][j], gm[j]);
+        if (LONG && R > 4) {
 #pragma unroll 1
-        for (int j = KEEP; j * 256 < n4; j++) {
-            const float4 g4 = gamma_at(tid + j * 256);
+            for (int j = KEEP; j * 256 < n4; j++) {
+                const float4 g4 = gamma_at(tid + j * 256);
 #pragma unroll
-            for (int r = 0; r < R; r++) hold(r, tid + j * 256, x_at(r, tid + j * 256), g4);
+                for (int r = 0; r < R; r++) hold(r, tid + j * 256, x_at(r, tid + j * 256), g4);
+            }
         }
         __syncthreads();
     } else {
@@ -232,23 +239,25 @@ gemm_rows_kernel(const RowsArgs p) {
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
         const int n0 = tile * TROWS;
         // what the epilogue needs beside the sums is asked for now: its trips to L2 run under the main loop
-        float pre_c = 0.f, pre_hist[3] = {0.f, 0.f, 0.f}, pre_cw[3] = {0.f, 0.f, 0.f}, pre_last = 0.f;
+        constexpr int PRE = EPI == EPI_CONV_STEP ? 2 : 3;                // kept inputs fetched ahead, with their taps, and the last tap
+        float pre_c = 0.f, pre_hist[PRE] = {}, pre_cw[PRE] = {}, pre_last = 0.f;
         bool pre_fresh = false;
         const int om = threadIdx.x / TROWS, on = n0 + threadIdx.x % TROWS;   // this thread's output (the first TROWS * M threads)
         const bool mine = om < M && on < n_out;
+        const int Kc = EPI == EPI_CONV_STEP ? 3 : p.conv_k;
         if (mine) {
             if (EPI == EPI_ACCUM_F32) pre_c = ((const float*)p.C)[(size_t)om * p.ldc + on];
-            if (EPI == EPI_CONV_STEP) {                                  // (the first three of the kept inputs, the last tap; a new request's kept
-                pre_fresh = p.seg_pos[om] == 0;                          //  inputs count as zeros below, so that nothing here waits for its position)
-                const float* st = p.conv_state + (size_t)p.seg_slot[om] * (p.conv_k - 1) * p.ff + on;
-                const float* cw = p.conv_w + (size_t)on * p.conv_k;
+            if (CONV) {                                                  // (a new request's kept inputs count as zeros below, so that
+                pre_fresh = p.seg_pos[om] == 0;                          //  nothing here waits for its position)
+                const float* st = p.conv_state + (size_t)p.seg_slot[om] * (Kc - 1) * p.ff + on;
+                const float* cw = p.conv_w + (size_t)on * Kc;
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const int kk = min(k, p.conv_k - 2);
+                for (int k = 0; k < PRE; k++) {
+                    const int kk = min(k, Kc - 2);
                     pre_hist[k] = st[(size_t)kk * p.ff];
                     pre_cw[k] = cw[kk];
                 }
-                pre_last = cw[p.conv_k - 1];
+                pre_last = cw[Kc - 1];
             }
         }
         float acc[MT][4];
@@ -303,33 +312,33 @@ gemm_rows_kernel(const RowsArgs p) {
             float v = sum_of(lr);
             if (p.bias) v += p.bias[n];
             const size_t o = (size_t)m * p.ldc + n;
-            if (EPI == EPI_CONV_STEP) {
+            if (CONV) {
                 float cg = sum_of(8 + lr), xv = sum_of(16 + lr);
                 if (p.bias) { cg += p.bias[p.ff + n]; xv += p.bias[2 * p.ff + n]; }
                 // B, C and X as the separate product stores them, then shortconv.cu's decode step: every product and
                 // sum rounded on its own (src/backend/cpu/common.c:2393-2431)
                 const float b = to_f32(from_f32<bf16>(v)), cq = to_f32(from_f32<bf16>(cg)), xq = to_f32(from_f32<bf16>(xv));
-                const int d = p.ff, Kc = p.conv_k;
+                const int d = p.ff;
                 float* st = p.conv_state + (size_t)p.seg_slot[m] * (Kc - 1) * d;
                 const float bx = __fmul_rn(b, xq);
                 float sum;
 #pragma unroll
-                for (int k = 0; k < 3; k++) pre_hist[k] = pre_fresh ? 0.f : pre_hist[k];
-                if (Kc == 3) {
+                for (int k = 0; k < PRE; k++) pre_hist[k] = pre_fresh ? 0.f : pre_hist[k];
+                if (EPI == EPI_CONV_STEP || Kc == 3) {
                     sum = __fadd_rn(__fadd_rn(__fmul_rn(pre_hist[0], pre_cw[0]), __fmul_rn(pre_hist[1], pre_cw[1])), __fmul_rn(bx, pre_last));
                 } else {
                     sum = __fmul_rn(bx, pre_last);
 #pragma unroll
-                    for (int k = 0; k < 3; k++)
+                    for (int k = 0; k < PRE; k++)
                         if (k < Kc - 1) sum = __fadd_rn(sum, __fmul_rn(pre_hist[k], pre_cw[k]));
                 }
 #pragma unroll
-                for (int k = 1; k < 3; k++)
+                for (int k = 1; k < PRE; k++)
                     if (k < Kc - 1) st[(size_t)(k - 1) * d + n] = pre_hist[k];
-                if (Kc > 4) {                                            // more taps: four at a time, their loads in front of the stores
+                if (EPI == EPI_CONV_ANY && Kc > 4) {                     // more taps: four at a time, their loads in front of the stores
                     const float* cw = p.conv_w + (size_t)n * Kc;
 #pragma unroll 1
-                    for (int k0 = 3; k0 < Kc - 1; k0 += 4) {
+                    for (int k0 = PRE; k0 < Kc - 1; k0 += 4) {
                         float h[4], t4[4];
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
@@ -375,16 +384,24 @@ static int rw_n_sm() {
     return n;
 }
 
-template <int WR, int EPI, int R, bool NORM, int ROOM>
-static int rows_launch(const RowsArgs& a, cudaStream_t s) {
+template <int WR, int EPI, int R, bool NORM, int ROOM, bool LONG>
+static int rows_launch_as(const RowsArgs& a, cudaStream_t s) {
     using Shape = RowsShape<WR, R, NORM, ROOM>;
-    constexpr int JOINS = EPI == EPI_CONV_STEP ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
-    auto kern = gemm_rows_kernel<WR, EPI, R, NORM, ROOM>;
+    constexpr int JOINS = EPI == EPI_CONV_STEP || EPI == EPI_CONV_ANY ? 3 : (EPI == EPI_SWIGLU ? 2 : 1);
+    auto kern = gemm_rows_kernel<WR, EPI, R, NORM, ROOM, LONG>;
     static std::atomic<unsigned long long> ready{0};
     const int st = kp_smem_limit(kern, Shape::bytes(RW_NORM_MAX_K), ready, true);
     if (st) return st;
     const int n_out = JOINS > 1 ? a.ff : a.N, n_tiles = (n_out + WR / JOINS - 1) / (WR / JOINS);
     return (int)kp_launch_pdl(kern, dim3(n_tiles < rw_n_sm() ? n_tiles : rw_n_sm()), dim3(RW_WARPS * 32), Shape::bytes(a.K), s, a);
+}
+
+// (Instances of their own for what few models need: in the one kernel their code, fetched at every launch, cost a short chat of the
+// 350M shape 1.2 % for more than 2048 columns, 0.25 % for other than three taps.)
+template <int WR, int EPI, int R, bool NORM, int ROOM>
+static int rows_launch(const RowsArgs& a, cudaStream_t s) {
+    if constexpr (NORM) if (a.K > 2048) return rows_launch_as<WR, EPI, R, NORM, ROOM, true>(a, s);
+    return rows_launch_as<WR, EPI, R, NORM, ROOM, false>(a, s);
 }
 
 template <int R, bool NORM, int BIG, int SMALL>
@@ -402,7 +419,8 @@ static int rows_run_r(const RowsArgs& a, int epi, cudaStream_t s) {
             return KP_ERR_BAD_ARG;
         case EPI_ACT: RW_PICK(EPI_ACT, BIG);
         case EPI_SWIGLU: return rows_launch<16, EPI_SWIGLU, R, NORM, BIG>(a, s);
-        case EPI_CONV_STEP: return rows_launch<24, EPI_CONV_STEP, R, NORM, BIG>(a, s);
+        case EPI_CONV_STEP:
+            return a.conv_k == 3 ? rows_launch<24, EPI_CONV_STEP, R, NORM, BIG>(a, s) : rows_launch<24, EPI_CONV_ANY, R, NORM, BIG>(a, s);
         default: return KP_ERR_BAD_ARG;
     }
 #undef RW_PICK
