@@ -11,12 +11,12 @@
 //              the 128-byte swizzle, no multicast.  The ring has as many stages as fit shared memory.
 //   warp 1   : allocates tensor memory (accumulators for two tiles, if there is room: the epilogue of a tile runs
 //              under the main loop of the next), then an elected lane of the warp issues the MMAs: four tcgen05.mma (128 x BN x 16)
-//              per stage, descriptors advanced by 32 bytes inside the swizzled rows (from inside a branch that one lane
+//              per k-block, descriptors advanced by 32 bytes inside the swizzled rows (from inside a branch that one lane
 //              took, a k-block cost about 0.3 us whatever its width: 128 rows by 2048 x 5632, 17.0 us against 12.4); tcgen05.commit frees the
 //              stage ("empty" mbarrier) and, after the last k-block, signals "accumulator full".
 //   the rest : epilogue, two warps for each quarter of the 128 lanes of tensor memory (a warp may only read
-//              the lanes 32 * (warp % 4) ...), taking the 32-column pieces in turn so that more loads and
-//              stores are in flight.  Each reads its lanes with tcgen05.ld (32 columns at a time), applies
+//              the lanes 32 * (warp % 4) ...), taking pieces of 16 columns in turn so that more loads and
+//              stores are in flight.  Each reads its lanes with tcgen05.ld (a piece at a time; 32 columns where sums go to other CTAs), applies
 //              bias / residual accumulation / SwiGLU, writes its rows of C and hands the accumulator back.
 // A k-block costs the producer and the MMA warp about 0.1 us of waits, arming and commits beside its copies and MMAs, so a
 // stage holds two k-blocks where that is at most 64 KB: one copy an operand, of a tensor map with the k-blocks as a
@@ -44,9 +44,9 @@
 // (a bulk copy between the CTAs' rings, counted at a barrier of the owner), and adds up its own, the parts in order of their number -- so the result
 // does not depend on timing -- then the epilogue.  The old values of an accumulated output come in under the exchange.
 // (Sums left in shared memory and read by the others between two barriers of the cluster took 4.5 us from the last MMA to the
-// end, of products of 8 to 16: 128 rows by 2048 x 5632 16.0 us, this 12.0; 17 rows by 2048 x 2048 6.0 and 5.7.  Sent by single
-// stores that count at the barrier, st.async, 13.0 and 7.7; added by the threads that read tensor memory, a few lanes of few
-// warps at few rows, 12.9 and 6.7.)
+// end: with weights from HBM, 128 rows by 2048 x 5632 16.2 us, this 13.7; 17 rows by 2048 x 2048 6.4 and 5.9.  Sent by single
+// stores that count at the barrier, st.async, the two took 8 and 35 % longer; added by the threads that read tensor memory, a few lanes
+// of few warps at few rows, 7 and 18 %.)
 // With it every SM brings in a part of A only, and wide tiles still keep all SMs streaming.
 //
 // Every wait on an mbarrier is bounded, and a warp goes on or gives up as one: instructions for a whole warp come next.  A wait
@@ -123,8 +123,8 @@ __device__ __forceinline__ void tc_bias(const TcArgs& p, int n_lim, float (&g)[W
         }
     }
 }
-// What becomes of a sum.  silu has instantiations of its own: with the activation chosen at run time every one of the 32
-// unrolled outputs carried the code of all of them, and the epilogue waited for instructions (200 rows by gate/up
+// What becomes of a sum.  silu has instantiations of its own: with the activation chosen at run time every one of the
+// 32 outputs that were unrolled then carried the code of all of them, and the epilogue waited for instructions (200 rows by gate/up
 // 11264 x 2048: 24.1 us a product against 20.7; the kernel of pairs 31.6 against 20.2).
 template <int EPI>
 __device__ __forceinline__ float tc_value(const TcArgs& p, float g, float u) {
@@ -137,7 +137,7 @@ __device__ __forceinline__ float tc_value(const TcArgs& p, float g, float u) {
     return EPI == EPI_ACT ? kp_act_plain(p.act, g) : g;
 }
 
-// A piece of W output columns (32, or 4 in the split's reduction) of row m, from its sums g (and u: the up half,
+// A piece of W output columns (16; 32 behind a pair's float32 store; 4 in the split's reduction) of row m, from its sums g (and u: the up half,
 // SwiGLU), to C: bias, SwiGLU or accumulation, and the store (vector stores where rows of C are 16-byte aligned).
 template <int EPI, int W>
 __device__ __forceinline__ void tc_finish(const TcArgs& p, int n_lim, const float (&g)[W], const float (&u)[W], int m,
@@ -198,7 +198,6 @@ __device__ __forceinline__ void tc_finish(const TcArgs& p, int n_lim, const floa
 // W columns of tensor memory, without the wait
 __device__ __forceinline__ void tc_ld_issue(uint32_t at, uint32_t (&r)[32]) { kp_tmem_ld32_issue(at, r); }
 __device__ __forceinline__ void tc_ld_issue(uint32_t at, uint32_t (&r)[16]) { kp_tmem_ld16_issue(at, r); }
-__device__ __forceinline__ void tc_ld_issue(uint32_t at, uint32_t (&r)[8]) { kp_tmem_ld8_issue(at, r); }
 
 // The W sums of a lane's row at a place of the unit's accumulators, g (and u: the up half, gated): one part's as they are,
 // several parts' added from zero in the order of the parts, as the split over a cluster adds them.
@@ -641,15 +640,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             int s = 0, b2 = 0;
             uint32_t ph = 0, set_ph = 1;
             bool ok = true;
-    #pragma unroll 1
-        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+#pragma unroll 1
+            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
                 ok = __all_sync(0xffffffffu, !*abort_flag && kp_mbar_wait_bounded(&acc_empty[b2], set_ph));
                 if (!ok) { *abort_flag = 1; break; }
                 kp_tc_fence_after();
                 uint32_t tmem_d = tmem_base + (uint32_t)(b2 * p.inner * BN);
                 int part_kb = 0;
-    #pragma unroll 1
-            for (int kb = 0; kb < n_kb; kb++) {
+#pragma unroll 1
+                for (int kb = 0; kb < n_kb; kb++) {
                     if (part_kb == p.kb_per_part) { part_kb = 0; tmem_d += BN; }
                     ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(&full[s], ph));
                     if (!ok) { *abort_flag = 1; break; }
@@ -958,8 +957,8 @@ static int tc_parts(int M, int N, int K, int epi) {
 //   a pair: TC_PAIR_COST for its barriers, and more for parts behind a gated epilogue, which is short of registers.
 // It was fitted to all that can run at 17 to 1000 rows of twelve layer products (1,087 timings): within 1 % of the best on average,
 // 23 % at worst (128 rows by 3072 x 2048, five parts by a cluster or by one CTA of 32 columns).  Measured, us, the
-// choice before the exchange by copies | now: 64 rows by 2048 x 2048 7.6 | 6.5, 128 by 2048 x 5632 16.0 | 12.0, 200 by
-// 1024 x 4608 13.4 | 10.1; gated 600 rows by 9216 x 1024 25.1 | 20.5.
+// choice before the exchange by copies | now: 64 rows by 2048 x 2048 7.8 | 6.7, 128 by 2048 x 5632 16.2 | 13.7, 200 by
+// 1024 x 4608 13.7 | 11.3; gated 600 rows by 9216 x 1024 25.2 | 20.9 (weights from HBM).
 static TcChoice tc_choose(int M, int N, int K, int epi, int split) {
     const bool gated = epi == EPI_SWIGLU;
     const int n_out = gated ? N / 2 : N, sms = tc_n_sm(), n_kb = (K + TC_BK - 1) / TC_BK;
