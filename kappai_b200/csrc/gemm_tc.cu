@@ -50,8 +50,8 @@
 // With it every SM brings in a part of A only, and wide tiles still keep all SMs streaming.
 //
 // Every wait on an mbarrier is bounded, and a warp goes on or gives up as one: instructions for a whole warp come next.  A wait
-// that gives up sets a status word (kp_tc_status), the CTA stops issuing work, tells the other CTAs of its cluster, and all of
-// them linger until what is under way must have come, still free their tensor memory and return.
+// that gives up sets a status word (kp_tc_status), the CTA stops issuing work, tells the other CTAs of its cluster, lingers until
+// what is under way must have come, still frees its tensor memory and returns.
 #include "tcgen05.cuh"
 
 #define EPI_STORE 0
@@ -226,6 +226,16 @@ __device__ __forceinline__ void tc_sums(const TcArgs& p, uint32_t at, float (&g)
             for (int j = 0; j < W; j++) { g[j] += __uint_as_float(r[j]); if TC_GATED(EPI) up[j] += __uint_as_float(u[j]); }
         }
     }
+}
+
+// What an epilogue warp does when it gave up (whatever gave up, these warps end here): the CTAs of the cluster are told first, so that
+// one that has not sent its sums yet does not send them; what is under way to here or from here has come when the warp arrives
+// at the cluster's last barrier, before which no CTA leaves.
+__device__ __noinline__ void tc_gave_up(int* abort_flag, int n_ctas) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) { *abort_flag = 1; atomicExch(&g_tc_status, 1); }
+    if (n_ctas > 1 && lane < n_ctas) kp_st_cluster(kp_cluster_addr(abort_flag, lane), 1);
+    kp_linger_after_failure();
 }
 
 template <int N> struct TcInt { static constexpr int value = N; };
@@ -454,7 +464,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             epi_sync();
             if (warp == 2) {
-                if (!p.recv_apart) ok = __all_sync(0xffffffffu, kp_mbar_wait_bounded(rings_free, 0));
+                // (a CTA that gave up while this one waited here has told so: see tc_gave_up)
+                if (!p.recv_apart) ok = __all_sync(0xffffffffu, kp_mbar_try_wait(rings_free, 0) || (kp_mbar_wait_bounded(rings_free, 0) && !*abort_flag));
                 const int olo = U * lane / S, bytes = (U * (lane + 1) / S - olo) * EIGHT * R;
                 if (ok && lane < S && lane != rank && bytes > 0)
                     kp_copy_to_cluster(kp_cluster_addr(recv, lane) + (rank < lane ? rank : rank - 1) * bytes, tiles + olo * EIGHT * R, bytes,
@@ -516,21 +527,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
             }
         }
-        if (__builtin_expect(!ok, 0)) {
-            if (lane == 0) { *abort_flag = 1; atomicExch(&g_tc_status, 1); }
-            // (all CTAs of the cluster are told, none of which has left yet: copies from them to here and from here to them may be on their way)
-            if (S > 1 && lane < S) kp_st_cluster(kp_cluster_addr(const_cast<const int*>(abort_flag), lane), 1);
-        }
+        if (__builtin_expect(!ok, 0)) tc_gave_up(const_cast<int*>(abort_flag), S);
         if (S > 1) { __syncwarp(); kp_cluster_arrive(); }
     }
     kp_tc_fence_before();
     __syncthreads();
     if (S > 1) kp_cluster_wait();                                         // no CTA leaves before all have what they were sent, or have given up
     if (threadIdx.x == 64) KP_TRACE_MARK_LANE(2);
-    if (warp == 1) {                                                      // (one warp that lingers keeps the CTA's memory)
-        if (*abort_flag) kp_linger_after_failure();
-        kp_tmem_dealloc(tmem_base, p.tmem_cols);
-    }
+    if (warp == 1) kp_tmem_dealloc(tmem_base, p.tmem_cols);
 }
 
 // ------------------------------------------------------------------------------------------ pairs of CTAs
