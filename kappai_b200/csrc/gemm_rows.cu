@@ -21,7 +21,7 @@
 //    launch between the product in front and this one.  (The weighted rows rounded before the scale, which then goes to the sums,
 //    saves two barriers a CTA but rounds a row elsewhere than with nine rows and more, and makes NaN of rows whose squares
 //    overflow; and with a warp's own columns read by itself, 128 bytes at a time, it was slower: rounds of one request of the
-//    1.2B shape 31.33 ms, this 31.06, of a short chat 8.02 and 7.88, of eight requests 44.10 and 43.77.  Left to the product in
+//    1.2B shape 31.5 ms, this 31.1, of a short chat 8.12 and 7.83, of eight requests 44.3 and 43.8.  Left to the product in
 //    front -- it writes the weighted rows and sums of squares, this one reads both -- a step took 3 % longer.)
 //
 // Measured back to back, us, gemm_stream | this, one row and 8: 2048 x 5632 7.8 | 6.5, 7.9 | 7.1; 6144 x 2048 6.8 | 5.2,
@@ -32,8 +32,8 @@
 // stand, big ones of more than half an SM; and only if the SM's split between cache and shared memory allows it (it is
 // set for the kernel that comes first: without the preference asked for in kp_smem_limit the second never came in).
 // A decode step through eight layers, us, norms apart and a CTA an SM | norms apart, two | norms inside, two (five to eight rows: see
-// rows_run): one request, 1024 columns 183 | 183 | 165, 2048 275 | 278 | 251, 2560 422 | 430 | 372; eight 193 | 188 | 177,
-// 299 | 288 | 276, 457 | 448 | 431.
+// rows_run): one request, 1024 columns 182 | 180 | 159, 1536 221 | 222 | 198, 2048 272 | 273 | 246, 2560 415 | 424 | 377; eight
+// 191 | 189 | 173, 232 | 224 | 216, 293 | 285 | 273, 451 | 441 | 425.
 // Big and small, KB, 64 steps of one request, 1.2B shape, ms: 148 + 78 32.1, 128 + 96 31.9, 116 + 110 32.2, 164 + 62 33.2.
 //
 // Epilogues as in gemm_stream.cu.  K a multiple of 512.  Loops are not unrolled where that gains nothing back to back: in a step
